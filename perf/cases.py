@@ -402,3 +402,224 @@ def tolerance(c):
     if kind == "moe":
         return {"rel": 0.018, "max": 0.38}
     return {"rel": 0.01, "max": 0.24}
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+def _exact_moe(c, seed):
+    s = _prepare_moe(c, seed)
+    x, router, w1, w2 = (t.detach().double() for t in s["args"])
+    t, e, f, top = c["tokens"], c["experts"], c["ffn"], c["top"]
+    probs = torch.softmax(x @ router.t(), dim=-1)
+    idx = torch.sort(probs, dim=-1, descending=True, stable=True).indices[:, :top]
+    picked = probs.gather(1, idx)
+    weight = picked / picked.sum(-1, keepdim=True)
+    w1, w2 = w1.view(e, 2 * f, -1), w2.view(e, -1, f)
+    out, grad = torch.zeros_like(x), None if s["grad"] is None else s["grad"].double()
+    if grad is not None:
+        dx, dw1, dw2, dweight = torch.zeros_like(x), torch.zeros_like(w1), torch.zeros_like(w2), torch.zeros_like(weight)
+    for i in range(e):
+        rows, slot = (idx == i).nonzero(as_tuple=True)
+        if rows.numel() == 0:
+            continue
+        gu = x[rows] @ w1[i].t()
+        gate, up = gu[:, :f], gu[:, f:]
+        sig = torch.sigmoid(gate)
+        act = gate * sig * up
+        y, w = act @ w2[i].t(), weight[rows, slot][:, None]
+        out.index_add_(0, rows, w * y)
+        if grad is None:
+            continue
+        g = grad[rows]
+        dweight[rows, slot] = (g * y).sum(-1)
+        dy = w * g
+        dw2[i] = dy.t() @ act
+        da = dy @ w2[i]
+        dgu = torch.cat([da * up * sig * (1 + gate * (1 - sig)), da * gate * sig], dim=1)
+        dw1[i] = dgu.t() @ x[rows]
+        dx.index_add_(0, rows, dgu @ w1[i])
+    if grad is None:
+        return {"out": out, "grads": []}
+    # the renormalised weights are a softmax over the selected logits
+    dlogits = torch.zeros_like(probs).scatter_(1, idx, weight * (dweight - (weight * dweight).sum(-1, keepdim=True)))
+    return {"out": out, "grads": [dx + dlogits @ router, dlogits.t() @ x, dw1.flatten(0, 1), dw2.flatten(0, 1)]}
+
+
+def _exact_linear_logp(c, seed):
+    s = _prepare_linear_logp(c, seed)
+    hidden, weight = s["hidden"].detach(), s["weight"].detach().double()
+    bias = None if s["bias"] is None else s["bias"].detach().double()
+    logp, entropy, gh, gw, gb = [], [], [], torch.zeros_like(weight) if c["backward"] else None, 0.0
+    for i in range(0, c["tokens"], 512):
+        h, ids = hidden[i:i + 512].double(), s["targets"][i:i + 512]
+        z = h @ weight.t()
+        if bias is not None:
+            z += bias
+        lse = torch.logsumexp(z, -1)
+        logp.append(z.gather(1, ids[:, None])[:, 0] - lse)
+        p = torch.exp(z - lse[:, None])
+        entropy.append(lse - (p * z).sum(-1))
+        if c["backward"]:
+            g = s["grad"][i:i + 512].double()[:, None]
+            dz = (-g * p).scatter_add_(1, ids[:, None], g)
+            gh.append(dz @ weight)
+            gw += dz.t() @ h
+            gb = gb + dz.sum(0)
+    grads = [torch.cat(gh), gw] + ([] if bias is None else [gb]) if c["backward"] else []
+    return {"logp": torch.cat(logp), "entropy": torch.cat(entropy) if c["entropy"] else None, "grads": grads}
+
+
+def _exact_loss(c, seed):
+    s = _prepare_loss(c, seed)
+    rewards, mask = s["rewards"].double().view(-1, c["group"]), s["mask"].double()
+    std = rewards.var(-1, correction=0, keepdim=True).clamp_min(1e-12).sqrt()
+    adv = ((rewards - rewards.mean(-1, keepdim=True)) / std).view(-1)
+    count = mask.sum()
+    policy_loss = kl = 0.0
+    grad = torch.empty(s["policy"].shape, dtype=torch.float64, device=DEV)
+    for i in range(c["batch"]):
+        z, r, ids = s["policy"][i].detach().double(), s["ref"][i].double(), s["ids"][i][:, None]
+        lse = torch.logsumexp(z, -1, keepdim=True)
+        lp = (z.gather(1, ids) - lse)[:, 0]
+        lr = r.gather(1, ids)[:, 0] - torch.logsumexp(r, -1)
+        ratio, diff = torch.exp(lp - s["old"][i].double()), lr - lp
+        free, clipped = ratio * adv[i], ratio.clamp(0.8, 1.2) * adv[i]
+        policy_loss += (-torch.minimum(free, clipped) * mask[i]).sum()
+        kl += ((torch.exp(diff) - diff - 1) * mask[i]).sum()
+        d = torch.where(free <= clipped, -free, torch.zeros_like(free)) + 0.04 * (1 - torch.exp(diff))
+        d = (d * mask[i] / count)[:, None]
+        grad[i] = (-d * torch.exp(z - lse)).scatter_add_(1, ids, d)
+    return {"loss": (policy_loss + 0.04 * kl) / count, "policy_loss": policy_loss / count, "kl": kl / count, "grad": grad}
+
+
+def _exact_attention(c, seed):
+    s = _prepare_attention(c, seed)
+    form, p, g, l = c["form"], c["prompt"], c["group"], c["length"]
+    q, k, v = (s[n].detach().double() for n in "qkv")
+    grad = None if s["grad"] is None else s["grad"].double()
+    if form == "prefix":
+        q, k, v = q.unsqueeze(3), k.unsqueeze(2), v.unsqueeze(2)  # one head
+        spans = [((b, i), [(b, slice(None))], None) for b in range(c["batch"]) for i in range(g)]
+    elif form == "causal":
+        spans = [((b, slice(None)), [(b, slice(None))], p) for b in range(c["batch"])]
+    else:
+        spans = [((slice(0, p),), [(slice(0, p),)], p)]
+        spans += [((slice(p + i * l, p + (i + 1) * l),), [(slice(0, p),), (slice(p + i * l, p + (i + 1) * l),)], l) for i in range(g)]
+    out, grads = torch.empty_like(q), None if grad is None else [torch.zeros_like(t) for t in (q, k, v)]
+    rep = c["heads"] // c["kv_heads"]
+    for rows, keys, causal in spans:
+        for head in range(c["heads"]):
+            kh = head // rep
+            kk, vv = (torch.cat([t[at][:, kh] for at in keys]) for t in (k, v))
+            qq = q[rows][:, head]
+            score = qq @ kk.t() * 128 ** -0.5
+            if causal is not None:  # the last `causal` keys are the queries' own
+                n = kk.shape[0] - causal
+                score[:, n:].masked_fill_(torch.ones(causal, causal, dtype=torch.bool, device=DEV).triu(1), -math.inf)
+            prob = torch.softmax(score, -1)
+            o = out[rows][:, head] = prob @ vv
+            if grad is None:
+                continue
+            do = (grad.unsqueeze(3) if form == "prefix" else grad)[rows][:, head]
+            ds = prob * (do @ vv.t() - (do * o).sum(-1, keepdim=True)) * 128 ** -0.5
+            grads[0][rows][:, head] = ds @ kk
+            at = 0
+            for span in keys:
+                m = k[span].shape[0]
+                grads[1][span][:, kh] += ds[:, at:at + m].t() @ qq
+                grads[2][span][:, kh] += prob[:, at:at + m].t() @ do
+                at += m
+    if form == "prefix":
+        out, grads = out.squeeze(3), grads and [grads[0].squeeze(3), grads[1].squeeze(2), grads[2].squeeze(2)]
+    return {"out": out, "grads": grads or []}
+
+
+def _rms(x, w):
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+
+
+def _rotate(x, positions):
+    half = 64
+    freq = (500000.0 ** (-torch.arange(half, dtype=torch.float32, device=DEV) / half)).double()
+    ang = (positions.double()[:, None] * freq)[:, None]
+    a, b = x[..., :half], x[..., half:]
+    return torch.cat([a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin()], dim=-1)
+
+
+def _exact_layer(model, c, i, x, positions, attend):
+    w = {n: model.view("l%d.%s" % (i, n)).detach() for n in ("attn_norm", "wqkv", "wo", "mlp_norm", "w_gate_up", "w_down")}
+    hq, hkv = c["heads"], c["kv_heads"]
+    qkv = (_rms(x, w["attn_norm"]) @ w["wqkv"].double().t()).view(x.shape[0], hq + 2 * hkv, 128)
+    q, k, v = _rotate(qkv[:, :hq], positions), _rotate(qkv[:, hq:hq + hkv], positions), qkv[:, hq + hkv:]
+    x = x + attend(q, k, v).reshape(x.shape[0], -1) @ w["wo"].double().t()
+    gu = _rms(x, w["mlp_norm"]) @ w["w_gate_up"].double().t()
+    gate, up = gu[:, :c["ffn"]], gu[:, c["ffn"]:]
+    return x + (gate * torch.sigmoid(gate) * up) @ w["w_down"].double().t()
+
+
+def _attend(q, k, v, rep, own=0):
+    """Queries over all keys; of the last ``own`` keys each query sees those up to its own."""
+    k, v = k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1)
+    score = torch.einsum("qhd,khd->hqk", q, k) * 128 ** -0.5
+    if own:
+        score[:, :, -own:].masked_fill_(torch.ones(own, own, dtype=torch.bool, device=DEV).triu(1), -math.inf)
+    return torch.einsum("hqk,khd->qhd", torch.softmax(score, -1), v)
+
+
+def _exact_score(c, seed):
+    s = _prepare_score(c, seed)
+    model, (g, l), p, rep = s["engine"].model, s["completions"].shape, c["prompt"], c["heads"] // c["kv_heads"]
+    tokens = torch.cat([s["prompt"], s["completions"].reshape(-1)])
+    positions = torch.cat([torch.arange(p, device=DEV), (p + torch.arange(l, device=DEV)).repeat(g)])
+
+    def attend(q, k, v):
+        out = [_attend(q[:p], k[:p], v[:p], rep, p)]
+        for i in range(g):
+            own = slice(p + i * l, p + (i + 1) * l)
+            out.append(_attend(q[own], torch.cat([k[:p], k[own]]), torch.cat([v[:p], v[own]]), rep, l))
+        return torch.cat(out)
+
+    with torch.no_grad():
+        x = model.view("embed")[tokens].double()
+        for i in range(c["layers"]):
+            x = _exact_layer(model, c, i, x, positions, attend)
+        x = _rms(x, model.view("final_norm"))
+        before = p + torch.arange(g * l, device=DEV).view(g, l) - 1
+        before[:, 0] = p - 1
+        head, logp = model.lm_head_weight().detach().double(), []
+        for i in range(g):
+            z = x[before[i]] @ head.t()
+            logp.append(z.gather(1, s["completions"][i, :, None])[:, 0] - torch.logsumexp(z, -1))
+    return torch.stack(logp)
+
+
+def _exact_decode(c, seed):
+    if c["fp8"]:
+        return None  # the codes are the framework's own
+    s = _prepare_decode(c, seed)
+    model, cache, tokens, positions, slots = s["keep"][:5]
+    n, p, rep, rows = c["n"], c["prompt"], c["heads"] // c["kv_heads"], c["own"] + 16
+    with torch.no_grad():
+        x = model.view("embed")[tokens].double()
+        for i in range(c["layers"]):
+            ck, cv = cache[i][0].double(), cache[i][1].double()
+
+            def attend(q, k, v):
+                ck[slots], cv[slots] = k, v
+                out = []
+                for j in range(n):
+                    at = slice(p + j * rows, p + j * rows + c["own"])
+                    out.append(_attend(q[j:j + 1], torch.cat([ck[:p], ck[at]]), torch.cat([cv[:p], cv[at]]), rep))
+                return torch.cat(out)
+
+            x = _exact_layer(model, c, i, x, positions, attend)
+        return _rms(x, model.view("final_norm")) @ model.lm_head_weight().detach().double().t()
+
+
+_EXACT = {"moe": _exact_moe, "linear_logp": _exact_linear_logp, "loss": _exact_loss, "attention": _exact_attention,
+          "score": _exact_score, "decode": _exact_decode}
+
+
+def exact(case, seed):
+    """What ``run`` returns, from plain torch in 64 bits.  Not for a training step (its results are the sums of a whole
+    step in 16-bit storage) nor for drawn tokens."""
+    return _EXACT[case["kind"]](case, seed) if case["kind"] in _EXACT else None
