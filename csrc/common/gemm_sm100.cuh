@@ -47,6 +47,7 @@ struct GemmProblem {
   int group_mode;
   const int* tile_group;
   const int* group_offsets;
+  const int* group_counts;  // mode 2, or null: rows of group g that hold anything; the others up to the next offset are zero
   int b_group_rows;
   int tiles_m_per_group;
   // Tensor-parallel fusions.  m_rot rotates the M-tile order (each rank starts on a different slab).
@@ -81,6 +82,7 @@ __host__ __device__ inline GemmProblem make_gemm_problem(int M, int N, int K, in
   p.group_mode = 0;
   p.tile_group = nullptr;
   p.group_offsets = nullptr;
+  p.group_counts = nullptr;
   p.b_group_rows = 0;
   p.tiles_m_per_group = 1;
   p.m_rot = 0;
@@ -123,9 +125,10 @@ __device__ __forceinline__ WorkItem decode_item(const GemmProblem& p, int id) {
   return w;
 }
 
-__device__ __forceinline__ ItemGeometry item_geometry(const GemmProblem& p, int m_tile) {
+// `tile_m` is the engine's M-tile (128 rows, or 256 for CTA pairs).
+__device__ __forceinline__ ItemGeometry item_geometry(const GemmProblem& p, int m_tile, int tile_m = kBM) {
   ItemGeometry g;
-  g.a_m0 = m_tile * kBM;
+  g.a_m0 = m_tile * tile_m;
   g.b_row_off = 0;
   g.k_row0 = 0;
   g.k_blocks = p.k_blocks;
@@ -133,9 +136,14 @@ __device__ __forceinline__ ItemGeometry item_geometry(const GemmProblem& p, int 
     g.b_row_off = p.tile_group[m_tile] * p.b_group_rows;
   } else if (p.group_mode == 2) {
     const int grp = m_tile / p.tiles_m_per_group;
-    g.a_m0 = (m_tile - grp * p.tiles_m_per_group) * kBM;
+    g.a_m0 = (m_tile - grp * p.tiles_m_per_group) * tile_m;
     g.k_row0 = p.group_offsets[grp];
-    g.k_blocks = (p.group_offsets[grp + 1] - g.k_row0 + kBK - 1) / kBK;
+    const int rows = p.group_counts != nullptr ? p.group_counts[grp] : p.group_offsets[grp + 1] - g.k_row0;
+    g.k_blocks = (rows + kBK - 1) / kBK;
+    if (rows == 0) {  // an empty group's product is zero: one k-block of rows past the end, which TMA fills with zeros
+      g.k_row0 = p.K;
+      g.k_blocks = 1;
+    }
   }
   return g;
 }

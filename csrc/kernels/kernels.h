@@ -54,6 +54,7 @@ struct GemmArgs {
   int group_mode = 0;
   const int* tile_group = nullptr;
   const int* group_offsets = nullptr;
+  const int* group_counts = nullptr;  // mode 2, optional: rows in use per group (groups may then be empty)
   int num_groups = 1;
   // Plain GEMM only: compute 256 x 256 tiles on pairs of SMs (tcgen05 cta_group::2, cluster of two CTAs).
   bool cta_pair = false;
@@ -432,8 +433,21 @@ void tp_gemm_rs(const TpGemmRsArgs& a, cudaStream_t stream);
 
 // Dispatch plan on the device: slot of every assignment, token of every slot (src_row must be pre-filled with -1),
 // expert of every 128-row tile, padded expert offsets [E + 1] and counts [E].  chunk_hist: scratch [ceil(A / 256), E].
+// compact: experts without assignments take no block, unused tiles get -1, and slot_assign[slot] (pre-filled with -1) names the
+// assignment instead of src_row naming its token.
 void moe_build_plan(const int* idx, int assignments, int k, int experts, int num_slots, int unused_group, int* chunk_hist,
-                    int* offsets, int* counts, int* tile_group, int* slot, int* src_row, cudaStream_t stream);
+                    int* offsets, int* counts, int* tile_group, int* slot, int* src_row, bool compact, cudaStream_t stream);
+// Slots of a compact plan.  gather: dst[slot] = src[assign / k].  backward: dst[slot] = weight[assign] * src[assign / k] and
+// dweight[assign] = <src[assign / k], y[slot]>.  Rows of tiles in use without an assignment are zeroed, other tiles untouched.
+void moe_gather_assigned(const __nv_bfloat16* src, long long ld_src, const int* assign, const int* tile_group, int k,
+                         __nv_bfloat16* dst, int slots, int hidden, cudaStream_t stream);
+void moe_dispatch_grad(const __nv_bfloat16* src, long long ld_src, const int* assign, const int* tile_group, int k,
+                       const float* weight, const __nv_bfloat16* y, __nv_bfloat16* dst, float* dweight, int slots, int hidden,
+                       cudaStream_t stream);
+// SwiGLU of packed [gate | up] rows and its gradient over the tiles in use of a compact plan.
+void moe_swiglu(const __nv_bfloat16* gu, const int* tile_group, __nv_bfloat16* out, int slots, int F, cudaStream_t stream);
+void moe_swiglu_backward(const __nv_bfloat16* gu, const __nv_bfloat16* dy, const int* tile_group, __nv_bfloat16* dgu, int slots, int F,
+                         cudaStream_t stream);
 // expert parallelism over peer-mapped buffers (dst / src / b hold one base pointer per rank)
 void moe_scatter_rows_peer(const __nv_bfloat16* src, long long ld_src, const int* token, const int* dest_rank,
                            const int* dest_slot, const float* scale, void* const* dst, int world, long long ld_dst,

@@ -277,24 +277,47 @@ __global__ void moe_plan_count_kernel(const int* __restrict__ idx, int assignmen
   for (int e = threadIdx.x; e < experts; e += blockDim.x) chunk_hist[blockIdx.x * experts + e] = hist[e];
 }
 
-__global__ void moe_plan_scan_kernel(int* __restrict__ chunk_hist, int chunks, int experts, int num_tiles, int unused_group,
-                                     int* __restrict__ offsets, int* __restrict__ counts, int* __restrict__ tile_group) {
+// One warp per expert walks the chunks 32 at a time with a shuffle scan (one thread per expert walking 141 chunks took 20 us).
+__global__ void __launch_bounds__(1024)
+moe_plan_scan_kernel(int* __restrict__ chunk_hist, int chunks, int experts, int num_tiles, int unused_group, bool compact,
+                     int* __restrict__ offsets, int* __restrict__ counts, int* __restrict__ tile_group) {
   extern __shared__ int off_s[];  // experts + 1
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  for (int e = warp; e < experts; e += warps) {
     int run = 0;
-    for (int c = 0; c < chunks; ++c) {
-      const int v = chunk_hist[c * experts + e];
-      chunk_hist[c * experts + e] = run;  // assignments of this expert in earlier chunks
-      run += v;
+    for (int c0 = 0; c0 < chunks; c0 += 32) {
+      const int c = c0 + lane;
+      const int v = c < chunks ? chunk_hist[c * experts + e] : 0;
+      int incl = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
+      }
+      if (c < chunks) chunk_hist[c * experts + e] = run + incl - v;  // assignments of this expert in earlier chunks
+      run += __shfl_sync(0xffffffffu, incl, 31);
     }
-    counts[e] = run;
-    const int blocks = run > 0 ? (run + 127) / 128 : 1;
-    off_s[e + 1] = blocks * 128;  // padded size, turned into offsets below
+    if (lane == 0) {
+      counts[e] = run;
+      const int blocks = run > 0 ? (run + 127) / 128 : (compact ? 0 : 1);
+      off_s[e + 1] = blocks * 128;  // padded size, turned into offsets below
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    off_s[0] = 0;
-    for (int e = 0; e < experts; ++e) off_s[e + 1] += off_s[e];
+  if (warp == 0) {
+    int run = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane;
+      int incl = e < experts ? off_s[e + 1] : 0;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
+      }
+      if (e < experts) off_s[e + 1] = run + incl;
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) off_s[0] = 0;
   }
   __syncthreads();
   for (int e = threadIdx.x; e <= experts; e += blockDim.x) offsets[e] = off_s[e];
@@ -312,7 +335,7 @@ __global__ void moe_plan_scan_kernel(int* __restrict__ chunk_hist, int chunks, i
 
 __global__ void moe_plan_place_kernel(const int* __restrict__ idx, int assignments, int k, int experts,
                                       const int* __restrict__ chunk_prefix, const int* __restrict__ offsets,
-                                      int* __restrict__ slot, int* __restrict__ src_row) {
+                                      int* __restrict__ slot, int* __restrict__ src_row, bool compact) {
   __shared__ int e_s[kPlanChunk];
   const int a = blockIdx.x * kPlanChunk + threadIdx.x;
   const int e = a < assignments ? idx[a] : -1;
@@ -323,7 +346,127 @@ __global__ void moe_plan_place_kernel(const int* __restrict__ idx, int assignmen
   for (int j = 0; j < threadIdx.x; ++j) rank += (e_s[j] == e) ? 1 : 0;
   const int s = offsets[e] + chunk_prefix[blockIdx.x * experts + e] + rank;
   slot[a] = s;
-  src_row[s] = a / k;
+  src_row[s] = compact ? a : a / k;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Rows of a compact plan.  All four kernels are one pass over rows in memory order, 16 bytes per access with several in
+// flight per thread, and leave the tiles without rows (the unused tail of the statically sized buffer) alone.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSlotWarps = 8;  // one warp per slot
+
+__device__ __forceinline__ float dot8(const uint4& x, const uint4& y, float acc) {
+  const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&x);
+  const __nv_bfloat162* hy = reinterpret_cast<const __nv_bfloat162*>(&y);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __bfloat1622float2(hx[e]), g = __bfloat1622float2(hy[e]);
+    acc = fmaf(f.x, g.x, acc);
+    acc = fmaf(f.y, g.y, acc);
+  }
+  return acc;
+}
+
+// GRAD: scale by the assignment's weight and form its gradient <src row, y row> in the same sweep.
+template <bool GRAD>
+__global__ void __launch_bounds__(32 * kSlotWarps)
+moe_slot_rows_kernel(const __nv_bfloat16* __restrict__ src, long long ld_src, const int* __restrict__ assign,
+                     const int* __restrict__ tile_group, int k, const float* __restrict__ weight,
+                     const __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ dst, float* __restrict__ dweight, int slots,
+                     int h8) {
+  const int slot = blockIdx.x * kSlotWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (slot >= slots || tile_group[slot >> 7] < 0) return;
+  uint4* out = reinterpret_cast<uint4*>(dst) + static_cast<long long>(slot) * h8;
+  const int a = assign[slot];
+  if (a < 0) {
+    for (int i = lane; i < h8; i += 32) out[i] = make_uint4(0u, 0u, 0u, 0u);
+    return;
+  }
+  const uint4* in = reinterpret_cast<const uint4*>(src + static_cast<long long>(a / k) * ld_src);
+  const uint4* yr = GRAD ? reinterpret_cast<const uint4*>(y) + static_cast<long long>(slot) * h8 : nullptr;
+  const float w = GRAD ? weight[a] : 1.f;
+  float acc = 0.f;
+  constexpr int kAhead = 4;
+  for (int i0 = lane; i0 < h8; i0 += 32 * kAhead) {
+    uint4 q[kAhead], v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = i0 + 32 * u;
+      if (i < h8) {
+        q[u] = __ldg(in + i);
+        if (GRAD) v[u] = __ldg(yr + i);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = i0 + 32 * u;
+      if (i >= h8) break;
+      if (GRAD) {
+        acc = dot8(q[u], v[u], acc);
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(h[j]);
+          h[j] = __floats2bfloat162_rn(f.x * w, f.y * w);
+        }
+      }
+      out[i] = q[u];
+    }
+  }
+  if (GRAD) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane == 0) dweight[a] = acc;
+  }
+}
+
+constexpr int kActRows = 8;  // rows per CTA
+constexpr int kActThreads = 128;
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kActThreads)
+moe_swiglu_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dy, const int* __restrict__ tile_group,
+                  __nv_bfloat16* __restrict__ out, int f8) {
+  const long long row0 = static_cast<long long>(blockIdx.x) * kActRows;
+  if (tile_group[row0 >> 7] < 0) return;
+  const uint4* in = reinterpret_cast<const uint4*>(gu) + row0 * 2 * f8;
+  const uint4* dr = GRAD ? reinterpret_cast<const uint4*>(dy) + row0 * f8 : nullptr;
+  uint4* o = reinterpret_cast<uint4*>(out) + row0 * (GRAD ? 2 : 1) * f8;
+  constexpr int kAhead = 4;
+  for (int c = threadIdx.x; c < f8; c += kActThreads) {
+#pragma unroll
+    for (int r0 = 0; r0 < kActRows; r0 += kAhead) {
+      uint4 g[kAhead], u[kAhead], d[kAhead];
+#pragma unroll
+      for (int r = 0; r < kAhead; ++r) {
+        g[r] = __ldg(in + (r0 + r) * 2 * f8 + c);
+        u[r] = __ldg(in + (r0 + r) * 2 * f8 + f8 + c);
+        if (GRAD) d[r] = __ldg(dr + (r0 + r) * f8 + c);
+      }
+#pragma unroll
+      for (int r = 0; r < kAhead; ++r) {
+        const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&g[r]);
+        const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&u[r]);
+        uint4 a, b;
+        __nv_bfloat162* ap = reinterpret_cast<__nv_bfloat162*>(&a);
+        __nv_bfloat162* bp = reinterpret_cast<__nv_bfloat162*>(&b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 gf = __bfloat1622float2(gp[i]), uf = __bfloat1622float2(up[i]);
+          const float s0 = 1.f / (1.f + __expf(-gf.x)), s1 = 1.f / (1.f + __expf(-gf.y));
+          if (GRAD) {
+            const float2 df = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&d[r])[i]);
+            ap[i] = __floats2bfloat162_rn(df.x * uf.x * s0 * (1.f + gf.x * (1.f - s0)), df.y * uf.y * s1 * (1.f + gf.y * (1.f - s1)));
+            bp[i] = __floats2bfloat162_rn(df.x * gf.x * s0, df.y * gf.y * s1);
+          } else {
+            ap[i] = __floats2bfloat162_rn(gf.x * s0 * uf.x, gf.y * s1 * uf.y);
+          }
+        }
+        o[(r0 + r) * (GRAD ? 2 : 1) * f8 + c] = a;
+        if (GRAD) o[(r0 + r) * 2 * f8 + f8 + c] = b;
+      }
+    }
+  }
 }
 
 PeerBases make_bases(void* const* p, int world) {
@@ -335,13 +478,39 @@ PeerBases make_bases(void* const* p, int world) {
 }  // namespace
 
 void moe_build_plan(const int* idx, int assignments, int k, int experts, int num_slots, int unused_group, int* chunk_hist,
-                    int* offsets, int* counts, int* tile_group, int* slot, int* src_row, cudaStream_t stream) {
+                    int* offsets, int* counts, int* tile_group, int* slot, int* src_row, bool compact, cudaStream_t stream) {
   if (assignments <= 0) return;
   const int chunks = (assignments + kPlanChunk - 1) / kPlanChunk;
   moe_plan_count_kernel<<<chunks, kPlanChunk, experts * sizeof(int), stream>>>(idx, assignments, experts, chunk_hist);
-  moe_plan_scan_kernel<<<1, 512, (experts + 1) * sizeof(int), stream>>>(chunk_hist, chunks, experts, num_slots / 128,
-                                                                       unused_group, offsets, counts, tile_group);
-  moe_plan_place_kernel<<<chunks, kPlanChunk, 0, stream>>>(idx, assignments, k, experts, chunk_hist, offsets, slot, src_row);
+  moe_plan_scan_kernel<<<1, 1024, (experts + 1) * sizeof(int), stream>>>(
+      chunk_hist, chunks, experts, num_slots / 128, unused_group, compact, offsets, counts, tile_group);
+  moe_plan_place_kernel<<<chunks, kPlanChunk, 0, stream>>>(idx, assignments, k, experts, chunk_hist, offsets, slot, src_row, compact);
+}
+
+void moe_gather_assigned(const __nv_bfloat16* src, long long ld_src, const int* assign, const int* tile_group, int k,
+                         __nv_bfloat16* dst, int slots, int hidden, cudaStream_t stream) {
+  if (slots <= 0) return;
+  moe_slot_rows_kernel<false><<<(slots + kSlotWarps - 1) / kSlotWarps, 32 * kSlotWarps, 0, stream>>>(
+      src, ld_src, assign, tile_group, k, nullptr, nullptr, dst, nullptr, slots, hidden / 8);
+}
+
+void moe_dispatch_grad(const __nv_bfloat16* src, long long ld_src, const int* assign, const int* tile_group, int k,
+                       const float* weight, const __nv_bfloat16* y, __nv_bfloat16* dst, float* dweight, int slots, int hidden,
+                       cudaStream_t stream) {
+  if (slots <= 0) return;
+  moe_slot_rows_kernel<true><<<(slots + kSlotWarps - 1) / kSlotWarps, 32 * kSlotWarps, 0, stream>>>(
+      src, ld_src, assign, tile_group, k, weight, y, dst, dweight, slots, hidden / 8);
+}
+
+void moe_swiglu(const __nv_bfloat16* gu, const int* tile_group, __nv_bfloat16* out, int slots, int F, cudaStream_t stream) {
+  if (slots <= 0) return;
+  moe_swiglu_kernel<false><<<slots / kActRows, kActThreads, 0, stream>>>(gu, nullptr, tile_group, out, F / 8);
+}
+
+void moe_swiglu_backward(const __nv_bfloat16* gu, const __nv_bfloat16* dy, const int* tile_group, __nv_bfloat16* dgu, int slots, int F,
+                         cudaStream_t stream) {
+  if (slots <= 0) return;
+  moe_swiglu_kernel<true><<<slots / kActRows, kActThreads, 0, stream>>>(gu, dy, tile_group, dgu, F / 8);
 }
 
 void moe_scatter_rows_peer(const __nv_bfloat16* src, long long ld_src, const int* token, const int* dest_rank,

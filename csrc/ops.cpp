@@ -279,7 +279,7 @@ Tensor tp_gemm_rs(const Tensor& a_in, const Tensor& b, bool b_mn, int64_t rank, 
 //           [G * K, N] (b_mn = true, used for dX = dY * W_g), tile_group int32 [rows / 128]  -> out [rows, N]
 //   mode 2: a [rows, M], b [rows, N], group_offsets int32 [G + 1]  -> out [G * M, N] = per-group a^T b
 Tensor grouped_gemm(const Tensor& a, const Tensor& b, int64_t mode, const Tensor& table, int64_t num_groups, bool b_mn,
-                    bool out_fp32, std::optional<Tensor> out) {
+                    bool out_fp32, std::optional<Tensor> out, std::optional<Tensor> counts) {
   check_rowmajor(a, "a");
   check_rowmajor(b, "b");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "grouped_gemm: bf16 operands only");
@@ -333,6 +333,12 @@ Tensor grouped_gemm(const Tensor& a, const Tensor& b, int64_t mode, const Tensor
     g.a_mn_major = true;
     g.b_mn_major = true;
     g.group_offsets = table.data_ptr<int>();
+    if (counts.has_value()) {
+      TORCH_CHECK(counts->is_cuda() && counts->scalar_type() == torch::kInt32 && counts->is_contiguous() && counts->numel() == num_groups,
+                  "grouped_gemm(2): counts must be int32, one per group");
+      g.group_counts = counts->data_ptr<int>();
+    }
+    g.cta_pair = gemm_pair_default();
   }
   g.D = d.data_ptr();
   g.ldd = d.stride(0);
@@ -378,13 +384,17 @@ Tensor moe_topk_bwd(const Tensor& idx, const Tensor& weight, const Tensor& dweig
 }
 
 // (slot [T, k], src_row [S], tile_group [S / 128], offsets [E + 1], counts [E]) for expert ids `idx` int32 [T, k].
-std::vector<Tensor> moe_build_plan(const Tensor& idx, int64_t experts, int64_t num_slots, int64_t unused_group) {
+// compact: experts without assignments take no block, unused tiles get group -1, and instead of src_row the second table names
+// the assignment (token * k + j) of every slot.
+std::vector<Tensor> moe_build_plan(const Tensor& idx, int64_t experts, int64_t num_slots, int64_t unused_group, bool compact) {
   TORCH_CHECK(idx.is_cuda() && idx.scalar_type() == torch::kInt32 && idx.is_contiguous() && idx.dim() == 2, "moe_build_plan: idx int32 [T, k]");
   TORCH_CHECK(experts >= 1 && experts <= 4096 && num_slots % 128 == 0, "moe_build_plan: 1 <= experts <= 4096, num_slots % 128 == 0");
   const c10::cuda::CUDAGuard guard(idx.device());
   const int64_t a = idx.numel(), k = idx.size(1);
   // every expert block is padded to a multiple of 128 rows (empty experts keep one block): at most a + 128 * experts rows
-  TORCH_CHECK(num_slots >= (a + 128 * experts) / 128 * 128, "moe_build_plan: num_slots is below the worst-case padded size");
+  // (compact: only experts that occur, each with at most 127 rows of padding)
+  TORCH_CHECK(num_slots >= (compact ? (a + 127 * std::min(experts, a)) : (a + 128 * experts)) / 128 * 128,
+              "moe_build_plan: num_slots is below the worst-case padded size");
   auto opt = idx.options();
   Tensor slot = torch::empty({idx.size(0), k}, opt);
   Tensor src_row = torch::full({num_slots}, -1, opt);
@@ -395,9 +405,9 @@ std::vector<Tensor> moe_build_plan(const Tensor& idx, int64_t experts, int64_t n
   Tensor scratch = torch::empty({std::max<int64_t>(chunks, 1) * experts}, opt);
   if (a > 0) {
     rlk::moe_build_plan(idx.data_ptr<int>(), static_cast<int>(a), static_cast<int>(k), static_cast<int>(experts),
-                        static_cast<int>(num_slots), static_cast<int>(unused_group), scratch.data_ptr<int>(),
+                        static_cast<int>(num_slots), compact ? -1 : static_cast<int>(unused_group), scratch.data_ptr<int>(),
                         offsets.data_ptr<int>(), counts.data_ptr<int>(), tile_group.data_ptr<int>(), slot.data_ptr<int>(),
-                        src_row.data_ptr<int>(), stream_of(idx));
+                        src_row.data_ptr<int>(), compact, stream_of(idx));
     after_launch(3);
   }
   return {slot, src_row, tile_group, offsets, counts};
@@ -408,6 +418,75 @@ void check_bf16_rows(const Tensor& t, const char* n) {
   TORCH_CHECK(t.scalar_type() == torch::kBFloat16 && t.size(1) % 8 == 0 && t.stride(0) % 8 == 0 &&
                   reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0,
               "rl_engine.moe: ", n, " must be bf16 rows of a multiple of 8 elements, 16-byte aligned");
+}
+
+namespace {
+
+void check_slots(const Tensor& assign, const Tensor& tile_group) {
+  TORCH_CHECK(assign.is_cuda() && assign.scalar_type() == torch::kInt32 && assign.is_contiguous() && assign.numel() % 128 == 0 &&
+                  tile_group.is_cuda() && tile_group.scalar_type() == torch::kInt32 && tile_group.is_contiguous() &&
+                  tile_group.numel() == assign.numel() / 128,
+              "rl_engine.moe: int32 tables, one assignment per slot and one group per 128 slots");
+}
+void check_slot_rows(const Tensor& t, const Tensor& assign, const char* n) {
+  check_bf16_rows(t, n);
+  TORCH_CHECK(t.is_contiguous() && t.size(0) == assign.numel(), "rl_engine.moe: ", n, " must hold one contiguous row per slot");
+}
+__nv_bfloat16* bf16_ptr(const Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
+
+}  // namespace
+
+// Rows of a compact plan: src[assign / k] for every slot in use.
+Tensor moe_gather_assigned(const Tensor& src, const Tensor& assign, const Tensor& tile_group, int64_t k) {
+  check_bf16_rows(src, "src");
+  check_slots(assign, tile_group);
+  const c10::cuda::CUDAGuard guard(src.device());
+  Tensor out = torch::empty({assign.numel(), src.size(1)}, src.options());
+  rlk::moe_gather_assigned(bf16_ptr(src), src.stride(0), assign.data_ptr<int>(), tile_group.data_ptr<int>(), static_cast<int>(k),
+                           bf16_ptr(out), static_cast<int>(assign.numel()), static_cast<int>(src.size(1)), stream_of(src));
+  after_launch();
+  return out;
+}
+
+// (weight[assign] * dout[assign / k] for every slot in use, <dout[assign / k], y[slot]> for every assignment)
+std::vector<Tensor> moe_dispatch_grad(const Tensor& dout, const Tensor& assign, const Tensor& tile_group, const Tensor& weight,
+                                      const Tensor& y) {
+  check_bf16_rows(dout, "dout");
+  check_slots(assign, tile_group);
+  check_slot_rows(y, assign, "y");
+  TORCH_CHECK(weight.is_cuda() && weight.scalar_type() == torch::kFloat32 && weight.is_contiguous() && weight.dim() == 2 &&
+                  weight.size(0) == dout.size(0) && y.size(1) == dout.size(1),
+              "moe_dispatch_grad: weight must be float32 [tokens, k]");
+  const c10::cuda::CUDAGuard guard(dout.device());
+  Tensor dy = torch::empty({assign.numel(), dout.size(1)}, dout.options());
+  Tensor dw = torch::empty_like(weight);
+  rlk::moe_dispatch_grad(bf16_ptr(dout), dout.stride(0), assign.data_ptr<int>(), tile_group.data_ptr<int>(),
+                         static_cast<int>(weight.size(1)), weight.data_ptr<float>(), bf16_ptr(y), bf16_ptr(dy), dw.data_ptr<float>(),
+                         static_cast<int>(assign.numel()), static_cast<int>(dout.size(1)), stream_of(dout));
+  after_launch();
+  return {dy, dw};
+}
+
+// silu(gate) * up of packed rows over the tiles in use; with dy: the gradient of the packed rows.
+Tensor moe_swiglu(const Tensor& gu, const Tensor& tile_group, std::optional<Tensor> dy) {
+  check_bf16_rows(gu, "gate_up");
+  TORCH_CHECK(gu.is_contiguous() && gu.size(1) % 16 == 0 && gu.size(0) % 128 == 0 && tile_group.is_cuda() &&
+                  tile_group.scalar_type() == torch::kInt32 && tile_group.is_contiguous() && tile_group.numel() == gu.size(0) / 128,
+              "moe_swiglu: contiguous [slots, 2 F] with 8 | F and one group per 128 slots");
+  const c10::cuda::CUDAGuard guard(gu.device());
+  const int64_t f = gu.size(1) / 2;
+  Tensor out = torch::empty({gu.size(0), dy.has_value() ? 2 * f : f}, gu.options());
+  if (dy.has_value()) {
+    check_bf16_rows(*dy, "dy");
+    TORCH_CHECK(dy->is_contiguous() && dy->size(0) == gu.size(0) && dy->size(1) == f, "moe_swiglu: dy must be contiguous [slots, F]");
+    rlk::moe_swiglu_backward(bf16_ptr(gu), bf16_ptr(*dy), tile_group.data_ptr<int>(), bf16_ptr(out), static_cast<int>(gu.size(0)),
+                             static_cast<int>(f), stream_of(gu));
+  } else {
+    rlk::moe_swiglu(bf16_ptr(gu), tile_group.data_ptr<int>(), bf16_ptr(out), static_cast<int>(gu.size(0)), static_cast<int>(f),
+                    stream_of(gu));
+  }
+  after_launch();
+  return out;
 }
 
 // dst_ptr == 0: allocate [slots, H] locally; else write to that device address (e.g. a peer's buffer).
@@ -1285,12 +1364,17 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("out") = py::none(), py::arg("out_fp32") = false, py::arg("accumulate") = false, py::arg("alpha") = 1.0,
         py::arg("pair") = -1);
   m.def("grouped_gemm", rlk::traced("rlk::grouped_gemm", &grouped_gemm), py::arg("a"), py::arg("b"), py::arg("mode"),
-        py::arg("table"), py::arg("num_groups"), py::arg("b_mn"), py::arg("out_fp32"), py::arg("out") = py::none());
+        py::arg("table"), py::arg("num_groups"), py::arg("b_mn"), py::arg("out_fp32"), py::arg("out") = py::none(),
+        py::arg("counts") = py::none());
   m.def("tp_ag_gemm", rlk::traced("rlk::tp_ag_gemm", &tp_ag_gemm));
   m.def("tp_gemm_rs", rlk::traced("rlk::tp_gemm_rs", &tp_gemm_rs));
   m.def("moe_topk", rlk::traced("rlk::moe_topk", &moe_topk));
   m.def("moe_topk_bwd", rlk::traced("rlk::moe_topk_bwd", &moe_topk_bwd));
-  m.def("moe_build_plan", rlk::traced("rlk::moe_build_plan", &moe_build_plan));
+  m.def("moe_build_plan", rlk::traced("rlk::moe_build_plan", &moe_build_plan), py::arg("idx"), py::arg("experts"), py::arg("num_slots"),
+        py::arg("unused_group"), py::arg("compact") = false);
+  m.def("moe_gather_assigned", rlk::traced("rlk::moe_gather_assigned", &moe_gather_assigned));
+  m.def("moe_dispatch_grad", rlk::traced("rlk::moe_dispatch_grad", &moe_dispatch_grad));
+  m.def("moe_swiglu", rlk::traced("rlk::moe_swiglu", &moe_swiglu), py::arg("gate_up"), py::arg("tile_group"), py::arg("dy") = py::none());
   m.def("moe_gather_rows", rlk::traced("rlk::moe_gather_rows", &moe_gather_rows), py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(),
         py::arg("dst_ptr") = 0, py::arg("dst_ld") = 0);
   m.def("moe_combine", rlk::traced("rlk::moe_combine", &moe_combine), py::arg("src"), py::arg("src_ptr"), py::arg("src_ld"), py::arg("hidden"), py::arg("slot"),

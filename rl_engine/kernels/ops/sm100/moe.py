@@ -106,18 +106,37 @@ def build_dispatch_plan(expert_idx: torch.Tensor, num_experts: int) -> DispatchP
     return DispatchPlan(slot.view(t, k), src_row, tile_group.to(torch.int32), offsets.to(torch.int32), counts, num_slots)
 
 
+@dataclass
+class CompactPlan:
+    """Slot tables of the single-GPU operator: as ``DispatchPlan``, but experts without a token take no block (a few
+    tokens meet a few experts: neither their tiles nor their weights are touched) and unused tiles are -1 (skipped)."""
+
+    slot: torch.Tensor          # int32 [T, k]   slot of every assignment
+    assign: torch.Tensor        # int32 [S]      assignment (token * k + j) of every slot, -1 for padding
+    tile_group: torch.Tensor    # int32 [S/128]  expert of every 128-row tile, -1 for unused ones
+    offsets: torch.Tensor       # int32 [E + 1]  padded slot offsets per expert
+    counts: torch.Tensor        # int32 [E]      real assignments per expert
+
+
+def build_compact_plan(expert_idx: torch.Tensor, num_experts: int) -> CompactPlan:
+    t, k = expert_idx.shape
+    num_slots = (t * k + (BLOCK - 1) * min(num_experts, t * k) + BLOCK - 1) // BLOCK * BLOCK  # static bound: no .item()
+    return CompactPlan(*require_ext().moe_build_plan(expert_idx.contiguous(), int(num_experts), int(num_slots), -1, True))
+
+
 class _ExpertFFN(torch.autograd.Function):
     """x [T, H], weights [T, k], plan, W1 [E*2F, H], W2 [E*H, F] -> out [T, H]."""
 
     @staticmethod
-    def forward(ctx, x, weights, w1, w2, plan: DispatchPlan, num_experts: int):
+    def forward(ctx, x, weights, w1, w2, plan: CompactPlan, num_experts: int):
         ext = require_ext()
-        xs = ext.moe_gather_rows(x, plan.src_row)
+        weights = weights.detach()
+        xs = ext.moe_gather_assigned(x, plan.assign, plan.tile_group, weights.shape[1])
         h1 = ext.grouped_gemm(xs, w1, 1, plan.tile_group, num_experts, False, False)
-        act = ext.swiglu_packed_fwd(h1)
+        act = ext.moe_swiglu(h1, plan.tile_group)
         y = ext.grouped_gemm(act, w2, 1, plan.tile_group, num_experts, False, False)
-        out = ext.moe_combine(y, 0, 0, 0, plan.slot, weights.detach())
-        ctx.save_for_backward(xs, h1, act, y, weights.detach(), w1, w2)
+        out = ext.moe_combine(y, 0, 0, 0, plan.slot, weights)
+        ctx.save_for_backward(xs, h1, act, y, weights, w1, w2)
         ctx.plan, ctx.num_experts = plan, num_experts
         return out
 
@@ -126,17 +145,12 @@ class _ExpertFFN(torch.autograd.Function):
         ext = require_ext()
         xs, h1, act, y, weights, w1, w2 = ctx.saved_tensors
         plan, e = ctx.plan, ctx.num_experts
-        dout = dout.contiguous()
-        # weight of the assignment living in each slot (padding slots: src_row = -1, never read)
-        slot_weight = torch.zeros(plan.num_slots, dtype=torch.float32, device=dout.device)
-        slot_weight[plan.slot.reshape(-1).long()] = weights.reshape(-1)
-        dweights = ext.moe_rowdot(dout, y, plan.slot)
-        dy = ext.moe_gather_rows(dout, plan.src_row, slot_weight)
+        dy, dweights = ext.moe_dispatch_grad(dout.contiguous(), plan.assign, plan.tile_group, weights.contiguous(), y)
         dact = ext.grouped_gemm(dy, w2, 1, plan.tile_group, e, True, False)
-        dw2 = ext.grouped_gemm(dy, act, 2, plan.offsets, e, True, False)
-        dh1 = ext.swiglu_packed_bwd(h1, dact)
+        dw2 = ext.grouped_gemm(dy, act, 2, plan.offsets, e, True, False, None, plan.counts)
+        dh1 = ext.moe_swiglu(h1, plan.tile_group, dact)
         dxs = ext.grouped_gemm(dh1, w1, 1, plan.tile_group, e, True, False)
-        dw1 = ext.grouped_gemm(dh1, xs, 2, plan.offsets, e, True, False)
+        dw1 = ext.grouped_gemm(dh1, xs, 2, plan.offsets, e, True, False, None, plan.counts)
         dx = ext.moe_combine(dxs, 0, 0, 0, plan.slot, None)
         return dx, dweights, dw1, dw2, None, None
 
@@ -165,7 +179,7 @@ class FusedMoESM100Op:
             x2 = x2.contiguous()
         logits = _RouterLogits.apply(x2, router_weight)
         idx, weights = route_topk(logits, top_k)
-        plan = build_dispatch_plan(idx, e)
+        plan = build_compact_plan(idx, e)
         out = _ExpertFFN.apply(x2, weights, w_gate_up, w_down, plan, e)
         return out.reshape(x.shape)
 
