@@ -1,12 +1,13 @@
-// Temperature / top-k / top-p sampling, one CTA per row of logits.
+// Temperature / top-k / top-p sampling, one CTA (many rows) or one cluster of CTAs (few rows) per row of logits.
 //
-//   1. a candidate threshold from ONE vectorised pass over the row without atomics: every thread keeps the maximum of
-//      its elements, and the k-th largest of the 1024 thread maxima (found by rank counting in shared memory) is a
-//      lower bound of the row's k-th largest value, so {x >= threshold} contains the top k and, for ordinary logits,
-//      only a few more.  If that set does not fit the candidate buffer (masses of ties), the exact radix select on
-//      order-preserving 32-bit keys (integer histograms in shared memory, 12-bit first digit) takes over;
-//   2. those candidates are gathered into shared memory and bitonic-sorted by (logit descending, index
-//      ascending) -- a total order, so the gather order does not matter -- and cut to the first k plus ties;
+//   1. a lower bound of the row's k-th largest value: the k-th largest of the maxima of 512 interleaved subsets of the first
+//      eighth of a slice (k <= 256), or of 2048 subsets of all of it (larger k) -- a bound for the row whichever part of it
+//      it comes from.  The slice is then streamed against the bound (what the first sweep read comes from L2) and what reaches it goes to
+//      a candidate buffer in shared memory: about 8 k elements, or 1.4 k, for ordinary logits.  If they do
+//      not fit (masses of ties, a row whose head is unlike its tail), the exact radix select on order-preserving 32-bit keys
+//      (integer histograms in shared memory, 12-bit first digit) takes over;
+//   2. the candidates are cut to at most 2048 by an exact radix select in shared memory where they are more, and bitonic-sorted by (logit descending, index
+//      ascending) -- a total order, so neither the gather order nor the split over CTAs matters -- and cut to the first k plus ties;
 //   3. softmax with temperature over the candidates, inclusive scan in a fixed tree, top-p cut
 //      "keep token i iff the mass strictly before it is <= p" (first token always kept);
 //   4. inverse-CDF draw with a Philox4x32-10 uniform keyed by (seed, row, offset).
@@ -19,12 +20,20 @@
 
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 namespace rlk {
 
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kCap = 2048;  // candidate capacity (k <= 1024 plus ties)
+constexpr int kThreads = 512;
+constexpr int kCap = 2048;       // candidates that are sorted (k <= 1024 plus ties)
+constexpr int kGather = 10240;   // candidates that are gathered: 80 KB, two CTAs per SM
+// Up to this k the bound comes from one maximum per thread over an eighth of the slice; above it from four per thread over all
+// of it (a bound from an eighth would let 8192 candidates through at k = 1024).
+constexpr int kFewLimit = 256;
+constexpr int kSampleShare = 8;
+constexpr int kMinSample = kThreads * 16;  // elements
 
 template <typename T> __device__ __forceinline__ float ldv(const T* p, int i);
 template <> __device__ __forceinline__ float ldv<float>(const float* p, int i) { return p[i]; }
@@ -53,133 +62,254 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint2 k) {
   return c;
 }
 
-// Calls f(value, index) for every element of the row, thread t taking 16-byte vectors t, t + 1024, ... when the row
-// is 16-byte aligned (scalar otherwise).  The visiting order per thread is fixed, the union over threads is the row.
-template <typename T, typename F>
-__device__ __forceinline__ void for_each_in_row(const T* __restrict__ z, int V, F&& f) {
-  constexpr int kVec = 16 / sizeof(T);
-  if ((reinterpret_cast<uintptr_t>(z) & 15u) == 0) {
-    const int body = V / kVec;
-    const uint4* p = reinterpret_cast<const uint4*>(z);
-    for (int v = threadIdx.x; v < body; v += kThreads) {
-      const uint4 q = p[v];
-      const T* e = reinterpret_cast<const T*>(&q);
+__device__ __forceinline__ uint32_t cluster_size_x() {
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ uint32_t cluster_max_u32(uint32_t addr, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.max.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ uint32_t cluster_add_u32(uint32_t addr, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ void cluster_store_u64(uint32_t addr, unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+struct SelectScratch {
+  unsigned int bins[256];
+  unsigned int prefix, remaining;
+};
+
+// The k-th largest (1-based) of the keys visited by `each` (a callable that calls its argument with (key, valid) the
+// same number of times in every lane of a warp), to DIGITS 8-bit digits from the top; the digits below are zero.  Every
+// thread of the block calls it; at least k valid keys must exist.
+template <int DIGITS, typename Each>
+__device__ __forceinline__ uint32_t block_kth_key(SelectScratch& s, unsigned int k, Each&& each) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t prefix = 0u, mask = 0u;
+  unsigned int remaining = k;
+#pragma unroll 1
+  for (int d = 0; d < DIGITS; ++d) {
+    const int shift = 24 - 8 * d;
+    if (tid < 256) s.bins[tid] = 0u;
+    __syncthreads();
+    each([&](uint32_t key, bool valid) {
+      // warp-aggregated counting: large keys share their leading bits, so most lanes of a warp hit the same bin
+      const bool active = valid && (key & mask) == prefix;
+      const uint32_t digit = (key >> shift) & 0xffu;
+      const unsigned int peers = __match_any_sync(0xffffffffu, active ? digit : 0xffffffffu);
+      if (active && lane == __ffs(peers) - 1) atomicAdd(&s.bins[digit], static_cast<unsigned int>(__popc(peers)));
+    });
+    __syncthreads();
+    if (warp == 0) {
+      // lane l owns bins 255 - 8 l ... 248 - 8 l (highest first); inclusive scan of the lanes' sums
+      unsigned int mine = 0u;
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) f(ldv(e, j), v * kVec + j);
+      for (int j = 0; j < 8; ++j) mine += s.bins[255 - (lane * 8 + j)];
+      unsigned int incl = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned int o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
+      }
+      const unsigned int before = incl - mine;
+      if (before < remaining && remaining <= incl) {  // exactly one lane: the digit is one of its bins
+        unsigned int acc = before;
+        int bin = 255 - lane * 8;
+        for (int j = 0; j < 8; ++j) {
+          bin = 255 - (lane * 8 + j);
+          if (acc + s.bins[bin] >= remaining) break;
+          acc += s.bins[bin];
+        }
+        s.prefix = prefix | (static_cast<uint32_t>(bin) << shift);
+        s.remaining = remaining - acc;
+      }
     }
-    for (int i = body * kVec + threadIdx.x; i < V; i += kThreads) f(ldv(z, i), i);
-  } else {
-    for (int i = threadIdx.x; i < V; i += kThreads) f(ldv(z, i), i);
+    __syncthreads();
+    prefix = s.prefix;
+    remaining = s.remaining;
+    mask |= 0xffu << shift;
+    __syncthreads();
   }
+  return prefix;
+}
+
+__device__ __forceinline__ unsigned long long pack_candidate(uint32_t key, int i) {
+  return (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(i));
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int top_k, float top_p, float inv_temp,
                         unsigned long long seed, unsigned long long offset, long long* __restrict__ out_ids,
                         float* __restrict__ out_logprob) {
-  __shared__ unsigned int hist[4096];
+  extern __shared__ unsigned long long gather_buf[];  // [kGather]
+  unsigned int* hist = reinterpret_cast<unsigned int*>(gather_buf);  // [4096], the radix select over the row only
   __shared__ unsigned long long cand[kCap];
   __shared__ float prob[kCap];
   __shared__ float warp_tot[kThreads / 32];
   __shared__ unsigned int warp_cnt[kThreads / 32];
-  __shared__ unsigned int s_prefix, s_remaining, s_above, s_pop, s_count, s_nkeep;
+  __shared__ SelectScratch select;
+  __shared__ unsigned int s_prefix, s_remaining, s_above, s_pop, s_count, s_nkeep, s_total, s_bound, s_overflow;
   __shared__ float s_mass;
 
-  const int row = blockIdx.x;
+  const int parts = static_cast<int>(cluster_size_x()), part = static_cast<int>(cluster_ctarank());
+  const int row = static_cast<int>(blockIdx.x) / parts;
   const T* z = logits + static_cast<long long>(row) * ld;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const int k = top_k < 1 ? 1 : (top_k > V ? V : top_k);
 
-  // ---- 1. radix select on order-preserving keys, digits of 12, 8, 8 and 4 bits from the top.  After each digit
-  //         the threshold bin is located by a parallel suffix scan; as soon as the elements above the bin plus the
-  //         bin itself fit into the candidate buffer the search stops and they are all gathered (the sort below
-  //         finds the exact k-th among them).  With k <= 1024 that is the case after the first digit for any
-  //         reasonable logit distribution, so a row is read twice (histogram, gather) instead of five times.
   if (tid == 0) {
     s_prefix = 0;
     s_remaining = static_cast<unsigned int>(k);
     s_above = 0;
     s_pop = static_cast<unsigned int>(V);
     s_count = 0;
+    s_total = 0;
+    s_bound = 0;
+    s_overflow = 0;
   }
-  // ---- 1a. threshold from the thread maxima (one pass, no atomics).  hist[] doubles as the key array.
+  __syncthreads();
+  if (parts > 1) cluster_sync();  // the first CTA's counters are set before anyone adds to them
+
+  // ---- 1. bound from the maxima of a first sweep, then one streaming pass.  The 16-byte vectors of the row
+  //         are dealt to the CTAs in contiguous slices; the unaligned head and the tail of the row go to the first.
   {
-    uint32_t best = 0u;  // smaller than the key of any float
-    for_each_in_row(z, V, [&](float x, int) {
-      const uint32_t key = f2key(x);
-      best = key > best ? key : best;
-    });
-    hist[tid] = best;
-    __syncthreads();
-    // k-th largest of the 1024 thread maxima by a radix select over their keys (four 8-bit digits from the top;
-    // bins in hist[1024 .. 1279], scanned by warp 0): a few microseconds, against tens for comparing all pairs.
-    {
-      unsigned int* bins = hist + kThreads;
-      uint32_t prefix = 0u, mask = 0u;
-      unsigned int remaining = static_cast<unsigned int>(k <= kThreads ? k : kThreads);
-#pragma unroll 1
-      for (int shift = 24; shift >= 0; shift -= 8) {
-        if (tid < 256) bins[tid] = 0u;
-        __syncthreads();
-        {
-          // warp-aggregated counting: the maxima share their leading bits, so most lanes of a warp hit the same bin
-          const bool active = (best & mask) == prefix;
-          const uint32_t digit = (best >> shift) & 0xffu;
-          const unsigned int peers = __match_any_sync(0xffffffffu, active ? digit : 0xffffffffu);
-          if (active && lane == __ffs(peers) - 1) atomicAdd(&bins[digit], static_cast<unsigned int>(__popc(peers)));
-        }
-        __syncthreads();
-        if (warp == 0) {
-          // lane l owns bins 255 - 8 l ... 248 - 8 l (highest first); inclusive scan of the lanes' sums
-          unsigned int mine = 0u;
+    constexpr int kVec = 16 / sizeof(T);
+    int head = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(z) & 15u)) & 15u) / sizeof(T));
+    if (head > V) head = V;
+    const int nvec = (V - head) / kVec;
+    const int per = (nvec + parts - 1) / parts;
+    const int v0 = min(nvec, part * per), v1 = min(nvec, v0 + per);
+    const uint4* p = reinterpret_cast<const uint4*>(z + head);
+    constexpr int kUnroll = 4;
+    // f(vector, index) for the vectors [v0, end) dealt to this thread, the next four in flight while four are looked at
+    auto sweep = [&](int end, auto&& f) {
+      uint4 q[kUnroll];
+      int v = v0 + tid;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) mine += bins[255 - (lane * 8 + j)];
-          unsigned int incl = mine;
+      for (int u = 0; u < kUnroll; ++u)
+        if (v + u * kThreads < end) q[u] = __ldg(p + v + u * kThreads);
+      while (v < end) {
+        uint4 now[kUnroll];
+        const int at = v;
+        v += kUnroll * kThreads;
 #pragma unroll
-          for (int off = 1; off < 32; off <<= 1) {
-            const unsigned int o = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += o;
-          }
-          const unsigned int before = incl - mine;
-          if (before < remaining && remaining <= incl) {  // exactly one lane: the digit is one of its bins
-            unsigned int acc = before;
-            int bin = 255 - lane * 8;
-            for (int j = 0; j < 8; ++j) {
-              bin = 255 - (lane * 8 + j);
-              if (acc + bins[bin] >= remaining) break;
-              acc += bins[bin];
-            }
-            s_prefix = prefix | (static_cast<uint32_t>(bin) << shift);
-            s_remaining = remaining - acc;
-          }
+        for (int u = 0; u < kUnroll; ++u) {
+          now[u] = q[u];
+          if (v + u * kThreads < end) q[u] = __ldg(p + v + u * kThreads);
         }
-        __syncthreads();
-        prefix = s_prefix;
-        remaining = s_remaining;
-        mask |= 0xffu << shift;
-        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+          if (at + u * kThreads < end) f(now[u], at + u * kThreads, u);
       }
-      // s_prefix now is the k-th largest thread maximum: a lower bound of the row's k-th largest key
-      if (tid == 0) s_remaining = static_cast<unsigned int>(k);
-    }
-    __syncthreads();
-    const uint32_t from = s_prefix;
-    if (k <= kThreads) {
-      for_each_in_row(z, V, [&](float x, int i) {
-        const uint32_t key = f2key(x);
-        if (key >= from) {
-          const unsigned int slot = atomicAdd(&s_count, 1u);
-          if (slot < kCap) cand[slot] = (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(i));
-        }
+    };
+    uint32_t best[kUnroll] = {0u, 0u, 0u, 0u};  // smaller than the key of any number
+    const bool few = k <= kFewLimit;
+    const int sample = few ? min(v1 - v0, max((v1 - v0) / kSampleShare, kMinSample / kVec)) : v1 - v0;
+    sweep(v0 + sample, [&](const uint4& q, int, int u) {
+      const T* e = reinterpret_cast<const T*>(&q);
+#pragma unroll
+      for (int j = 0; j < kVec; ++j) best[u] = max(best[u], f2key(ldv(e, j)));
+    });
+    // two digits (sign, exponent, seven mantissa bits) are enough: a bound a little lower costs a few more candidates
+    uint32_t from;
+    if (few) {
+      const uint32_t top = max(max(best[0], best[1]), max(best[2], best[3]));
+      from = block_kth_key<2>(select, static_cast<unsigned int>(k), [&](auto&& f) { f(top, true); });
+    } else {
+      from = block_kth_key<2>(select, static_cast<unsigned int>(k), [&](auto&& f) {
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) f(best[u], true);
       });
     }
+    auto keep = [&](uint32_t kk, int i) {
+      const unsigned int slot = atomicAdd(&s_count, 1u);
+      if (slot < kGather) gather_buf[slot] = pack_candidate(kk, i);
+    };
+    sweep(v1, [&](const uint4& q, int v, int) {
+      const T* e = reinterpret_cast<const T*>(&q);
+      uint32_t kk[kVec], top = 0u;
+#pragma unroll
+      for (int j = 0; j < kVec; ++j) {
+        kk[j] = f2key(ldv(e, j));
+        top = max(top, kk[j]);
+      }
+      if (top >= from) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j)
+          if (kk[j] >= from) keep(kk[j], head + v * kVec + j);
+      }
+    });
+    if (part == 0) {
+      const int tail = head + nvec * kVec;
+      for (int i = tid; i < head + (V - tail); i += kThreads) {
+        const int at = i < head ? i : tail + (i - head);
+        const uint32_t kk = f2key(ldv(z, at));
+        if (kk >= from) keep(kk, at);
+      }
+    }
+    __syncthreads();
+    if (parts > 1) {
+      // the highest bound of the cluster holds for the row; what reaches it goes to the first CTA's sort buffer
+      const uint32_t bound0 = mapa_u32(smem_u32(&s_bound), 0), total0 = mapa_u32(smem_u32(&s_total), 0);
+      const uint32_t over0 = mapa_u32(smem_u32(&s_overflow), 0), cand0 = mapa_u32(smem_u32(cand), 0);
+      if (tid == 0) {
+        cluster_max_u32(bound0, from);
+        if (s_count > static_cast<unsigned int>(kGather)) cluster_max_u32(over0, 1u);
+      }
+      cluster_sync();
+      uint32_t bound;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bound) : "r"(bound0) : "memory");
+      const int mine = static_cast<int>(min(s_count, static_cast<unsigned int>(kGather)));
+      for (int i = tid; i < mine; i += kThreads) {
+        const unsigned long long c = gather_buf[i];
+        if (static_cast<uint32_t>(c >> 32) >= bound) {
+          const unsigned int slot = cluster_add_u32(total0, 1u);
+          if (slot < kCap) cluster_store_u64(cand0 + slot * 8u, c);
+        }
+      }
+      cluster_sync();
+      if (part != 0) return;  // nothing of this CTA is read any more
+    } else {
+      const unsigned int have = s_count;
+      if (have > static_cast<unsigned int>(kGather)) {
+        if (tid == 0) s_overflow = 1u;
+      } else {
+        uint32_t bound = 0u;
+        if (have > static_cast<unsigned int>(kCap)) {  // exact k-th key of the candidates
+          const int rounds = static_cast<int>((have + kThreads - 1) / kThreads);
+          bound = block_kth_key<4>(select, static_cast<unsigned int>(k), [&](auto&& f) {
+            for (int r = 0; r < rounds; ++r) {
+              const unsigned int i = r * kThreads + tid;
+              const bool in = i < have;
+              f(in ? static_cast<uint32_t>(gather_buf[i] >> 32) : 0u, in);
+            }
+          });
+        }
+        for (unsigned int i = tid; i < have; i += kThreads) {
+          const unsigned long long c = gather_buf[i];
+          if (static_cast<uint32_t>(c >> 32) >= bound) {
+            const unsigned int slot = atomicAdd(&s_total, 1u);
+            if (slot < kCap) cand[slot] = c;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0) s_count = s_total;
     __syncthreads();
   }
-  const bool gathered = k <= kThreads && s_count <= static_cast<unsigned int>(kCap);  // uniform over the block
-  __syncthreads();
-  if (!gathered && tid == 0) s_prefix = 0;
+  // uniform over the block.  Otherwise: radix select over the row, digits of 12, 8, 8 and 4 bits from the top; after each the
+  // threshold bin is located by a parallel suffix scan, until what lies above the bin and the bin itself fit the buffer.
+  const bool gathered = s_overflow == 0u && s_count <= static_cast<unsigned int>(kCap);
   __syncthreads();
   int shift = 32;
 #pragma unroll 1
@@ -212,13 +342,13 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
     if (lane == 31) warp_cnt[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-      unsigned int w = warp_cnt[lane];
+      unsigned int w = lane < kThreads / 32 ? warp_cnt[lane] : 0u;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const unsigned int o = __shfl_up_sync(0xffffffffu, w, off);
         if (lane >= off) w += o;
       }
-      warp_cnt[lane] = w;
+      if (lane < kThreads / 32) warp_cnt[lane] = w;
     }
     __syncthreads();
     const unsigned int before = (warp == 0 ? 0u : warp_cnt[warp - 1]) + (incl - mine);  // count in higher bins
@@ -262,7 +392,8 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
   while (sort_n < n) sort_n <<= 1;
   for (int i = n + tid; i < sort_n; i += kThreads) cand[i] = 0ull;
   __syncthreads();
-  // bitonic sort, descending, sort_n elements
+  // bitonic sort, descending, sort_n elements.  Pairs t = 32 w .. 32 w + 31 at strides up to 32 stay inside the 64 elements
+  // [64 w, 64 w + 64), which one warp owns, so those rounds need no block barrier.
   for (int size = 2; size <= sort_n; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
       for (int t = tid; t < sort_n / 2; t += kThreads) {
@@ -275,7 +406,8 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
           cand[hi] = a;
         }
       }
-      __syncthreads();
+      if (stride > 32 || (stride == 1 && size >= 64)) __syncthreads();  // the next round crosses the warps' blocks
+      else __syncwarp();
     }
   }
 
@@ -294,13 +426,15 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
 
   // ---- 3. softmax over candidates + inclusive scan (fixed tree) + top-p cut
   const float zmax = key2f(static_cast<uint32_t>(cand[0] >> 32));
-  float e0 = 0.f, e1 = 0.f;
-  {
-    const int i0 = 2 * tid, i1 = 2 * tid + 1;
-    if (i0 < n) e0 = expf((key2f(static_cast<uint32_t>(cand[i0] >> 32)) - zmax) * inv_temp);
-    if (i1 < n) e1 = expf((key2f(static_cast<uint32_t>(cand[i1] >> 32)) - zmax) * inv_temp);
+  constexpr int kEach = kCap / kThreads;  // consecutive candidates per thread
+  float e[kEach], own = 0.f;
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const int i = kEach * tid + j;
+    e[j] = i < n ? expf((key2f(static_cast<uint32_t>(cand[i] >> 32)) - zmax) * inv_temp) : 0.f;
+    own += e[j];
   }
-  float incl = e0 + e1;  // thread total, then warp inclusive scan
+  float incl = own;  // thread total, then warp inclusive scan
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
     const float o = __shfl_up_sync(0xffffffffu, incl, off);
@@ -309,19 +443,19 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    float w = warp_tot[lane];
+    float w = lane < kThreads / 32 ? warp_tot[lane] : 0.f;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const float o = __shfl_up_sync(0xffffffffu, w, off);
       if (lane >= off) w += o;
     }
-    warp_tot[lane] = w;  // inclusive over warps
+    if (lane < kThreads / 32) warp_tot[lane] = w;  // inclusive over warps
   }
   __syncthreads();
-  const float base = (warp == 0 ? 0.f : warp_tot[warp - 1]) + (incl - (e0 + e1));  // mass before element 2*tid
-  if (2 * tid < kCap) {
-    prob[2 * tid] = base + e0;
-    prob[2 * tid + 1] = base + e0 + e1;
+  {
+    float run = (warp == 0 ? 0.f : warp_tot[warp - 1]) + (incl - own);  // mass before this thread's candidates
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) prob[kEach * tid + j] = run += e[j];
   }
   __syncthreads();
   const float total = warp_tot[kThreads / 32 - 1];
@@ -331,9 +465,11 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
   {
     const float lim = top_p * total;
     unsigned int local = 0;
-    const int i0 = 2 * tid, i1 = 2 * tid + 1;
-    if (i0 < n && (i0 == 0 || prob[i0 - 1] <= lim)) ++local;
-    if (i1 < n && prob[i1 - 1] <= lim) ++local;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      const int i = kEach * tid + j;
+      if (i < n && (i == 0 || prob[i - 1] <= lim)) ++local;
+    }
     if (local) atomicAdd(&s_nkeep, local);
   }
   __syncthreads();
@@ -368,10 +504,15 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
 // smallest set of highest-probability tokens whose mass reaches top_p (all tokens tied with the
 // cut value are kept), draw by inverse CDF in INDEX order inside the kept set.
 //
-// The cut is found by a 4-pass radix search over the order-preserving keys, with the bins holding
-// probability MASS instead of counts.  Masses are 40-bit fixed point in 64-bit integers, so the
-// shared-memory atomics that build the histograms are order-independent and the result is
+// Masses are 40-bit fixed point in 64-bit integers, so sums do not depend on their order and the result is
 // deterministic: a pure function of (row, top_p, T, seed, offset, row index).
+//
+// Three sweeps over the row, 16 bytes per access: maximum; histogram of the mass over 256 equal steps of (max - x) / T up to
+// 28, beyond which the mass is 0 (equal steps hold a percent of the tokens each, where the leading bits of the key put nearly
+// all into four bins); then the tokens of the step that holds the cut are gathered and every warp sums what lies
+// above it in its own stretch of the row.  The cut itself is a radix search among the gathered tokens in shared memory, and the draw rescans
+// one warp's stretch.  The histogram has one copy per lane, so the 32-bit atomics of a warp (14 bits of the mass
+// at a time) hit 32 banks.  If the step does not fit the buffer (flat logits), a 4-pass radix search over the row's keys follows.
 // ---------------------------------------------------------------------------------------------
 constexpr int kNucleusThreads = 1024;
 
@@ -381,17 +522,72 @@ __device__ __forceinline__ unsigned long long fixed_mass(float x, float row_max,
   return static_cast<unsigned long long>(e * 1099511627776.0f);
 }
 
+constexpr int kSteps = 256;
+constexpr int kMassBits = 14;   // of the 41 bits per histogram word: 2^18 tokens per lane fit 32 bits
+constexpr int kMassWords = 3;
+constexpr int kNucleusBytes = kMassWords * kSteps * 32 * 4;
+constexpr int kNucleusGather = kNucleusBytes / 8;  // the histogram's memory is reused for the gathered tokens
+
+// Calls f(value, index) for the elements of one warp's stretch of the row (stretches follow one another in index order).
+// The 16-byte vectors are dealt to the warps evenly; the unaligned head belongs to the first, the tail to the last.
+template <typename T, typename F>
+__device__ __forceinline__ void for_each_in_stretch(const T* __restrict__ z, int V, F&& f) {
+  constexpr int kVec = 16 / sizeof(T);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int head = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(z) & 15u)) & 15u) / sizeof(T));
+  if (head > V) head = V;
+  const int nvec = (V - head) / kVec, warps = kNucleusThreads / 32, per = (nvec + warps - 1) / warps;
+  const int v0 = min(nvec, warp * per), v1 = min(nvec, v0 + per);
+  const uint4* p = reinterpret_cast<const uint4*>(z + head);
+  if (warp == 0 && lane < head) f(ldv(z, lane), lane);
+  constexpr int kAhead = 4;
+  int v = v0 + lane;
+  for (; v + 32 * (kAhead - 1) < v1; v += 32 * kAhead) {
+    uint4 q[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) q[u] = __ldg(p + v + 32 * u);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const T* e = reinterpret_cast<const T*>(&q[u]);
+#pragma unroll
+      for (int j = 0; j < kVec; ++j) f(ldv(e, j), head + (v + 32 * u) * kVec + j);
+    }
+  }
+  for (; v < v1; v += 32) {
+    const uint4 q = __ldg(p + v);
+    const T* e = reinterpret_cast<const T*>(&q);
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) f(ldv(e, j), head + v * kVec + j);
+  }
+  const int tail = head + nvec * kVec;
+  if (warp == warps - 1 && tail + lane < V) f(ldv(z, tail + lane), tail + lane);
+}
+// [begin, end) of warp `warp`'s stretch
+template <typename T>
+__device__ __forceinline__ int2 stretch_of(const T* z, int V, int warp) {
+  constexpr int kVec = 16 / sizeof(T);
+  int head = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(z) & 15u)) & 15u) / sizeof(T));
+  if (head > V) head = V;
+  const int nvec = (V - head) / kVec, warps = kNucleusThreads / 32, per = (nvec + warps - 1) / warps;
+  const int v0 = min(nvec, warp * per), v1 = min(nvec, v0 + per);
+  return make_int2(warp == 0 ? 0 : head + v0 * kVec, warp == warps - 1 ? V : head + v1 * kVec);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kNucleusThreads)
 sample_nucleus_kernel(const T* __restrict__ logits, long long ld, int V, float top_p, float inv_temp,
                       unsigned long long seed, unsigned long long offset, long long* __restrict__ out_ids,
                       float* __restrict__ out_logprob) {
+  extern __shared__ unsigned long long dyn[];
+  unsigned int* lanes = reinterpret_cast<unsigned int*>(dyn);  // [kMassWords][kSteps][32]
+  unsigned long long* gathered = dyn;                          // [kNucleusGather]: key << 32 | index
   __shared__ unsigned long long hist[256];
   __shared__ unsigned long long warp_part[kNucleusThreads / 32];
   __shared__ float warp_max[kNucleusThreads / 32];
   __shared__ unsigned long long s_total, s_above, s_target, s_base;
   __shared__ uint32_t s_prefix;
-  __shared__ int s_pick;
+  __shared__ int s_pick, s_step, s_warp;
+  __shared__ unsigned int s_count;
   __shared__ float s_max;
   const int row = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -399,65 +595,165 @@ sample_nucleus_kernel(const T* __restrict__ logits, long long ld, int V, float t
 
   // ---- row maximum
   float m = -INFINITY;
-  for (int i = tid; i < V; i += kNucleusThreads) m = fmaxf(m, ldv(z, i));
+  for_each_in_stretch(z, V, [&](float x, int) { m = fmaxf(m, x); });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (lane == 0) warp_max[warp] = m;
+  for (int i = tid; i < kMassWords * kSteps * 32; i += kNucleusThreads) lanes[i] = 0u;
   __syncthreads();
-  if (tid == 0) {
-    float r = warp_max[0];
-    for (int w = 1; w < kNucleusThreads / 32; ++w) r = fmaxf(r, warp_max[w]);
-    s_max = r;
-    s_prefix = 0u;
-    s_above = 0ull;
+  if (warp == 0) {
+    float r = warp_max[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+    if (lane == 0) {
+      s_max = r;
+      s_prefix = 0u;
+      s_above = 0ull;
+      s_count = 0u;
+      s_step = kSteps - 1;
+    }
   }
   __syncthreads();
   const float row_max = s_max;
 
-  // ---- radix search for the cut key: after pass r the top 8*(r+1) bits of the cut are known
+  // ---- mass per step of (max - x) / T: monotone in x, so the steps are in the order of the keys
+  auto step_of = [&](float x) {
+    const int b = static_cast<int>((row_max - x) * inv_temp * (kSteps / 28.f));
+    return b < 0 ? 0 : (b < kSteps ? b : kSteps - 1);
+  };
+  for_each_in_stretch(z, V, [&](float x, int) {
+    const unsigned long long mass = fixed_mass(x, row_max, inv_temp);
+    if (mass == 0ull) return;
+    unsigned int* h = lanes + step_of(x) * 32 + lane;
+#pragma unroll
+    for (int w = 0; w < kMassWords; ++w) {
+      const unsigned int part = static_cast<unsigned int>(mass >> (w * kMassBits)) & ((1u << kMassBits) - 1u);
+      if (part) atomicAdd(h + w * kSteps * 32, part);
+    }
+  });
+  __syncthreads();
+  for (int b = warp; b < kSteps; b += kNucleusThreads / 32) {
+    unsigned long long sum = 0ull;
+#pragma unroll
+    for (int w = 0; w < kMassWords; ++w) sum += static_cast<unsigned long long>(lanes[(w * kSteps + b) * 32 + lane]) << (w * kMassBits);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) hist[b] = sum;
+  }
+  __syncthreads();
+  // mass that the kept set must reach (at least one unit so that the best token is always kept), and the step that holds it
+  auto locate = [&](bool descending, unsigned long long above0) {
+    // lane l owns bins 8 l .. 8 l + 7 of the order; returns through s_step / s_above
+    if (warp == 0) {
+      unsigned long long mine = 0ull;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mine += hist[descending ? 255 - (lane * 8 + j) : lane * 8 + j];
+      unsigned long long incl = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
+      }
+      const unsigned long long before = above0 + incl - mine;
+      if (before < s_target && s_target <= before + mine) {  // at most one lane
+        unsigned long long acc = before;
+        int j = 0;
+        for (; j < 7; ++j) {
+          const unsigned long long h = hist[descending ? 255 - (lane * 8 + j) : lane * 8 + j];
+          if (acc + h >= s_target) break;
+          acc += h;
+        }
+        s_step = descending ? 255 - (lane * 8 + j) : lane * 8 + j;
+        s_above = acc;  // mass of the tokens before the chosen bin
+      }
+    }
+    __syncthreads();
+  };
+  if (warp == 0) {
+    unsigned long long total = 0ull;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) total += hist[lane * 8 + j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    if (lane == 0) {
+      s_total = total;
+      const double want = static_cast<double>(top_p) * static_cast<double>(total);
+      const unsigned long long t = want < 1.0 ? 1ull : static_cast<unsigned long long>(want);
+      s_target = t;
+    }
+  }
+  __syncthreads();
+  locate(false, 0ull);
+  const int cut_step = s_step;
+
+  // ---- gather the tokens of that step; mass of the kept tokens above it per stretch
+  unsigned long long part = 0ull;
+  for_each_in_stretch(z, V, [&](float x, int i) {
+    const int b = step_of(x);
+    if (b < cut_step) {
+      part += fixed_mass(x, row_max, inv_temp);
+    } else if (b == cut_step) {
+      const unsigned int slot = atomicAdd(&s_count, 1u);
+      if (slot < kNucleusGather) gathered[slot] = (static_cast<unsigned long long>(f2key(x)) << 32) | static_cast<uint32_t>(i);
+    }
+  });
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  if (lane == 0) warp_part[warp] = part;
+  __syncthreads();
+  const unsigned int have = s_count;
+  const bool fits = have <= static_cast<unsigned int>(kNucleusGather);  // uniform
+
+  // ---- radix search for the cut key: after pass r its top 8 (r + 1) bits are known
+  if (!fits && tid == 0) s_above = 0ull;
+  __syncthreads();
   for (int pass = 0; pass < 4; ++pass) {
     const int shift = 24 - 8 * pass;
     for (int b = tid; b < 256; b += kNucleusThreads) hist[b] = 0ull;
     __syncthreads();
     const uint32_t prefix = s_prefix;
     const uint32_t mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
-    for (int i = tid; i < V; i += kNucleusThreads) {
-      const float x = ldv(z, i);
-      const uint32_t key = f2key(x);
-      if ((key & mask) == (prefix & mask)) atomicAdd(&hist[(key >> shift) & 0xffu], fixed_mass(x, row_max, inv_temp));
+    const unsigned long long above = s_above;
+    if (fits) {
+      for (unsigned int i = tid; i < have; i += kNucleusThreads) {
+        const uint32_t key = static_cast<uint32_t>(gathered[i] >> 32);
+        if ((key & mask) == (prefix & mask)) atomicAdd(&hist[(key >> shift) & 0xffu], fixed_mass(key2f(key), row_max, inv_temp));
+      }
+    } else {
+      for (int i = tid; i < V; i += kNucleusThreads) {
+        const float x = ldv(z, i);
+        const uint32_t key = f2key(x);
+        if ((key & mask) == (prefix & mask)) atomicAdd(&hist[(key >> shift) & 0xffu], fixed_mass(x, row_max, inv_temp));
+      }
     }
+    if (tid == 0) s_step = 0;
     __syncthreads();
-    if (tid == 0) {
-      if (pass == 0) {
-        unsigned long long total = 0ull;
-        for (int b = 0; b < 256; ++b) total += hist[b];
-        s_total = total;
-        // mass that the kept set must reach (at least one unit so that the best token is always kept)
-        const double want = static_cast<double>(top_p) * static_cast<double>(total);
-        s_target = want < 1.0 ? 1ull : static_cast<unsigned long long>(want);
-      }
-      unsigned long long above = s_above;
-      int b = 255;
-      for (; b > 0; --b) {
-        if (above + hist[b] >= s_target) break;
-        above += hist[b];
-      }
-      s_above = above;  // mass of the tokens strictly above the chosen bin
-      s_prefix = prefix | (static_cast<uint32_t>(b) << shift);
-    }
+    locate(true, above);
+    if (tid == 0) s_prefix = prefix | (static_cast<uint32_t>(s_step) << shift);
     __syncthreads();
   }
   const uint32_t cut = s_prefix;  // keep every token with key >= cut
 
-  // ---- mass of the kept set, then the draw
-  unsigned long long part = 0ull;
-  for (int i = tid; i < V; i += kNucleusThreads) {
-    const float x = ldv(z, i);
-    if (f2key(x) >= cut) part += fixed_mass(x, row_max, inv_temp);
-  }
+  // ---- mass of the kept set per stretch, then the draw
+  if (fits) {
+    for (unsigned int i = tid; i < have; i += kNucleusThreads) {
+      const unsigned long long g = gathered[i];
+      const uint32_t key = static_cast<uint32_t>(g >> 32);
+      if (key < cut) continue;
+      const int at = static_cast<int>(g & 0xffffffffu);
+      int w = 0;  // the stretch that holds index `at`
+      while (at >= stretch_of(z, V, w).y) ++w;
+      atomicAdd(&warp_part[w], fixed_mass(key2f(key), row_max, inv_temp));
+    }
+  } else {
+    part = 0ull;
+    for_each_in_stretch(z, V, [&](float x, int) {
+      if (f2key(x) >= cut) part += fixed_mass(x, row_max, inv_temp);
+    });
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if (lane == 0) warp_part[warp] = part;
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) warp_part[warp] = part;
+  }
   __syncthreads();
   if (tid == 0) {
     unsigned long long kept = 0ull;
@@ -472,15 +768,26 @@ sample_nucleus_kernel(const T* __restrict__ logits, long long ld, int V, float t
     s_target = t;  // pick the first kept token (index order) whose inclusive cumulative mass exceeds t
     s_base = 0ull;
     s_pick = -1;
+    s_warp = kNucleusThreads / 32;  // the stretch that holds it (none if nothing is kept)
+    unsigned long long before = 0ull;
+    for (int w = 0; w < kNucleusThreads / 32; ++w) {
+      if (t < before + warp_part[w]) {
+        s_warp = w;
+        s_base = before;
+        break;
+      }
+      before += warp_part[w];
+    }
   }
   __syncthreads();
+  const int2 range = s_warp < kNucleusThreads / 32 ? stretch_of(z, V, s_warp) : make_int2(0, 0);
 
-  // ---- index-order scan in tiles of kNucleusThreads tokens
-  for (int base = 0; base < V && s_pick < 0; base += kNucleusThreads) {
+  // ---- index-order scan of that stretch in tiles of kNucleusThreads tokens
+  for (int base = range.x; base < range.y && s_pick < 0; base += kNucleusThreads) {
     const int i = base + tid;
     unsigned long long mine = 0ull;
     float x = 0.f;
-    if (i < V) {
+    if (i < range.y) {
       x = ldv(z, i);
       if (f2key(x) >= cut) mine = fixed_mass(x, row_max, inv_temp);
     }
@@ -530,32 +837,62 @@ void sample_nucleus(const void* logits, long long ld, int dtype, int rows, int V
                     cudaStream_t stream) {
   if (rows <= 0) return;
   const float inv_temp = 1.f / temperature;
-  if (dtype == 0)
-    sample_nucleus_kernel<float><<<rows, kNucleusThreads, 0, stream>>>(static_cast<const float*>(logits), ld, V, top_p,
-                                                                       inv_temp, seed, offset, out_ids, out_logprob);
-  else if (dtype == 1)
-    sample_nucleus_kernel<__nv_bfloat16><<<rows, kNucleusThreads, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(logits), ld, V, top_p, inv_temp, seed, offset, out_ids, out_logprob);
-  else
-    sample_nucleus_kernel<__half><<<rows, kNucleusThreads, 0, stream>>>(static_cast<const __half*>(logits), ld, V, top_p,
-                                                                        inv_temp, seed, offset, out_ids, out_logprob);
+  auto launch = [&](auto kernel, auto* typed) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(typed)>>;
+    static PerDeviceOnce configured;  // one per element type
+    if (configured.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNucleusBytes);
+    kernel<<<rows, kNucleusThreads, kNucleusBytes, stream>>>(static_cast<const T*>(logits), ld, V, top_p, inv_temp, seed, offset,
+                                                             out_ids, out_logprob);
+  };
+  if (dtype == 0) launch(sample_nucleus_kernel<float>, static_cast<const float*>(nullptr));
+  else if (dtype == 1) launch(sample_nucleus_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(nullptr));
+  else launch(sample_nucleus_kernel<__half>, static_cast<const __half*>(nullptr));
 }
+
+namespace {
+
+// CTAs per row: enough for two on every SM, at most eight (the portable cluster size), and slices of at least twice the
+// smallest sample: below that the merge is not repaid.
+int sample_parts(int rows, int V) {
+  int parts = 1;
+  while (parts < 8 && static_cast<long long>(rows) * parts * 2 <= 296 && V / (parts * 2) >= 2 * kMinSample) parts *= 2;
+  return parts;
+}
+
+template <typename T>
+void launch_sample(const void* logits, long long ld, int rows, int V, int top_k, float top_p, float inv_temp,
+                   unsigned long long seed, unsigned long long offset, long long* out_ids, float* out_logprob, cudaStream_t stream) {
+  auto kernel = sample_topk_topp_kernel<T>;
+  constexpr int kBytes = kGather * 8;
+  static PerDeviceOnce configured;
+  if (configured.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+  const int parts = sample_parts(rows, V);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * parts);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(parts);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<const T*>(logits), ld, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob);
+}
+
+}  // namespace
 
 void sample_topk_topp(const void* logits, long long ld, int dtype, int rows, int V, int top_k, float top_p,
                       float temperature, unsigned long long seed, unsigned long long offset, long long* out_ids,
                       float* out_logprob, cudaStream_t stream) {
   if (rows <= 0) return;
   const float inv_temp = 1.f / temperature;
-  if (dtype == 0)
-    sample_topk_topp_kernel<float><<<rows, kThreads, 0, stream>>>(static_cast<const float*>(logits), ld, V, top_k,
-                                                                  top_p, inv_temp, seed, offset, out_ids, out_logprob);
+  if (dtype == 0) launch_sample<float>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, stream);
   else if (dtype == 1)
-    sample_topk_topp_kernel<__nv_bfloat16><<<rows, kThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), ld,
-                                                                          V, top_k, top_p, inv_temp, seed, offset,
-                                                                          out_ids, out_logprob);
-  else
-    sample_topk_topp_kernel<__half><<<rows, kThreads, 0, stream>>>(static_cast<const __half*>(logits), ld, V, top_k,
-                                                                   top_p, inv_temp, seed, offset, out_ids, out_logprob);
+    launch_sample<__nv_bfloat16>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, stream);
+  else launch_sample<__half>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, stream);
 }
 
 int sample_topk_limit() { return 1024; }
