@@ -135,6 +135,29 @@ struct LogpRowsArgs {
 };
 void logp_rows(const LogpRowsArgs& args, cudaStream_t stream);
 
+// GRPO loss over materialised logits: per row (token) the surrogate terms, their unit gradients and the log-sum-exp.
+struct GrpoRowsArgs {
+  const void* policy;
+  const void* ref;
+  long long ld_policy, ld_ref;
+  int dtype;
+  const long long* ids;
+  const unsigned char* mask;
+  const float* old_logp;
+  const double* adv;  // per sequence of `tokens` rows
+  long long rows, tokens;
+  int V;
+  float clip_lo, clip_hi;
+  float *pl, *kl, *d_pl, *d_kl, *lse;  // [rows]
+};
+void grpo_rows(const GrpoRowsArgs& args, cudaStream_t stream);
+void grpo_rows_backward(const GrpoRowsArgs& args, const float* stats, const float* g_loss, const float* g_pl, const float* g_kl,
+                        float beta, void* grad, long long ld_grad, cudaStream_t stream);
+void ids_outside(const long long* ids, const unsigned char* mask, long long n, long long V, int* flag, cudaStream_t stream);
+// out4 = {loss, policy_loss, kl, count} of per-token terms (zero where masked)
+void surrogate_reduce(const float* pl, const float* kl, const unsigned char* mask, long long n, float beta, float* partials, float* out4,
+                      cudaStream_t stream);
+
 struct RatioKlFwdArgs {
   const void* policy;
   const void* ref;  // null: reference == policy
@@ -178,7 +201,7 @@ namespace rlk {
 // bounds == null -> uniform groups of `uniform` sequences.
 // n_rewards: length of ``rewards`` / ``adv`` (group bounds are checked against it in debug-bounds builds)
 void group_advantages(const float* rewards, const long long* bounds, int num_groups, long long uniform, float eps,
-                      float* adv, long long n_rewards, cudaStream_t stream);
+                      float* adv, double* adv64, long long n_rewards, cudaStream_t stream);
 
 struct SurrogateFwdArgs {
   const float* logp;      // [n] policy log-probs

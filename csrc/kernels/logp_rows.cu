@@ -281,33 +281,98 @@ __global__ void __launch_bounds__(kThreads) ratio_kl_fwd_kernel(const T* __restr
   }
 }
 
-// dlogits[row, j] = coef * (onehot_j - softmax_j), coef = g_ratio * ratio + g_kl * (1 - exp(d))
-template <typename T>
-__global__ void __launch_bounds__(kThreads) ratio_kl_bwd_kernel(const T* __restrict__ pol, long long ld_p,
-                                                                const long long* __restrict__ ids,
-                                                                const unsigned char* __restrict__ mask,
-                                                                const float* __restrict__ g_ratio,
-                                                                const float* __restrict__ g_kl,
-                                                                const float* __restrict__ ratio,
-                                                                const float* __restrict__ save_d,
-                                                                const float* __restrict__ save_lse, int V,
-                                                                T* __restrict__ grad, long long ld_g) {
+// Coefficient of a row's gradient from upstream gradients of (ratio, kl) ...
+struct RatioKlCoef {
+  const float *g_ratio, *g_kl, *ratio, *save_d;
+  __device__ __forceinline__ float operator()(long long row) const {
+    return g_ratio[row] * ratio[row] + g_kl[row] * (1.f - expf(save_d[row]));
+  }
+};
+// ... and of (loss, policy loss, kl): unit gradients per token over the token count (stats[3]); a null upstream is zero.
+struct SurrogateCoef {
+  const float *d_pl, *d_kl, *stats, *g_loss, *g_pl, *g_kl;
+  float beta;
+  __device__ __forceinline__ float operator()(long long row) const {
+    const float inv = 1.f / fmaxf(stats[3], 1e-8f);
+    const float gl = g_loss ? *g_loss : 0.f, gp = g_pl ? *g_pl : 0.f, gk = g_kl ? *g_kl : 0.f;
+    return (gl + gp) * inv * d_pl[row] + (gl * beta + gk) * inv * d_kl[row];
+  }
+};
+
+// dlogits[row, j] = coef(row) * (onehot_j - softmax_j)
+//
+// One read of the logits and one write of their gradient, so it is bound by memory: 16-byte streaming accesses, four
+// loads in flight per thread.  A row whose logits and gradient share their offset from a 16-byte boundary (any V when both
+// tensors are dense) is peeled up to it; rows that do not go element by element.
+template <typename T, class Coef>
+__global__ void __launch_bounds__(kThreads) logp_bwd_kernel(const T* __restrict__ pol, long long ld_p,
+                                                            const long long* __restrict__ ids,
+                                                            const unsigned char* __restrict__ mask, const Coef coef_of,
+                                                            const float* __restrict__ save_lse, int V, T* __restrict__ grad,
+                                                            long long ld_g) {
+  constexpr int kVec = 16 / sizeof(T);
+  constexpr int kUnroll = 4;
   const long long row = blockIdx.x;
   T* grow = grad + row * ld_g;
-  if (!mask[row]) {
-    for (int i = threadIdx.x; i < V; i += kThreads) grow[i] = from_f<T>(0.f);
+  const T* prow = pol + row * ld_p;
+  const bool active = mask[row] != 0;
+  const uintptr_t at_g = reinterpret_cast<uintptr_t>(grow) & 15u;
+  const bool together = !active || (reinterpret_cast<uintptr_t>(prow) & 15u) == at_g;
+  int head = together ? static_cast<int>(((16 - at_g) & 15u) / sizeof(T)) : V;
+  if (head > V) head = V;
+  const int body = (V - head) / kVec;
+  const int tail = head + body * kVec;
+  uint4* gv = reinterpret_cast<uint4*>(grow + head);
+  if (!active) {
+    for (int i = threadIdx.x; i < head; i += kThreads) grow[i] = from_f<T>(0.f);
+    for (int i = threadIdx.x; i < body; i += kThreads) __stcs(gv + i, make_uint4(0u, 0u, 0u, 0u));
+    for (int i = tail + threadIdx.x; i < V; i += kThreads) grow[i] = from_f<T>(0.f);
     return;
   }
-  const float coef = g_ratio[row] * ratio[row] + g_kl[row] * (1.f - expf(save_d[row]));
+  const uint4* pv = reinterpret_cast<const uint4*>(prow + head);
+  // the first vectors are requested before the row's scalars, later ones before their predecessors are worked on
+  uint4 q[kUnroll];
+  int i = threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u)
+    if (i + u * kThreads < body) q[u] = __ldcs(pv + i + u * kThreads);
+  const float coef = coef_of(row);
   const float lse2 = save_lse[row] * kLog2e;
   long long t = ids[row];
   if (t < 0 || t >= V) t = 0;
-  const T* prow = pol + row * ld_p;
-  for (int i = threadIdx.x; i < V; i += kThreads) {
-    const float p = fast_exp2(fmaf(to_f(prow[i]), kLog2e, -lse2));
-    float g = -coef * p;
-    if (i == t) g += coef;
-    grow[i] = from_f<T>(g);
+  auto one = [&](int at) {
+    float g = -coef * fast_exp2(fmaf(to_f(prow[at]), kLog2e, -lse2));
+    if (at == t) g += coef;
+    grow[at] = from_f<T>(g);
+  };
+  for (int at = threadIdx.x; at < head; at += kThreads) one(at);
+  for (int at = tail + threadIdx.x; at < V; at += kThreads) one(at);
+  const int t_vec = t >= head && t < tail ? static_cast<int>(t - head) / kVec : -1;
+  while (i < body) {
+    uint4 now[kUnroll];
+    const int at = i;
+    i += kUnroll * kThreads;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      now[u] = q[u];
+      if (i + u * kThreads < body) q[u] = __ldcs(pv + i + u * kThreads);
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const int v = at + u * kThreads;
+      if (v < body) {
+        const T* e = reinterpret_cast<const T*>(&now[u]);
+        uint4 o;
+        T* r = reinterpret_cast<T*>(&o);
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+          float g = -coef * fast_exp2(fmaf(to_f(e[j]), kLog2e, -lse2));
+          if (v == t_vec && head + v * kVec + j == t) g += coef;
+          r[j] = from_f<T>(g);
+        }
+        __stcs(gv + v, o);
+      }
+    }
   }
 }
 
@@ -327,10 +392,90 @@ void ratio_kl_forward(const RatioKlFwdArgs& a, cudaStream_t stream) {
 
 void ratio_kl_backward(const RatioKlBwdArgs& a, cudaStream_t stream) {
   if (a.rows <= 0) return;
+  const RatioKlCoef coef{a.g_ratio, a.g_kl, a.ratio, a.save_d};
 #define RLK_LAUNCH(T)                                                                                         \
-  ratio_kl_bwd_kernel<T><<<a.rows, kThreads, 0, stream>>>(static_cast<const T*>(a.policy), a.ld_policy, a.ids, a.mask, \
-                                                          a.g_ratio, a.g_kl, a.ratio, a.save_d, a.save_lse, a.V,     \
-                                                          static_cast<T*>(a.grad), a.ld_grad)
+  logp_bwd_kernel<T><<<a.rows, kThreads, 0, stream>>>(static_cast<const T*>(a.policy), a.ld_policy, a.ids, a.mask, coef, \
+                                                      a.save_lse, a.V, static_cast<T*>(a.grad), a.ld_grad)
+  if (a.dtype == 0) RLK_LAUNCH(float);
+  else if (a.dtype == 1) RLK_LAUNCH(__nv_bfloat16);
+  else RLK_LAUNCH(__half);
+#undef RLK_LAUNCH
+}
+
+// ---------------------------------------------------------------------------------------------
+// GRPO loss over materialised logits: policy and reference rows streamed side by side, and the row's surrogate terms at the
+// end of its CTA, so the forward is this sweep and a reduction over one record per token.
+// ---------------------------------------------------------------------------------------------
+namespace {
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) grpo_rows_kernel(const T* __restrict__ pol, const T* __restrict__ ref, long long ld_p,
+                                                             long long ld_r, const GrpoRowsArgs a) {
+  __shared__ MS red[kThreads / 32];
+  const long long row = blockIdx.x;
+  if (!a.mask[row]) {
+    if (threadIdx.x == 0) a.pl[row] = a.kl[row] = a.d_pl[row] = a.d_kl[row] = a.lse[row] = 0.f;
+    return;
+  }
+  const T* prow = pol + row * ld_p;
+  const T* rrow = ref + row * ld_r;
+  MS p, r;
+  stream_two_rows(prow, rrow, a.V, p, r);
+  p = block_merge(p, red);
+  r = block_merge(r, red);
+  if (threadIdx.x != 0) return;
+  long long t = a.ids[row];
+  if (t < 0 || t >= a.V) t = 0;  // refused by the host
+  // The last steps in 64 bits, one thread per row: log-probs are differences of numbers near 10, and their differences again
+  // (to the old and the reference log-prob) are what the loss is made of.
+  const double ln2 = 0.6931471805599453;
+  const double lse = (static_cast<double>(p.m2) + log2(static_cast<double>(p.s))) * ln2;
+  const double lp = static_cast<double>(to_f(prow[t])) - lse;
+  const double lr = static_cast<double>(to_f(rrow[t])) - (static_cast<double>(r.m2) + log2(static_cast<double>(r.s))) * ln2;
+  const double adv = a.adv[row / a.tokens];
+  const float ratio = expf(static_cast<float>(lp - static_cast<double>(a.old_logp[row])));
+  const double unclipped = ratio * adv, clipped = fminf(fmaxf(ratio, a.clip_lo), a.clip_hi) * adv;
+  const float d = static_cast<float>(lr - lp), e = expf(d);
+  a.pl[row] = static_cast<float>(-fmin(unclipped, clipped));
+  a.kl[row] = expm1f(d) - d;
+  a.d_pl[row] = unclipped <= clipped ? static_cast<float>(-unclipped) : 0.f;
+  a.d_kl[row] = 1.f - e;
+  a.lse[row] = static_cast<float>(lse);
+}
+
+// flag = 1 if an unmasked id lies outside [0, V); one block, no initialisation needed
+__global__ void __launch_bounds__(1024) ids_outside_kernel(const long long* __restrict__ ids, const unsigned char* __restrict__ mask,
+                                                           long long n, long long V, int* __restrict__ flag) {
+  int bad = 0;
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) bad |= mask[i] && (ids[i] < 0 || ids[i] >= V);
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) *flag = bad ? 1 : 0;
+}
+
+}  // namespace
+
+void ids_outside(const long long* ids, const unsigned char* mask, long long n, long long V, int* flag, cudaStream_t stream) {
+  ids_outside_kernel<<<1, 1024, 0, stream>>>(ids, mask, n, V, flag);
+}
+
+void grpo_rows(const GrpoRowsArgs& a, cudaStream_t stream) {
+  if (a.rows <= 0) return;
+#define RLK_LAUNCH(T)                                                                                                       \
+  grpo_rows_kernel<T><<<static_cast<unsigned>(a.rows), kThreads, 0, stream>>>(static_cast<const T*>(a.policy),              \
+                                                                             static_cast<const T*>(a.ref), a.ld_policy, a.ld_ref, a)
+  if (a.dtype == 0) RLK_LAUNCH(float);
+  else if (a.dtype == 1) RLK_LAUNCH(__nv_bfloat16);
+  else RLK_LAUNCH(__half);
+#undef RLK_LAUNCH
+}
+
+void grpo_rows_backward(const GrpoRowsArgs& a, const float* stats, const float* g_loss, const float* g_pl, const float* g_kl, float beta,
+                        void* grad, long long ld_grad, cudaStream_t stream) {
+  if (a.rows <= 0) return;
+  const SurrogateCoef coef{a.d_pl, a.d_kl, stats, g_loss, g_pl, g_kl, beta};
+#define RLK_LAUNCH(T)                                                                                                       \
+  logp_bwd_kernel<T><<<static_cast<unsigned>(a.rows), kThreads, 0, stream>>>(static_cast<const T*>(a.policy), a.ld_policy, a.ids, \
+                                                                            a.mask, coef, a.lse, a.V, static_cast<T*>(grad), ld_grad)
   if (a.dtype == 0) RLK_LAUNCH(float);
   else if (a.dtype == 1) RLK_LAUNCH(__nv_bfloat16);
   else RLK_LAUNCH(__half);

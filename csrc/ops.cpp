@@ -782,11 +782,102 @@ Tensor ratio_kl_bwd(const Tensor& policy, const Tensor& ids, const Tensor& mask,
 }
 
 // ------------------------------------------------------------------------------- RL losses
-Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int64_t uniform, double eps) {
+// int32 flag on the device: 1 if an unmasked id lies outside [0, V)
+Tensor ids_outside(const Tensor& ids, const Tensor& mask, int64_t v) {
+  check_cuda(ids, "ids");
+  TORCH_CHECK(ids.scalar_type() == torch::kInt64 && ids.is_contiguous() && mask.is_cuda() && mask.scalar_type() == torch::kBool &&
+                  mask.is_contiguous() && mask.numel() == ids.numel(),
+              "ids_outside: contiguous int64 ids and bool mask");
+  const c10::cuda::CUDAGuard guard(ids.device());
+  Tensor flag = torch::empty({1}, ids.options().dtype(torch::kInt32));
+  rlk::ids_outside(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), reinterpret_cast<const unsigned char*>(mask.data_ptr<bool>()),
+                   ids.numel(), v, flag.data_ptr<int>(), stream_of(ids));
+  after_launch();
+  return flag;
+}
+
+namespace {
+
+rlk::GrpoRowsArgs grpo_args(const Tensor& policy, const Tensor& ids, const Tensor& mask) {
+  check_rowmajor(policy, "policy_logits");
+  const int64_t rows = policy.size(0);
+  TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == torch::kInt64 && ids.is_contiguous() && ids.numel() == rows, "ids: int64 [rows]");
+  TORCH_CHECK(mask.is_cuda() && mask.scalar_type() == torch::kBool && mask.is_contiguous() && mask.numel() == rows, "mask: bool [rows]");
+  rlk::GrpoRowsArgs a{};
+  a.policy = policy.data_ptr();
+  a.ld_policy = policy.stride(0);
+  a.dtype = dtype_code(policy);
+  a.ids = reinterpret_cast<const long long*>(ids.data_ptr<int64_t>());
+  a.mask = reinterpret_cast<const unsigned char*>(mask.data_ptr<bool>());
+  a.rows = rows;
+  a.V = static_cast<int>(policy.size(1));
+  return a;
+}
+
+}  // namespace
+
+// GRPO loss over logits rows [B * T, V]: ({loss, policy_loss, kl, count}, per-token unit gradients d_pl and d_kl, log-sum-exp)
+std::vector<Tensor> grpo_logits_fwd(const Tensor& policy, const Tensor& ref, const Tensor& ids, const Tensor& mask, const Tensor& old_logp,
+                                    const Tensor& adv, int64_t tokens, double clip_eps, double beta) {
+  rlk::GrpoRowsArgs a = grpo_args(policy, ids, mask);
+  check_rowmajor(ref, "ref_logits");
+  TORCH_CHECK(policy.scalar_type() == ref.scalar_type() && policy.sizes() == ref.sizes(), "policy/ref logits must match");
+  TORCH_CHECK(old_logp.is_cuda() && old_logp.scalar_type() == torch::kFloat32 && old_logp.is_contiguous() && old_logp.numel() == a.rows,
+              "old_logps: float32 [rows]");
+  TORCH_CHECK(tokens >= 1 && adv.is_cuda() && adv.scalar_type() == torch::kFloat64 && adv.is_contiguous() &&
+                  adv.numel() * tokens >= a.rows,
+              "advantages: float64, one per sequence");
+  const c10::cuda::CUDAGuard guard(policy.device());
+  auto fopt = policy.options().dtype(torch::kFloat32);
+  Tensor rec = torch::empty({5, a.rows}, fopt), out4 = torch::empty({4}, fopt), partials = torch::empty({rlk::surrogate_partial_floats()}, fopt);
+  a.ref = ref.data_ptr();
+  a.ld_ref = ref.stride(0);
+  a.old_logp = old_logp.data_ptr<float>();
+  a.adv = adv.data_ptr<double>();
+  a.tokens = tokens;
+  a.clip_lo = static_cast<float>(1.0 - clip_eps);
+  a.clip_hi = static_cast<float>(1.0 + clip_eps);
+  float* r = rec.data_ptr<float>();
+  a.pl = r;
+  a.kl = r + a.rows;
+  a.d_pl = r + 2 * a.rows;
+  a.d_kl = r + 3 * a.rows;
+  a.lse = r + 4 * a.rows;
+  rlk::grpo_rows(a, stream_of(policy));
+  rlk::surrogate_reduce(a.pl, a.kl, a.mask, a.rows, static_cast<float>(beta), partials.data_ptr<float>(), out4.data_ptr<float>(),
+                        stream_of(policy));
+  after_launch(3);
+  return {out4, rec};
+}
+
+Tensor grpo_logits_bwd(const Tensor& policy, const Tensor& ids, const Tensor& mask, const Tensor& out4, const Tensor& rec,
+                       std::optional<Tensor> g_loss, std::optional<Tensor> g_pl, std::optional<Tensor> g_kl, double beta) {
+  rlk::GrpoRowsArgs a = grpo_args(policy, ids, mask);
+  TORCH_CHECK(rec.is_contiguous() && rec.scalar_type() == torch::kFloat32 && rec.numel() == 5 * a.rows, "grpo_logits_bwd: bad records");
+  const c10::cuda::CUDAGuard guard(policy.device());
+  std::vector<Tensor> keep;
+  auto scalar = [&](const std::optional<Tensor>& g) -> const float* {
+    if (!g.has_value() || !g->defined()) return nullptr;
+    TORCH_CHECK(g->is_cuda() && g->numel() == 1, "grpo_logits_bwd: upstream gradients are scalars on the device");
+    keep.push_back(g->to(torch::kFloat32).contiguous());
+    return keep.back().data_ptr<float>();
+  };
+  const float *gl = scalar(g_loss), *gp = scalar(g_pl), *gk = scalar(g_kl);
+  Tensor grad = torch::empty({policy.size(0), policy.size(1)}, policy.options());
+  float* r = rec.data_ptr<float>();
+  a.d_pl = r + 2 * a.rows;
+  a.d_kl = r + 3 * a.rows;
+  a.lse = r + 4 * a.rows;
+  rlk::grpo_rows_backward(a, out4.data_ptr<float>(), gl, gp, gk, static_cast<float>(beta), grad.data_ptr(), grad.stride(0), stream_of(policy));
+  after_launch();
+  return grad;
+}
+
+Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int64_t uniform, double eps, bool f64) {
   check_cuda(rewards, "rewards");
   TORCH_CHECK(rewards.scalar_type() == torch::kFloat32 && rewards.is_contiguous(), "rewards: contiguous float32");
   const c10::cuda::CUDAGuard guard(rewards.device());
-  Tensor adv = torch::empty_like(rewards);
+  Tensor adv = torch::empty_like(rewards, rewards.options().dtype(f64 ? torch::kFloat64 : torch::kFloat32));
   const long long* bptr = nullptr;
   int64_t groups = 0;
   if (bounds.has_value() && bounds->defined()) {
@@ -799,7 +890,8 @@ Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int
   }
   if (groups > 0) {
     rlk::group_advantages(rewards.data_ptr<float>(), bptr, static_cast<int>(groups), uniform, static_cast<float>(eps),
-                          adv.data_ptr<float>(), rewards.numel(), stream_of(rewards));
+                          f64 ? nullptr : adv.data_ptr<float>(), f64 ? adv.data_ptr<double>() : nullptr, rewards.numel(),
+                          stream_of(rewards));
     after_launch();
   }
   return adv;
@@ -1390,7 +1482,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("logp_rows", rlk::traced("rlk::logp_rows", &logp_rows));
   m.def("ratio_kl_fwd", rlk::traced("rlk::ratio_kl_fwd", &ratio_kl_fwd));
   m.def("ratio_kl_bwd", rlk::traced("rlk::ratio_kl_bwd", &ratio_kl_bwd));
-  m.def("group_advantages", rlk::traced("rlk::group_advantages", &group_advantages));
+  m.def("ids_outside", rlk::traced("rlk::ids_outside", &ids_outside));
+  m.def("grpo_logits_fwd", rlk::traced("rlk::grpo_logits_fwd", &grpo_logits_fwd));
+  m.def("grpo_logits_bwd", rlk::traced("rlk::grpo_logits_bwd", &grpo_logits_bwd));
+  m.def("group_advantages", rlk::traced("rlk::group_advantages", &group_advantages), py::arg("rewards"), py::arg("bounds"),
+        py::arg("uniform"), py::arg("eps"), py::arg("f64") = false);
   m.def("surrogate_fwd", rlk::traced("rlk::surrogate_fwd", &surrogate_fwd));
   m.def("surrogate_bwd", rlk::traced("rlk::surrogate_bwd", &surrogate_bwd));
   m.def("dpo_fwd", rlk::traced("rlk::dpo_fwd", &dpo_fwd));

@@ -43,6 +43,24 @@ class _Surrogate(torch.autograd.Function):
         return grad.reshape(ctx.shape), None, None, None, None, None, None, None, None
 
 
+class _FromLogits(torch.autograd.Function):
+    """(loss, policy_loss, kl) from logits rows; one sweep forward, one backward; differentiable w.r.t. the policy logits."""
+
+    @staticmethod
+    def forward(ctx, policy, ref, ids, mask, old_logp, adv, tokens, clip_eps, beta):
+        out4, records = require_ext().grpo_logits_fwd(policy, ref, ids, mask, old_logp, adv, tokens, clip_eps, beta)
+        ctx.save_for_backward(policy, ids, mask, out4, records)
+        ctx.beta = beta
+        ctx.set_materialize_grads(False)
+        return out4[0], out4[1], out4[2]
+
+    @staticmethod
+    def backward(ctx, g_loss, g_pl, g_kl):
+        policy, ids, mask, out4, records = ctx.saved_tensors
+        grad = require_ext().grpo_logits_bwd(policy, ids, mask, out4, records, g_loss, g_pl, g_kl, ctx.beta)
+        return grad, None, None, None, None, None, None, None, None
+
+
 def surrogate_from_logps(
     policy_logps: torch.Tensor,
     ref_logps: Optional[torch.Tensor],
@@ -78,6 +96,9 @@ class FusedGRPOLossSM100Op:
         self, rewards: torch.Tensor, *, samples_per_prompt: Optional[int] = None,
         group_boundaries: Optional[Boundaries] = None, eps: float = 1e-6,
     ) -> torch.Tensor:
+        return self._group_advantages(rewards, samples_per_prompt, group_boundaries, eps)
+
+    def _group_advantages(self, rewards, samples_per_prompt, group_boundaries, eps, f64: bool = False) -> torch.Tensor:
         if not rewards.is_cuda:
             return self._native.group_advantages(
                 rewards, samples_per_prompt=samples_per_prompt, group_boundaries=group_boundaries, eps=eps
@@ -93,7 +114,7 @@ class FusedGRPOLossSM100Op:
                 raise ValueError(
                     f"num_sequences ({n}) must be divisible by samples_per_prompt ({samples_per_prompt})."
                 )
-            return require_ext().group_advantages(flat, None, int(samples_per_prompt), float(eps))
+            return require_ext().group_advantages(flat, None, int(samples_per_prompt), float(eps), f64)
         host = torch.as_tensor(group_boundaries, dtype=torch.long).cpu()
         if host.ndim != 1 or host.numel() < 2:
             raise ValueError("group_boundaries must be a 1D tensor of length num_groups + 1.")
@@ -102,7 +123,7 @@ class FusedGRPOLossSM100Op:
             raise ValueError(f"group sizes sum to {int(sizes.sum())} but there are {n} sequences.")
         if bool((sizes < 1).any()):
             raise ValueError("each group must contain at least one sequence.")
-        return require_ext().group_advantages(flat, host.to(flat.device), 0, float(eps))
+        return require_ext().group_advantages(flat, host.to(flat.device), 0, float(eps), f64)
 
     expand_advantages = staticmethod(NativeGRPOLossOp.expand_advantages)
 
@@ -115,24 +136,27 @@ class FusedGRPOLossSM100Op:
                 policy_logits, ref_logits, action_ids, old_logps, sample_advantages, completion_mask,
                 clip_eps=clip_eps, beta=beta,
             )
-        # logits -> selected log-probs on the streaming kernels, then the fused tail.  The ratio/KL
-        # front end already produces exp(lp - old) and the k3 terms with the right masking, but the
-        # tail needs log-probs, so route through the differentiable log-prob kernel pair instead.
-        from rl_engine.kernels.ops.sm100.logp_autograd import selected_logprobs
-
         keep = completion_mask.to(torch.bool)
         v = policy_logits.shape[-1]
-        if bool((keep & ((action_ids < 0) | (action_ids >= v))).any()):
+        rows = lambda t: t if t.stride(1) == 1 else t.contiguous()
+        ids, mask = action_ids.reshape(-1).long().contiguous(), keep.reshape(-1).contiguous()
+        # The check's answer is copied out first and read after the sweeps over the logits have been queued, so the GPU
+        # does not idle through the round trip (the kernels take any id).
+        answer = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        answer.copy_(require_ext().ids_outside(ids, mask, v), non_blocking=True)
+        copied = torch.cuda.Event()
+        copied.record(torch.cuda.current_stream(ids.device))
+        out = _FromLogits.apply(
+            rows(policy_logits.reshape(-1, v)), rows(ref_logits.detach().to(policy_logits.dtype).reshape(-1, v)), ids, mask,
+            old_logps.detach().reshape(-1).float().contiguous(), sample_advantages.detach().reshape(-1).double().contiguous(),
+            policy_logits.shape[-2] if policy_logits.ndim > 2 else 1, float(clip_eps), float(beta),
+        )
+        copied.synchronize()
+        if int(answer):
             raise ValueError(
                 f"action_ids at active (unmasked) positions must be in [0, {v}); found out-of-range ids."
             )
-        ids = torch.where(keep, action_ids, torch.zeros_like(action_ids))
-        lp = selected_logprobs(policy_logits, ids, keep)
-        with torch.no_grad():
-            lr = selected_logprobs(ref_logits.to(policy_logits.dtype), ids, keep)
-        return surrogate_from_logps(
-            lp, lr, old_logps, keep, sample_advantages=sample_advantages, clip_eps=clip_eps, beta=beta
-        )
+        return out
 
     def apply_from_logps(
         self, policy_logps, ref_logps, old_logps, sample_advantages, completion_mask,
@@ -152,9 +176,7 @@ class FusedGRPOLossSM100Op:
         *, clip_eps: float = 0.2, beta: float = 0.0, samples_per_prompt: Optional[int] = None,
         group_boundaries: Optional[Boundaries] = None, eps: float = 1e-6,
     ):
-        adv = self.group_advantages(
-            rewards, samples_per_prompt=samples_per_prompt, group_boundaries=group_boundaries, eps=eps
-        )
+        adv = self._group_advantages(rewards, samples_per_prompt, group_boundaries, eps, policy_logits.is_cuda)
         return self.apply(
             policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps=clip_eps, beta=beta
         )
