@@ -13,8 +13,6 @@
 //                              interface as the single-CTA kernel; one lane per warp releases the
 //                              accumulator to the even CTA's MMA thread
 //
-// Besides the plain GEMM it takes the grouped-K mode (per-group weight gradients) with M a multiple of 256 per group.
-//
 // All waits are bounded (mbar_wait).  The pair synchronises on the cluster barrier after set-up and
 // before TMEM is released, so neither CTA can leave while its partner may still touch its memory.
 #pragma once
@@ -96,17 +94,16 @@ gemm_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       uint32_t phase = 0;
       for (int id = pair; id < p.num_items; id += num_pairs) {
         const WorkItem w = decode_item(p, id);
-        const ItemGeometry geo = item_geometry(p, w.m_tile, kPairBM);
-        const int m0 = geo.a_m0 + static_cast<int>(cta) * kBM;
+        const int m0 = w.m_tile * kPairBM + static_cast<int>(cta) * kBM;
         for (int nt = w.n_begin; nt < w.n_end; ++nt) {
           const int n0 = nt * BN + static_cast<int>(cta) * kHalfN;
-          for (int kb = 0; kb < geo.k_blocks; ++kb) {
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
             mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, err, kernel_id, 1);
             uint8_t* sa = smem + stage * L::kStageBytes;
             uint8_t* sb = sa + L::kABytes;
             if (cta == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * L::kStageBytes);
             const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), 0);
-            const int k0 = geo.k_row0 + kb * kBKElems;
+            const int k0 = kb * kBKElems;
             if constexpr (!A_MN) {
               tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);
             } else {
@@ -137,12 +134,11 @@ gemm_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       uint32_t buf_phase = 0;
       for (int id = pair; id < p.num_items; id += num_pairs) {
         const WorkItem w = decode_item(p, id);
-        const int item_k_blocks = item_geometry(p, w.m_tile, kPairBM).k_blocks;
         for (int nt = w.n_begin; nt < w.n_end; ++nt) {
           mbar_wait(&tmem_empty[buf], buf_phase ^ 1, abort_flag, err, kernel_id, 2);
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * BN;
-          for (int kb = 0; kb < item_k_blocks; ++kb) {
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
             mbar_wait(&full_bar[stage], phase, abort_flag, err, kernel_id, 3);
             tc_fence_after();
             const uint32_t sa = smem_u32(smem + stage * L::kStageBytes);

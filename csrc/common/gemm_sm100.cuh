@@ -125,10 +125,9 @@ __device__ __forceinline__ WorkItem decode_item(const GemmProblem& p, int id) {
   return w;
 }
 
-// `tile_m` is the engine's M-tile (128 rows, or 256 for CTA pairs).
-__device__ __forceinline__ ItemGeometry item_geometry(const GemmProblem& p, int m_tile, int tile_m = kBM) {
+__device__ __forceinline__ ItemGeometry item_geometry(const GemmProblem& p, int m_tile) {
   ItemGeometry g;
-  g.a_m0 = m_tile * tile_m;
+  g.a_m0 = m_tile * kBM;
   g.b_row_off = 0;
   g.k_row0 = 0;
   g.k_blocks = p.k_blocks;
@@ -136,7 +135,7 @@ __device__ __forceinline__ ItemGeometry item_geometry(const GemmProblem& p, int 
     g.b_row_off = p.tile_group[m_tile] * p.b_group_rows;
   } else if (p.group_mode == 2) {
     const int grp = m_tile / p.tiles_m_per_group;
-    g.a_m0 = (m_tile - grp * p.tiles_m_per_group) * tile_m;
+    g.a_m0 = (m_tile - grp * p.tiles_m_per_group) * kBM;
     g.k_row0 = p.group_offsets[grp];
     const int rows = p.group_counts != nullptr ? p.group_counts[grp] : p.group_offsets[grp + 1] - g.k_row0;
     g.k_blocks = (rows + kBK - 1) / kBK;

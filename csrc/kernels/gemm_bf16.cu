@@ -73,17 +73,12 @@ constexpr int kPairStagesTma = 5;  // one ring stage makes room for the 64 KB ou
 
 template <bool A_MN, bool B_MN, class Epi, int STAGES = kPairStages>
 void launch_pair(const GemmArgs& a, const typename Epi::Params& ep, cudaStream_t stream) {
-  const int total_m = a.group_mode == 2 ? a.M * a.num_groups : a.M;
-  GemmProblem p = make_gemm_problem(total_m, a.N, a.K, kBN, 1, 1);
-  p.tiles_m = (total_m + kPairBM - 1) / kPairBM;
+  GemmProblem p = make_gemm_problem(a.M, a.N, a.K, kBN, 1, 1);
+  p.tiles_m = (a.M + kPairBM - 1) / kPairBM;
   p.num_items = p.tiles_m * p.items_per_m;
-  p.group_mode = a.group_mode;
-  p.group_offsets = a.group_offsets;
-  p.group_counts = a.group_counts;
-  p.tiles_m_per_group = a.group_mode == 2 ? a.M / kPairBM : 1;
   // at least eight 256-row tiles per group: with fewer, B streams from DRAM too often on long-K problems (measured:
   // groups of 8 beat 4-6 by 2-4 % on K = 14336 / 28672, groups of 32 and more lose 5-10 % on every shape)
-  p.group_m = a.group_mode == 2 ? p.tiles_m_per_group : raster_group_m(p.tiles_m, 2 * a.K, 8);
+  p.group_m = raster_group_m(p.tiles_m, 2 * a.K, 8);
   if (group_m_override() > 0) p.group_m = group_m_override() < p.tiles_m ? group_m_override() : p.tiles_m;
   const CUtensorMap ta = A_MN ? make_tmap_2d_bf16(a.A, a.K, a.M, a.lda, kBK, 64)
                               : make_tmap_2d_bf16(a.A, a.M, a.K, a.lda, kBM, kBK);
@@ -132,10 +127,7 @@ void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
       return;
     }
   }
-  // Pairs take the grouped-K mode too: its k loops are short (281 rows per expert are 5 k-blocks), so operand traffic through L2
-  // bounds it, of which a pair needs a third less.
-  const bool pair = a.cta_pair && (a.group_mode == 0 || (a.group_mode == 2 && a.M % kPairBM == 0));
-  if (!pair) {
+  if (!(a.cta_pair && a.group_mode == 0)) {
     // single-CTA engine, bf16 output that TMA can address: half-tile staging (32 KB next to the 4-stage ring)
     const bool tma_out = !a.out_fp32 && !a.accumulate && a.ldd % 8 == 0 && (reinterpret_cast<uintptr_t>(a.D) & 15u) == 0 &&
                          !pair_tma_store_disabled();
@@ -148,13 +140,13 @@ void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
       return;
     }
   }
-  if (pair) {
+  if (a.cta_pair && a.group_mode == 0) {
     // bf16 output that TMA can address: stage the tile in shared memory and store full lines
     const bool tma_out = !a.out_fp32 && !a.accumulate && a.ldd % 8 == 0 && (reinterpret_cast<uintptr_t>(a.D) & 15u) == 0 &&
                          !pair_tma_store_disabled();
     if (tma_out) {
       EpiStoreTma<256>::Params ep{};
-      ep.tmap_c = make_tmap_2d_bf16(a.D, a.group_mode == 2 ? static_cast<uint64_t>(a.M) * a.num_groups : a.M, a.N, a.ldd, kBM, 64);
+      ep.tmap_c = make_tmap_2d_bf16(a.D, a.M, a.N, a.ldd, kBM, 64);
       ep.alpha = a.alpha;
       launch_pair<A_MN, B_MN, EpiStoreTma<256>, kPairStagesTma>(a, ep, stream);
       return;

@@ -338,7 +338,6 @@ Tensor grouped_gemm(const Tensor& a, const Tensor& b, int64_t mode, const Tensor
                   "grouped_gemm(2): counts must be int32, one per group");
       g.group_counts = counts->data_ptr<int>();
     }
-    g.cta_pair = gemm_pair_default();
   }
   g.D = d.data_ptr();
   g.ldd = d.stride(0);
