@@ -19,6 +19,8 @@
 // SM: the shared-memory footprint (> 114 KB) guarantees that.
 #pragma once
 
+#include <type_traits>
+
 #include "ptx.cuh"
 
 namespace rlk {
@@ -485,11 +487,34 @@ struct EpiStore {
 // are clipped by the tensor map.  Needs a 16-byte aligned C with a 16-byte row pitch; the launchers fall back to
 // EpiStore otherwise.  COLS = 256 stages a whole tile (64 KB), COLS = 128 half a tile (32 KB).
 // ---------------------------------------------------------------------------------------------
-template <int COLS>
+// AddT: D = alpha * acc + addend without a pass of its own.  A float addend (a partial sum kept in 32 bits) is added before
+// the one rounding; a bf16 addend (a residual stream, a gradient accumulated so far) is added to the product rounded to
+// bf16, the bits of a GEMM followed by an addition.  Rows of 16-byte aligned 16-byte multiples, like C.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void add_vec8(float (&x)[8], const float* p) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
+  x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
+}
+__device__ __forceinline__ void add_vec8(float (&x)[8], const __nv_bfloat16* p) {
+  const uint4 q = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = __bfloat1622float2(h[j]);
+    x[2 * j] += f.x;
+    x[2 * j + 1] += f.y;
+  }
+}
+
+template <int COLS, class AddT = void>
 struct EpiStoreTma {
+  static constexpr bool kAdd = !std::is_void<AddT>::value;
   struct Params {
     CUtensorMap tmap_c;  // bf16 [M, N], box 64 x 128, 128B swizzle
     float alpha;
+    const AddT* addend;    // [M, N], N % 8 == 0 (AddT != void)
+    long long ld_addend;
   };
   struct State {
     uint8_t* staging;
@@ -524,11 +549,23 @@ struct EpiStoreTma {
         uint8_t* box = st.staging + (c >> 6) * (kBM * 128) + r * 128;  // 64-column box, 128 bytes per row
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
+          float x[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(t[v * 8 + j]) * ep.alpha;
+          if constexpr (kAdd) {
+            const int col = n0 + seg + c + v * 8;
+            if (row < p.M && col < p.N) {
+              if constexpr (sizeof(AddT) == 2) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = __bfloat162float(__float2bfloat16_rn(x[j]));
+              }
+              add_vec8(x, ep.addend + static_cast<long long>(row) * ep.ld_addend + col);
+            }
+          }
           uint32_t w[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(t[v * 8 + 2 * j]) * ep.alpha,
-                                                     __uint_as_float(t[v * 8 + 2 * j + 1]) * ep.alpha);
+            __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
             w[j] = *reinterpret_cast<uint32_t*>(&b);
           }
           const int chunk = ((c & 63) >> 3) + v;  // 16-byte chunk inside the 128-byte row

@@ -119,8 +119,31 @@ void launch_skinny(const GemmArgs& a, cudaStream_t stream) {
       ta, tb, p, typename Epi::Params{static_cast<__nv_bfloat16*>(a.D), a.ldd, a.alpha}, a.err, 101u);
 }
 
+// D (bf16) = alpha * A B^T + addend: the TMA-store epilogues with the addend read beside the accumulator.
+template <bool A_MN, bool B_MN, class AddT>
+void launch_add(const GemmArgs& a, cudaStream_t stream) {
+  if (a.cta_pair) {
+    using E = EpiStoreTma<256, AddT>;
+    typename E::Params ep{make_tmap_2d_bf16(a.D, a.M, a.N, a.ldd, kBM, 64), a.alpha, static_cast<const AddT*>(a.addend), a.ld_addend};
+    launch_pair<A_MN, B_MN, E, kPairStagesTma>(a, ep, stream);
+  } else {
+    using E = EpiStoreTma<128, AddT>;
+    typename E::Params ep{make_tmap_2d_bf16(a.D, a.M, a.N, a.ldd, kBM, 64), a.alpha, static_cast<const AddT*>(a.addend), a.ld_addend};
+    launch<A_MN, B_MN, E>(a, ep, stream);
+  }
+}
+
 template <bool A_MN, bool B_MN>
 void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
+  if (a.addend != nullptr) {  // the caller has checked: plain GEMM, bf16 D, N % 8 == 0, 16-byte aligned rows of D and addend
+    if constexpr (A_MN && B_MN) {
+      if (a.addend_bf16) launch_add<A_MN, B_MN, __nv_bfloat16>(a, stream);
+      else launch_add<A_MN, B_MN, float>(a, stream);
+    } else if constexpr (!A_MN && !B_MN) {
+      if (a.addend_bf16) launch_add<A_MN, B_MN, __nv_bfloat16>(a, stream);
+    }
+    return;
+  }
   if constexpr (!A_MN && !B_MN) {
     if (a.group_mode == 0 && a.M <= kBM && !a.out_fp32 && !a.accumulate && a.N >= 4 * kSkinnyBN) {
       launch_skinny(a, stream);
@@ -132,7 +155,7 @@ void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
     const bool tma_out = !a.out_fp32 && !a.accumulate && a.ldd % 8 == 0 && (reinterpret_cast<uintptr_t>(a.D) & 15u) == 0 &&
                          !pair_tma_store_disabled();
     if (tma_out) {
-      EpiStoreTma<128>::Params ep;
+      EpiStoreTma<128>::Params ep{};
       // grouped-K stacks one [M, N] block per group along the rows of D
       ep.tmap_c = make_tmap_2d_bf16(a.D, a.group_mode == 2 ? static_cast<uint64_t>(a.M) * a.num_groups : a.M, a.N, a.ldd, kBM, 64);
       ep.alpha = a.alpha;

@@ -58,6 +58,13 @@ struct GemmArgs {
   int num_groups = 1;
   // Plain GEMM only: compute 256 x 256 tiles on pairs of SMs (tcgen05 cta_group::2, cluster of two CTAs).
   bool cta_pair = false;
+  // D (bf16) = alpha * op(A) op(B)^T + addend: a 32-bit partial sum of a weight gradient (added before the rounding), the
+  // gradient accumulated so far in bf16 (both operands MN-major; may be D itself) or a bf16 residual (both K-major; bf16
+  // addends are added to the rounded product).  N % 8 == 0, 16-byte aligned rows of D and addend; plain GEMM,
+  // no accumulate.
+  const void* addend = nullptr;
+  bool addend_bf16 = false;
+  long long ld_addend = 0;
 };
 void gemm_bf16(const GemmArgs& args, cudaStream_t stream);
 
@@ -113,6 +120,10 @@ struct LinearLogpDzArgs {
   uint32_t* err;
 };
 void linear_logp_dz(const LinearLogpDzArgs& args, cudaStream_t stream);
+// Column sums of dz (the bias gradient): out[V] (+)= sum over rows; workspace of dz_colsum_workspace_floats floats.
+long long dz_colsum_workspace_floats(int rows, int V);
+void dz_colsum(const __nv_bfloat16* dz, long long ld, int rows, int V, float* workspace, float* out, bool accumulate,
+               cudaStream_t stream);
 
 }  // namespace rlk
 

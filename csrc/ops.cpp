@@ -80,7 +80,7 @@ bool gemm_pair_default() {
 }
 
 Tensor gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, std::optional<Tensor> out, bool out_fp32,
-            bool accumulate, double alpha, int64_t pair) {
+            bool accumulate, double alpha, int64_t pair, std::optional<Tensor> addend) {
   check_rowmajor(a, "a");
   check_rowmajor(b, "b");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "rl_engine.gemm: bf16 operands only");
@@ -103,12 +103,30 @@ Tensor gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, std::optiona
     TORCH_CHECK(!accumulate, "rl_engine.gemm: accumulate needs an explicit out tensor");
     d = torch::empty({M, N}, a.options().dtype(out_fp32 ? torch::kFloat32 : torch::kBFloat16));
   }
+  if (addend.has_value()) {
+    check_rowmajor(*addend, "addend");
+    const bool bf16 = addend->scalar_type() == torch::kBFloat16;
+    TORCH_CHECK(a_mn == b_mn && (a_mn || bf16) && !out_fp32 && !accumulate,
+                "rl_engine.gemm: an addend needs MN-major operands (or K-major ones, if it is bf16) and a bf16 output");
+    TORCH_CHECK((bf16 || addend->scalar_type() == torch::kFloat32) && addend->size(0) == M && addend->size(1) == N,
+                "rl_engine.gemm: addend must have the output's shape");
+    TORCH_CHECK(N % 8 == 0 && d.stride(0) % 8 == 0 && addend->stride(0) % (bf16 ? 8 : 4) == 0 &&
+                    reinterpret_cast<uintptr_t>(d.data_ptr()) % 16 == 0 &&
+                    reinterpret_cast<uintptr_t>(addend->data_ptr()) % 16 == 0,
+                "rl_engine.gemm: addend needs N % 8 == 0 and 16-byte aligned rows");
+  }
   if (M == 0 || N == 0) return d;
   if (K == 0) {
-    if (!accumulate) d.zero_();
+    if (addend.has_value()) d.copy_(*addend);
+    else if (!accumulate) d.zero_();
     return d;
   }
   rlk::GemmArgs g;
+  if (addend.has_value()) {
+    g.addend = addend->data_ptr();
+    g.addend_bf16 = addend->scalar_type() == torch::kBFloat16;
+    g.ld_addend = addend->stride(0);
+  }
   g.A = reinterpret_cast<const __nv_bfloat16*>(a.data_ptr());
   g.B = reinterpret_cast<const __nv_bfloat16*>(b.data_ptr());
   g.D = d.data_ptr();
@@ -679,6 +697,27 @@ void linear_logp_dz(const Tensor& hidden, const Tensor& weight, const Tensor& ta
   a.err = err_ptr(hidden);
   rlk::linear_logp_dz(a, stream_of(hidden));
   after_launch();
+}
+
+// out[V] (+)= column sums of dz [rows, V] in fp32, fixed order.
+void dz_colsum(const Tensor& dz, Tensor out, bool accumulate) {
+  check_rowmajor(dz, "dz");
+  check_cuda(out, "out");
+  TORCH_CHECK(dz.scalar_type() == torch::kBFloat16 && dz.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(dz.data_ptr()) % 16 == 0 &&
+                  dz.stride(0) >= (dz.size(1) + 7) / 8 * 8,
+              "rl_engine.dz_colsum: dz must be bf16 with 16-byte aligned rows");
+  TORCH_CHECK(out.scalar_type() == torch::kFloat32 && out.is_contiguous() && out.numel() == dz.size(1),
+              "rl_engine.dz_colsum: out must be contiguous float32 [V]");
+  const c10::cuda::CUDAGuard guard(dz.device());
+  const int rows = static_cast<int>(dz.size(0)), v = static_cast<int>(dz.size(1));
+  if (rows == 0 || v == 0) {
+    if (!accumulate) out.zero_();
+    return;
+  }
+  Tensor ws = torch::empty({rlk::dz_colsum_workspace_floats(rows, v)}, out.options());
+  rlk::dz_colsum(reinterpret_cast<const __nv_bfloat16*>(dz.data_ptr()), dz.stride(0), rows, v, ws.data_ptr<float>(),
+                 out.data_ptr<float>(), accumulate, stream_of(dz));
+  after_launch(2);
 }
 
 // --------------------------------------------------------------------------- logp over logits
@@ -1453,7 +1492,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("trace_enabled", [] { return rlk::trace_enabled(); });
   m.def("gemm", rlk::traced("rlk::gemm", &gemm), py::arg("a"), py::arg("b"), py::arg("a_mn") = false, py::arg("b_mn") = false,
         py::arg("out") = py::none(), py::arg("out_fp32") = false, py::arg("accumulate") = false, py::arg("alpha") = 1.0,
-        py::arg("pair") = -1);
+        py::arg("pair") = -1, py::arg("addend") = py::none());
   m.def("grouped_gemm", rlk::traced("rlk::grouped_gemm", &grouped_gemm), py::arg("a"), py::arg("b"), py::arg("mode"),
         py::arg("table"), py::arg("num_groups"), py::arg("b_mn"), py::arg("out_fp32"), py::arg("out") = py::none(),
         py::arg("counts") = py::none());
@@ -1477,6 +1516,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("slot_base"), py::arg("total_records"), py::arg("peer_partials"), py::arg("peer_counters"),
         py::arg("next_counters"), py::arg("counter_capacity"), py::arg("want_lse"), py::arg("want_entropy"),
         py::arg("wait_limit_ms"), py::arg("global_vocab") = 0);
+  m.def("dz_colsum", rlk::traced("rlk::dz_colsum", &dz_colsum));
   m.def("linear_logp_dz", rlk::traced("rlk::linear_logp_dz", &linear_logp_dz));
   m.def("logp_rows", rlk::traced("rlk::logp_rows", &logp_rows));
   m.def("ratio_kl_fwd", rlk::traced("rlk::ratio_kl_fwd", &ratio_kl_fwd));

@@ -8,9 +8,9 @@ vocab_start_index=0, global_vocab_size=None)`` returning float32 log-probs shape
 * forward is ONE kernel including the split/rank merge (the reference launches a GEMM kernel, a
   combine kernel and, under tensor parallelism, three NCCL all-reduces);
 * backward never calls a library GEMM: per token chunk a recompute kernel writes
-  ``dz = g * (onehot - softmax)`` as bf16 into a pre-allocated chunk workspace, then two tcgen05
-  GEMMs form ``grad_hidden`` and accumulate ``grad_weight`` in fp32 in fixed chunk order.  Extra
-  memory is constant in the number of tokens: ``chunk * V`` bf16 plus the fp32 ``grad_weight``;
+  ``dz = g * (onehot - softmax)`` as bf16 into a chunk workspace, then two tcgen05 GEMMs form
+  ``grad_hidden`` and accumulate ``grad_weight`` in fp32 in fixed chunk order (one chunk stores it
+  as bf16 directly).  Extra memory is bounded by ``chunk * V`` bf16 plus one fp32 ``grad_weight``;
 * ``with_entropy`` also returns the softmax entropy per token from the same sweep.
 
 Inputs must be bf16 on a CUDA device for the fused path; anything else goes to the PyTorch oracle.
@@ -100,20 +100,52 @@ def _dz_workspace(device: torch.device, chunk: int, v_local: int) -> torch.Tenso
     return buf
 
 
+def backward_chunk(n: int, d: int, chunk_tokens: int, need_weight: bool) -> int:
+    """Rows of dz formed at once.  One chunk needs no fp32 ``grad_weight`` (4 V D bytes) beside its dz, so with the
+    memory of ``chunk_tokens`` rows and that buffer, ``chunk_tokens + 2 D`` rows fit in one piece; longer batches go
+    ``chunk_tokens`` at a time."""
+    chunk = max(128, chunk_tokens)
+    if need_weight and n <= chunk + 2 * d:
+        chunk = max(chunk, n)
+    return min(chunk, (n + 127) // 128 * 128)
+
+
+def accumulate_grad_weight(ext, dz, h2, grad_w, first: bool, last: bool, dtype, sink=None):
+    """``grad_w`` of a chunk onto the sum of the earlier ones: the first chunk writes, later ones add in fp32, the last one
+    rounds to ``dtype`` as it stores.  No zero-fill and no conversion pass over ``[V, D]``.  ``sink``: a gradient buffer that the
+    only chunk adds to."""
+    if sink is not None and first and last:
+        return ext.gemm(dz, h2, True, True, sink, False, False, 1.0, -1, sink)
+    if dtype == torch.bfloat16 and last:
+        out = torch.empty(dz.shape[1], h2.shape[1], dtype=dtype, device=dz.device)
+        return ext.gemm(dz, h2, True, True, out, False, False, 1.0, -1, None if first else grad_w)
+    if first:
+        grad_w = torch.empty(dz.shape[1], h2.shape[1], dtype=torch.float32, device=dz.device)
+    return ext.gemm(dz, h2, True, True, grad_w, True, not first, 1.0)
+
+
 def linear_logp_backward_local(
     grad_logp: torch.Tensor, hidden2d: torch.Tensor, weight: torch.Tensor, target: torch.Tensor,
     bias: Optional[torch.Tensor], lse: torch.Tensor, *, vocab_start: int = 0, need_hidden: bool = True,
     need_weight: bool = True, chunk_tokens: int = DEFAULT_BWD_CHUNK_TOKENS, grad_hidden_dtype=torch.bfloat16,
+    grad_weight_dtype=torch.float32, grad_weight_sink=None,
 ):
-    """Chunked recompute backward on one rank's vocab shard.  Returns (grad_h, grad_w fp32, grad_b fp32)."""
+    """Chunked recompute backward on one rank's vocab shard.  Returns (grad_h, grad_w, grad_b fp32); ``grad_w`` is summed in
+    fp32 and comes as ``grad_weight_dtype`` (float32 or bfloat16); with a ``grad_weight_sink`` it is added there and
+    ``None`` is returned."""
     ext = require_ext()
     n, d = hidden2d.shape
     v = weight.shape[0]
     g = grad_logp.reshape(-1).float().contiguous()
-    chunk = max(128, min(chunk_tokens, (n + 127) // 128 * 128))
-    dz_buf = _dz_workspace(hidden2d.device, chunk, v)
+    chunk = backward_chunk(n, d, chunk_tokens, need_weight)
+    if chunk <= max(128, chunk_tokens):
+        dz_buf = _dz_workspace(hidden2d.device, chunk, v)
+    else:  # larger than what is kept between calls
+        dz_buf = torch.empty(chunk, (v + 7) // 8 * 8, dtype=torch.bfloat16, device=hidden2d.device)
     grad_h = torch.empty(n, d, dtype=grad_hidden_dtype, device=hidden2d.device) if need_hidden else None
-    grad_w = torch.zeros(v, d, dtype=torch.float32, device=weight.device) if need_weight else None
+    grad_w = None
+    if need_weight and n == 0:
+        grad_w = torch.zeros(v, d, dtype=grad_weight_dtype, device=weight.device)
     grad_b = torch.zeros(v, dtype=torch.float32, device=weight.device) if bias is not None else None
     for i0 in range(0, n, chunk):
         i1 = min(i0 + chunk, n)
@@ -123,15 +155,20 @@ def linear_logp_backward_local(
         if need_hidden:
             ext.gemm(dz, weight, False, True, grad_h[i0:i1], grad_hidden_dtype == torch.float32, False, 1.0)
         if need_weight:
-            ext.gemm(dz, hidden2d[i0:i1], True, True, grad_w, True, True, 1.0)
+            grad_w = accumulate_grad_weight(ext, dz, hidden2d[i0:i1], grad_w, i0 == 0, i1 == n, grad_weight_dtype,
+                                            grad_weight_sink)
         if grad_b is not None:
-            grad_b += dz.float().sum(0)
+            ext.dz_colsum(dz, grad_b, i0 > 0)
+    if grad_weight_sink is not None and grad_w is not None:
+        if grad_w is not grad_weight_sink and grad_w.data_ptr() != grad_weight_sink.data_ptr():
+            grad_weight_sink.add_(grad_w)  # several chunks
+        grad_w = None
     return grad_h, grad_w, grad_b
 
 
 class _LinearLogp(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, hidden, weight, bias, target, want_entropy, chunk_tokens, check_vocab=0):
+    def forward(ctx, hidden, weight, bias, target, want_entropy, chunk_tokens, check_vocab=0, sink=None):
         h2 = hidden.reshape(-1, hidden.shape[-1])
         if h2.stride(1) != 1 or h2.stride(0) % 8 or h2.data_ptr() % 16:
             h2 = h2.contiguous()
@@ -141,7 +178,7 @@ class _LinearLogp(torch.autograd.Function):
         ctx.save_for_backward(h2, w, t, lse, *(() if bias is None else (bias,)))
         ctx.has_bias = bias is not None
         ctx.hidden_shape = hidden.shape
-        ctx.chunk_tokens = chunk_tokens
+        ctx.chunk_tokens, ctx.sink = chunk_tokens, sink
         lead = hidden.shape[:-1]
         if want_entropy:
             ctx.mark_non_differentiable(ent)
@@ -154,13 +191,13 @@ class _LinearLogp(torch.autograd.Function):
         bias = rest[0] if ctx.has_bias else None
         gh, gw, gb = linear_logp_backward_local(
             grad_logp, h2, w, t, bias, lse, need_hidden=ctx.needs_input_grad[0], need_weight=ctx.needs_input_grad[1],
-            chunk_tokens=ctx.chunk_tokens,
+            chunk_tokens=ctx.chunk_tokens, grad_weight_dtype=w.dtype, grad_weight_sink=ctx.sink,
         )
         return (
             None if gh is None else gh.reshape(ctx.hidden_shape),
-            None if gw is None else gw.to(w.dtype),
+            gw,
             None if gb is None else gb.to(bias.dtype),
-            None, None, None, None,
+            None, None, None, None, None,
         )
 
 
@@ -212,8 +249,10 @@ class FusedLinearLogpSM100Op:
 
     def apply(
         self, hidden, lm_head_weight, target_ids, bias=None, *, tp_group: Any = None, vocab_start_index: int = 0,
-        global_vocab_size: Optional[int] = None,
+        global_vocab_size: Optional[int] = None, grad_weight_sink: Optional[torch.Tensor] = None,
     ) -> torch.Tensor:
+        """``grad_weight_sink``: the gradient buffer of ``lm_head_weight``; the fused backward adds to it instead of returning
+        a gradient."""
         check_linear_logp_args(hidden, lm_head_weight, target_ids, bias)
         if should_use_tensor_parallel_linear_logp(
             tp_group, int(vocab_start_index), global_vocab_size, lm_head_weight.shape[0]
@@ -234,7 +273,7 @@ class FusedLinearLogpSM100Op:
             return self._native.apply(hidden, lm_head_weight, target_ids, bias)
         self._validate_targets(target_ids, lm_head_weight.shape[0])
         logp, _ = _LinearLogp.apply(hidden, lm_head_weight, bias, target_ids, False, self.bwd_chunk_tokens,
-                                    self._device_check(lm_head_weight.shape[0]))
+                                    self._device_check(lm_head_weight.shape[0]), grad_weight_sink)
         return logp
 
     def _device_check(self, vocab: int) -> int:

@@ -122,7 +122,7 @@ class _TPLinearLogp(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_logp, _grad_ent):
-        from rl_engine.kernels.ops.sm100.linear_logp import _dz_workspace
+        from rl_engine.kernels.ops.sm100.linear_logp import _dz_workspace, accumulate_grad_weight
 
         ext = require_ext()
         has_bias, hidden_shape, v_start, tp_group, chunk = ctx.meta
@@ -134,7 +134,7 @@ class _TPLinearLogp(torch.autograd.Function):
         g = grad_logp.reshape(-1).float().contiguous()
         dz_buf = _dz_workspace(h2.device, chunk, v)
         grad_h = torch.empty(n, d, dtype=h2.dtype, device=h2.device)
-        grad_w = torch.zeros(v, d, dtype=torch.float32, device=w.device) if ctx.needs_input_grad[1] else None
+        grad_w = torch.zeros_like(w) if ctx.needs_input_grad[1] and n == 0 else None
         grad_b = torch.zeros(v, dtype=torch.float32, device=w.device) if has_bias else None
         for i0 in range(0, n, chunk):
             i1 = min(i0 + chunk, n)
@@ -146,12 +146,12 @@ class _TPLinearLogp(torch.autograd.Function):
             ext.gemm(dz, w, False, True, part.local[:rows], False, False, 1.0)
             ws.mem.barrier()
             ext.peer_sum(part.ptrs, rows * d, False, grad_h[i0:i1])
-            if grad_w is not None:
-                ext.gemm(dz, h2[i0:i1], True, True, grad_w, True, True, 1.0)
+            if ctx.needs_input_grad[1]:
+                grad_w = accumulate_grad_weight(ext, dz, h2[i0:i1], grad_w, i0 == 0, i1 == n, w.dtype)
             if grad_b is not None:
-                grad_b += dz.float().sum(0)
+                ext.dz_colsum(dz, grad_b, i0 > 0)
         return (
-            grad_h.reshape(hidden_shape), None if grad_w is None else grad_w.to(w.dtype),
+            grad_h.reshape(hidden_shape), grad_w,
             None if grad_b is None else grad_b.to(bias.dtype), None, None, None, None, None, None, None,
         )
 
