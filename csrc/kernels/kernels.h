@@ -250,7 +250,7 @@ int rmsnorm_bwd_rows_per_cta(long long rows);
 int rmsnorm_bwd_chunks(long long rows, int rows_per_cta = 0);
 void rmsnorm_backward(const void* x, long long ldx, int x_dtype, const void* w, int w_dtype, const void* dy,
                       long long lddy, const float* rstd, void* dx, long long lddx, long long rows, int D,
-                      float* dw_part, void* dw, cudaStream_t stream, int rows_per_cta = 0);
+                      float* dw_part, void* dw, cudaStream_t stream, int rows_per_cta = 0, bool accumulate_dw = false);
 // Per-head RMSNorm (head_dim 128) of the q and k heads inside a packed qkv buffer [tokens, (hq + 2 hkv) * 128]; v is copied.
 // Backward writes per-block partial weight gradients ``part [qk_norm_blocks(...)][2][128]`` (q, then k).
 int qk_norm_blocks(long long tokens, int heads);
@@ -280,9 +280,10 @@ void rope_apply(const void* x, long long ldt, int dtype, const long long* pos, c
                 cudaStream_t stream);
 void embedding_forward(const long long* ids, const void* table, long long ldw, int dtype, void* out, long long rows,
                        int D, long long vocab, cudaStream_t stream);
-void embedding_backward(const long long* seg_ids, const long long* seg_start, long long segments,
-                        const long long* order, const void* dy, int dy_dtype, int D, void* dtable, bool table_fp32,
-                        long long ldw, long long dy_rows, long long table_rows, cudaStream_t stream);
+// ids: sorted (stable), order: the row of dy each sorted id belongs to; writes the table rows that occur.
+long long embedding_backward_partial_floats(long long n, int D);
+void embedding_backward(const long long* ids, const long long* order, long long n, const void* dy, int dy_dtype, int D, void* dtable,
+                        bool table_fp32, long long ldw, float* partials, long long table_rows, bool accumulate, cudaStream_t stream);
 // master: fp32 master weights or nullptr.  residual: 16-bit residuals of a bf16 parameter (fp32 master = parameter
 // bits << 16 plus the sign-extended residual) or nullptr; at most one of the two.
 void adamw_step(void* p, int p_dtype, float* master, short* residual, const void* g, int g_dtype, float* m, float* v,

@@ -1083,19 +1083,23 @@ std::vector<Tensor> qk_norm_bwd(const Tensor& qkv, const Tensor& dout, const Ten
   return {dqkv, dw[0].to(torch::kBFloat16), dw[1].to(torch::kBFloat16)};
 }
 
-std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd) {
+std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd, std::optional<Tensor> dw_sum) {
   check_rowmajor(x, "x");
   check_rowmajor(dy, "dy");
   TORCH_CHECK(dy.scalar_type() == x.scalar_type(), "dy dtype must match x");
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t rows = x.size(0), D = x.size(1);
   Tensor dx = torch::empty({rows, D}, x.options());
-  Tensor dw = torch::zeros({D}, w.options());
+  // dw_sum: the weight gradient is added to this tensor, which is then returned in its place
+  if (dw_sum.has_value())
+    TORCH_CHECK(dw_sum->is_cuda() && dw_sum->is_contiguous() && dw_sum->numel() == D && dw_sum->scalar_type() == w.scalar_type(),
+                "rmsnorm_bwd: dw_sum must match the weight");
+  Tensor dw = dw_sum.has_value() ? *dw_sum : (rows ? torch::empty({D}, w.options()) : torch::zeros({D}, w.options()));
   if (rows) {
     Tensor part = torch::empty({rlk::rmsnorm_bwd_chunks(rows), D}, x.options().dtype(torch::kFloat32));
     rlk::rmsnorm_backward(x.data_ptr(), x.stride(0), dtype_code(x), w.data_ptr(), dtype_code(w), dy.data_ptr(),
                           dy.stride(0), rstd.data_ptr<float>(), dx.data_ptr(), dx.stride(0), rows, static_cast<int>(D),
-                          part.data_ptr<float>(), dw.data_ptr(), stream_of(x));
+                          part.data_ptr<float>(), dw.data_ptr(), stream_of(x), 0, dw_sum.has_value());
     after_launch(2);
   }
   return {dx, dw};
@@ -1240,22 +1244,27 @@ Tensor embedding_fwd(const Tensor& ids, const Tensor& table) {
   return out;
 }
 
-// seg_ids [S], seg_start [S+1], order [tokens]: tokens stably sorted by id and run-length encoded.
-void embedding_bwd(const Tensor& seg_ids, const Tensor& seg_start, const Tensor& order, const Tensor& dy, Tensor dtable) {
+// sorted_ids [tokens] (stable sort), order [tokens]: the row of dy each of them belongs to.  Rows of dtable whose id does not
+// occur are left as they are; accumulate adds to the others instead of writing them.
+void embedding_bwd(const Tensor& sorted_ids, const Tensor& order, const Tensor& dy, Tensor dtable, bool accumulate) {
   check_rowmajor(dy, "dy");
   check_rowmajor(dtable, "dtable");
   TORCH_CHECK(dy.is_contiguous(), "dy must be contiguous");
+  const int64_t n = sorted_ids.numel();
+  auto index_ok = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == torch::kInt64 && t.is_contiguous() && t.numel() == n; };
+  TORCH_CHECK(index_ok(sorted_ids) && index_ok(order) && dy.size(0) == n && dy.size(1) == dtable.size(1),
+              "embedding_bwd: contiguous int64 ids and order, one per row of dy");
   const c10::cuda::CUDAGuard guard(dy.device());
-  const int64_t segs = seg_ids.numel();
-  if (segs == 0) return;
+  if (n == 0) return;
   const bool tfp32 = dtable.scalar_type() == torch::kFloat32;
   TORCH_CHECK(tfp32 || dtable.scalar_type() == dy.scalar_type(), "dtable must be float32 or match dy");
-  rlk::embedding_backward(reinterpret_cast<const long long*>(seg_ids.data_ptr<int64_t>()),
-                          reinterpret_cast<const long long*>(seg_start.data_ptr<int64_t>()), segs,
-                          reinterpret_cast<const long long*>(order.data_ptr<int64_t>()), dy.data_ptr(), dtype_code(dy),
-                          static_cast<int>(dy.size(1)), dtable.data_ptr(), tfp32, dtable.stride(0), dy.size(0),
-                          dtable.size(0), stream_of(dy));
-  after_launch();
+  const int D = static_cast<int>(dy.size(1));
+  Tensor partials = torch::empty({rlk::embedding_backward_partial_floats(n, D)}, dy.options().dtype(torch::kFloat32));
+  rlk::embedding_backward(reinterpret_cast<const long long*>(sorted_ids.data_ptr<int64_t>()),
+                          reinterpret_cast<const long long*>(order.data_ptr<int64_t>()), n, dy.data_ptr(), dtype_code(dy), D,
+                          dtable.data_ptr(), tfp32, dtable.stride(0), partials.data_ptr<float>(), dtable.size(0), accumulate,
+                          stream_of(dy));
+  after_launch(2);
 }
 
 void adamw(Tensor p, std::optional<Tensor> master, const Tensor& g, Tensor m, Tensor v, double lr, double b1, double b2,
@@ -1536,7 +1545,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm_fwd", rlk::traced("rlk::rmsnorm_fwd", &rmsnorm_fwd));
   m.def("qk_norm_fwd", rlk::traced("rlk::qk_norm_fwd", &qk_norm_fwd));
   m.def("qk_norm_bwd", rlk::traced("rlk::qk_norm_bwd", &qk_norm_bwd));
-  m.def("rmsnorm_bwd", rlk::traced("rlk::rmsnorm_bwd", &rmsnorm_bwd));
+  m.def("rmsnorm_bwd", rlk::traced("rlk::rmsnorm_bwd", &rmsnorm_bwd), py::arg("x"), py::arg("w"), py::arg("dy"), py::arg("rstd"),
+        py::arg("dw_sum") = py::none());
   m.def("swiglu_fwd", rlk::traced("rlk::swiglu_fwd", &swiglu_fwd));
   m.def("swiglu_bwd", rlk::traced("rlk::swiglu_bwd", &swiglu_bwd));
   m.def("swiglu_packed_fwd", rlk::traced("rlk::swiglu_packed_fwd", &swiglu_packed_fwd));
@@ -1544,7 +1554,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rope", rlk::traced("rlk::rope", &rope), py::arg("x"), py::arg("positions"), py::arg("cos"), py::arg("sin"), py::arg("inverse") = false,
         py::arg("out") = py::none());
   m.def("embedding_fwd", rlk::traced("rlk::embedding_fwd", &embedding_fwd));
-  m.def("embedding_bwd", rlk::traced("rlk::embedding_bwd", &embedding_bwd));
+  m.def("embedding_bwd", rlk::traced("rlk::embedding_bwd", &embedding_bwd), py::arg("sorted_ids"), py::arg("order"), py::arg("dy"),
+        py::arg("dtable"), py::arg("accumulate") = false);
   m.def("adamw", rlk::traced("rlk::adamw", &adamw));
   m.def("sample", rlk::traced("rlk::sample", &sample));
   m.def("attention_fwd", rlk::traced("rlk::attention_fwd", &attention_fwd));

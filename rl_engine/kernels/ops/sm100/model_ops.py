@@ -215,11 +215,12 @@ class FusedRoPESM100Op:
 # ---------------------------------------------------------------------------------- embedding
 class _Embedding(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, ids, weight):
+    def forward(ctx, ids, weight, sink):
         flat = ids.reshape(-1).to(torch.long).contiguous()
         ctx.save_for_backward(flat)
         ctx.w_shape = weight.shape
         ctx.w_dtype = weight.dtype
+        ctx.sink = sink
         out = require_ext().embedding_fwd(flat, weight if weight.stride(1) == 1 else weight.contiguous())
         return out.reshape(*ids.shape, weight.shape[1])
 
@@ -228,18 +229,34 @@ class _Embedding(torch.autograd.Function):
         (flat,) = ctx.saved_tensors
         d = ctx.w_shape[1]
         dy2 = dy.reshape(-1, d).contiguous()
-        # stable sort + run-length encoding fix the summation order: no atomics, bitwise reproducible
+        # a stable sort fixes the summation order: no atomics, bitwise reproducible
         sorted_ids, order = torch.sort(flat, stable=True)
-        seg_ids, counts = torch.unique_consecutive(sorted_ids, return_counts=True)
-        seg_start = torch.zeros(seg_ids.numel() + 1, dtype=torch.long, device=flat.device)
-        seg_start[1:] = counts.cumsum(0)
-        keep = (seg_ids >= 0) & (seg_ids < ctx.w_shape[0])
+        if flat.numel():
+            _refuse_ids_outside(sorted_ids, ctx.w_shape[0])
+        if ctx.sink is not None:  # the table's gradient buffer: only the rows that occur are touched
+            require_ext().embedding_bwd(sorted_ids, order, dy2, ctx.sink, True)
+            return None, None, None
         dtable = torch.zeros(ctx.w_shape, dtype=ctx.w_dtype, device=dy.device)
-        if bool(keep.all()):
-            require_ext().embedding_bwd(seg_ids, seg_start, order, dy2, dtable)
-        else:
+        require_ext().embedding_bwd(sorted_ids, order, dy2, dtable)
+        return None, dtable, None
+
+
+def _refuse_ids_outside(sorted_ids: torch.Tensor, rows: int) -> None:
+    """Raises ``ValueError`` from the backward pass that is running if an id lies outside ``[0, rows)``.  The smallest and the
+    largest id are copied out now and looked at when that pass has queued all its kernels (which skip such ids): the
+    host does not stop in the middle of it."""
+    n = sorted_ids.numel()
+    ends = torch.empty(2, dtype=torch.long, pin_memory=True)
+    ends.copy_(sorted_ids[:: n - 1] if n > 1 else sorted_ids.expand(2), non_blocking=True)
+    copied = torch.cuda.Event()
+    copied.record(torch.cuda.current_stream(sorted_ids.device))
+
+    def check() -> None:
+        copied.synchronize()
+        if int(ends[0]) < 0 or int(ends[1]) >= rows:
             raise ValueError("embedding backward saw out-of-range token ids")
-        return None, dtable
+
+    torch.autograd.Variable._execution_engine.queue_callback(check)
 
 
 class FusedEmbeddingSM100Op(torch.nn.Module):
@@ -247,10 +264,11 @@ class FusedEmbeddingSM100Op(torch.nn.Module):
         super().__init__()
         self._native = NativeEmbeddingOp()
 
-    def forward(self, token_ids, weight):
+    def forward(self, token_ids, weight, *, grad_sink=None):
+        """``grad_sink``: the gradient buffer of ``weight``; the backward pass adds to it instead of returning a gradient."""
         if not (_ok(weight) and token_ids.is_cuda):
             return self._native.forward(token_ids, weight)
-        return _Embedding.apply(token_ids, weight)
+        return _Embedding.apply(token_ids, weight, grad_sink)
 
     def forward_fp32(self, token_ids, weight):
         return self.forward(token_ids, weight).float()
