@@ -714,23 +714,32 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 struct ReduceJob {
   int k_row, k_len, slot_begin, slot_end;
 };
-__global__ void attn_bwd_reduce_kernel(const ReduceJob* __restrict__ jobs, const float* __restrict__ partials,
-                                       int num_heads_kv, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                                       long long ld_dkv) {
+// One thread per four columns of dK and dV, eight key rows per CTA: a job alone (128 keys of one head) keeps 16 CTAs busy,
+// so the few split tiles of a short prompt are not summed by a handful of SMs.
+constexpr int kReduceRows = 8;
+__global__ void __launch_bounds__(kReduceRows * 32)
+attn_bwd_reduce_kernel(const ReduceJob* __restrict__ jobs, const float* __restrict__ partials, int num_heads_kv,
+                       __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long ld_dkv) {
   const ReduceJob job = jobs[blockIdx.x];
   const int kv_head = blockIdx.y;
-  for (int e = threadIdx.x; e < job.k_len * kD; e += blockDim.x) {
-    const int r = e / kD, c = e - r * kD;
-    float acc_v = 0.f, acc_k = 0.f;
-    for (int s = job.slot_begin; s < job.slot_end; ++s) {
-      const float* base = partials + (static_cast<long long>(s) * num_heads_kv + kv_head) * 2 * (128 * kD);
-      acc_v += base[r * kD + c];
-      acc_k += base[128 * kD + r * kD + c];
-    }
-    const long long o = (static_cast<long long>(job.k_row) + r) * ld_dkv + kv_head * kD + c;
-    dv[o] = __float2bfloat16_rn(acc_v);
-    dk[o] = __float2bfloat16_rn(acc_k);
+  const int r = blockIdx.z * kReduceRows + (threadIdx.x >> 5), c = (threadIdx.x & 31) * 4;
+  if (r >= job.k_len) return;
+  float4 acc_v = make_float4(0.f, 0.f, 0.f, 0.f), acc_k = acc_v;
+  const long long pitch = static_cast<long long>(num_heads_kv) * 2 * (128 * kD);
+  const float* base = partials + job.slot_begin * pitch + static_cast<long long>(kv_head) * 2 * (128 * kD) + r * kD + c;
+#pragma unroll 4
+  for (int s = job.slot_begin; s < job.slot_end; ++s, base += pitch) {
+    const float4 x = *reinterpret_cast<const float4*>(base), y = *reinterpret_cast<const float4*>(base + 128 * kD);
+    acc_v.x += x.x; acc_v.y += x.y; acc_v.z += x.z; acc_v.w += x.w;
+    acc_k.x += y.x; acc_k.y += y.y; acc_k.z += y.z; acc_k.w += y.w;
   }
+  const long long o = (static_cast<long long>(job.k_row) + r) * ld_dkv + kv_head * kD + c;
+  auto put = [](__nv_bfloat16* dst, const float4& x) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(x.x, x.y), hi = __floats2bfloat162_rn(x.z, x.w);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  };
+  put(dv + o, acc_v);
+  put(dk + o, acc_k);
 }
 
 template <class K>
@@ -780,7 +789,7 @@ void attention_backward_dkv(const AttnBwdArgs& a, cudaStream_t stream) {
       a.heads_kv, a.heads_q / a.heads_kv, a.softmax_scale, a.lse, a.delta, a.total_q, a.dk, a.dv, a.ld_dkv, a.partials,
       a.err);
   if (a.num_reduce_jobs > 0) {
-    attn_bwd_reduce_kernel<<<dim3(a.num_reduce_jobs, a.heads_kv), 256, 0, stream>>>(
+    attn_bwd_reduce_kernel<<<dim3(a.num_reduce_jobs, a.heads_kv, 128 / kReduceRows), kReduceRows * 32, 0, stream>>>(
         reinterpret_cast<const ReduceJob*>(a.reduce_jobs), a.partials, a.heads_kv, a.dk, a.dv, a.ld_dkv);
   }
 }

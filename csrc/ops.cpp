@@ -1383,7 +1383,7 @@ std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor
 std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
                                   const Tensor& dout, const Tensor& lse, const Tensor& seqs, const Tensor& q_tiles,
                                   const Tensor& kv_items, const Tensor& q_blocks, const Tensor& reduce_jobs,
-                                  int64_t num_slots, bool causal, double softmax_scale) {
+                                  int64_t num_slots, bool causal, double softmax_scale, bool packed, bool covered) {
   auto check3 = [](const Tensor& t, const char* n) {
     TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 3 && t.size(2) == 128 &&
                     t.stride(2) == 1 && t.stride(1) == 128 && t.stride(0) % 8 == 0 &&
@@ -1410,9 +1410,23 @@ std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor
   checki(reduce_jobs, 4, "reduce_jobs");
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t hq = q.size(1), hkv = k.size(1);
-  Tensor dq = torch::zeros({q.size(0), hq, 128}, q.options());
-  Tensor dk = torch::zeros({k.size(0), hkv, 128}, k.options());
-  Tensor dv = torch::zeros({k.size(0), hkv, 128}, k.options());
+  // packed: the three gradients are slices of one [tokens, hq + 2 hkv, 128] tensor (queries and keys are the same tokens)
+  TORCH_CHECK(!packed || q.size(0) == k.size(0), "rl_engine.attention_bwd: packed gradients need as many queries as keys");
+  // covered: the work lists write every row of all three, nothing has to be zeroed first
+  auto make = [&](int64_t rows, int64_t heads, const Tensor& like) {
+    return covered ? torch::empty({rows, heads, 128}, like.options()) : torch::zeros({rows, heads, 128}, like.options());
+  };
+  Tensor dq, dk, dv, all;
+  if (packed) {
+    all = make(q.size(0), hq + 2 * hkv, q);
+    dq = all.slice(1, 0, hq);
+    dk = all.slice(1, hq, hq + hkv);
+    dv = all.slice(1, hq + hkv, hq + 2 * hkv);
+  } else {
+    dq = make(q.size(0), hq, q);
+    dk = make(k.size(0), hkv, k);
+    dv = make(k.size(0), hkv, k);
+  }
   Tensor delta = torch::empty({hq, q.size(0)}, lse.options());
   Tensor partials = torch::empty({std::max<int64_t>(num_slots, 1) * hkv * 2 * 128 * 128}, lse.options());
   cudaStream_t stream = stream_of(q);
@@ -1454,6 +1468,7 @@ std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor
   rlk::attention_backward_dq(a, stream);
   rlk::attention_backward_dkv(a, stream);
   after_launch(a.num_reduce_jobs > 0 ? 4 : 3);
+  if (packed) return {all};
   return {dq, dk, dv};
 }
 
@@ -1559,7 +1574,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("adamw", rlk::traced("rlk::adamw", &adamw));
   m.def("sample", rlk::traced("rlk::sample", &sample));
   m.def("attention_fwd", rlk::traced("rlk::attention_fwd", &attention_fwd));
-  m.def("attention_bwd", rlk::traced("rlk::attention_bwd", &attention_bwd));
+  m.def("attention_bwd", rlk::traced("rlk::attention_bwd", &attention_bwd), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"),
+        py::arg("dout"), py::arg("lse"), py::arg("seqs"), py::arg("q_tiles"), py::arg("kv_items"), py::arg("q_blocks"),
+        py::arg("reduce_jobs"), py::arg("num_slots"), py::arg("causal"), py::arg("softmax_scale"), py::arg("packed") = false, py::arg("covered") = false);
   m.def("error_state", rlk::traced("rlk::error_state", &error_state));
   m.def("reset_error", rlk::traced("rlk::reset_error", &reset_error));
   m.def("launch_count", rlk::traced("rlk::launch_count", &launch_count));

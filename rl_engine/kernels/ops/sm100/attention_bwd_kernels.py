@@ -18,12 +18,31 @@ from rl_engine.kernels.ops.base import require_ext
 KEY_TILE = 128
 Q_BLOCK = 64
 MAX_BLOCKS_PER_ITEM = 64
+MIN_BLOCKS_PER_ITEM = 4
 
-_PLAN_CACHE: Dict[int, tuple] = {}
+_PLAN_CACHE: Dict[Tuple[int, int], tuple] = {}
 
 
-def build_plan(layout) -> tuple:
-    hit = _PLAN_CACHE.get(id(layout))
+def blocks_per_item(blocks: int, kv_heads: int) -> int:
+    """How long a key tile's query-block list may be before it is split.  One CTA walks one list for all query heads of
+    its group (1.3 us per block and head), so a list of 40 blocks on a machine with 80 CTAs in all is the whole kernel's
+    time; two CTAs per SM (296) of equal length is what the split aims at.  Below 4 blocks the CTA's set-up and the
+    reduction of its partial (128 KB) cost more than they save, above 64 the tail of the last wave does."""
+    return max(MIN_BLOCKS_PER_ITEM, min(MAX_BLOCKS_PER_ITEM, -(-blocks * kv_heads // 296)))
+
+
+def union_length(spans) -> int:
+    total, at = 0, 0
+    for lo, hi in sorted(spans):
+        total += max(0, hi - max(lo, at))
+        at = max(at, hi)
+    return total
+
+
+def build_plan(layout, kv_heads: int = 1) -> tuple:
+    """``(items, q_blocks, jobs, partial slots, (query rows, key rows) that the lists write)``"""
+    key = (id(layout), kv_heads)
+    hit = _PLAN_CACHE.get(key)
     if hit is not None and hit[0] is layout:
         return hit[1]
     # readers: (k_start, k_len, q_start, q_len, causal).  Key ranges of different sequences may be equal
@@ -40,6 +59,7 @@ def build_plan(layout) -> tuple:
     q_blocks: List[List[int]] = []
     items: List[List[int]] = []
     jobs: List[List[int]] = []
+    lists: List[Tuple[int, int, int, int]] = []  # (first key, keys, list begin, list end)
     slots = 0
     for lo, hi in zip(cuts[:-1], cuts[1:]):
         covering = [r for r in readers if r[0] <= lo and hi <= r[0] + r[1]]
@@ -58,22 +78,27 @@ def build_plan(layout) -> tuple:
             end = len(q_blocks)
             if end == begin:
                 continue
-            tile_len = min(KEY_TILE, hi - k_abs)
-            pieces = [(b, min(b + MAX_BLOCKS_PER_ITEM, end)) for b in range(begin, end, MAX_BLOCKS_PER_ITEM)]
-            if len(pieces) == 1:
-                items.append([k_abs, tile_len, 0, begin, end, -1, 0, 0])
-            else:
-                jobs.append([k_abs, tile_len, slots, slots + len(pieces)])
-                for (b, e) in pieces:
-                    items.append([k_abs, tile_len, 0, b, e, slots, 0, 0])
-                    slots += 1
+            lists.append((k_abs, min(KEY_TILE, hi - k_abs), begin, end))
+    most = blocks_per_item(len(q_blocks), kv_heads)
+    for (k_abs, tile_len, begin, end) in lists:
+        count = -(-(end - begin) // most)
+        per = -(-(end - begin) // count)  # pieces of equal length
+        pieces = [(b, min(b + per, end)) for b in range(begin, end, per)]
+        if len(pieces) == 1:
+            items.append([k_abs, tile_len, 0, begin, end, -1, 0, 0])
+        else:
+            jobs.append([k_abs, tile_len, slots, slots + len(pieces)])
+            for (b, e) in pieces:
+                items.append([k_abs, tile_len, 0, b, e, slots, 0, 0])
+                slots += 1
     items.sort(key=lambda it: it[3] - it[4])  # longest lists first
     dev = layout.seqs.device
     as_t = lambda rows, w: torch.tensor(rows, dtype=torch.int32, device=dev).reshape(-1, w)
-    plan = (as_t(items, 8), as_t(q_blocks, 4), as_t(jobs, 4), slots)
+    covered = (union_length((s[0], s[0] + s[1]) for s in layout.host_seqs), union_length((x[0], x[0] + x[1]) for x in lists))
+    plan = (as_t(items, 8), as_t(q_blocks, 4), as_t(jobs, 4), slots, covered)
     if len(_PLAN_CACHE) > 64:
         _PLAN_CACHE.clear()
-    _PLAN_CACHE[id(layout)] = (layout, plan)
+    _PLAN_CACHE[key] = (layout, plan)
     return plan
 
 
@@ -82,14 +107,15 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t if ok else t.contiguous()
 
 
-def fused_backward(q, k, v, out, lse, dout, layout, scale: float):
-    items, q_blocks, jobs, slots = build_plan(layout)
+def fused_backward(q, k, v, out, lse, dout, layout, scale: float, packed: bool = False):
+    """``(dq, dk, dv)``; ``packed`` (queries and keys are the same tokens): one ``[tokens, Hq + 2 Hkv, 128]`` tensor."""
+    items, q_blocks, jobs, slots, written = build_plan(layout, k.shape[1])
     dout = _aligned(dout)
     out = _aligned(out)
     if out.stride(0) != dout.stride(0):
         out, dout = out.contiguous(), dout.contiguous()
-    dq, dk, dv = require_ext().attention_bwd(
+    grads = require_ext().attention_bwd(
         _aligned(q), _aligned(k), _aligned(v), out, dout, lse, layout.seqs, layout.tiles, items, q_blocks, jobs, slots,
-        layout.causal, float(scale),
+        layout.causal, float(scale), packed, written == (q.shape[0], k.shape[0]),
     )
-    return dq, dk, dv
+    return grads[0] if packed else tuple(grads)

@@ -53,3 +53,22 @@ def test_embedding_gradient_refuses_ids_outside_the_table():
         out = FusedEmbeddingSM100Op()(torch.tensor([1, bad, 2], device=DEV), table)
         with pytest.raises(ValueError):
             out.sum().backward()
+
+
+@pytest.mark.parametrize("p,g,l,hq,hkv", [(1, 2, 33, 4, 1), (300, 5, 70, 8, 2), (129, 40, 64, 2, 2), (700, 3, 200, 16, 2)])
+def test_attention_gradient_with_split_block_lists(p, g, l, hq, hkv):
+    """Key tiles whose query-block lists are cut into pieces of 4 and more, against the fp32 restatement of the packed
+    attention (P and dS are rounded to bf16 once each)."""
+    from rl_engine.kernels.ops.sm100.attention import _reference_backward, grpo_group_layout, packed_attention_forward
+    from rl_engine.kernels.ops.sm100.attention_bwd_kernels import fused_backward
+
+    t = p + g * l
+    q, k, v = _randn(t, hq, 128, seed=1), _randn(t, hkv, 128, seed=2), _randn(t, hkv, 128, seed=3)
+    dout = _randn(t, hq, 128, seed=4)
+    layout = grpo_group_layout(p, g, l, torch.device(DEV))
+    out, lse = packed_attention_forward(q, k, v, layout)
+    scale = 128 ** -0.5
+    got = fused_backward(q, k, v, out, lse, dout, layout, scale)
+    for a, b in zip(got, _reference_backward(q, k, v, out, lse, dout, layout, scale)):
+        assert _rel(a, b) < 2 * BF16
+    assert all(torch.equal(a, b) for a, b in zip(got, fused_backward(q, k, v, out, lse, dout, layout, scale)))
