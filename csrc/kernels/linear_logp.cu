@@ -108,15 +108,23 @@ struct EpiLogpStats {
       // columns of -inf only (a masked stretch of the vocabulary): exponents are taken against 0, the sum stays 0
       const float base = new_m2 == -INFINITY ? 0.f : new_m2;
       const float rescale = fast_exp2(st.m2 - base);  // 0 on the first chunk (m2 = -inf)
-      float sum = 0.f, tsum = 0.f;
+      // The exponentials bound this loop at short contractions (K = 512: 2048 cycles of them per tile and as many of products), so
+      // the entropy's sum is formed only where it is asked for; the other sums are the same either way.
+      float sum = 0.f;
+      if (ep.entropy != nullptr) {
+        float tsum = 0.f;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float e = fast_exp2(fmaf(v[j], kLog2e, -base));
-        sum += e;
-        tsum = fmaf(e, (col0 + j < p.N) ? v[j] : 0.f, tsum);
+        for (int j = 0; j < 32; ++j) {
+          const float e = fast_exp2(fmaf(v[j], kLog2e, -base));
+          sum += e;
+          tsum = fmaf(e, (col0 + j < p.N) ? v[j] : 0.f, tsum);
+        }
+        st.t = fmaf(st.t, rescale, tsum);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum += fast_exp2(fmaf(v[j], kLog2e, -base));
       }
       st.s = fmaf(st.s, rescale, sum);
-      st.t = fmaf(st.t, rescale, tsum);
       st.m2 = new_m2;
       const int tl = st.tgt - col0;
       if (tl >= 0 && tl < 32) {

@@ -669,7 +669,8 @@ void linear_logp_dz(const Tensor& hidden, const Tensor& weight, const Tensor& ta
   check_rowmajor(dz, "dz");
   TORCH_CHECK(dz.scalar_type() == torch::kBFloat16 && dz.size(0) >= hidden.size(0) && dz.size(1) == weight.size(0),
               "rl_engine.linear_logp_dz: dz must be bf16 [>=N, V_local]");
-  TORCH_CHECK(dz.stride(0) % 8 == 0, "rl_engine.linear_logp_dz: dz row pitch must be a multiple of 8");
+  TORCH_CHECK(dz.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(dz.data_ptr()) % 16 == 0,
+              "rl_engine.linear_logp_dz: dz row pitch must be a multiple of 8 and its base 16-byte aligned");
   TORCH_CHECK(lse.scalar_type() == torch::kFloat32 && grad.scalar_type() == torch::kFloat32 && lse.is_contiguous() &&
                   grad.is_contiguous(),
               "rl_engine.linear_logp_dz: lse and grad must be contiguous float32");

@@ -23,6 +23,72 @@ def _rel(got, want):
     return ((got.double() - want.double()).norm() / want.double().norm().clamp_min(1e-300)).item()
 
 
+# ------------------------------------------------------------------------------------------------ linear log-prob
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 300, 777, 5000])
+@pytest.mark.parametrize("v", [300, 513, 9000])
+def test_linear_logp_rows_on_both_engines(n, v):
+    """Single CTAs up to one row tile, CTA pairs above: values against fp64, and each row the same bits on its own."""
+    from rl_engine.kernels.ops.sm100.linear_logp import FusedLinearLogpSM100Op
+
+    h, w = _randn(n, 192, seed=n), _randn(v, 192, seed=v, scale=0.1)
+    t = torch.randint(0, v, (n,), device=DEV, generator=_gen(3))
+    op = FusedLinearLogpSM100Op()
+    lp, ent = op.with_entropy(h, w, t)
+    z = torch.log_softmax(h.double() @ w.double().t(), -1)
+    assert torch.allclose(lp.double(), z.gather(1, t[:, None])[:, 0], atol=2e-5, rtol=1e-5)  # 32-bit sums over v terms
+    assert torch.allclose(ent.double(), -(z.exp() * z).sum(-1), atol=2e-5, rtol=1e-5)
+    rows = slice(n // 2, n // 2 + 1)
+    assert torch.equal(op(h[rows], w, t[rows]), lp[rows])
+
+
+def test_linear_logp_with_masked_vocabulary_and_replayed_graph():
+    """Whole records of -inf (a masked stretch of the vocabulary, also the first one) leave the row finite; a captured call
+    gives new results on every replay."""
+    from rl_engine.kernels.ops.sm100.linear_logp import FusedLinearLogpSM100Op
+
+    n, v = 200, 3000
+    h, w = _randn(n, 128, seed=1), _randn(v, 128, seed=2, scale=0.1)
+    bias = torch.zeros(v, device=DEV)
+    bias[:1100] = float("-inf")
+    bias[2000:2600] = float("-inf")
+    t = torch.randint(1100, 2000, (n,), device=DEV, generator=_gen(4))
+    op = FusedLinearLogpSM100Op()
+    want = torch.log_softmax(h.double() @ w.double().t() + bias.double(), -1).gather(1, t[:, None])[:, 0]
+    with torch.no_grad():
+        assert torch.allclose(op(h, w, t, bias).double(), want, atol=2e-5, rtol=1e-5)
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            op(h, w, t, bias)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = op(h, w, t, bias)
+        for seed in (5, 6, 7):
+            h.copy_(_randn(n, 128, seed=seed))
+            graph.replay()
+            want = torch.log_softmax(h.double() @ w.double().t() + bias.double(), -1).gather(1, t[:, None])[:, 0]
+            assert torch.allclose(out.double(), want, atol=2e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("n,chunk", [(100, 4096), (700, 128), (700, 4096), (513, 256)])
+@pytest.mark.parametrize("v", [1001, 1024])
+def test_linear_logp_weight_gradient_in_one_and_several_chunks(n, chunk, v):
+    """First chunk writes, later ones add, the last one rounds: against fp64 of the same bf16 dz (rounding of dz: 2^-9 per
+    term, of the stored gradient 2^-9), bias column sums included."""
+    from rl_engine.kernels.ops.sm100.linear_logp import FusedLinearLogpSM100Op
+
+    d = 64
+    h, w = _randn(n, d, seed=n).requires_grad_(True), _randn(v, d, seed=v, scale=0.1).requires_grad_(True)
+    b = (0.1 * torch.randn(v, device=DEV, generator=_gen(8))).requires_grad_(True)
+    t = torch.randint(0, v, (n,), device=DEV, generator=_gen(9))
+    g = torch.randn(n, device=DEV, generator=_gen(10))
+    FusedLinearLogpSM100Op(bwd_chunk_tokens=chunk)(h, w, t, b).backward(g)
+    hd, wd, bd = (x.detach().double().requires_grad_(True) for x in (h, w, b))
+    torch.log_softmax(hd @ wd.t() + bd, -1).gather(1, t[:, None])[:, 0].backward(g.double())
+    for got, want in ((h.grad, hd.grad), (w.grad, wd.grad), (b.grad, bd.grad)):
+        assert _rel(got, want) < BF16
+
+
 # ------------------------------------------------------------------------------------------------ embedding gradient
 @pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 1000])
 @pytest.mark.parametrize("kind", ["one", "distinct", "few", "border"])
