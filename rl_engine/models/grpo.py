@@ -12,6 +12,7 @@ The reference's counterpart is ``DeepSpeedTrainingWorker.train``
 from __future__ import annotations
 
 import contextlib
+import threading
 from dataclasses import dataclass
 from typing import Dict, Optional
 
@@ -248,6 +249,15 @@ def suffix_geometry(p: int, m: int, l: int, device):
     return hit
 
 
+def _head_logps(model, picked: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
+    from rl_engine.kernels.registry import kernel_registry
+
+    op, sink = kernel_registry.get_op("linear_logp"), getattr(model, "_grad_sink", lambda name: None)("lm_head")
+    if sink is None:
+        return op(picked, model.lm_head_weight(), ids)
+    return op(picked, model.lm_head_weight(), ids, grad_weight_sink=sink)
+
+
 def policy_logps_after_prefix(model: LlamaModel, batch: "GRPOBatch", last_state: torch.Tensor, kv) -> torch.Tensor:
     """``policy_logps`` for completions whose prompt was processed by ``model.prefix_states`` (``last_state``, ``kv``):
     same kernels and per-row arithmetic as the single pass, without re-processing the prompt."""
@@ -257,8 +267,7 @@ def policy_logps_after_prefix(model: LlamaModel, batch: "GRPOBatch", last_state:
     layout, positions, rows = suffix_geometry(p, m, l, batch.prompt_ids.device)
     hidden = model.hidden_states_after_prefix(batch.completion_ids.reshape(-1), positions, layout, kv)
     picked = kernel_registry.get_op("embedding")(rows, torch.cat([last_state, hidden]))
-    logp = kernel_registry.get_op("linear_logp")(picked, model.lm_head_weight(), batch.completion_ids.reshape(-1))
-    return logp.reshape(m, l)
+    return _head_logps(model, picked, batch.completion_ids.reshape(-1)).reshape(m, l)
 
 
 def policy_logps(model: LlamaModel, batch: "GRPOBatch") -> torch.Tensor:
@@ -274,8 +283,7 @@ def policy_logps(model: LlamaModel, batch: "GRPOBatch") -> torch.Tensor:
     hidden = model.hidden_states(tokens, positions, layout)
     # deterministic differentiable row gather (ordered segment sums in backward, no atomics)
     picked = kernel_registry.get_op("embedding")(rows, hidden)
-    logp = kernel_registry.get_op("linear_logp")(picked, model.lm_head_weight(), batch.completion_ids.reshape(-1))
-    return logp.reshape(g, l)
+    return _head_logps(model, picked, batch.completion_ids.reshape(-1)).reshape(g, l)
 
 
 def choose_micro_group(group: int, prompt_len: int, completion_len: int, layers: int, kept_for_tokens,
@@ -341,6 +349,9 @@ class GRPOTrainer:
     # anything is launched, so that a step whose peers have left raises ``RankLeftError`` instead of waiting on them.
     liveness = None
     _steps_started = 0
+    # The fused layers add weight gradients to the flat buffer in their own GEMMs (``LlamaModel._grad_sink``).  Trainers that
+    # watch or exchange gradients while backward runs leave this off.
+    sink_weight_grads = True
     cache_prompt = True  # micro-batches attend to the prompt's cached keys / values instead of re-processing it
     _last_group = True   # False while ``step_groups`` is accumulating a group that is not the step's last one
 
@@ -395,6 +406,15 @@ class GRPOTrainer:
 
     def forward_backward(self, batch: GRPOBatch) -> torch.Tensor:
         """Accumulates the gradient of the group's token-mean loss into the flat gradient buffer; returns the loss."""
+        if not (self.sink_weight_grads and hasattr(self.model, "sink_weight_grads")):
+            return self._forward_backward(batch)
+        self.model.sink_weight_grads = threading.get_ident()
+        try:
+            return self._forward_backward(batch)
+        finally:
+            self.model.sink_weight_grads = None
+
+    def _forward_backward(self, batch: GRPOBatch) -> torch.Tensor:
         g = batch.completion_ids.shape[0]
         m = self.completions_per_pass(batch)
         if m >= g and not self.force_prompt_pass(batch):

@@ -16,6 +16,7 @@ The reference ships no model (only ``Embedding -> Linear`` toys:
 from __future__ import annotations
 
 import math
+import threading
 from typing import Dict, List, Optional, Tuple, Union
 
 import torch
@@ -93,8 +94,8 @@ class _FusedAttentionBlock(torch.autograd.Function):
         # backward pass, and this block's backward un-rotates the gradients, so the unrotated values are never read
         # again.  One [T, Hq + 2 Hkv, 128] tensor is kept instead of that plus rotated copies of q and k.
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        ext.rope(q, positions, cos_t, sin_t, False, q)
-        ext.rope(k, positions, cos_t, sin_t, False, k)
+        qk = qkv[:, : hq + hkv]  # adjacent heads: one launch rotates both
+        ext.rope(qk, positions, cos_t, sin_t, False, qk)
         out, lse = packed_attention_forward(q, k, v, layout, scale, True)
         ctx.save_for_backward(qkv, out, lse, positions, cos_t, sin_t)
         ctx.meta = (layout, hq, hkv, scale)
@@ -103,17 +104,15 @@ class _FusedAttentionBlock(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         from rl_engine.kernels.ops.base import require_ext
-        from rl_engine.kernels.ops.sm100.attention_bwd import packed_attention_backward
+        from rl_engine.kernels.ops.sm100.attention_bwd_kernels import fused_backward
 
         qkv, out, lse, positions, cos_t, sin_t = ctx.saved_tensors
         layout, hq, hkv, scale = ctx.meta
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        dq, dk, dv = packed_attention_backward(q, k, v, out, lse, dout.contiguous(), layout, scale)
-        dqkv = torch.empty_like(qkv)
-        ext = require_ext()
-        ext.rope(dq, positions, cos_t, sin_t, True, dqkv[:, :hq])
-        ext.rope(dk, positions, cos_t, sin_t, True, dqkv[:, hq : hq + hkv])
-        dqkv[:, hq + hkv :].copy_(dv)
+        # the kernels write the slices of one packed tensor; its q and k heads are un-rotated in place
+        dqkv = fused_backward(q, k, v, out, lse, dout.contiguous(), layout, scale, packed=True)
+        dqk = dqkv[:, : hq + hkv]
+        require_ext().rope(dqk, positions, cos_t, sin_t, True, dqk)
         return dqkv, None, None, None, None, None, None, None
 
 
@@ -139,8 +138,8 @@ class _FusedAttentionBlockKV(torch.autograd.Function):
 
         ext = require_ext()
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        ext.rope(q, positions, cos_t, sin_t, False, q)
-        ext.rope(k, positions, cos_t, sin_t, False, k)
+        qk = qkv[:, : hq + hkv]  # adjacent heads: one launch rotates both
+        ext.rope(qk, positions, cos_t, sin_t, False, qk)
         out, lse = packed_attention_forward(q, k, v, layout, scale, True)
         ctx.save_for_backward(qkv, out, lse, positions, cos_t, sin_t)
         ctx.meta = (layout, hq, hkv, scale)
@@ -148,17 +147,19 @@ class _FusedAttentionBlockKV(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout, dk_later, dv_later):
-        from rl_engine.kernels.ops.sm100.attention_bwd import packed_attention_backward
+        from rl_engine.kernels.ops.base import require_ext
+        from rl_engine.kernels.ops.sm100.attention_bwd_kernels import fused_backward
 
         qkv, out, lse, positions, cos_t, sin_t = ctx.saved_tensors
         layout, hq, hkv, scale = ctx.meta
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        dq, dk, dv = packed_attention_backward(q, k, v, out, lse, dout.contiguous(), layout, scale)
-        if dk_later is not None:
-            dk = (dk.float() + dk_later.float()).to(dk.dtype)
+        dqkv = fused_backward(q, k, v, out, lse, dout.contiguous(), layout, scale, packed=True)
+        if dk_later is not None:  # added in 32 bits, rounded once
+            dqkv[:, hq : hq + hkv].add_(dk_later)
         if dv_later is not None:
-            dv = (dv.float() + dv_later.float()).to(dv.dtype)
-        dqkv = _unrotate_into(torch.empty_like(qkv), dq, dk, dv, positions, cos_t, sin_t, hq, hkv)
+            dqkv[:, hq + hkv :].add_(dv_later)
+        dqk = dqkv[:, : hq + hkv]
+        require_ext().rope(dqk, positions, cos_t, sin_t, True, dqk)
         return dqkv, None, None, None, None, None, None, None
 
 
@@ -174,8 +175,8 @@ class _FusedAttentionBlockPrefix(torch.autograd.Function):
 
         ext = require_ext()
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        ext.rope(q, positions, cos_t, sin_t, False, q)
-        ext.rope(k, positions, cos_t, sin_t, False, k)
+        qk = qkv[:, : hq + hkv]  # adjacent heads: one launch rotates both
+        ext.rope(qk, positions, cos_t, sin_t, False, qk)
         out, lse = packed_attention_forward(q, torch.cat([k_prefix, k]), torch.cat([v_prefix, v]), layout, scale, True)
         ctx.save_for_backward(qkv, k_prefix, v_prefix, out, lse, positions, cos_t, sin_t)
         ctx.meta = (layout, hq, hkv, scale)
@@ -208,8 +209,8 @@ class _FusedAttentionBlockCP(torch.autograd.Function):
 
         ext = require_ext()
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        ext.rope(q, positions, cos_t, sin_t, False, q)
-        ext.rope(k, positions, cos_t, sin_t, False, k)
+        qk = qkv[:, : hq + hkv]  # adjacent heads: one launch rotates both
+        ext.rope(qk, positions, cos_t, sin_t, False, qk)
         k_all, v_all = cp.gather_kv(k, v)
         out, lse = packed_attention_forward(q, k_all, v_all, cp.layout(q.device), scale, True)
         ctx.save_for_backward(qkv, out, lse, positions, cos_t, sin_t)
@@ -267,8 +268,8 @@ class _FusedAttentionBlockCPKV(torch.autograd.Function):
 
         ext = require_ext()
         q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
-        ext.rope(q, positions, cos_t, sin_t, False, q)
-        ext.rope(k, positions, cos_t, sin_t, False, k)
+        qk = qkv[:, : hq + hkv]  # adjacent heads: one launch rotates both
+        ext.rope(qk, positions, cos_t, sin_t, False, qk)
         k_all, v_all = cp.gather_kv(k, v)
         k_all, v_all = k_all.clone(), v_all.clone()  # the symmetric buffers are reused by the next layer
         out, lse = packed_attention_forward(q, k_all, v_all, cp.layout(q.device), scale, True)
@@ -315,6 +316,10 @@ class LlamaModel(nn.Module):
         # final norm), i.e. when nothing of this pass touches the parameters of layers >= ``layer_index`` again.
         self.layer_grad_hook = None
         self._fp8_linears: Dict[str, object] = {}
+        # Set while a trainer that calls ``backward`` itself builds the graph: the fused layers then add weight gradients
+        # to ``param.grad`` in their GEMMs (``_grad_sink``) instead of returning them to autograd to be added there.
+        # Holds the thread that does so: graphs built elsewhere at the same time return their gradients as usual.
+        self.sink_weight_grads: Optional[int] = None
         h, f = cfg.hidden_size, cfg.ffn_size
         qkv_rows = cfg.q_dim + 2 * cfg.kv_dim
         shapes: List[Tuple[str, Tuple[int, ...]]] = [("embed", (cfg.vocab_size, h))]
@@ -397,6 +402,26 @@ class LlamaModel(nn.Module):
             for name in self._names:
                 self.view(name).grad = self._slice(self.flat_grad, name)
         return self.flat_grad
+
+    def _grad_sink(self, name: str) -> Optional[torch.Tensor]:
+        """The gradient buffer that a fused backward pass may add to in place of autograd, or ``None``: sinks are off, the
+        parameter is frozen or watched by hooks, or its gradient is not a buffer the kernels can address."""
+        if self.sink_weight_grads is None or self.sink_weight_grads != threading.get_ident():
+            return None
+        p = self.view(name)
+        g = p.grad
+        if (g is None or not p.requires_grad or p._backward_hooks or getattr(p, "_post_accumulate_grad_hooks", None)
+                or g.dtype != torch.bfloat16 or g.shape != p.shape or not g.is_contiguous() or g.data_ptr() % 16
+                or g.shape[-1] % 8 or not g.is_cuda):
+            return None
+        return g
+
+    def embed_tokens(self, token_ids: torch.Tensor) -> torch.Tensor:
+        from rl_engine.kernels.registry import kernel_registry
+
+        sink = self._grad_sink("embed")
+        op = kernel_registry.get_op("embedding")
+        return op(token_ids, self.view("embed")) if sink is None else op(token_ids, self.view("embed"), grad_sink=sink)
 
     @torch.no_grad()
     def reset_parameters(self, seed: int = 0) -> None:
@@ -485,7 +510,8 @@ class LlamaModel(nn.Module):
         if lean:
             from rl_engine.kernels.ops.sm100.lean_blocks import norm_linear
 
-            qkv = norm_linear(x, p("attn_norm"), p("wqkv"), cfg.rms_eps)
+            sink = lambda n: self._grad_sink(f"l{index}.{n}")
+            qkv = norm_linear(x, p("attn_norm"), p("wqkv"), cfg.rms_eps, (sink("attn_norm"), sink("wqkv")))
         else:
             qkv = linear(rms_norm(x, p("attn_norm"), cfg.rms_eps), p("wqkv"))
         if cfg.qkv_bias:
@@ -493,7 +519,12 @@ class LlamaModel(nn.Module):
         attn = self._attention(qkv, positions, layout, index, k_prefix, v_prefix, return_kv)
         if return_kv:
             attn, k_rot, v_rot = attn
-        x = x + linear(attn, p("wo"))
+        if lean:
+            from rl_engine.kernels.ops.sm100.lean_blocks import residual_linear
+
+            x = residual_linear(x, attn, p("wo"), sink("wo"))
+        else:
+            x = x + linear(attn, p("wo"))
         x = self._ffn(x, index, lean)
         return (x, k_rot, v_rot) if return_kv else x
 
@@ -511,7 +542,9 @@ class LlamaModel(nn.Module):
             moe = self.moe_op if self.moe_op is not None else kernel_registry.get_op("moe")
             return x + moe(h, p("router"), p("w_gate_up"), p("w_down"), cfg.experts_per_token)
         if lean:
-            return x + swiglu_linear(norm_linear(x, p("mlp_norm"), p("w_gate_up"), cfg.rms_eps), p("w_down"))
+            sink = lambda n: self._grad_sink(f"l{index}.{n}")
+            gu = norm_linear(x, p("mlp_norm"), p("w_gate_up"), cfg.rms_eps, (sink("mlp_norm"), sink("w_gate_up")))
+            return swiglu_linear(gu, p("w_down"), residual=x, sink=sink("w_down"))
         gu = linear(rms_norm(x, p("mlp_norm"), cfg.rms_eps), p("w_gate_up"))
         return x + linear(swiglu_packed(gu), p("w_down"))
 
@@ -559,9 +592,7 @@ class LlamaModel(nn.Module):
 
     def hidden_states(self, token_ids: torch.Tensor, positions: torch.Tensor, layout) -> torch.Tensor:
         """Packed ``token_ids [T]`` -> final-norm hidden states ``[T, H]``."""
-        from rl_engine.kernels.registry import kernel_registry
-
-        x = kernel_registry.get_op("embedding")(token_ids, self.view("embed"))
+        x = self.embed_tokens(token_ids)
         training = torch.is_grad_enabled()
         first_kept = self.cfg.num_layers - (self.plan_checkpointing(token_ids.numel()) if training else 0)
         for i in range(self.cfg.num_layers):
@@ -589,8 +620,6 @@ class LlamaModel(nn.Module):
         Back-propagating through the outputs then sums the ranks' gradients onto the rows' owners; together with
         the data-parallel gradient sum this equals every rank running the whole prompt."""
         from rl_engine.kernels.ops.sm100.attention import make_layout
-        from rl_engine.kernels.registry import kernel_registry
-
         n = prompt_ids.numel()
         positions = torch.arange(n, device=prompt_ids.device)
         if cp is None:
@@ -603,7 +632,7 @@ class LlamaModel(nn.Module):
             layout = cp
             prompt_ids = shard_sequence(prompt_ids.reshape(-1), cp.rank, cp.world)
             positions = shard_sequence(positions, cp.rank, cp.world)
-        x = kernel_registry.get_op("embedding")(prompt_ids, self.view("embed"))
+        x = self.embed_tokens(prompt_ids)
         kv = []
         for i in range(self.cfg.num_layers):
             self._watch(x, i)
@@ -616,9 +645,7 @@ class LlamaModel(nn.Module):
     def hidden_states_after_prefix(self, token_ids: torch.Tensor, positions: torch.Tensor, layout, kv) -> torch.Tensor:
         """Final-norm hidden states ``[T, H]`` of tokens that follow a prefix given by its per-layer ``kv``.
         ``layout`` indexes queries in ``token_ids`` and keys in ``[prefix | token_ids]``."""
-        from rl_engine.kernels.registry import kernel_registry
-
-        x = kernel_registry.get_op("embedding")(token_ids, self.view("embed"))
+        x = self.embed_tokens(token_ids)
         training = torch.is_grad_enabled()
         first_kept = self.cfg.num_layers - (self.plan_checkpointing(token_ids.numel()) if training else 0)
         for i, (k_prefix, v_prefix) in enumerate(kv):
@@ -651,8 +678,6 @@ class LlamaModel(nn.Module):
         log-sum-exp (``decode_layouts`` builds the pair)."""
         from rl_engine.kernels.ops.base import require_ext
         from rl_engine.kernels.ops.sm100.attention import packed_attention_forward
-        from rl_engine.kernels.registry import kernel_registry
-
         if not self.supports_prefix_cache():
             raise RuntimeError("decode_step needs the fused path (CUDA, bf16, head_dim 128, dense FFN)")
         cfg, ext = self.cfg, require_ext()

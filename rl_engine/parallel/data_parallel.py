@@ -234,6 +234,8 @@ class ShardedGRPOTrainer(GRPOTrainer):
 
     optimizer_class = ShardedFusedAdamW
 
+    sink_weight_grads = False  # gradient buckets are exchanged from hooks while backward runs
+
     def __init__(self, model: LlamaModel, *, group=None, lr: float = 1e-6, clip_eps: float = 0.2, beta: float = 0.04,
                  adv_eps: float = 1e-6, weight_decay: float = 0.0, master_weights: bool = True,
                  micro_group="auto", overlap: bool = True, layers_per_bucket: int = 4, shard_prompt: bool = False) -> None:

@@ -121,6 +121,101 @@ def test_embedding_gradient_refuses_ids_outside_the_table():
             out.sum().backward()
 
 
+# ------------------------------------------------------------------------------------------------ sampler
+def _draws(z, k, p, seed, offset):
+    """The kernel's rule in fp64 on the host; a draw within 1e-5 of the border between two tokens allows both."""
+    from rl_engine.kernels.ops.sm100.sampler import philox_uniform
+
+    out = []
+    for row, x in enumerate(z.double().cpu()):
+        order = torch.argsort(x, descending=True, stable=True)
+        kth = x[order[min(k, x.numel()) - 1]]
+        order = order[: int((x >= kth).sum())]
+        e = torch.exp(x[order] - x[order[0]])
+        c = e.cumsum(0)
+        keep = 1 + int((c[:-1] <= p * c[-1]).sum())
+        at = philox_uniform(seed, offset, row) * c[keep - 1]
+        near = lambda s: int(order[min(int(torch.searchsorted(c[:keep], at * s, right=True)), keep - 1)])
+        out.append({near(1 - 1e-5), near(1.0), near(1 + 1e-5)})
+    return out
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 140000), (3, 40001), (75, 33000), (200, 4096), (5, 37)])
+@pytest.mark.parametrize("k", [1, 50, 513, 1000])
+@pytest.mark.parametrize("shape", ["normal", "rising", "ties"])
+def test_top_k_sampler_over_splits_and_fallbacks(rows, vocab, k, shape):
+    """1 to 8 CTAs per row, unaligned rows, k above the vocabulary, a row whose head is far below its tail (the candidates
+    overflow) and masses of ties at the k-th place."""
+    from rl_engine.kernels.ops.sm100.sampler import sample_topk_topp
+
+    z = torch.randn(rows, vocab, device=DEV, generator=_gen(rows + k)) * 2
+    if shape == "rising":
+        z = z * 0.01 + torch.linspace(0, 40, vocab, device=DEV)
+    elif shape == "ties":
+        z = torch.round(z)
+        if int((z[0] == z[0].kthvalue(vocab - min(k, vocab) + 1).values).sum()) > 1000:
+            z[:, ::3] = z[:, ::3] + 0.25  # at most 2048 candidates are ordered
+    if k >= vocab:
+        pytest.skip("top_k >= vocab is the full-vocabulary kernel")
+    ids, _ = sample_topk_topp(z, top_k=k, top_p=0.95, temperature=1.0, seed=7, offset=11)
+    kth = z.kthvalue(vocab - k + 1, dim=-1).values
+    if int((z >= kth[:, None]).sum(-1).max()) > 2048:
+        assert bool((z.gather(1, ids[:, None])[:, 0] >= kth).all())
+        return
+    allowed = _draws(z, k, 0.95, 7, 11)
+    assert all(int(i) in a for i, a in zip(ids.cpu(), allowed))
+
+
+# ------------------------------------------------------------------------------------------------ log-prob gradient
+@pytest.mark.parametrize("v", [5, 1024, 4099, 8192])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("pitch", [0, 1, 8])
+def test_selected_logprob_gradient_alignment(v, dtype, pitch):
+    """Rows that share their offset from a 16-byte boundary with the gradient's (peeled) and rows that do not."""
+    from rl_engine.kernels.ops.sm100.logp_autograd import selected_logprobs
+
+    n = 9
+    store = _randn(n, v + pitch, seed=v, dtype=dtype)
+    z = store[:, :v].detach().requires_grad_(True)
+    ids = torch.randint(0, v, (n,), device=DEV, generator=_gen(2))
+    ids[:2] = torch.tensor([0, v - 1], device=DEV)
+    mask = torch.ones(n, dtype=torch.bool, device=DEV)
+    mask[3] = False
+    g = torch.randn(n, device=DEV, generator=_gen(3))
+    (grad,) = torch.autograd.grad(selected_logprobs(z, ids, mask), [z], g)
+    want = -torch.softmax(z.detach().double(), -1)
+    want[torch.arange(n), ids] += 1
+    want *= (g * mask).double()[:, None]
+    assert _rel(grad, want) < {torch.float32: 1e-6, torch.bfloat16: BF16 / 2, torch.float16: 2.0 ** -11}[dtype] * 2
+    assert bool((grad[3] == 0).all())
+
+
+# ------------------------------------------------------------------------------------------------ experts, attention backward
+@pytest.mark.parametrize("tokens", [1, 5, 130, 700])
+@pytest.mark.parametrize("h,e,k,f", [(256, 32, 4, 64), (128, 8, 2, 192), (512, 4, 1, 128)])
+def test_moe_with_empty_experts_and_ragged_blocks(tokens, h, e, k, f):
+    """Experts without a token (their weight gradient is exactly zero), blocks of any length, per-expert gradients with and
+    without 256-row tiles: against the oracle in fp32.  Every stored tensor on the way is rounded to bf16 once."""
+    from rl_engine.kernels.ops.sm100.moe import FusedMoESM100Op, NativeMoEOp
+
+    x, r = _randn(tokens, h, seed=1), _randn(e, h, seed=2, scale=h ** -0.5)
+    w1, w2 = _randn(e * 2 * f, h, seed=3, scale=0.05), _randn(e * h, f, seed=4, scale=0.05)
+    args = [t.requires_grad_(True) for t in (x, r, w1, w2)]
+    oracle = [t.detach().float().requires_grad_(True) for t in args]
+    dout = _randn(tokens, h, seed=5)
+    torch.full((1 << 24,), float("nan"), device=DEV)  # rows that no kernel writes would otherwise look harmless
+    out = FusedMoESM100Op()(*args, k)
+    want = NativeMoEOp()(*oracle, k)
+    assert _rel(out.detach(), want.detach()) < 2 * BF16
+    grads, wanted = torch.autograd.grad(out, args, dout), torch.autograd.grad(want, oracle, dout.float())
+    # the router's gradient is made of differences w_i w_j (dw_i - dw_j) of dot products of rounded rows: with few tokens each
+    # rounding counts up to |dw_i| + |dw_j| over their difference times, here up to four
+    for i, (got, ref) in enumerate(zip(grads, wanted)):
+        assert _rel(got, ref) < (12 if i == 1 else 3) * BF16
+    hit = wanted[3].view(e, -1).abs().sum(1) > 0
+    assert bool((grads[3].view(e, -1)[~hit] == 0).all()) and bool((grads[2].view(e, -1)[~hit] == 0).all())
+
+
 @pytest.mark.parametrize("p,g,l,hq,hkv", [(1, 2, 33, 4, 1), (300, 5, 70, 8, 2), (129, 40, 64, 2, 2), (700, 3, 200, 16, 2)])
 def test_attention_gradient_with_split_block_lists(p, g, l, hq, hkv):
     """Key tiles whose query-block lists are cut into pieces of 4 and more, against the fp32 restatement of the packed
@@ -138,3 +233,63 @@ def test_attention_gradient_with_split_block_lists(p, g, l, hq, hkv):
     for a, b in zip(got, _reference_backward(q, k, v, out, lse, dout, layout, scale)):
         assert _rel(a, b) < 2 * BF16
     assert all(torch.equal(a, b) for a, b in zip(got, fused_backward(q, k, v, out, lse, dout, layout, scale)))
+
+
+@pytest.mark.parametrize("rows,vocab", [(3, 40001), (160, 4096), (2, 150000), (4, 5)])
+@pytest.mark.parametrize("p", [0.5, 0.95, 1.0])
+@pytest.mark.parametrize("shape", ["normal", "flat", "steep", "masked"])
+def test_nucleus_sampler_integer_masses(rows, vocab, p, shape):
+    """The cut and the draw on 40-bit integer masses, restated on the host; flat logits overflow the gathered step and take
+    the search over the row.  A draw within 1e-5 of a token's border allows its neighbour."""
+    from rl_engine.kernels.ops.sm100.sampler import philox_uniform, sample_topk_topp
+
+    z = {"normal": 2.0, "flat": 1e-4, "steep": 12.0, "masked": 2.0}[shape] * torch.randn(rows, vocab, device=DEV, generator=_gen(vocab))
+    if shape == "masked" and vocab > 8:
+        z[:, : vocab // 2] = float("-inf")
+    got, _ = sample_topk_topp(z, top_k=None, top_p=p, temperature=0.8, seed=3, offset=2)
+    x = z.double().cpu()
+    for row in range(rows):
+        mass = torch.floor(torch.exp((x[row] - x[row].max()) / 0.8) * 2.0 ** 40)
+        order = torch.argsort(x[row], descending=True, stable=True)
+        c = mass[order].cumsum(0)
+        i = int(got[row])
+        first = min(int(torch.searchsorted(c, max(1.0, p * float(c[-1])) * (1 + 1e-5))), vocab - 1)
+        assert x[row, i] >= x[row, order[first]]  # inside the nucleus
+        cut = x[row, order[min(int(torch.searchsorted(c, max(1.0, p * float(c[-1])))), vocab - 1)]]
+        kept = torch.where(x[row] >= cut, mass, torch.zeros_like(mass)).cumsum(0)
+        t = philox_uniform(3, 2, row) * float(kept[-1])
+        lo, hi = (0.0 if i == 0 else float(kept[i - 1])), float(kept[i])
+        assert lo - 2e-5 * float(kept[-1]) <= t <= hi + 2e-5 * float(kept[-1])
+
+
+@pytest.mark.parametrize("micro", [None, 2])
+@pytest.mark.parametrize("chunk", [4096, 128])
+def test_gradients_added_by_the_gemms_equal_those_added_by_autograd(micro, chunk):
+    """One pass, and micro-batches after a prompt pass; LM-head gradients of one chunk and of several: the same bits."""
+    from rl_engine.kernels.registry import kernel_registry
+    from rl_engine.models.config import ModelConfig
+    from rl_engine.models.grpo import GRPOTrainer, synthetic_batch
+    from rl_engine.models.llama import LlamaModel
+
+    cfg = ModelConfig("sink", 640, 256, 2, 4, 2, 128, 384)
+    batch = synthetic_batch(640, 70, 6, 90, seed=2).to(DEV)
+    op = kernel_registry.get_op("linear_logp")
+    before, op.bwd_chunk_tokens = op.bwd_chunk_tokens, chunk
+    try:
+        grads = []
+        for sink in (True, False):
+            trainer = GRPOTrainer(LlamaModel(cfg, dtype=torch.bfloat16, device=DEV, seed=4), micro_group=micro)
+            trainer.sink_weight_grads = sink
+            trainer.opt.zero_grad()
+            trainer.forward_backward(batch)
+            grads.append({n: p.grad.clone() for n, p in trainer.model.named_views().items()})
+            assert trainer.model.sink_weight_grads is None
+        for name, want in grads[1].items():
+            assert torch.equal(grads[0][name], want), name
+        # outside the trainer's own pass, gradients are returned
+        model = trainer.model
+        out = trainer.policy_logps(batch).sum()
+        (g,) = torch.autograd.grad(out, [model.view("l0.wo")])
+        assert float(g.float().norm()) > 0
+    finally:
+        op.bwd_chunk_tokens = before
