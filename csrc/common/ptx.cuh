@@ -95,6 +95,33 @@ __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// ---- programmatic dependent launch -----------------------------------------------------------
+// Both do nothing in a kernel that was launched without the attribute.  A kernel calls grid_dep_launch() only after its own
+// grid_dep_wait(): whatever ran before it in the stream has then completed when the next kernel starts early.  What a
+// predecessor wrote is read with __ldcg (or TMA): the read-only path that the compiler picks for const __restrict__ pointers is
+// for data that does not change while the kernel is resident, and an early start makes it resident before the data is there.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+#ifdef __CUDACC__
+// Launch with the programmatic-stream-serialization attribute: the kernel may start while its predecessor in the stream
+// drains and has to call grid_dep_wait() before it touches anything an earlier kernel reads or writes.
+template <class... KArgs, class... Args>
+inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+#endif
+
 // ---- mbarrier ------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -72,8 +72,10 @@ struct Smem {
 };
 static_assert(Smem::kDynamic <= 232448, "attention forward exceeds the 227 KB shared-memory limit");
 
-struct SeqDesc {  // one per sequence, int32 x 8
-  int q_start, q_len, pk_start, pk_len, sk_start, sk_len, pad0, pad1;
+struct alignas(16) SeqDesc {  // one per sequence, int32 x 8
+  int q_start, q_len, pk_start, pk_len, sk_start, sk_len;
+  int out_offset;  // added to the row that output and log-sum-exp are stored to (partial results of one query set)
+  int pad1;
 };
 
 // Half a score row (64 keys) of one query: p = 2^(s * scale - m) packed to bf16 into the row's 128-byte swizzle
@@ -134,14 +136,19 @@ __device__ __forceinline__ Item decode_item(int w, const SeqDesc* __restrict__ s
   const int tile_id = w / num_heads_q;
   it.head = w - tile_id * num_heads_q;
   it.kv_head = it.head / q_per_kv;
-  const int2 tile = tiles[tile_id];
+  const int2 tile = __ldcg(tiles + tile_id);
   it.q0 = tile.y;
   it.n_prefix = it.n_tiles = 0;
   // The layout tables come from the caller.  Debug-bounds builds check them against the tensors before anything is
   // read or written through them; every role of the CTA decodes the same item and takes the same decision.
   it.ok = RLK_INDEX_OK(tile.x, num_seqs, err, 200u, 1);
   if (!it.ok) return it;
-  it.sd = seqs[tile.x];
+  {
+    // decoding advances the table between launches, and this kernel may be resident before that
+    const int4* d = reinterpret_cast<const int4*>(seqs + tile.x);
+    const int4 a = __ldcg(d), b = __ldcg(d + 1);
+    it.sd = SeqDesc{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  }
   it.ok = RLK_INDEX_OK(it.q0, it.sd.q_len > 0 ? it.sd.q_len : 1, err, 200u, 2) &&
           RLK_INDEX_OK(it.sd.q_start, total_q - it.sd.q_len + 1, err, 200u, 3) &&
           RLK_INDEX_OK(it.sd.pk_start, total_kv - it.sd.pk_len + 1, err, 200u, 4) &&
@@ -219,6 +226,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // a decoding step launches this kernel while its predecessor drains; nothing before this line reads its results
+  grid_dep_wait();
+  grid_dep_launch();
   const int first = total_items - 1 - static_cast<int>(blockIdx.x), step = static_cast<int>(gridDim.x);
 #define RLK_ATTN_ITEM(w) decode_item(w, seqs, tiles, num_heads_q, q_per_kv, causal, num_seqs, total_q, total_kv, err)
 
@@ -450,7 +460,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
       if (qi < sd.q_len) {
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        __nv_bfloat16* dst = out + static_cast<long long>(sd.q_start + qi) * ld_out + it.head * kD + half * kHalf;
+        __nv_bfloat16* dst = out + static_cast<long long>(sd.out_offset + sd.q_start + qi) * ld_out + it.head * kD + half * kHalf;
 #pragma unroll
         for (int c8 = 0; c8 < kHalf / 8; ++c8) {
           uint32_t wd[4];
@@ -463,7 +473,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           reinterpret_cast<uint4*>(dst)[c8] = make_uint4(wd[0], wd[1], wd[2], wd[3]);
         }
         if (lse != nullptr && half == 0) {
-          lse[static_cast<long long>(it.head) * lse_head_stride + sd.q_start + qi] =
+          lse[static_cast<long long>(it.head) * lse_head_stride + sd.out_offset + sd.q_start + qi] =
               l > 0.f ? (m2 + log2f(l)) * kLn2 : -INFINITY;
         }
       }
@@ -496,7 +506,15 @@ void attention_forward(const AttnFwdArgs& a, cudaStream_t stream) {
   }
   const long long items = static_cast<long long>(a.num_tiles) * a.heads_q;
   const long long grid = items < a.sm_count ? items : a.sm_count;  // one persistent CTA per SM (227 KB of shared memory each)
-  attn_fwd_kernel<<<static_cast<unsigned int>(grid), kThreads, Smem::kDynamic, stream>>>(
+  const dim3 blocks(static_cast<unsigned>(grid));
+  if (a.dependent) {
+    launch_dependent(attn_fwd_kernel, blocks, dim3(kThreads), Smem::kDynamic, stream, tq, tk, tv,
+                     reinterpret_cast<const SeqDesc*>(a.seqs), reinterpret_cast<const int2*>(a.tiles), static_cast<int>(items),
+                     a.heads_q, a.heads_q / a.heads_kv, a.causal ? 1 : 0, a.softmax_scale * kLog2e, a.out, a.ld_out, a.lse,
+                     a.lse_head_stride, a.err, a.num_seqs, static_cast<int>(a.total_q), static_cast<int>(a.total_kv));
+    return;
+  }
+  attn_fwd_kernel<<<blocks, kThreads, Smem::kDynamic, stream>>>(
       tq, tk, tv, reinterpret_cast<const SeqDesc*>(a.seqs), reinterpret_cast<const int2*>(a.tiles),
       static_cast<int>(items), a.heads_q, a.heads_q / a.heads_kv, a.causal ? 1 : 0, a.softmax_scale * kLog2e, a.out, a.ld_out, a.lse, a.lse_head_stride,
       a.err, a.num_seqs, static_cast<int>(a.total_q), static_cast<int>(a.total_kv));

@@ -146,6 +146,28 @@ void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
   }
   if constexpr (!A_MN && !B_MN) {
     if (a.group_mode == 0 && a.M <= kBM && !a.out_fp32 && !a.accumulate && a.N >= 4 * kSkinnyBN) {
+      // With at least one 128-row tile of B per SM (an LM head) the weight-streaming kernel of the decoding step takes it:
+      // B is its 128-row operand, so a stage is nearly all weight instead of two thirds padded tokens: 3 tokens on a
+      // 128256 x 4096 head 402 -> 174 us (2.6 -> 6.0 TB/s).  With fewer tiles than SMs, whole tiles leave SMs idle that the
+      // 64-column tiles below reach.
+      if (a.N >= kBM * a.sm_count && a.alpha == 1.f) {
+        DecodeLinearArgs d{};
+        d.x = a.A;
+        d.w = a.B;
+        d.ld_x = a.lda;
+        d.ld_w = a.ldb;
+        d.n = a.M;
+        d.N = a.N;
+        d.K = a.K;
+        d.mode = kDecodeStore;
+        d.whole_tiles = true;
+        d.out = static_cast<__nv_bfloat16*>(a.D);
+        d.ldo = a.ldd;
+        d.sm_count = a.sm_count;
+        d.err = a.err;
+        decode_linear(d, stream);
+        return;
+      }
       launch_skinny(a, stream);
       return;
     }

@@ -77,6 +77,46 @@ void gemm_fp8_rowscaled(const void* a_q, long long lda, const float* scale_a, co
 void quantize_rows_e4m3(const void* x, long long ldx, long long rows, int cols, void* q, long long ldq, float* scale,
                         cudaStream_t stream);
 
+// ------------------------------------------------------- linear layers of a decoding step (decode_linear.cu)
+enum DecodeLinearMode : int {
+  kDecodeStore = 0,   // out[t, f] = x W^T (+ residual[t, f])
+  kDecodeSwiglu = 1,  // W = [gate | up]: out[t, f] = silu(gate) * up
+  kDecodeQkv = 2,     // W = [q | k | v] heads of 128: rotary embedding on q and k, q packed for decode attention, k / v to the cache
+};
+struct DecodeLinearArgs {
+  const void* x;  // [n, K] bf16 (or e4m3 codes), n <= 128
+  const void* w;  // [N, K] bf16 (or e4m3 codes)
+  long long ld_x, ld_w;
+  int n, N, K;
+  bool fp8;              // kDecodeStore only
+  const float* scale_x;  // [n] (fp8)
+  const float* scale_w;  // [N] (fp8)
+  int mode;
+  bool whole_tiles;    // deal whole output tiles: K is summed in one piece, no partials or counters
+  bool early_weights;  // no kernel just before this one in the stream writes w
+  float* partials;         // decode_linear_partial_floats floats
+  unsigned int* counters;  // one per 128-row tile of W (64 outputs in the SwiGLU mode), zero before the launch
+  __nv_bfloat16* out;
+  long long ldo;
+  const __nv_bfloat16* residual;  // or null
+  long long ld_residual;
+  const __nv_bfloat16* bias;      // [N] or null (kDecodeQkv)
+  const float* cos;               // [table_rows, 64]
+  const float* sin;
+  const long long* positions;     // [n]
+  long long table_rows;
+  const long long* slots;         // [n] cache rows
+  __nv_bfloat16* cache_k;         // [cache_rows, hkv, 128]
+  __nv_bfloat16* cache_v;
+  long long cache_rows;
+  __nv_bfloat16* q_rows;          // [n * hq / hkv, hkv, 128]
+  int hq, hkv;
+  int sm_count;
+  uint32_t* err;
+};
+long long decode_linear_partial_floats(int n, int sm_count);
+void decode_linear(const DecodeLinearArgs& args, cudaStream_t stream);
+
 // ----------------------------------------------------------------- fused linear -> log-prob
 struct LinearLogpFwdArgs {
   const __nv_bfloat16* hidden;  // [n_tokens, hidden_dim]
@@ -272,6 +312,8 @@ void swiglu_packed_backward(const __nv_bfloat16* gu, long long ldgu, const __nv_
                             __nv_bfloat16* dgu, long long lddgu, long long rows, int F, cudaStream_t stream);
 // out[n, Hkv * rep * 128] = merge by log-sum-exp of two partial attention results o1 / o2 [n * rep, Hkv, 128] (bf16)
 // with l1 / l2 [Hkv, n * rep]; rows = n * rep.
+void attn_merge_parts(const __nv_bfloat16* o, const float* lse, __nv_bfloat16* out, int parts, long long rows, int hkv, int rep,
+                      cudaStream_t stream);
 void attn_merge2(const void* o1, const float* l1, const void* o2, const float* l2, void* out, long long rows, int hkv,
                  int rep, cudaStream_t stream);
 // table_rows: rows of the cos / sin tables (positions are checked against it in debug-bounds builds)
@@ -332,6 +374,7 @@ struct AttnFwdArgs {
   long long lse_head_stride;
   uint32_t* err;
   int sm_count = 148;  // CTAs of the persistent grid
+  bool dependent = false;  // programmatic dependent launch (decoding steps)
 };
 void attention_forward(const AttnFwdArgs& args, cudaStream_t stream);
 

@@ -105,6 +105,8 @@ __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
                         __nv_bfloat16* __restrict__ y, long long ldy, int D, float eps, float* __restrict__ rstd_out) {
   __shared__ float red[4];
+  grid_dep_wait();
+  grid_dep_launch();
   const long long row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
@@ -116,7 +118,7 @@ rmsnorm_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, cons
   for (int v = 0; v < kNormVecMax; ++v) {
     const int i = threadIdx.x + v * kNormThreads;
     if (i < n8) {
-      buf[v] = xr[i];
+      buf[v] = __ldcg(xr + i);
       const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&buf[v]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -446,7 +448,7 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const T*
 // chunk is written to its table row at once, the ends of runs that cross a chunk border go to fp32 partials (slot 2 c: the
 // run that came in from the left, 2 c + 1: the one that leaves to the right), which the second kernel adds in chunk
 // order.  So one id that fills half the batch (a padding id) is spread over the machine like any other rows: walked by
-// one CTA, 2000 rows of 4096 took 14 ms.
+// one CTA, 2000 rows of 4096 took 14 ms; 0.06 ms now.
 constexpr int kEmbChunk = 64;
 constexpr int kEmbThreads = 128;
 
@@ -766,6 +768,48 @@ __global__ void attn_merge2_kernel(const __nv_bfloat16* __restrict__ o1, const f
   }
 }
 
+// The same for `parts` partial results of one query set in one buffer: o [parts * rows, Hkv, 128] and
+// lse [Hkv, parts * rows], merged in part order.
+__global__ void attn_merge_parts_kernel(const __nv_bfloat16* __restrict__ o, const float* __restrict__ lse,
+                                        __nv_bfloat16* __restrict__ out, int parts, long long rows, int hkv, int rep) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const long long total = rows * hkv * 16;
+  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int v = static_cast<int>(idx & 15);
+    const long long rh = idx >> 4;
+    const int h = static_cast<int>(rh % hkv);
+    const long long r = rh / hkv;
+    const float* l = lse + h * parts * rows + r;
+    float top = -INFINITY;
+    for (int i = 0; i < parts; ++i) top = fmaxf(top, __ldcg(l + i * rows));
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, total_w = 0.f;
+    for (int i = 0; i < parts; ++i) {
+      const float w = top == -INFINITY ? 0.f : __expf(__ldcg(l + i * rows) - top);
+      total_w += w;
+      const uint4 q = __ldcg(reinterpret_cast<const uint4*>(o + ((i * rows + r) * hkv + h) * 128) + v);
+      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(p[j]);
+        if (w > 0.f) {
+          acc[2 * j] = fmaf(f.x, w, acc[2 * j]);
+          acc[2 * j + 1] = fmaf(f.y, w, acc[2 * j + 1]);
+        }
+      }
+    }
+    const float inv = total_w > 0.f ? 1.f / total_w : 0.f;
+    uint4 res;
+    __nv_bfloat162* pr = reinterpret_cast<__nv_bfloat162*>(&res);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pr[j] = __floats2bfloat162_rn(acc[2 * j] * inv, acc[2 * j + 1] * inv);
+    const long long seq = r / rep;
+    const int j = static_cast<int>(r - seq * rep);
+    reinterpret_cast<uint4*>(out + (seq * hkv * rep + static_cast<long long>(h) * rep + j) * 128)[v] = res;
+  }
+}
+
 inline int grid_for(long long total, int threads) {
   long long b = (total + threads - 1) / threads;
   const long long cap = 148LL * 16;
@@ -786,6 +830,12 @@ void rmsnorm_forward(const void* x, long long ldx, int x_dtype, const void* w, i
   if (rows <= 0) return;
   if (x_dtype == 1 && w_dtype == 1 && !out_fp32 && bf16_vec_ok(x, ldx, D) && bf16_vec_ok(y, ldy, D) &&
       bf16_vec_ok(w, 8, D)) {
+    if (rows <= 128) {  // a decoding step: its kernels are a few microseconds each, so launches overlap their predecessors
+      launch_dependent(rmsnorm_fwd_bf16_kernel, dim3(static_cast<unsigned>(rows)), dim3(kNormThreads), 0, stream,
+                       static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w),
+                       static_cast<__nv_bfloat16*>(y), ldy, D, eps, rstd);
+      return;
+    }
     rmsnorm_fwd_bf16_kernel<<<rows, kNormThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ldx,
                                                                static_cast<const __nv_bfloat16*>(w),
                                                                static_cast<__nv_bfloat16*>(y), ldy, D, eps, rstd);
@@ -896,6 +946,13 @@ void attn_merge2(const void* o1, const float* l1, const void* o2, const float* l
   attn_merge2_kernel<<<grid_for(rows * hkv * 16, 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(o1), l1, static_cast<const __nv_bfloat16*>(o2), l2,
       static_cast<__nv_bfloat16*>(out), rows, hkv, rep);
+}
+
+void attn_merge_parts(const __nv_bfloat16* o, const float* lse, __nv_bfloat16* out, int parts, long long rows, int hkv, int rep,
+                      cudaStream_t stream) {
+  if (rows <= 0) return;
+  launch_dependent(attn_merge_parts_kernel, dim3((static_cast<unsigned>(rows) * hkv * 16 + 127) / 128), dim3(128), 0, stream, o, lse,
+                   out, parts, rows, hkv, rep);
 }
 
 void rope_apply(const void* x, long long ldt, int dtype, const long long* pos, const float* cos_t, const float* sin_t,

@@ -1346,6 +1346,9 @@ std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor
   TORCH_CHECK(seqs.is_cuda() && seqs.scalar_type() == torch::kInt32 && seqs.is_contiguous() && seqs.dim() == 2 &&
                   seqs.size(1) == 8,
               "rl_engine.attention: seqs must be int32 [S, 8]");
+  // rows are read 16 bytes at a time; a table at an odd offset is copied
+  const Tensor seqs_a = reinterpret_cast<uintptr_t>(seqs.data_ptr()) % 16 == 0 ? seqs : seqs.clone();
+  const Tensor tiles_a = reinterpret_cast<uintptr_t>(tiles.data_ptr()) % 8 == 0 ? tiles : tiles.clone();
   TORCH_CHECK(tiles.is_cuda() && tiles.scalar_type() == torch::kInt32 && tiles.is_contiguous() && tiles.dim() == 2 &&
                   tiles.size(1) == 2,
               "rl_engine.attention: tiles must be int32 [n, 2]");
@@ -1364,10 +1367,10 @@ std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor
   a.total_kv = k.size(0);
   a.heads_q = static_cast<int>(q.size(1));
   a.heads_kv = static_cast<int>(k.size(1));
-  a.seqs = seqs.data_ptr<int>();
+  a.seqs = seqs_a.data_ptr<int>();
   a.num_seqs = static_cast<int>(seqs.size(0));
   a.sm_count = sm_count_of(q.get_device());
-  a.tiles = tiles.data_ptr<int>();
+  a.tiles = tiles_a.data_ptr<int>();
   a.num_tiles = static_cast<int>(tiles.size(0));
   a.causal = causal;
   a.softmax_scale = static_cast<float>(softmax_scale);
@@ -1379,6 +1382,169 @@ std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor
   rlk::attention_forward(a, stream_of(q));
   after_launch();
   return {out, lse};
+}
+
+// ------------------------------------------------------------------------------ decoding step
+namespace {
+
+// Fields shared by the decode projections.
+rlk::DecodeLinearArgs decode_args(const Tensor& x, const Tensor& w, const Tensor& partials, const Tensor& counters, int mode) {
+  check_rowmajor(x, "x");
+  check_rowmajor(w, "w");
+  TORCH_CHECK(x.scalar_type() == torch::kBFloat16 && w.scalar_type() == torch::kBFloat16, "rl_engine.decode_linear: bf16 operands only");
+  TORCH_CHECK(x.size(1) == w.size(1) && x.size(0) >= 1 && x.size(0) <= 128, "rl_engine.decode_linear: x must be [1..128, K]");
+  TORCH_CHECK(x.stride(0) % 8 == 0 && w.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 &&
+                  reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0,
+              "rl_engine.decode_linear: rows must be 16-byte aligned");
+  rlk::DecodeLinearArgs a{};
+  a.x = x.data_ptr();
+  a.w = w.data_ptr();
+  a.ld_x = x.stride(0);
+  a.ld_w = w.stride(0);
+  a.n = static_cast<int>(x.size(0));
+  a.N = static_cast<int>(w.size(0));
+  a.K = static_cast<int>(x.size(1));
+  a.mode = mode;
+  a.early_weights = true;
+  a.sm_count = sm_count_of(x.get_device());
+  TORCH_CHECK(partials.is_cuda() && partials.scalar_type() == torch::kFloat32 && partials.is_contiguous() &&
+                  partials.numel() >= rlk::decode_linear_partial_floats(a.n, a.sm_count) && reinterpret_cast<uintptr_t>(partials.data_ptr()) % 16 == 0,
+              "rl_engine.decode_linear: partials too small");
+  TORCH_CHECK(counters.is_cuda() && counters.scalar_type() == torch::kInt32 && counters.is_contiguous() &&
+                  counters.numel() >= (a.N + 127) / 128,
+              "rl_engine.decode_linear: one int32 counter per 128 rows of w");
+  a.partials = partials.data_ptr<float>();
+  a.counters = reinterpret_cast<unsigned int*>(counters.data_ptr<int>());
+  a.err = err_ptr(x);
+  return a;
+}
+
+}  // namespace
+
+int64_t decode_linear_partial_floats(int64_t n, int64_t device) {
+  return rlk::decode_linear_partial_floats(static_cast<int>(n), sm_count_of(static_cast<int>(device)));
+}
+
+// x W^T (+ residual), or silu(gate) * up of a packed [gate | up] weight.  counters: zeroed int32, one per 128 rows of w.
+Tensor decode_linear(const Tensor& x, const Tensor& w, bool swiglu, std::optional<Tensor> residual, const Tensor& partials,
+                     const Tensor& counters) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  rlk::DecodeLinearArgs a = decode_args(x, w, partials, counters, swiglu ? rlk::kDecodeSwiglu : rlk::kDecodeStore);
+  TORCH_CHECK(!swiglu || (a.N % 128 == 0 && !residual.has_value()), "rl_engine.decode_linear: SwiGLU needs 64 | F and no residual");
+  Tensor out = torch::empty({a.n, swiglu ? a.N / 2 : a.N}, x.options().dtype(torch::kBFloat16));
+  if (residual.has_value()) {
+    check_rowmajor(*residual, "residual");
+    TORCH_CHECK(residual->scalar_type() == torch::kBFloat16 && residual->sizes() == out.sizes(),
+                "rl_engine.decode_linear: residual must be bf16 of the output's shape");
+    a.residual = reinterpret_cast<const __nv_bfloat16*>(residual->data_ptr());
+    a.ld_residual = residual->stride(0);
+  }
+  a.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+  a.ldo = out.stride(0);
+  rlk::decode_linear(a, stream_of(x));
+  after_launch();
+  return out;
+}
+
+// The q / k / v projection of a decoding step: rotary embedding on q and k, k / v written to rows `slots` of the caches,
+// q returned as [n * hq / hkv, hkv, 128] (the query heads of a key / value head are rows).
+Tensor decode_qkv(const Tensor& x, const Tensor& w, std::optional<Tensor> bias, const Tensor& cos_t, const Tensor& sin_t,
+                  const Tensor& positions, const Tensor& slots, Tensor cache_k, Tensor cache_v, int64_t hq, const Tensor& partials,
+                  const Tensor& counters) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  rlk::DecodeLinearArgs a = decode_args(x, w, partials, counters, rlk::kDecodeQkv);
+  auto cache_ok = [&](const Tensor& c) {
+    return c.is_cuda() && c.scalar_type() == torch::kBFloat16 && c.is_contiguous() && c.dim() == 3 && c.size(2) == 128;
+  };
+  TORCH_CHECK(cache_ok(cache_k) && cache_ok(cache_v) && cache_k.sizes() == cache_v.sizes(),
+              "rl_engine.decode_qkv: caches must be contiguous bf16 [rows, kv heads, 128]");
+  const int64_t hkv = cache_k.size(1);
+  TORCH_CHECK(hkv > 0 && hq % hkv == 0 && a.N == (hq + 2 * hkv) * 128, "rl_engine.decode_qkv: w must be [(hq + 2 hkv) * 128, K]");
+  auto index_ok = [&](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == torch::kInt64 && t.is_contiguous() && t.numel() == a.n;
+  };
+  TORCH_CHECK(index_ok(positions) && index_ok(slots), "rl_engine.decode_qkv: positions and slots must be contiguous int64 [n]");
+  auto table_ok = [&](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.is_contiguous() && t.dim() == 2 && t.size(1) == 64;
+  };
+  TORCH_CHECK(table_ok(cos_t) && table_ok(sin_t) && cos_t.sizes() == sin_t.sizes(), "rl_engine.decode_qkv: cos / sin must be float32 [rows, 64]");
+  if (bias.has_value()) {
+    TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == torch::kBFloat16 && bias->is_contiguous() && bias->numel() == a.N,
+                "rl_engine.decode_qkv: bias must be contiguous bf16 [N]");
+    a.bias = reinterpret_cast<const __nv_bfloat16*>(bias->data_ptr());
+  }
+  Tensor q = torch::empty({a.n * hq / hkv, hkv, 128}, cache_k.options());
+  a.cos = cos_t.data_ptr<float>();
+  a.sin = sin_t.data_ptr<float>();
+  a.table_rows = cos_t.size(0);
+  a.positions = reinterpret_cast<const long long*>(positions.data_ptr<int64_t>());
+  a.slots = reinterpret_cast<const long long*>(slots.data_ptr<int64_t>());
+  a.cache_k = reinterpret_cast<__nv_bfloat16*>(cache_k.data_ptr());
+  a.cache_v = reinterpret_cast<__nv_bfloat16*>(cache_v.data_ptr());
+  a.cache_rows = cache_k.size(0);
+  a.q_rows = reinterpret_cast<__nv_bfloat16*>(q.data_ptr());
+  a.hq = static_cast<int>(hq);
+  a.hkv = static_cast<int>(hkv);
+  rlk::decode_linear(a, stream_of(x));
+  after_launch();
+  return q;
+}
+
+// Attention of a decoding step over `parts` disjoint key sets per query (seqs[:, 6] = part * rows) and their merge:
+// [rows / rep, hkv * rep * 128] in the model's head order.
+Tensor decode_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& seqs, const Tensor& tiles, int64_t parts,
+                        int64_t rep, double softmax_scale) {
+  auto check3 = [](const Tensor& t, const char* n) {
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 3 && t.size(2) == 128 && t.is_contiguous() &&
+                    reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0,
+                "rl_engine.decode_attention: ", n, " must be contiguous bf16 [rows, heads, 128]");
+  };
+  check3(q, "q");
+  check3(k, "k");
+  check3(v, "v");
+  TORCH_CHECK(k.sizes() == v.sizes() && q.size(1) == k.size(1), "rl_engine.decode_attention: q, k and v must have the same heads");
+  TORCH_CHECK(seqs.is_cuda() && seqs.scalar_type() == torch::kInt32 && seqs.is_contiguous() && seqs.dim() == 2 && seqs.size(1) == 8 &&
+                  tiles.is_cuda() && tiles.scalar_type() == torch::kInt32 && tiles.is_contiguous() && tiles.dim() == 2 &&
+                  tiles.size(1) == 2,
+              "rl_engine.decode_attention: seqs int32 [S, 8], tiles int32 [n, 2]");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(seqs.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(tiles.data_ptr()) % 8 == 0,
+              "rl_engine.decode_attention: tables must be 16-byte aligned");
+  const int64_t rows = q.size(0), hkv = q.size(1);
+  TORCH_CHECK(parts >= 1 && rep >= 1 && rows % rep == 0, "rl_engine.decode_attention: rows must be a multiple of rep");
+  const c10::cuda::CUDAGuard guard(q.device());
+  Tensor o = torch::empty({parts * rows, hkv, 128}, q.options());
+  Tensor lse = torch::empty({hkv, parts * rows}, q.options().dtype(torch::kFloat32));
+  Tensor out = torch::empty({rows / rep, hkv * rep * 128}, q.options());
+  if (rows == 0) return out;
+  rlk::AttnFwdArgs a{};
+  a.q = reinterpret_cast<const __nv_bfloat16*>(q.data_ptr());
+  a.k = reinterpret_cast<const __nv_bfloat16*>(k.data_ptr());
+  a.v = reinterpret_cast<const __nv_bfloat16*>(v.data_ptr());
+  a.ld_q = q.stride(0);
+  a.ld_k = k.stride(0);
+  a.ld_v = v.stride(0);
+  a.total_q = rows;
+  a.total_kv = k.size(0);
+  a.heads_q = a.heads_kv = static_cast<int>(hkv);
+  a.seqs = seqs.data_ptr<int>();
+  a.num_seqs = static_cast<int>(seqs.size(0));
+  a.sm_count = sm_count_of(q.get_device());
+  a.tiles = tiles.data_ptr<int>();
+  a.num_tiles = static_cast<int>(tiles.size(0));
+  a.causal = false;
+  a.softmax_scale = static_cast<float>(softmax_scale);
+  a.out = reinterpret_cast<__nv_bfloat16*>(o.data_ptr());
+  a.ld_out = o.stride(0);
+  a.lse = lse.data_ptr<float>();
+  a.lse_head_stride = parts * rows;
+  a.err = err_ptr(q);
+  a.dependent = true;
+  rlk::attention_forward(a, stream_of(q));
+  rlk::attn_merge_parts(reinterpret_cast<const __nv_bfloat16*>(o.data_ptr()), lse.data_ptr<float>(),
+                        reinterpret_cast<__nv_bfloat16*>(out.data_ptr()), static_cast<int>(parts), rows, static_cast<int>(hkv),
+                        static_cast<int>(rep), stream_of(q));
+  after_launch(2);
+  return out;
 }
 
 std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
@@ -1578,6 +1744,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention_bwd", rlk::traced("rlk::attention_bwd", &attention_bwd), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"),
         py::arg("dout"), py::arg("lse"), py::arg("seqs"), py::arg("q_tiles"), py::arg("kv_items"), py::arg("q_blocks"),
         py::arg("reduce_jobs"), py::arg("num_slots"), py::arg("causal"), py::arg("softmax_scale"), py::arg("packed") = false, py::arg("covered") = false);
+  m.def("decode_linear_partial_floats", rlk::traced("rlk::decode_linear_partial_floats", &decode_linear_partial_floats));
+  m.def("decode_linear", rlk::traced("rlk::decode_linear", &decode_linear));
+  m.def("decode_qkv", rlk::traced("rlk::decode_qkv", &decode_qkv));
+  m.def("decode_attention", rlk::traced("rlk::decode_attention", &decode_attention));
   m.def("error_state", rlk::traced("rlk::error_state", &error_state));
   m.def("reset_error", rlk::traced("rlk::reset_error", &reset_error));
   m.def("launch_count", rlk::traced("rlk::launch_count", &launch_count));

@@ -18,7 +18,7 @@ Head dim must be 128 and tensors bf16 for the kernel; other cases go to the PyTo
 from __future__ import annotations
 
 import math
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
@@ -37,6 +37,21 @@ class PackedLayout:
     tiles: torch.Tensor  # int32 [n_tiles, 2]: (sequence, first query row in the sequence)
     host_seqs: Tuple[Tuple[int, ...], ...]
     causal: bool
+    # of the own-keys layout of a decoding step: the same sequences and the shared prefix in one table
+    step: Optional["DecodeStepTables"] = None
+
+
+@dataclass(frozen=True)
+class DecodeStepTables:
+    """A decoding step's key ranges: the prefix cut into ``parts - 1`` ranges, each with all query rows, followed
+    by the completions' own sequences.  ``seqs[own_begin:]`` is the storage of the own layout's table, so a caller that
+    advances that table in place advances this one."""
+
+    seqs: torch.Tensor          # int32 [parts - 1 + n, 8]; column 6: first output row of the sequence's part
+    tiles: torch.Tensor         # int32 [n_tiles, 2] of all sequences
+    parts: int
+    own_begin: int
+    prefix: PackedLayout
 
 
 _LAYOUT_CACHE: Dict[Tuple, PackedLayout] = {}
@@ -66,6 +81,26 @@ def make_layout(seqs: Sequence[Sequence[int]], causal: bool, device) -> PackedLa
         _LAYOUT_CACHE.clear()
     _LAYOUT_CACHE[key] = layout
     return layout
+
+
+def decode_step_layouts(prefix: PackedLayout, own: PackedLayout, rows: int, prefix_len: int, kv_heads: int) -> PackedLayout:
+    """``own`` with a private table that is part of a ``DecodeStepTables`` for both layouts.
+
+    The prefix is cut so that its (range, 128-row query tile, head) items are about as many as the machine has SMs: one
+    item walks its key tiles one after the other, and 8 heads alone would keep 8 of 148 SMs busy.  More than 16 ranges
+    cost more in the merge than they save."""
+    dev = own.seqs.device
+    n_tiles, q_tiles = (prefix_len + TILE - 1) // TILE, (rows + TILE - 1) // TILE
+    ranges = max(1, min(n_tiles, 16, 148 // max(1, q_tiles * kv_heads)))
+    per = max(1, -(-n_tiles // ranges)) * TILE
+    starts = list(range(0, prefix_len, per))
+    seqs = [[0, rows, s, min(per, prefix_len - s), 0, 0, (i + 1) * rows, 0] for i, s in enumerate(starts)]
+    tiles = [[i, q0] for i in range(len(seqs)) for q0 in range(0, rows, TILE)]
+    own_begin = len(seqs)
+    tiles += [[own_begin + i, q0] for i, s in enumerate(own.host_seqs) for q0 in range(0, s[1], TILE)]
+    table = torch.cat([torch.tensor(seqs, dtype=torch.int32, device=dev).reshape(-1, 8), own.seqs])
+    step = DecodeStepTables(table, torch.tensor(tiles, dtype=torch.int32, device=dev).reshape(-1, 2), own_begin + 1, own_begin, prefix)
+    return replace(own, seqs=table[own_begin:], step=step)
 
 
 def grpo_group_layout(prompt_len: int, num_completions: int, completion_len: int, device, base: int = 0) -> PackedLayout:

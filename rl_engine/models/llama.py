@@ -684,7 +684,10 @@ class LlamaModel(nn.Module):
         hq, hkv = cfg.num_heads, cfg.num_kv_heads
         scale = 1.0 / math.sqrt(cfg.head_dim)
         n = token_ids.numel()
-        x = kernel_registry.get_op("embedding")(token_ids, self.view("embed"))
+        x = self.embed_tokens(token_ids)
+        step = self._decode_tables(n, positions, cache, slots, prefix_layout, self_layout)
+        if step is not None:
+            return self._decode_layers(x.reshape(n, -1), positions, cache, slots, step, scale)
         for i in range(cfg.num_layers):
             p = lambda name: self.view(f"l{i}.{name}")
             qkv = self._project(rms_norm(x, p("attn_norm"), cfg.rms_eps), f"l{i}.wqkv")
@@ -706,19 +709,67 @@ class LlamaModel(nn.Module):
             x = x + self._project(swiglu_packed(gu), f"l{i}.w_down")
         return rms_norm(x, self.view("final_norm"), cfg.rms_eps)
 
+    def _decode_tables(self, n, positions, cache, slots, prefix_layout, self_layout):
+        """The joint tables of ``decode_layouts`` if this call can run on the decode kernels (``_decode_layers``): up to
+        128 tokens, layouts that belong together, contiguous caches.  ``None``: the general kernels."""
+        cfg, step = self.cfg, getattr(self_layout, "step", None)
+        # (fp8 projections keep the general kernels: a code that rounds the other way moves a logit by percents, so their
+        # results are only comparable bit by bit)
+        if (step is None or not 1 <= n <= 128 or step.prefix is not prefix_layout or cfg.ffn_size % 64 or cfg.hidden_size % 8
+                or self._fp8_linears):
+            return None
+        own = step.seqs[step.own_begin:]
+        if self_layout.seqs.data_ptr() != own.data_ptr() or self_layout.seqs.shape != own.shape:
+            return None  # the caller has put another table in its place
+        shape = (cfg.num_kv_heads, cfg.head_dim)
+        for k, v in cache:
+            if not (k.is_contiguous() and v.is_contiguous() and k.dtype == v.dtype == torch.bfloat16 and k.dim() == 3
+                    and tuple(k.shape[1:]) == shape and k.shape == v.shape and k.is_cuda and v.is_cuda
+                    and k.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0):
+                return None
+        for t in (positions, slots):
+            if not (t.is_cuda and t.dtype == torch.long and t.is_contiguous() and t.numel() == n):
+                return None
+        return step
+
+    def _decode_layers(self, x, positions, cache, slots, step, scale):
+        """The layers of ``decode_step`` on the decode kernels: eight launches per layer, each weight streamed once by
+        all SMs; rotary embedding, cache write, residual add and SwiGLU are epilogues of the projections."""
+        from rl_engine.kernels.ops.base import require_ext
+
+        cfg, ext = self.cfg, require_ext()
+        n, rep = x.shape[0], cfg.num_heads // cfg.num_kv_heads
+        names = ("wqkv", "wo", "w_gate_up", "w_down")
+        tiles = [-(-self._shapes[f"l0.{name}"][0] // 128) for name in names]
+        partials = torch.empty(ext.decode_linear_partial_floats(n, x.get_device()), dtype=torch.float32, device=x.device)
+        counters = torch.zeros(cfg.num_layers * sum(tiles), dtype=torch.int32, device=x.device).split(tiles * cfg.num_layers)
+
+        def project(h, i, which, swiglu, residual):
+            return ext.decode_linear(h, self.view(f"l{i}.{names[which]}").detach(), swiglu, residual, partials,
+                                     counters[i * len(names) + which])
+
+        for i in range(cfg.num_layers):
+            p = lambda name: self.view(f"l{i}.{name}")
+            q = ext.decode_qkv(rms_norm(x, p("attn_norm"), cfg.rms_eps), p("wqkv").detach(), p("bqkv").detach() if cfg.qkv_bias else None,
+                               self.rope_cos, self.rope_sin, positions, slots, cache[i][0], cache[i][1], cfg.num_heads, partials,
+                               counters[i * len(names)])
+            attn = ext.decode_attention(q, cache[i][0], cache[i][1], step.seqs, step.tiles, step.parts, rep, scale)
+            x = project(attn, i, 1, False, x)
+            act = project(rms_norm(x, p("mlp_norm"), cfg.rms_eps), i, 2, True, None)
+            x = project(act, i, 3, False, x)
+        return rms_norm(x, self.view("final_norm"), cfg.rms_eps)
+
     def decode_layouts(self, n: int, prefix_len: int, rows_per_sequence: int, own_len: int = 1):
         """The two layouts of ``decode_step`` for ``n`` sequences whose cache rows are ``[prefix | n x rows_per_sequence]``
         when every sequence holds ``own_len`` tokens including the new one.  Column 5 of ``self_layout.seqs`` is that
         length: a caller that decodes step by step adds one to it in place (the tables are private copies)."""
-        from dataclasses import replace
-
-        from rl_engine.kernels.ops.sm100.attention import make_layout
+        from rl_engine.kernels.ops.sm100.attention import decode_step_layouts, make_layout
 
         dev = self.flat.device
         rep = self.cfg.num_heads // self.cfg.num_kv_heads
         prefix = make_layout([(0, n * rep, 0, prefix_len, 0, 0)], False, dev)
         own = make_layout([(i * rep, rep, 0, 0, prefix_len + i * rows_per_sequence, own_len) for i in range(n)], False, dev)
-        return prefix, replace(own, seqs=own.seqs.clone())
+        return prefix, decode_step_layouts(prefix, own, n * rep, prefix_len, self.cfg.num_kv_heads)
 
     def _project(self, x: torch.Tensor, name: str) -> torch.Tensor:
         """``x @ W[name].T`` for inference-only passes: the fp8 copy of the weight if ``enable_fp8_inference`` made one."""

@@ -89,6 +89,82 @@ def test_linear_logp_weight_gradient_in_one_and_several_chunks(n, chunk, v):
         assert _rel(got, want) < BF16
 
 
+# ------------------------------------------------------------------------------------------------ decoding step
+@pytest.mark.parametrize("n", [1, 16, 17, 33, 64, 128])
+@pytest.mark.parametrize("rows,k", [(128, 64), (200, 200), (2560, 1088), (12800, 320), (128 * 149, 136), (128 * 300 - 8, 72)])
+def test_decode_linear(n, rows, k):
+    """Equal K splits, ranges that ignore tile borders, a CTA per tile with two per SM, more tiles than that; ragged last tile,
+    k tail; residual add and SwiGLU epilogues."""
+    from rl_engine.kernels.ops.base import require_ext
+
+    ext = require_ext()
+    x, w = _randn(n, k, seed=n), _randn(rows, k, seed=rows, scale=k ** -0.5)
+    partials = torch.empty(ext.decode_linear_partial_floats(n, 0), device=DEV)
+    counters = lambda: torch.zeros(-(-rows // 128), dtype=torch.int32, device=DEV)
+    res = _randn(n, rows, seed=5)
+    y = x.double() @ w.double().t()
+    plain = ext.decode_linear(x, w, False, None, partials, counters())
+    assert _rel(plain, y) < BF16 / 2
+    assert torch.equal(plain, ext.decode_linear(x, w, False, None, partials, counters()))
+    assert _rel(ext.decode_linear(x, w, False, res, partials, counters()), y + res.double()) < BF16 / 2
+    if rows % 128 == 0:
+        gate, up = y[:, : rows // 2], y[:, rows // 2 :]
+        got = ext.decode_linear(x, w, True, None, partials, counters())
+        assert _rel(got, gate * torch.sigmoid(gate) * up) < BF16 / 2
+
+
+@pytest.mark.parametrize("m", [1, 17, 100, 128])
+@pytest.mark.parametrize("rows,k", [(200, 208), (4096, 4096), (128 * 149, 272), (128 * 300, 144)])
+def test_few_row_fp8_gemm_has_the_bits_of_the_tall_engines(m, rows, k):
+    from rl_engine.kernels.ops.sm100.gemm_fp8 import gemm_fp8, quantize_rows
+
+    (x, sx), (w, sw) = quantize_rows(_randn(300, k, seed=1)), quantize_rows(_randn(rows, k, seed=2))
+    full = gemm_fp8(x, sx, w, sw)
+    assert torch.equal(gemm_fp8(x[:m], sx[:m].contiguous(), w, sw), full[:m])
+
+
+@pytest.mark.parametrize("n,p,own,heads,kv,bias", [(1, 1, 1, 4, 2, False), (3, 300, 5, 8, 2, True), (40, 1500, 130, 8, 2, False),
+                                                   (128, 200, 3, 4, 4, False)])
+def test_decode_step_on_the_decode_kernels_matches_the_general_ones(n, p, own, heads, kv, bias):
+    """One prefix range and many, one query tile and several, own keys across a tile; the cache rows that are written are
+    the same up to one rounding.  Each route rounds about ten intermediate tensors per layer to bf16: 2 layers, 2^-8."""
+    from rl_engine.models.config import ModelConfig
+    from rl_engine.models.llama import LlamaModel
+
+    cfg = ModelConfig("decode", 512, 256, 2, heads, kv, 128, 448, qkv_bias=bias)
+    model = LlamaModel(cfg, dtype=torch.bfloat16, device=DEV, seed=3)
+    rows = own + 2
+    cache = model.new_kv_cache(p + n * rows)
+    for i, (k, v) in enumerate(cache):
+        k.copy_(_randn(*k.shape, seed=10 + i))
+        v.copy_(_randn(*v.shape, seed=20 + i))
+        if bias:
+            with torch.no_grad():
+                model.view(f"l{i}.bqkv").copy_(_randn(*model.view(f"l{i}.bqkv").shape, seed=30 + i, scale=0.1))
+    tokens = torch.randint(0, 512, (n,), device=DEV, generator=_gen(1))
+    positions = torch.full((n,), p + own - 1, dtype=torch.long, device=DEV)
+    slots = p + torch.arange(n, device=DEV) * rows + own - 1
+    prefix, layout = model.decode_layouts(n, p, rows, own)
+    other = [(k.clone(), v.clone()) for k, v in cache]
+    got = model.decode_step(tokens, positions, cache, slots, prefix, layout)
+    want = model.decode_step(tokens, positions, other, slots, prefix, replace(layout, step=None))
+    assert _rel(got, want) < 4 * BF16
+    for (k, v), (k2, v2) in zip(cache, other):
+        assert _rel(k, k2) < 4 * BF16 and _rel(v, v2) < 4 * BF16
+    layout.seqs[:, 5] += 1  # advanced in place by the caller: both tables follow
+    assert torch.equal(layout.step.seqs[layout.step.own_begin :, 5], layout.seqs[:, 5])
+
+
+@pytest.mark.parametrize("m", [1, 32, 100, 128])
+def test_wide_gemm_rows_have_the_same_bits_at_any_number_of_rows(m):
+    from rl_engine.kernels.ops.sm100.gemm import gemm
+
+    x, w = _randn(300, 200, seed=1), _randn(128 * 148 + 72, 200, seed=2, scale=0.1)
+    full = gemm(x, w)
+    assert torch.equal(gemm(x[:m], w), full[:m])
+    assert _rel(full, x.double() @ w.double().t()) < BF16 / 2
+
+
 # ------------------------------------------------------------------------------------------------ embedding gradient
 @pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 1000])
 @pytest.mark.parametrize("kind", ["one", "distinct", "few", "border"])
