@@ -195,8 +195,8 @@ struct GrpoRowsArgs {
   const long long* ids;
   const unsigned char* mask;
   const float* old_logp;
-  const double* adv;  // per sequence of `tokens` rows
-  long long rows, tokens;
+  const double* adv;  // [2, sequences] in 64 bits, and the 32-bit values; a sequence is `tokens` rows
+  long long rows, tokens, sequences;
   int V;
   float clip_lo, clip_hi;
   float *pl, *kl, *d_pl, *d_kl, *lse;  // [rows]

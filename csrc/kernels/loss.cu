@@ -13,8 +13,9 @@ namespace rlk {
 namespace {
 
 // ------------------------------------------------------------------------- group advantages
-// One warp per group (CSR bounds).  Population variance, clamped at eps^2 before the sqrt; in 64 bits, and returned so to the loss
-// over logits (a group's advantages sum to zero there, so each one's rounding would show).
+// One warp per group (CSR bounds).  Population variance, clamped at eps^2 before the sqrt.  The loss over logits takes them in 64
+// bits as well (a group's advantages sum to zero there, so each one's rounding would show): adv64[i], and the 32-bit value
+// at adv64[n_rewards + i].
 __global__ void group_adv_kernel(const float* __restrict__ rewards, const long long* __restrict__ bounds,
                                  int num_groups, long long uniform, float eps, float* __restrict__ adv,
                                  double* __restrict__ adv64,
@@ -28,22 +29,36 @@ __global__ void group_adv_kernel(const float* __restrict__ rewards, const long l
   if (!RLK_INDEX_OK(b0, n_rewards + 1, RLK_DBG_ERR, 640u, 1) || !RLK_INDEX_OK(b1, n_rewards + 1, RLK_DBG_ERR, 640u, 2) ||
       !RLK_INDEX_OK(b1 - b0, n_rewards + 1, RLK_DBG_ERR, 640u, 3))
     return;
-  double s = 0.0;
+  float s = 0.f, q = 0.f;
+  double s64 = 0.0;
   for (long long i = b0 + lane; i < b1; i += 32) {
-    s += rewards[i];
+    const float r = rewards[i];
+    s += r;
+    q = fmaf(r, r, q);
+    s64 += r;
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  const double n = static_cast<double>(b1 - b0), mean = s / n;
-  double q = 0.0;
-  for (long long i = b0 + lane; i < b1; i += 32) q += (rewards[i] - mean) * (rewards[i] - mean);
+  for (int off = 16; off > 0; off >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, off);
+    q += __shfl_xor_sync(0xffffffffu, q, off);
+    s64 += __shfl_xor_sync(0xffffffffu, s64, off);
+  }
+  const float n = static_cast<float>(b1 - b0);
+  const float mean = s / n;
+  const float var = fmaxf(q / n - mean * mean, eps * eps);
+  const float inv = 1.f / sqrtf(var);
+  if (adv)
+    for (long long i = b0 + lane; i < b1; i += 32) adv[i] = (rewards[i] - mean) * inv;
+  if (!adv64) return;
+  const double n64 = static_cast<double>(b1 - b0), mean64 = s64 / n64;
+  double q64 = 0.0;
+  for (long long i = b0 + lane; i < b1; i += 32) q64 += (rewards[i] - mean64) * (rewards[i] - mean64);
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) q += __shfl_xor_sync(0xffffffffu, q, off);
-  const double inv = 1.0 / sqrt(fmax(q / n, static_cast<double>(eps) * eps));
+  for (int off = 16; off > 0; off >>= 1) q64 += __shfl_xor_sync(0xffffffffu, q64, off);
+  const double inv64 = 1.0 / sqrt(fmax(q64 / n64, static_cast<double>(eps) * eps));
   for (long long i = b0 + lane; i < b1; i += 32) {
-    const double a = (rewards[i] - mean) * inv;
-    if (adv) adv[i] = static_cast<float>(a);
-    if (adv64) adv64[i] = a;
+    adv64[i] = (rewards[i] - mean64) * inv64;
+    adv64[n_rewards + i] = (rewards[i] - mean) * inv;
   }
 }
 

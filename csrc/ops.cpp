@@ -864,8 +864,8 @@ std::vector<Tensor> grpo_logits_fwd(const Tensor& policy, const Tensor& ref, con
   TORCH_CHECK(old_logp.is_cuda() && old_logp.scalar_type() == torch::kFloat32 && old_logp.is_contiguous() && old_logp.numel() == a.rows,
               "old_logps: float32 [rows]");
   TORCH_CHECK(tokens >= 1 && adv.is_cuda() && adv.scalar_type() == torch::kFloat64 && adv.is_contiguous() &&
-                  adv.numel() * tokens >= a.rows,
-              "advantages: float64, one per sequence");
+                  adv.dim() == 2 && adv.size(0) == 2 && adv.size(1) * tokens >= a.rows,
+              "advantages: float64 [2, sequences]");
   const c10::cuda::CUDAGuard guard(policy.device());
   auto fopt = policy.options().dtype(torch::kFloat32);
   Tensor rec = torch::empty({5, a.rows}, fopt), out4 = torch::empty({4}, fopt), partials = torch::empty({rlk::surrogate_partial_floats()}, fopt);
@@ -874,6 +874,7 @@ std::vector<Tensor> grpo_logits_fwd(const Tensor& policy, const Tensor& ref, con
   a.old_logp = old_logp.data_ptr<float>();
   a.adv = adv.data_ptr<double>();
   a.tokens = tokens;
+  a.sequences = adv.size(1);
   a.clip_lo = static_cast<float>(1.0 - clip_eps);
   a.clip_hi = static_cast<float>(1.0 + clip_eps);
   float* r = rec.data_ptr<float>();
@@ -916,7 +917,8 @@ Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int
   check_cuda(rewards, "rewards");
   TORCH_CHECK(rewards.scalar_type() == torch::kFloat32 && rewards.is_contiguous(), "rewards: contiguous float32");
   const c10::cuda::CUDAGuard guard(rewards.device());
-  Tensor adv = torch::empty_like(rewards, rewards.options().dtype(f64 ? torch::kFloat64 : torch::kFloat32));
+  // f64: [2, n], in 64 bits and the 32-bit values
+  Tensor adv = f64 ? torch::empty({2, rewards.numel()}, rewards.options().dtype(torch::kFloat64)) : torch::empty_like(rewards);
   const long long* bptr = nullptr;
   int64_t groups = 0;
   if (bounds.has_value() && bounds->defined()) {

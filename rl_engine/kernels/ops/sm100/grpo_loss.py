@@ -136,6 +136,11 @@ class FusedGRPOLossSM100Op:
                 policy_logits, ref_logits, action_ids, old_logps, sample_advantages, completion_mask,
                 clip_eps=clip_eps, beta=beta,
             )
+        adv = sample_advantages.detach().reshape(1, -1).double().expand(2, -1).contiguous()
+        return self._apply(policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps, beta)
+
+    def _apply(self, policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps, beta):
+        """``adv``: float64 ``[2, sequences]``, the advantages in 64 bits and their 32-bit values."""
         keep = completion_mask.to(torch.bool)
         v = policy_logits.shape[-1]
         rows = lambda t: t if t.stride(1) == 1 else t.contiguous()
@@ -148,7 +153,7 @@ class FusedGRPOLossSM100Op:
         copied.record(torch.cuda.current_stream(ids.device))
         out = _FromLogits.apply(
             rows(policy_logits.reshape(-1, v)), rows(ref_logits.detach().to(policy_logits.dtype).reshape(-1, v)), ids, mask,
-            old_logps.detach().reshape(-1).float().contiguous(), sample_advantages.detach().reshape(-1).double().contiguous(),
+            old_logps.detach().reshape(-1).float().contiguous(), adv,
             policy_logits.shape[-2] if policy_logits.ndim > 2 else 1, float(clip_eps), float(beta),
         )
         copied.synchronize()
@@ -176,7 +181,10 @@ class FusedGRPOLossSM100Op:
         *, clip_eps: float = 0.2, beta: float = 0.0, samples_per_prompt: Optional[int] = None,
         group_boundaries: Optional[Boundaries] = None, eps: float = 1e-6,
     ):
-        adv = self._group_advantages(rewards, samples_per_prompt, group_boundaries, eps, policy_logits.is_cuda)
+        both = policy_logits.is_cuda and rewards.is_cuda
+        adv = self._group_advantages(rewards, samples_per_prompt, group_boundaries, eps, both)
+        if both:
+            return self._apply(policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, float(clip_eps), float(beta))
         return self.apply(
             policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps=clip_eps, beta=beta
         )
