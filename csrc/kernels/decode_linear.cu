@@ -15,6 +15,8 @@
 // kernel) while this layer's tail drains.
 //
 //   warp 0     : TMA producer     warp 1 : tcgen05.mma issuer (128 x NT x 16)     warps 2..5 : epilogue, lane = output feature
+#include <algorithm>
+
 #include "../common/gemm_sm100.cuh"
 #include "../common/tensormap.h"
 #include "kernels.h"
@@ -27,17 +29,18 @@ constexpr uint32_t kKernelId = 120u;
 
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-template <int NT>
+// DEEP: the whole SM for one CTA.
+template <int NT, bool DEEP>
 struct DecSmem {
   static constexpr int kWBytes = 128 * 128;
   static constexpr int kXBytes = NT * 128;
   static constexpr int kStageBytes = kWBytes + kXBytes;
-  static constexpr int kStages = NT <= 32 ? 5 : (NT == 64 ? 4 : 3);
+  static constexpr int kStages = DEEP ? 200 * 1024 / kStageBytes : (NT <= 32 ? 5 : (NT == 64 ? 4 : 3));
   static constexpr int kXch = kStages * kStageBytes;            // float [kChunk][128]
   static constexpr int kBars = kXch + kChunk * 128 * 4;
   static constexpr int kBytes = kBars + (2 * kStages + 4) * 8 + 16;
   static constexpr int kDynamic = kBytes + 1024;
-  static_assert(kDynamic <= 113 * 1024, "two CTAs must fit an SM");
+  static_assert(kDynamic <= (DEEP ? 227 : 113) * 1024, "two CTAs must fit an SM, or one deep one");
 };
 
 // The (tile, k-block) units of CTA c: [c T / G, (c + 1) T / G), in units of `step` (one k-block, or a whole tile).
@@ -48,11 +51,11 @@ __device__ __forceinline__ int range_owner(long long total, long long unit, int 
   return static_cast<int>(((unit + 1) * grid - 1) / total);
 }
 
-template <int NT, int ELT, int MODE>
+template <int NT, int ELT, int MODE, bool DEEP>
 __global__ void __launch_bounds__(192)
 decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                      const __grid_constant__ DecodeLinearArgs p, const int tiles, const int k_blocks) {
-  using L = DecSmem<NT>;
+  using L = DecSmem<NT, DEEP>;
   constexpr int kElems = 128 / ELT;  // elements of one 128-byte k-block
   constexpr uint32_t kTmemCols = 2 * NT;
   extern __shared__ uint8_t smem_raw[];
@@ -372,21 +375,45 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   }
 }
 
-template <int NT, int ELT, int MODE>
-void launch(const DecodeLinearArgs& a, cudaStream_t stream) {
-  using L = DecSmem<NT>;
-  const int tiles = MODE == kDecodeSwiglu ? a.N / 128 : (a.N + 127) / 128;
-  const int k_blocks = (a.K * ELT + 127) / 128;
+// CTAs of a launch.  A tile cut between CTAs costs the last of them a round trip through memory (fence, counter, partials:
+// 5 us and more at the end of a 20 us layer), a CTA that holds two cut tiles pays it twice.  So:
+//   - up to two tiles per SM and no fewer than one: a CTA per tile, two to an SM; they share the memory's bandwidth evenly
+//     whether an SM holds one or two (gate / up projection of 32 tokens, 235 MB: 52 -> 45 us).
+//   - fewer: the largest number of equal K splits per tile that the SMs hold, if that uses three quarters of them (each
+//     CTA has one tile: 21 -> 19 and 20 -> 18 us for 50 and 34 MB); ranges that ignore the tile borders otherwise, because
+//     SMs left out cost more than the cut.  A step of four 4096-wide layers and a 128256-row head: 839 -> 792 us.
+int grid_of(int tiles, int k_blocks, bool whole_tiles, int sm_count) {
+  if (whole_tiles) return tiles <= 2 * sm_count ? tiles : sm_count;
+  if (tiles >= sm_count) return tiles <= 2 * sm_count ? tiles : sm_count;
+  const int splits = std::min(sm_count / tiles, k_blocks);
+  if (tiles * splits * 4 >= sm_count * 3 || splits == k_blocks) return tiles * splits;
+  return static_cast<int>(std::min<long long>(static_cast<long long>(tiles) * k_blocks, sm_count));
+}
+
+template <int NT, int ELT, int MODE, bool DEEP>
+void launch_as(const DecodeLinearArgs& a, int tiles, int k_blocks, int grid, cudaStream_t stream) {
+  using L = DecSmem<NT, DEEP>;
   const uint32_t w_box = MODE == kDecodeSwiglu ? 64 : 128;
   const CUtensorMap tw = ELT == 1 ? make_tmap_2d_u8(a.w, a.N, a.K, a.ld_w, w_box, 128)
                                   : make_tmap_2d_bf16(a.w, a.N, a.K, a.ld_w, w_box, 64);
   const CUtensorMap tx = ELT == 1 ? make_tmap_2d_u8(a.x, a.n, a.K, a.ld_x, NT, 128) : make_tmap_2d_bf16(a.x, a.n, a.K, a.ld_x, NT, 64);
-  auto kernel = decode_linear_kernel<NT, ELT, MODE>;
+  auto kernel = decode_linear_kernel<NT, ELT, MODE, DEEP>;
   static PerDeviceOnce configured;
   if (configured.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
-  const long long units = a.whole_tiles ? tiles : static_cast<long long>(tiles) * k_blocks;
-  launch_dependent(kernel, dim3(static_cast<unsigned>(units < a.sm_count ? units : a.sm_count)), dim3(192), L::kDynamic, stream, tw,
-                   tx, a, tiles, k_blocks);
+  launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(192), L::kDynamic, stream, tw, tx, a, tiles, k_blocks);
+}
+
+template <int NT, int ELT, int MODE>
+void launch(const DecodeLinearArgs& a, cudaStream_t stream) {
+  const int tiles = MODE == kDecodeSwiglu ? a.N / 128 : (a.N + 127) / 128;
+  const int k_blocks = (a.K * ELT + 127) / 128;
+  const int grid = grid_of(tiles, k_blocks, a.whole_tiles, a.sm_count);
+  if constexpr (ELT == 1) {
+    // Whole tiles of an 8-bit weight that leave SMs idle: each CTA keeps twice the bytes in flight, with the shared memory of
+    // the second CTA that its SM will not get (with three tokens, 16 projections 425 -> 400 us).
+    if (grid <= a.sm_count / 2) return launch_as<NT, ELT, MODE, true>(a, tiles, k_blocks, grid, stream);
+  }
+  launch_as<NT, ELT, MODE, false>(a, tiles, k_blocks, grid, stream);
 }
 
 template <int NT>
