@@ -195,8 +195,8 @@ struct GrpoRowsArgs {
   const long long* ids;
   const unsigned char* mask;
   const float* old_logp;
-  const double* adv;  // [2, sequences] in 64 bits, and the 32-bit values; a sequence is `tokens` rows
-  long long rows, tokens, sequences;
+  const float* adv;  // per sequence of `tokens` rows
+  long long rows, tokens;
   int V;
   float clip_lo, clip_hi;
   float *pl, *kl, *d_pl, *d_kl, *lse;  // [rows]
@@ -252,7 +252,7 @@ namespace rlk {
 // bounds == null -> uniform groups of `uniform` sequences.
 // n_rewards: length of ``rewards`` / ``adv`` (group bounds are checked against it in debug-bounds builds)
 void group_advantages(const float* rewards, const long long* bounds, int num_groups, long long uniform, float eps,
-                      float* adv, double* adv64, long long n_rewards, cudaStream_t stream);
+                      float* adv, long long n_rewards, cudaStream_t stream);
 
 struct SurrogateFwdArgs {
   const float* logp;      // [n] policy log-probs

@@ -426,26 +426,19 @@ __global__ void __launch_bounds__(kThreads) grpo_rows_kernel(const T* __restrict
   if (threadIdx.x != 0) return;
   long long t = a.ids[row];
   if (t < 0 || t >= a.V) t = 0;  // refused by the host
-  // The terms of the loss in 64 bits, one thread per row: log-probs are differences of numbers near 10, and their differences
-  // again (to the old and the reference log-prob) are what the loss is made of.
-  const double ln2 = 0.6931471805599453;
-  const double lp = static_cast<double>(to_f(prow[t])) - (static_cast<double>(p.m2) + log2(static_cast<double>(p.s))) * ln2;
-  const double lr = static_cast<double>(to_f(rrow[t])) - (static_cast<double>(r.m2) + log2(static_cast<double>(r.s))) * ln2;
-  const long long seq = row / a.tokens;
-  const double adv = a.adv[seq];
-  const float ratio = expf(static_cast<float>(lp - static_cast<double>(a.old_logp[row]))), d = static_cast<float>(lr - lp);
-  a.pl[row] = static_cast<float>(-fmin(ratio * adv, fminf(fmaxf(ratio, a.clip_lo), a.clip_hi) * adv));
-  a.kl[row] = expm1f(d) - d;
-  // The gradient's coefficients and its log-sum-exp in the 32-bit steps of the log-prob and surrogate kernels: a 16-bit
-  // gradient is mostly a few of its smallest steps, and one that rounds the other way is a tenth of its rms.
-  const float lse32 = (p.m2 + log2f(p.s)) * kLn2, lse_r32 = (r.m2 + log2f(r.s)) * kLn2;
-  const float lp32 = to_f(prow[t]) - lse32, lr32 = to_f(rrow[t]) - lse_r32;
-  const float adv32 = static_cast<float>(a.adv[a.sequences + seq]);
-  const float ratio32 = expf(lp32 - a.old_logp[row]);
-  const float unclipped = ratio32 * adv32, clipped = fminf(fmaxf(ratio32, a.clip_lo), a.clip_hi) * adv32;
+  // The steps of the log-prob and surrogate kernels, with their bits: the loss is a small difference of its terms, and a 16-bit
+  // gradient is mostly a few of its smallest steps, where one that rounds the other way is a tenth of its rms.
+  const float lse_p = (p.m2 + log2f(p.s)) * kLn2, lse_r = (r.m2 + log2f(r.s)) * kLn2;
+  const float lp = to_f(prow[t]) - lse_p, lr = to_f(rrow[t]) - lse_r;
+  const float adv = a.adv[row / a.tokens];
+  const float ratio = expf(lp - a.old_logp[row]);
+  const float unclipped = ratio * adv, clipped = fminf(fmaxf(ratio, a.clip_lo), a.clip_hi) * adv;
+  const float d = lr - lp, e = expf(d);
+  a.pl[row] = -fminf(unclipped, clipped);
+  a.kl[row] = e - d - 1.f;
   a.d_pl[row] = unclipped <= clipped ? -unclipped : 0.f;
-  a.d_kl[row] = 1.f - expf(lr32 - lp32);
-  a.lse[row] = lse32;
+  a.d_kl[row] = 1.f - e;
+  a.lse[row] = lse_p;
 }
 
 // flag = 1 if an unmasked id lies outside [0, V); one block, no initialisation needed

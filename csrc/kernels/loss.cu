@@ -13,12 +13,9 @@ namespace rlk {
 namespace {
 
 // ------------------------------------------------------------------------- group advantages
-// One warp per group (CSR bounds).  Population variance, clamped at eps^2 before the sqrt.  The loss over logits takes them in 64
-// bits as well (a group's advantages sum to zero there, so each one's rounding would show): adv64[i], and the 32-bit value
-// at adv64[n_rewards + i].
+// One warp per group (CSR bounds).  Population variance, clamped at eps^2 before the sqrt.
 __global__ void group_adv_kernel(const float* __restrict__ rewards, const long long* __restrict__ bounds,
                                  int num_groups, long long uniform, float eps, float* __restrict__ adv,
-                                 double* __restrict__ adv64,
                                  long long n_rewards RLK_DBG_PARAM) {
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -30,45 +27,28 @@ __global__ void group_adv_kernel(const float* __restrict__ rewards, const long l
       !RLK_INDEX_OK(b1 - b0, n_rewards + 1, RLK_DBG_ERR, 640u, 3))
     return;
   float s = 0.f, q = 0.f;
-  double s64 = 0.0;
   for (long long i = b0 + lane; i < b1; i += 32) {
     const float r = rewards[i];
     s += r;
     q = fmaf(r, r, q);
-    s64 += r;
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     s += __shfl_xor_sync(0xffffffffu, s, off);
     q += __shfl_xor_sync(0xffffffffu, q, off);
-    s64 += __shfl_xor_sync(0xffffffffu, s64, off);
   }
   const float n = static_cast<float>(b1 - b0);
   const float mean = s / n;
   const float var = fmaxf(q / n - mean * mean, eps * eps);
   const float inv = 1.f / sqrtf(var);
-  if (adv)
-    for (long long i = b0 + lane; i < b1; i += 32) adv[i] = (rewards[i] - mean) * inv;
-  if (!adv64) return;
-  const double n64 = static_cast<double>(b1 - b0), mean64 = s64 / n64;
-  double q64 = 0.0;
-  for (long long i = b0 + lane; i < b1; i += 32) q64 += (rewards[i] - mean64) * (rewards[i] - mean64);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) q64 += __shfl_xor_sync(0xffffffffu, q64, off);
-  const double inv64 = 1.0 / sqrt(fmax(q64 / n64, static_cast<double>(eps) * eps));
-  for (long long i = b0 + lane; i < b1; i += 32) {
-    adv64[i] = (rewards[i] - mean64) * inv64;
-    adv64[n_rewards + i] = (rewards[i] - mean) * inv;
-  }
+  for (long long i = b0 + lane; i < b1; i += 32) adv[i] = (rewards[i] - mean) * inv;
 }
 
 // ------------------------------------------------------------------- clipped surrogate + KL
 constexpr int kLossThreads = 256;
 constexpr int kLossBlocks = 256;  // fixed: the reduction tree does not depend on the input size
 
-// The mean of the surrogate is a small difference of large sums (advantages of a group sum to zero), so it is summed in 64 bits:
-// a few hundred additions, and no order of them shows in the result.
-__device__ __forceinline__ double3 block_sum3(double3 v, double3* smem) {
+__device__ __forceinline__ float3 block_sum3(float3 v, float3* smem) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
@@ -78,7 +58,7 @@ __device__ __forceinline__ double3 block_sum3(double3 v, double3* smem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) smem[warp] = v;
   __syncthreads();
-  double3 r = smem[0];
+  float3 r = smem[0];
   for (int w = 1; w < kLossThreads / 32; ++w) {
     r.x += smem[w].x;
     r.y += smem[w].y;
@@ -95,12 +75,12 @@ surrogate_fwd_kernel(const float* __restrict__ logp, const float* __restrict__ r
                      const float* __restrict__ old_logp, const float* __restrict__ adv_seq,
                      const float* __restrict__ adv_tok, const unsigned char* __restrict__ mask, long long n,
                      long long T, float clip_lo, float clip_hi, float* __restrict__ d_pl, float* __restrict__ d_kl,
-                     float* __restrict__ ratio_out, float* __restrict__ kl_out, double3* __restrict__ partials) {
-  __shared__ double3 red[kLossThreads / 32];
+                     float* __restrict__ ratio_out, float* __restrict__ kl_out, float3* __restrict__ partials) {
+  __shared__ float3 red[kLossThreads / 32];
   const long long per_block = (n + kLossBlocks - 1) / kLossBlocks;
   const long long begin = blockIdx.x * per_block;
   const long long end = begin + per_block < n ? begin + per_block : n;
-  double3 acc = make_double3(0.0, 0.0, 0.0);
+  float3 acc = make_float3(0.f, 0.f, 0.f);
   for (long long i = begin + threadIdx.x; i < end; i += kLossThreads) {
     float dpl = 0.f, dkl = 0.f, ratio = 1.f, kl = 0.f;
     if (mask[i]) {
@@ -120,7 +100,7 @@ surrogate_fwd_kernel(const float* __restrict__ logp, const float* __restrict__ r
       dkl = 1.f - e;
       acc.x += pl;
       acc.y += kl;
-      acc.z += 1.0;
+      acc.z += 1.f;
     }
     d_pl[i] = dpl;
     d_kl[i] = dkl;
@@ -131,29 +111,46 @@ surrogate_fwd_kernel(const float* __restrict__ logp, const float* __restrict__ r
   if (threadIdx.x == 0) partials[blockIdx.x] = acc;
 }
 
-// out = {loss, policy_loss, kl, count}; one thread per block partial, fixed tree
-static_assert(kLossBlocks == kLossThreads, "the finisher holds one partial per thread");
+// out = {loss, policy_loss, kl, count}.  The partials are added one after the other (the loss is a small difference of them, so its
+// bits are those of that order); they are fetched by all threads at once.
+static_assert(kLossBlocks == kLossThreads, "one partial per thread");
 __global__ void __launch_bounds__(kLossThreads)
-surrogate_finish_kernel(const double3* __restrict__ partials, float beta, float* __restrict__ out) {
-  __shared__ double3 red[kLossThreads / 32];
-  const double3 s = block_sum3(partials[threadIdx.x], red);
+surrogate_finish_kernel(const float3* __restrict__ partials, float beta, float* __restrict__ out) {
+  __shared__ float3 part[kLossBlocks];
+  part[threadIdx.x] = partials[threadIdx.x];
+  __syncthreads();
   if (threadIdx.x != 0) return;
-  const double denom = fmax(s.z, 1e-8);
-  out[0] = static_cast<float>((s.x + static_cast<double>(beta) * s.y) / denom);
-  out[1] = static_cast<float>(s.x / denom);
-  out[2] = static_cast<float>(s.y / denom);
-  out[3] = static_cast<float>(s.z);
+  float pl = 0.f, kl = 0.f, cnt = 0.f;
+#pragma unroll 8
+  for (int b = 0; b < kLossBlocks; ++b) {
+    pl += part[b].x;
+    kl += part[b].y;
+    cnt += part[b].z;
+  }
+  const float denom = fmaxf(cnt, 1e-8f);
+  const float policy_loss = pl / denom;
+  const float klm = kl / denom;
+  out[0] = policy_loss + beta * klm;
+  out[1] = policy_loss;
+  out[2] = klm;
+  out[3] = cnt;
 }
 
+// Sums of per-token terms that are there already, in the order of surrogate_fwd_kernel.
 __global__ void __launch_bounds__(kLossThreads)
 surrogate_reduce_kernel(const float* __restrict__ pl, const float* __restrict__ kl, const unsigned char* __restrict__ mask, long long n,
-                        double3* __restrict__ partials) {
-  __shared__ double3 red[kLossThreads / 32];
-  double3 acc = make_double3(0.0, 0.0, 0.0);
-  for (long long i = blockIdx.x * static_cast<long long>(kLossThreads) + threadIdx.x; i < n; i += kLossBlocks * kLossThreads) {
-    acc.x += pl[i];
-    acc.y += kl[i];
-    acc.z += mask[i] ? 1.0 : 0.0;
+                        float3* __restrict__ partials) {
+  __shared__ float3 red[kLossThreads / 32];
+  const long long per_block = (n + kLossBlocks - 1) / kLossBlocks;
+  const long long begin = blockIdx.x * per_block;
+  const long long end = begin + per_block < n ? begin + per_block : n;
+  float3 acc = make_float3(0.f, 0.f, 0.f);
+  for (long long i = begin + threadIdx.x; i < end; i += kLossThreads) {
+    if (mask[i]) {
+      acc.x += pl[i];
+      acc.y += kl[i];
+      acc.z += 1.f;
+    }
   }
   acc = block_sum3(acc, red);
   if (threadIdx.x == 0) partials[blockIdx.x] = acc;
@@ -206,27 +203,27 @@ __global__ void dpo_kernel(const float* __restrict__ pc, const float* __restrict
 }  // namespace
 
 void group_advantages(const float* rewards, const long long* bounds, int num_groups, long long uniform, float eps,
-                      float* adv, double* adv64, long long n_rewards, cudaStream_t stream) {
+                      float* adv, long long n_rewards, cudaStream_t stream) {
   if (num_groups <= 0) return;
   const int threads = 128;
   const int blocks = (num_groups * 32 + threads - 1) / threads;
-  group_adv_kernel<<<blocks, threads, 0, stream>>>(rewards, bounds, num_groups, uniform, eps, adv, adv64,
+  group_adv_kernel<<<blocks, threads, 0, stream>>>(rewards, bounds, num_groups, uniform, eps, adv,
                                                    n_rewards RLK_DBG_ARG);
 }
 
-int surrogate_partial_floats() { return kLossBlocks * 6; }
+int surrogate_partial_floats() { return kLossBlocks * 3; }
 
 void surrogate_forward(const SurrogateFwdArgs& a, cudaStream_t stream) {
   surrogate_fwd_kernel<<<kLossBlocks, kLossThreads, 0, stream>>>(
       a.logp, a.ref_logp, a.old_logp, a.adv_seq, a.adv_tok, a.mask, a.n, a.T, 1.f - a.clip_eps, 1.f + a.clip_eps,
-      a.d_pl, a.d_kl, a.ratio_out, a.kl_out, reinterpret_cast<double3*>(a.partials));
-  surrogate_finish_kernel<<<1, kLossThreads, 0, stream>>>(reinterpret_cast<const double3*>(a.partials), a.beta, a.out4);
+      a.d_pl, a.d_kl, a.ratio_out, a.kl_out, reinterpret_cast<float3*>(a.partials));
+  surrogate_finish_kernel<<<1, kLossThreads, 0, stream>>>(reinterpret_cast<const float3*>(a.partials), a.beta, a.out4);
 }
 
 void surrogate_reduce(const float* pl, const float* kl, const unsigned char* mask, long long n, float beta, float* partials, float* out4,
                       cudaStream_t stream) {
-  surrogate_reduce_kernel<<<kLossBlocks, kLossThreads, 0, stream>>>(pl, kl, mask, n, reinterpret_cast<double3*>(partials));
-  surrogate_finish_kernel<<<1, kLossThreads, 0, stream>>>(reinterpret_cast<const double3*>(partials), beta, out4);
+  surrogate_reduce_kernel<<<kLossBlocks, kLossThreads, 0, stream>>>(pl, kl, mask, n, reinterpret_cast<float3*>(partials));
+  surrogate_finish_kernel<<<1, kLossThreads, 0, stream>>>(reinterpret_cast<const float3*>(partials), beta, out4);
 }
 
 void surrogate_backward(const float* d_pl, const float* d_kl, const float* stats, const float* g3, float beta,

@@ -863,18 +863,17 @@ std::vector<Tensor> grpo_logits_fwd(const Tensor& policy, const Tensor& ref, con
   TORCH_CHECK(policy.scalar_type() == ref.scalar_type() && policy.sizes() == ref.sizes(), "policy/ref logits must match");
   TORCH_CHECK(old_logp.is_cuda() && old_logp.scalar_type() == torch::kFloat32 && old_logp.is_contiguous() && old_logp.numel() == a.rows,
               "old_logps: float32 [rows]");
-  TORCH_CHECK(tokens >= 1 && adv.is_cuda() && adv.scalar_type() == torch::kFloat64 && adv.is_contiguous() &&
-                  adv.dim() == 2 && adv.size(0) == 2 && adv.size(1) * tokens >= a.rows,
-              "advantages: float64 [2, sequences]");
+  TORCH_CHECK(tokens >= 1 && adv.is_cuda() && adv.scalar_type() == torch::kFloat32 && adv.is_contiguous() &&
+                  adv.numel() * tokens >= a.rows,
+              "advantages: float32, one per sequence");
   const c10::cuda::CUDAGuard guard(policy.device());
   auto fopt = policy.options().dtype(torch::kFloat32);
   Tensor rec = torch::empty({5, a.rows}, fopt), out4 = torch::empty({4}, fopt), partials = torch::empty({rlk::surrogate_partial_floats()}, fopt);
   a.ref = ref.data_ptr();
   a.ld_ref = ref.stride(0);
   a.old_logp = old_logp.data_ptr<float>();
-  a.adv = adv.data_ptr<double>();
+  a.adv = adv.data_ptr<float>();
   a.tokens = tokens;
-  a.sequences = adv.size(1);
   a.clip_lo = static_cast<float>(1.0 - clip_eps);
   a.clip_hi = static_cast<float>(1.0 + clip_eps);
   float* r = rec.data_ptr<float>();
@@ -913,12 +912,11 @@ Tensor grpo_logits_bwd(const Tensor& policy, const Tensor& ids, const Tensor& ma
   return grad;
 }
 
-Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int64_t uniform, double eps, bool f64) {
+Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int64_t uniform, double eps) {
   check_cuda(rewards, "rewards");
   TORCH_CHECK(rewards.scalar_type() == torch::kFloat32 && rewards.is_contiguous(), "rewards: contiguous float32");
   const c10::cuda::CUDAGuard guard(rewards.device());
-  // f64: [2, n], in 64 bits and the 32-bit values
-  Tensor adv = f64 ? torch::empty({2, rewards.numel()}, rewards.options().dtype(torch::kFloat64)) : torch::empty_like(rewards);
+  Tensor adv = torch::empty_like(rewards);
   const long long* bptr = nullptr;
   int64_t groups = 0;
   if (bounds.has_value() && bounds->defined()) {
@@ -931,8 +929,7 @@ Tensor group_advantages(const Tensor& rewards, std::optional<Tensor> bounds, int
   }
   if (groups > 0) {
     rlk::group_advantages(rewards.data_ptr<float>(), bptr, static_cast<int>(groups), uniform, static_cast<float>(eps),
-                          f64 ? nullptr : adv.data_ptr<float>(), f64 ? adv.data_ptr<double>() : nullptr, rewards.numel(),
-                          stream_of(rewards));
+                          adv.data_ptr<float>(), rewards.numel(), stream_of(rewards));
     after_launch();
   }
   return adv;
@@ -1717,8 +1714,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ids_outside", rlk::traced("rlk::ids_outside", &ids_outside));
   m.def("grpo_logits_fwd", rlk::traced("rlk::grpo_logits_fwd", &grpo_logits_fwd));
   m.def("grpo_logits_bwd", rlk::traced("rlk::grpo_logits_bwd", &grpo_logits_bwd));
-  m.def("group_advantages", rlk::traced("rlk::group_advantages", &group_advantages), py::arg("rewards"), py::arg("bounds"),
-        py::arg("uniform"), py::arg("eps"), py::arg("f64") = false);
+  m.def("group_advantages", rlk::traced("rlk::group_advantages", &group_advantages));
   m.def("surrogate_fwd", rlk::traced("rlk::surrogate_fwd", &surrogate_fwd));
   m.def("surrogate_bwd", rlk::traced("rlk::surrogate_bwd", &surrogate_bwd));
   m.def("dpo_fwd", rlk::traced("rlk::dpo_fwd", &dpo_fwd));

@@ -96,9 +96,6 @@ class FusedGRPOLossSM100Op:
         self, rewards: torch.Tensor, *, samples_per_prompt: Optional[int] = None,
         group_boundaries: Optional[Boundaries] = None, eps: float = 1e-6,
     ) -> torch.Tensor:
-        return self._group_advantages(rewards, samples_per_prompt, group_boundaries, eps)
-
-    def _group_advantages(self, rewards, samples_per_prompt, group_boundaries, eps, f64: bool = False) -> torch.Tensor:
         if not rewards.is_cuda:
             return self._native.group_advantages(
                 rewards, samples_per_prompt=samples_per_prompt, group_boundaries=group_boundaries, eps=eps
@@ -114,7 +111,7 @@ class FusedGRPOLossSM100Op:
                 raise ValueError(
                     f"num_sequences ({n}) must be divisible by samples_per_prompt ({samples_per_prompt})."
                 )
-            return require_ext().group_advantages(flat, None, int(samples_per_prompt), float(eps), f64)
+            return require_ext().group_advantages(flat, None, int(samples_per_prompt), float(eps))
         host = torch.as_tensor(group_boundaries, dtype=torch.long).cpu()
         if host.ndim != 1 or host.numel() < 2:
             raise ValueError("group_boundaries must be a 1D tensor of length num_groups + 1.")
@@ -123,7 +120,7 @@ class FusedGRPOLossSM100Op:
             raise ValueError(f"group sizes sum to {int(sizes.sum())} but there are {n} sequences.")
         if bool((sizes < 1).any()):
             raise ValueError("each group must contain at least one sequence.")
-        return require_ext().group_advantages(flat, host.to(flat.device), 0, float(eps), f64)
+        return require_ext().group_advantages(flat, host.to(flat.device), 0, float(eps))
 
     expand_advantages = staticmethod(NativeGRPOLossOp.expand_advantages)
 
@@ -136,11 +133,6 @@ class FusedGRPOLossSM100Op:
                 policy_logits, ref_logits, action_ids, old_logps, sample_advantages, completion_mask,
                 clip_eps=clip_eps, beta=beta,
             )
-        adv = sample_advantages.detach().reshape(1, -1).double().expand(2, -1).contiguous()
-        return self._apply(policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps, beta)
-
-    def _apply(self, policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps, beta):
-        """``adv``: float64 ``[2, sequences]``, the advantages in 64 bits and their 32-bit values."""
         keep = completion_mask.to(torch.bool)
         v = policy_logits.shape[-1]
         rows = lambda t: t if t.stride(1) == 1 else t.contiguous()
@@ -153,7 +145,7 @@ class FusedGRPOLossSM100Op:
         copied.record(torch.cuda.current_stream(ids.device))
         out = _FromLogits.apply(
             rows(policy_logits.reshape(-1, v)), rows(ref_logits.detach().to(policy_logits.dtype).reshape(-1, v)), ids, mask,
-            old_logps.detach().reshape(-1).float().contiguous(), adv,
+            old_logps.detach().reshape(-1).float().contiguous(), sample_advantages.detach().reshape(-1).float().contiguous(),
             policy_logits.shape[-2] if policy_logits.ndim > 2 else 1, float(clip_eps), float(beta),
         )
         copied.synchronize()
@@ -181,10 +173,9 @@ class FusedGRPOLossSM100Op:
         *, clip_eps: float = 0.2, beta: float = 0.0, samples_per_prompt: Optional[int] = None,
         group_boundaries: Optional[Boundaries] = None, eps: float = 1e-6,
     ):
-        both = policy_logits.is_cuda and rewards.is_cuda
-        adv = self._group_advantages(rewards, samples_per_prompt, group_boundaries, eps, both)
-        if both:
-            return self._apply(policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, float(clip_eps), float(beta))
+        adv = self.group_advantages(
+            rewards, samples_per_prompt=samples_per_prompt, group_boundaries=group_boundaries, eps=eps
+        )
         return self.apply(
             policy_logits, ref_logits, action_ids, old_logps, adv, completion_mask, clip_eps=clip_eps, beta=beta
         )
