@@ -212,8 +212,12 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
       }
     };
     uint32_t best[kUnroll] = {0u, 0u, 0u, 0u};  // smaller than the key of any number
-    const bool few = k <= kFewLimit;
-    const int sample = few ? min(v1 - v0, max((v1 - v0) / kSampleShare, kMinSample / kVec)) : v1 - v0;
+    // In a cluster every CTA lets about k x (slice / sample) candidates through, and what all of them send has to fit the
+    // first one's sort buffer: 200 of 77420 in four slices overflowed it (43 us instead of 22 through the exact radix select).
+    const int part_sample = min(v1 - v0, max((v1 - v0) / kSampleShare, kMinSample / kVec));
+    const bool few = k <= kFewLimit &&
+                     (parts == 1 || static_cast<long long>(k) * parts * (v1 - v0) <= static_cast<long long>(kCap) * 3 / 4 * part_sample);
+    const int sample = few ? part_sample : v1 - v0;
     sweep(v0 + sample, [&](const uint4& q, int, int u) {
       const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
@@ -852,10 +856,12 @@ void sample_nucleus(const void* logits, long long ld, int dtype, int rows, int V
 namespace {
 
 // CTAs per row: enough for two on every SM, at most eight (the portable cluster size), and slices of at least twice the
-// smallest sample: below that the merge is not repaid.
-int sample_parts(int rows, int V) {
+// smallest sample: below that the merge is not repaid.  No more than leave room for k x 3 / 2 candidates of each in the first
+// one's sort buffer.
+int sample_parts(int rows, int V, int k) {
   int parts = 1;
   while (parts < 8 && static_cast<long long>(rows) * parts * 2 <= 296 && V / (parts * 2) >= 2 * kMinSample) parts *= 2;
+  while (parts > 1 && static_cast<long long>(parts) * k * 3 > 2 * kCap) parts /= 2;
   return parts;
 }
 
@@ -866,7 +872,7 @@ void launch_sample(const void* logits, long long ld, int rows, int V, int top_k,
   constexpr int kBytes = kGather * 8;
   static PerDeviceOnce configured;
   if (configured.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-  const int parts = sample_parts(rows, V);
+  const int parts = sample_parts(rows, V, top_k);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * parts);
   cfg.blockDim = dim3(kThreads);
