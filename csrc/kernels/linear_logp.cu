@@ -28,9 +28,10 @@ constexpr int kLogpStages = 4;
 constexpr int kLogpPairStages = 6;    // CTA-pair engine, statistics epilogue (no staging)
 constexpr int kLogpPairStagesDz = 5;  // CTA-pair engine with the 64 KB dz staging tile
 constexpr int kMaxWorld = 8;
-// Vocab tiles per record: a constant, so that a row's merge order depends neither on the other rows of the batch nor on the
-// engine or the length of the work items.
-constexpr int kTilesPerRecord = 2;
+// Vocab tiles per record (8192 columns), which is also one work item: a constant, so that the order of a row's sums depends
+// neither on the other rows of the batch nor on the engine.  It is part of the numbers that a training run sees: the last bit
+// of a log-sum-exp moves the rounding of a bf16 gradient, and with it what a run of many steps arrives at.
+constexpr int kTilesPerRecord = 32;
 
 struct LogpFwdParams {
   const long long* target;  // [N] global vocab ids
@@ -64,14 +65,11 @@ struct EpiLogpStats {
     int tgt;  // local target column or -1
   };
 
-  __device__ static void clear(State& st) {
+  __device__ static void begin_item(State& st, const Params& ep, const GemmProblem& p, const WorkItem&, int row) {
     st.m2 = -INFINITY;
     st.s = 0.f;
     st.t = 0.f;
     st.zt = 0.f;
-  }
-  __device__ static void begin_item(State& st, const Params& ep, const GemmProblem& p, const WorkItem&, int row) {
-    clear(st);
     st.tgt = -1;
     if (row < p.M) {
       const long long local = ep.target[row] - ep.vocab_start;
@@ -80,7 +78,7 @@ struct EpiLogpStats {
   }
 
   template <int BN>
-  __device__ static void tile(State& st, const Params& ep, const GemmProblem& p, uint32_t acc, int row, int n0) {
+  __device__ static void tile(State& st, const Params& ep, const GemmProblem& p, uint32_t acc, int /*row*/, int n0) {
 #pragma unroll 1
     for (int c = 0; c < BN; c += 32) {
       uint32_t r[32];
@@ -133,23 +131,15 @@ struct EpiLogpStats {
           if (j == tl) st.zt = v[j];
       }
     }
-    // a record is complete every kTilesPerRecord tiles, whatever the length of the item
-    const int nt = n0 / BN;
-    if ((nt + 1) % kTilesPerRecord == 0 || nt + 1 == p.tiles_n) {
-      if ((row >> 7) < ep.row_tiles) {
-        const float4 rec = make_float4(st.m2, st.s, st.t, st.zt);
-        const size_t slot = static_cast<size_t>(ep.slot_base + nt / kTilesPerRecord) * ep.n_pad + row;
-        for (int r = 0; r < ep.world; ++r) ep.peer_partials[r][slot] = rec;
-      }
-      clear(st);
-    }
   }
 
   // `row` >> 7 is this CTA's 128-row tile under both engines (the pair engine's M-tiles hold two of them).
   __device__ static void end_item(State& st, const Params& ep, const GemmProblem& p, const WorkItem& w, int row) {
     const int t128 = row >> 7;
     if (t128 >= ep.row_tiles) return;  // second half of the last pair: no rows (uniform over the CTA)
-    const unsigned int records = (w.n_end - w.n_begin + kTilesPerRecord - 1) / kTilesPerRecord;
+    const float4 rec = make_float4(st.m2, st.s, st.t, st.zt);
+    const size_t slot = static_cast<size_t>(ep.slot_base + w.split) * ep.n_pad + row;
+    for (int r = 0; r < ep.world; ++r) ep.peer_partials[r][slot] = rec;
     if (ep.world == 1) {
       // One GPU: whoever delivers the last record of a row tile merges it at once.  Nobody waits, so the kernel does
       // not depend on all its CTAs being resident together, and the merges overlap other tiles' products.
@@ -160,9 +150,9 @@ struct EpiLogpStats {
         unsigned int old;
         asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
                      : "=r"(old)
-                     : "l"(ep.peer_counters[0] + t128), "r"(records)
+                     : "l"(ep.peer_counters[0] + t128), "r"(1u)
                      : "memory");
-        s_last = old + records == static_cast<unsigned int>(ep.total_records) ? 1u : 0u;
+        s_last = old + 1u == static_cast<unsigned int>(ep.total_records) ? 1u : 0u;
         if (s_last) ep.peer_counters[0][t128] = 0u;  // the same set may be counted in again (a replayed CUDA graph)
       }
       epi_bar_sync();
@@ -173,7 +163,7 @@ struct EpiLogpStats {
     epi_bar_sync();
     if (threadIdx.x == 64) {  // one epilogue thread publishes the arrival
       for (int r = 0; r < ep.world; ++r) {
-        asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(ep.peer_counters[r] + t128), "r"(records)
+        asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(ep.peer_counters[r] + t128), "r"(1u)
                      : "memory");
       }
     }
@@ -181,37 +171,24 @@ struct EpiLogpStats {
 
   static constexpr uint32_t kMergeKernelId = 101u;
 
-  // Fixed (rank, split) order, eight records per step: their loads are in flight together and the running sums are
-  // rescaled once per step.  A row's value depends on its records only, not on the engine or the other rows.
+  // Fixed (rank, split) order: the maximum of all records, then the sums one record after the other against it.  A row's
+  // value depends on its records only, not on the engine or the other rows.  Eight records' loads are in flight together.
   __device__ static void merge_row(const Params& ep, const GemmProblem& p, int row, uint32_t kernel_id) {
     if (row >= p.M) return;
     const float4* parts = ep.peer_partials[ep.rank] + row;
     const int records = ep.total_records;
     float M2 = -INFINITY, S = 0.f, T = 0.f, ZT = 0.f;
-    constexpr int kStep = 8;
-    for (int i = 0; i < records; i += kStep) {
-      float4 rec[kStep];
-#pragma unroll
-      for (int j = 0; j < kStep; ++j) {
-        // plain (not read-only-cached) loads: other SMs and peers wrote these during this launch
-        rec[j] = i + j < records ? __ldcg(parts + static_cast<size_t>(i + j) * ep.n_pad)
-                                 : make_float4(-INFINITY, 0.f, 0.f, 0.f);
-      }
-      float top = M2;
-#pragma unroll
-      for (int j = 0; j < kStep; ++j) top = fmaxf(top, rec[j].x);
-      const float base = top == -INFINITY ? 0.f : top;
-      const float keep = fast_exp2(M2 - base);
-      S *= keep;
-      T *= keep;
-      M2 = top;
-#pragma unroll
-      for (int j = 0; j < kStep; ++j) {
-        const float w = fast_exp2(rec[j].x - base);
-        S = fmaf(rec[j].y, w, S);
-        T = fmaf(rec[j].z, w, T);
-        ZT += rec[j].w;
-      }
+    // not through the read-only cache: other SMs and peers wrote these during this launch
+#pragma unroll 8
+    for (int i = 0; i < records; ++i) M2 = fmaxf(M2, __ldcg(&parts[static_cast<size_t>(i) * ep.n_pad].x));
+    const float base = M2 == -INFINITY ? 0.f : M2;
+#pragma unroll 8
+    for (int i = 0; i < records; ++i) {
+      const float4 rec = __ldcg(parts + static_cast<size_t>(i) * ep.n_pad);
+      const float w = fast_exp2(rec.x - base);
+      S = fmaf(rec.y, w, S);
+      T = fmaf(rec.z, w, T);
+      ZT += rec.w;
     }
     const float lse = (M2 + log2f(S)) * kLn2;
     if (ep.global_vocab > 0) {
@@ -430,14 +407,6 @@ void linear_logp_workspace_shape(int n_tokens, int v_local, int world, int* item
 
 namespace {
 
-// Records per work item.  One keeps every SM busy on short batches: 777 tokens over 50257 columns are 7 x 99 items for 148
-// SMs, where the 8192 columns an item had at first gave 7 x 7.  Each item ends with a fence and an atomic, which at short
-// contractions (512) cost a tenth of a one-record item, so long batches take up to 16 as long as eight rounds of items remain.
-int records_per_item(long long row_tiles, int records, int units) {
-  const long long r = row_tiles * records / (8ll * units);
-  return static_cast<int>(r < 1 ? 1 : (r > 16 ? 16 : r));
-}
-
 GemmProblem pair_problem(int M, int N, int K, int tiles_per_item) {
   GemmProblem p = make_gemm_problem(M, N, K, kLogpBN, tiles_per_item, 1);
   p.tiles_m = (M + kPairBM - 1) / kPairBM;
@@ -461,9 +430,8 @@ bool pair_is_better(int M, int items_per_m, int sm_count) {
 void linear_logp_forward(const LinearLogpFwdArgs& a, cudaStream_t stream) {
   const int row_tiles = (a.n_tokens + kBM - 1) / kBM;
   const int records = ((a.v_local + kLogpBN - 1) / kLogpBN + kTilesPerRecord - 1) / kTilesPerRecord;
-  const int per_item = kTilesPerRecord * (a.world == 1 ? records_per_item(row_tiles, records, a.sm_count) : 1);
   // keep as many token tiles per group as stay L2-resident, so the weight streams from DRAM once per group
-  GemmProblem p = make_gemm_problem(a.n_tokens, a.v_local, a.hidden_dim, kLogpBN, per_item,
+  GemmProblem p = make_gemm_problem(a.n_tokens, a.v_local, a.hidden_dim, kLogpBN, kTilesPerRecord,
                                     raster_group_m(row_tiles, a.hidden_dim, 16, 64ll << 20));
   const CUtensorMap ta = make_tmap_2d_bf16(a.hidden, a.n_tokens, a.hidden_dim, a.ld_hidden, kBM, kBK);
   LogpFwdParams ep;
@@ -490,7 +458,7 @@ void linear_logp_forward(const LinearLogpFwdArgs& a, cudaStream_t stream) {
   ep.wait_limit_ns = a.wait_limit_ns ? a.wait_limit_ns : kWaitLimitNs;
   // Tensor parallelism stays on single CTAs: its merge waits for other CTAs' records, so all must be resident.
   if (a.world == 1 && pair_is_better(a.n_tokens, p.items_per_m, a.sm_count)) {
-    p = pair_problem(a.n_tokens, a.v_local, a.hidden_dim, per_item);
+    p = pair_problem(a.n_tokens, a.v_local, a.hidden_dim, kTilesPerRecord);
     const CUtensorMap tb = make_tmap_2d_bf16(a.weight, a.v_local, a.hidden_dim, a.ld_weight, kLogpBN / 2, kBK);
     constexpr auto kernel = gemm_pair_sm100_kernel<kLogpBN, false, false, kLogpPairStages, EpiLogpStatsWithMerge>;
     using L = PairSmem<kLogpBN, kLogpPairStages>;
