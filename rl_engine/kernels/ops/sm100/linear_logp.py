@@ -9,8 +9,9 @@ vocab_start_index=0, global_vocab_size=None)`` returning float32 log-probs shape
   combine kernel and, under tensor parallelism, three NCCL all-reduces);
 * backward never calls a library GEMM: per token chunk a recompute kernel writes
   ``dz = g * (onehot - softmax)`` as bf16 into a chunk workspace, then two tcgen05 GEMMs form
-  ``grad_hidden`` and accumulate ``grad_weight`` in fp32 in fixed chunk order (one chunk stores it
-  as bf16 directly).  Extra memory is bounded by ``chunk * V`` bf16 plus one fp32 ``grad_weight``;
+  ``grad_hidden`` and accumulate ``grad_weight`` in fp32 in fixed chunk order (a batch of one
+  chunk stores it as bf16 directly).  Extra memory is constant in the number of tokens: ``chunk * V`` bf16 plus one fp32
+  ``grad_weight``;
 * ``with_entropy`` also returns the softmax entropy per token from the same sweep.
 
 Inputs must be bf16 on a CUDA device for the fused path; anything else goes to the PyTorch oracle.
@@ -100,20 +101,12 @@ def _dz_workspace(device: torch.device, chunk: int, v_local: int) -> torch.Tenso
     return buf
 
 
-def backward_chunk(n: int, d: int, chunk_tokens: int, need_weight: bool) -> int:
-    """Rows of dz formed at once.  One chunk needs no fp32 ``grad_weight`` (4 V D bytes) beside its dz, so with the
-    memory of ``chunk_tokens`` rows and that buffer, ``chunk_tokens + 2 D`` rows fit in one piece; longer batches go
-    ``chunk_tokens`` at a time."""
-    chunk = max(128, chunk_tokens)
-    if need_weight and n <= chunk + 2 * d:
-        chunk = max(chunk, n)
-    return min(chunk, (n + 127) // 128 * 128)
-
-
 def accumulate_grad_weight(ext, dz, h2, grad_w, first: bool, last: bool, dtype, sink=None):
     """``grad_w`` of a chunk onto the sum of the earlier ones: the first chunk writes, later ones add in fp32, the last one
     rounds to ``dtype`` as it stores.  No zero-fill and no conversion pass over ``[V, D]``.  ``sink``: a gradient buffer that the
-    only chunk adds to."""
+    only chunk adds to.  The chunks' products are formed apart
+    and added in order, also where one contraction over all tokens would fit: its sums would round elsewhere, and a training
+    run's numbers with them (8192 tokens, forward and backward: 27.0 ms in one piece, 27.4 ms in two)."""
     if sink is not None and first and last:
         return ext.gemm(dz, h2, True, True, sink, False, False, 1.0, -1, sink)
     if dtype == torch.bfloat16 and last:
@@ -137,11 +130,8 @@ def linear_logp_backward_local(
     n, d = hidden2d.shape
     v = weight.shape[0]
     g = grad_logp.reshape(-1).float().contiguous()
-    chunk = backward_chunk(n, d, chunk_tokens, need_weight)
-    if chunk <= max(128, chunk_tokens):
-        dz_buf = _dz_workspace(hidden2d.device, chunk, v)
-    else:  # larger than what is kept between calls
-        dz_buf = torch.empty(chunk, (v + 7) // 8 * 8, dtype=torch.bfloat16, device=hidden2d.device)
+    chunk = max(128, min(chunk_tokens, (n + 127) // 128 * 128))
+    dz_buf = _dz_workspace(hidden2d.device, chunk, v)
     grad_h = torch.empty(n, d, dtype=grad_hidden_dtype, device=hidden2d.device) if need_hidden else None
     grad_w = None
     if need_weight and n == 0:

@@ -89,6 +89,28 @@ def test_linear_logp_weight_gradient_in_one_and_several_chunks(n, chunk, v):
         assert _rel(got, want) < BF16
 
 
+@pytest.mark.parametrize("n,chunk", [(300, 128), (512, 256), (513, 512)])
+def test_linear_logp_weight_gradient_adds_its_chunks_in_order(n, chunk):
+    """The sum of the chunks' products, each formed apart in 32 bits, rounded once: the same bits, also where one longer
+    contraction over the whole batch would fit."""
+    from rl_engine.kernels.ops.base import require_ext
+    from rl_engine.kernels.ops.sm100.linear_logp import FusedLinearLogpSM100Op, _forward_local
+
+    ext, d, v = require_ext(), 192, 1024
+    h, w = _randn(n, d, seed=n).requires_grad_(True), _randn(v, d, seed=v, scale=0.1).requires_grad_(True)
+    t = torch.randint(0, v, (n,), device=DEV, generator=_gen(9))
+    g = torch.randn(n, device=DEV, generator=_gen(10))
+    FusedLinearLogpSM100Op(bwd_chunk_tokens=chunk)(h, w, t).backward(g)
+    _, lse, _ = _forward_local(h.detach(), w.detach(), t, None, True, False)
+    want = torch.zeros(v, d, device=DEV)
+    for i in range(0, n, chunk):
+        rows = slice(i, min(i + chunk, n))
+        dz = torch.empty(rows.stop - i, v, dtype=torch.bfloat16, device=DEV)
+        ext.linear_logp_dz(h.detach()[rows], w.detach(), t[rows], None, lse[rows], g[rows], 0, dz)
+        want += ext.gemm(dz, h.detach()[rows], True, True, None, True)
+    assert torch.equal(w.grad, want.to(torch.bfloat16))
+
+
 # ------------------------------------------------------------------------------------------------ decoding step
 @pytest.mark.parametrize("n", [1, 16, 17, 33, 64, 128])
 @pytest.mark.parametrize("rows,k", [(128, 64), (200, 200), (2560, 1088), (12800, 320), (128 * 149, 136), (128 * 300 - 8, 72)])
