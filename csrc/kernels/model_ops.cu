@@ -235,25 +235,42 @@ inline bool bf16_vec_ok(const void* a, long long lda, int D) {
   return D % 8 == 0 && D <= 8 * kNormVecMax * kNormThreads && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0;
 }
 
-// Sum of the chunks' partial rows.  32 columns x 16 groups per CTA, group g adds chunks g, g + 16, ... and the groups are added
-// in order: one thread per column would walk hundreds of chunks one load after the other (45 us at 4096 columns and
-// 1100 chunks) on a handful of SMs.
+// Sum of the chunks' partial rows, chunk after chunk: the order of the additions is that of one thread walking a column, whose last
+// bit a training run's numbers depend on.  What such a thread waits for is memory (45 us at 4096 columns and 1100 chunks on a
+// handful of SMs), so 16 warps fetch 128 rows of 32 columns ahead and one warp adds them from shared memory.
 constexpr int kColsumGroups = 16;
+constexpr int kColsumAhead = 8;
+constexpr int kColsumRows = kColsumGroups * kColsumAhead;
 template <typename TW>
 __global__ void __launch_bounds__(32 * kColsumGroups)
 colsum_kernel(const float* __restrict__ part, int chunks, int D, TW* __restrict__ dw, bool accumulate) {
-  __shared__ float red[kColsumGroups][32];
+  __shared__ float tile[2][kColsumRows][32];
   const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
+  float next[kColsumAhead];
+  auto fetch = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < kColsumAhead; ++u) {
+      const int c = base + u * kColsumGroups + group;
+      next[u] = i < D && c < chunks ? part[static_cast<long long>(c) * D + i] : 0.f;
+    }
+  };
+  fetch(0);
   float s = 0.f;
-  if (i < D) {
-#pragma unroll 8
-    for (int c = group; c < chunks; c += kColsumGroups) s += part[static_cast<long long>(c) * D + i];
+  // two buffers and one barrier a round: the adding warp reaches the barrier of round t + 1 only when it is done with round t,
+  // whose buffer is written again after that barrier
+  for (int base = 0, b = 0; base < chunks; base += kColsumRows, b ^= 1) {
+#pragma unroll
+    for (int u = 0; u < kColsumAhead; ++u) tile[b][u * kColsumGroups + group][lane] = next[u];
+    if (base + kColsumRows < chunks) fetch(base + kColsumRows);
+    __syncthreads();
+    if (group == 0) {
+      const int n = min(kColsumRows, chunks - base);
+#pragma unroll 16
+      for (int r = 0; r < n; ++r) s += tile[b][r][lane];
+    }
   }
-  red[group][lane] = s;
-  __syncthreads();
   if (group == 0 && i < D) {
-    for (int g = 1; g < kColsumGroups; ++g) s += red[g][lane];
     if (accumulate) {  // the bits of a gradient tensor of its own that is added afterwards
       TW r;
       stf(&r, 0, s);

@@ -111,6 +111,23 @@ def test_linear_logp_weight_gradient_adds_its_chunks_in_order(n, chunk):
     assert torch.equal(w.grad, want.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("rows", [8, 24, 1024, 1032, 4000])
+@pytest.mark.parametrize("d", [40, 264])
+def test_rmsnorm_weight_gradient_adds_its_chunks_in_order(rows, d):
+    """Eight rows a chunk at these sizes: the chunks on their own, added one after the other in 32 bits, are the same bits."""
+    from rl_engine.kernels.ops.base import require_ext
+
+    ext = require_ext()
+    x, dy = _randn(rows, d, seed=1), _randn(rows, d, seed=2)
+    w = torch.randn(d, device=DEV, generator=_gen(3))
+    rstd = torch.rand(rows, device=DEV, generator=_gen(4)) + 0.5
+    parts = [ext.rmsnorm_bwd(x[i : i + 8], w, dy[i : i + 8], rstd[i : i + 8])[1] for i in range(0, rows, 8)]
+    want = torch.zeros(d, device=DEV)
+    for part in parts:
+        want = want + part
+    assert torch.equal(ext.rmsnorm_bwd(x, w, dy, rstd)[1], want)
+
+
 # ------------------------------------------------------------------------------------------------ decoding step
 @pytest.mark.parametrize("n", [1, 16, 17, 33, 64, 128])
 @pytest.mark.parametrize("rows,k", [(128, 64), (200, 200), (2560, 1088), (12800, 320), (128 * 149, 136), (128 * 300 - 8, 72)])
