@@ -17,20 +17,12 @@ from rl_engine.kernels.ops.base import require_ext
 
 KEY_TILE = 128
 Q_BLOCK = 64
+# A list is cut after every 64 blocks, on any machine and for any head count: where the cuts lie decides the order of a key's
+# fp32 sums, and with it the last bit of its gradient.  Shorter pieces for grids that leave SMs idle (two equal pieces per SM)
+# made the dK / dV kernel of a ragged batch 228 -> 52 us a layer, and the numbers of a training run others.
 MAX_BLOCKS_PER_ITEM = 64
-MIN_BLOCKS_PER_ITEM = 4
 
-_PLAN_CACHE: Dict[Tuple[int, int], tuple] = {}
-
-
-def blocks_per_item(blocks: int, kv_heads: int) -> int:
-    """How long a key tile's query-block list may be before it is split.  One CTA walks one list for all query heads of
-    its group (1.3 us per block and head), so a list of 40 blocks on a machine with 80 CTAs in all is the whole kernel's
-    time; two CTAs per SM (296) of equal length is what the split aims at.  Below 4 blocks the CTA's set-up and the
-    reduction of its partial (128 KB) cost more than they save, above 64 the tail of the last wave does.  With 64 blocks
-    for every shape the dK / dV kernel of a 0.5B model's ragged batch took 228 us a layer and 40 us for two layers' worth of
-    a hundred tokens; now 52 and 22 us."""
-    return max(MIN_BLOCKS_PER_ITEM, min(MAX_BLOCKS_PER_ITEM, -(-blocks * kv_heads // 296)))
+_PLAN_CACHE: Dict[int, tuple] = {}
 
 
 def union_length(spans) -> int:
@@ -41,10 +33,9 @@ def union_length(spans) -> int:
     return total
 
 
-def build_plan(layout, kv_heads: int = 1) -> tuple:
+def build_plan(layout) -> tuple:
     """``(items, q_blocks, jobs, partial slots, (query rows, key rows) that the lists write)``"""
-    key = (id(layout), kv_heads)
-    hit = _PLAN_CACHE.get(key)
+    hit = _PLAN_CACHE.get(id(layout))
     if hit is not None and hit[0] is layout:
         return hit[1]
     # readers: (k_start, k_len, q_start, q_len, causal).  Key ranges of different sequences may be equal
@@ -61,7 +52,7 @@ def build_plan(layout, kv_heads: int = 1) -> tuple:
     q_blocks: List[List[int]] = []
     items: List[List[int]] = []
     jobs: List[List[int]] = []
-    lists: List[Tuple[int, int, int, int]] = []  # (first key, keys, list begin, list end)
+    key_spans: List[Tuple[int, int]] = []
     slots = 0
     for lo, hi in zip(cuts[:-1], cuts[1:]):
         covering = [r for r in readers if r[0] <= lo and hi <= r[0] + r[1]]
@@ -80,27 +71,24 @@ def build_plan(layout, kv_heads: int = 1) -> tuple:
             end = len(q_blocks)
             if end == begin:
                 continue
-            lists.append((k_abs, min(KEY_TILE, hi - k_abs), begin, end))
-    most = blocks_per_item(len(q_blocks), kv_heads)
-    for (k_abs, tile_len, begin, end) in lists:
-        count = -(-(end - begin) // most)
-        per = -(-(end - begin) // count)  # pieces of equal length
-        pieces = [(b, min(b + per, end)) for b in range(begin, end, per)]
-        if len(pieces) == 1:
-            items.append([k_abs, tile_len, 0, begin, end, -1, 0, 0])
-        else:
-            jobs.append([k_abs, tile_len, slots, slots + len(pieces)])
-            for (b, e) in pieces:
-                items.append([k_abs, tile_len, 0, b, e, slots, 0, 0])
-                slots += 1
+            tile_len = min(KEY_TILE, hi - k_abs)
+            key_spans.append((k_abs, k_abs + tile_len))
+            pieces = [(b, min(b + MAX_BLOCKS_PER_ITEM, end)) for b in range(begin, end, MAX_BLOCKS_PER_ITEM)]
+            if len(pieces) == 1:
+                items.append([k_abs, tile_len, 0, begin, end, -1, 0, 0])
+            else:
+                jobs.append([k_abs, tile_len, slots, slots + len(pieces)])
+                for (b, e) in pieces:
+                    items.append([k_abs, tile_len, 0, b, e, slots, 0, 0])
+                    slots += 1
     items.sort(key=lambda it: it[3] - it[4])  # longest lists first
     dev = layout.seqs.device
     as_t = lambda rows, w: torch.tensor(rows, dtype=torch.int32, device=dev).reshape(-1, w)
-    covered = (union_length((s[0], s[0] + s[1]) for s in layout.host_seqs), union_length((x[0], x[0] + x[1]) for x in lists))
+    covered = (union_length((s[0], s[0] + s[1]) for s in layout.host_seqs), union_length(key_spans))
     plan = (as_t(items, 8), as_t(q_blocks, 4), as_t(jobs, 4), slots, covered)
     if len(_PLAN_CACHE) > 64:
         _PLAN_CACHE.clear()
-    _PLAN_CACHE[key] = (layout, plan)
+    _PLAN_CACHE[id(layout)] = (layout, plan)
     return plan
 
 
@@ -111,7 +99,7 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
 
 def fused_backward(q, k, v, out, lse, dout, layout, scale: float, packed: bool = False):
     """``(dq, dk, dv)``; ``packed`` (queries and keys are the same tokens): one ``[tokens, Hq + 2 Hkv, 128]`` tensor."""
-    items, q_blocks, jobs, slots, written = build_plan(layout, k.shape[1])
+    items, q_blocks, jobs, slots, written = build_plan(layout)
     dout = _aligned(dout)
     out = _aligned(out)
     if out.stride(0) != dout.stride(0):
