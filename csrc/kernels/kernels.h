@@ -323,9 +323,8 @@ void rope_apply(const void* x, long long ldt, int dtype, const long long* pos, c
 void embedding_forward(const long long* ids, const void* table, long long ldw, int dtype, void* out, long long rows,
                        int D, long long vocab, cudaStream_t stream);
 // ids: sorted (stable), order: the row of dy each sorted id belongs to; writes the table rows that occur.
-long long embedding_backward_partial_floats(long long n, int D);
 void embedding_backward(const long long* ids, const long long* order, long long n, const void* dy, int dy_dtype, int D, void* dtable,
-                        bool table_fp32, long long ldw, float* partials, long long table_rows, bool accumulate, cudaStream_t stream);
+                        bool table_fp32, long long ldw, long long table_rows, bool accumulate, cudaStream_t stream);
 // master: fp32 master weights or nullptr.  residual: 16-bit residuals of a bf16 parameter (fp32 master = parameter
 // bits << 16 plus the sign-extended residual) or nullptr; at most one of the two.
 void adamw_step(void* p, int p_dtype, float* master, short* residual, const void* g, int g_dtype, float* m, float* v,

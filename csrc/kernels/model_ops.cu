@@ -460,12 +460,11 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const T*
   }
 }
 
-// Deterministic backward without atomics: `ids` are the sorted token ids, `order` the rows they come from (stable sort).
-// The sorted rows are cut into chunks of kEmbChunk; a CTA sums the runs of equal ids of its chunk in order.  A run inside one
-// chunk is written to its table row at once, the ends of runs that cross a chunk border go to fp32 partials (slot 2 c: the
-// run that came in from the left, 2 c + 1: the one that leaves to the right), which the second kernel adds in chunk
-// order.  So one id that fills half the batch (a padding id) is spread over the machine like any other rows: walked by
-// one CTA, 2000 rows of 4096 took 14 ms; 0.06 ms now.
+// Deterministic backward without atomics: `ids` are the sorted token ids, `order` the rows they come from (stable sort).  Every
+// table row is one 32-bit sum in the order of the batch, whatever the id's run is cut by: the last bit of that sum is part of a
+// training run's numbers.  The sorted rows are cut into chunks of kEmbChunk; a CTA sums the runs that lie inside its chunk.  A
+// run that crosses a chunk border is walked by CTAs of 128-byte column slices, which fetch 128 rows ahead of the one warp that adds
+// them: one id that fills half the batch (a padding id) costs the additions and not a round trip to memory for each row.
 constexpr int kEmbChunk = 64;
 constexpr int kEmbThreads = 128;
 
@@ -532,8 +531,8 @@ __device__ __forceinline__ void store_cols(T* p, const float (&x)[VEC]) {
 template <typename T, typename TG, int VEC>
 __global__ void __launch_bounds__(kEmbThreads)
 embedding_bwd_chunks_kernel(const long long* __restrict__ ids, const long long* __restrict__ order, long long n,
-                            const T* __restrict__ dy, int D, TG* __restrict__ dtable, long long ldw, float* __restrict__ partials,
-                            long long table_rows, bool accumulate) {
+                            const T* __restrict__ dy, int D, TG* __restrict__ dtable, long long ldw, long long table_rows,
+                            bool accumulate) {
   __shared__ long long id_s[kEmbChunk], row_s[kEmbChunk];
   const long long r0 = static_cast<long long>(blockIdx.x) * kEmbChunk;
   const int count = static_cast<int>(n - r0 < kEmbChunk ? n - r0 : kEmbChunk);
@@ -544,76 +543,128 @@ embedding_bwd_chunks_kernel(const long long* __restrict__ ids, const long long* 
   __syncthreads();
   const int col = (blockIdx.y * kEmbThreads + threadIdx.x) * VEC;
   if (col >= D) return;
-  const bool from_left = r0 > 0 && ids[r0 - 1] == id_s[0];
-  const bool to_right = r0 + count < n && ids[r0 + count] == id_s[count - 1];
+  // the runs that reach over the chunk's borders are left to embedding_bwd_runs_kernel
+  int lo = 0, hi = count;
+  if (r0 > 0 && ids[r0 - 1] == id_s[0])
+    while (lo < count && id_s[lo] == id_s[0]) ++lo;
+  if (r0 + count < n && ids[r0 + count] == id_s[count - 1])
+    while (hi > lo && id_s[hi - 1] == id_s[count - 1]) --hi;
   float acc[VEC];
 #pragma unroll
   for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
-  bool left = from_left;  // the current run began in an earlier chunk
   constexpr int kAhead = 4;
-  for (int base = 0; base < count; base += kAhead) {
+  for (int base = lo; base < hi; base += kAhead) {
     float x[kAhead][VEC];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u)
-      if (base + u < count) load_cols<T, VEC>(dy + row_s[base + u] * static_cast<long long>(D) + col, x[u]);
+      if (base + u < hi) load_cols<T, VEC>(dy + row_s[base + u] * static_cast<long long>(D) + col, x[u]);
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
       const int i = base + u;
-      if (i >= count) break;
+      if (i >= hi) break;
 #pragma unroll
       for (int j = 0; j < VEC; ++j) acc[j] += x[u][j];
-      const bool last = i + 1 == count;
-      if (!last && id_s[i + 1] == id_s[i]) continue;
-      const bool right = last && to_right;
-      if (left || right) {
-        store_cols<float, VEC>(partials + (2ll * blockIdx.x + (left ? 0 : 1)) * D + col, acc);
-      } else if (id_s[i] >= 0 && id_s[i] < table_rows) {
-        put_cols<TG, VEC>(dtable + id_s[i] * ldw + col, acc, accumulate);
-      }
+      if (i + 1 < hi && id_s[i + 1] == id_s[i]) continue;
+      if (id_s[i] >= 0 && id_s[i] < table_rows) put_cols<TG, VEC>(dtable + id_s[i] * ldw + col, acc, accumulate);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
-      left = false;
     }
   }
 }
 
-// One CTA row per chunk: the chunk in which a border-crossing run begins adds up its partials.
-template <typename TG, int VEC>
-__global__ void __launch_bounds__(kEmbThreads)
-embedding_bwd_runs_kernel(const long long* __restrict__ ids, long long n, int D, TG* __restrict__ dtable, long long ldw,
-                          const float* __restrict__ partials, long long table_rows, bool accumulate) {
-  const int col = (blockIdx.y * kEmbThreads + threadIdx.x) * VEC;
-  const long long r1 = (static_cast<long long>(blockIdx.x) + 1) * kEmbChunk;
-  if (col >= D || r1 >= n) return;
+// One CTA per (chunk, 128-byte column slice): the chunk in which a border-crossing run begins walks all of it.  VEC: rows of dy are
+// 16-byte aligned and a multiple of 16 bytes.
+constexpr int kRunThreads = 256;
+constexpr int kRunRows = 128;      // rows of a buffer
+constexpr int kRunSlice = 128;     // bytes of a row
+
+template <typename T, typename TG, bool VEC>
+__global__ void __launch_bounds__(kRunThreads)
+embedding_bwd_runs_kernel(const long long* __restrict__ ids, const long long* __restrict__ order, long long n,
+                          const T* __restrict__ dy, int D, TG* __restrict__ dtable, long long ldw, long long table_rows,
+                          bool accumulate) {
+  const long long r1 = (static_cast<long long>(blockIdx.x) + 1) * kEmbChunk, r0 = r1 - kEmbChunk;
+  if (r1 >= n) return;
   const long long id = ids[r1 - 1];
-  if (ids[r1] != id || id < 0 || id >= table_rows) return;      // no run leaves this chunk to the right
-  const long long r0 = r1 - kEmbChunk;
-  if (r0 > 0 && ids[r0] == id && ids[r0 - 1] == id) return;     // it began further left
-  float acc[VEC];
-  load_cols<float, VEC>(partials + (2ll * blockIdx.x + 1) * D + col, acc);
-  // chunks the run covers completely, and the one it ends in
-  long long c = blockIdx.x + 1;
-  constexpr int kAhead = 8;
-  for (bool more = true; more;) {
-    float x[kAhead][VEC];
-    int got = 0;
+  if (ids[r1] != id || id < 0 || id >= table_rows) return;   // no run leaves this chunk to the right
+  if (r0 > 0 && ids[r0] == id && ids[r0 - 1] == id) return;  // it began further left
+  // [begin, end): the ids are sorted, so it is enough to count those that are equal
+  const int tid = threadIdx.x;
+  const long long begin = r1 - __syncthreads_count(tid < kEmbChunk && ids[r0 + tid] == id);
+  long long end = r1;  // first the chunks the run covers or reaches into, then its end in the last of them
+  for (;;) {
+    const long long at = end + static_cast<long long>(tid) * kEmbChunk;
+    const int got = __syncthreads_count(at < n && ids[at] == id);
+    end += static_cast<long long>(got) * kEmbChunk;
+    if (got < kRunThreads) break;
+  }
+  end -= kEmbChunk;  // ids[end] is equal: ids[r1] was
+  end += __syncthreads_count(tid < kEmbChunk && end + tid < n && ids[end + tid] == id);
+
+  constexpr int kCols = kRunSlice / static_cast<int>(sizeof(T));
+  __shared__ alignas(16) T tile[2][kRunRows][kCols];
+  const int col0 = static_cast<int>(blockIdx.y) * kCols;
+  const int cols = min(kCols, D - col0);
+  const long long total = end - begin;
+  constexpr int kUnits = kRunSlice / 16, kStep = kRunThreads / kUnits, kPer = kRunRows / kStep;  // 16-byte units of a row
+  const int unit = tid % kUnits, first = tid / kUnits;
+  long long row[kPer];
+  uint4 q[kPer];
+  auto load_rows = [&](long long base) {
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      if (more) {
-        load_cols<float, VEC>(partials + 2ll * c * D + col, x[u]);
-        ++c;
-        got = u + 1;
-        more = c * kEmbChunk < n && ids[c * kEmbChunk] == id;  // sorted: the run reaches into the next chunk
+    for (int u = 0; u < kPer; ++u) {
+      const long long k = base + first + u * kStep;
+      row[u] = k < total ? order[begin + k] : -1;
+    }
+  };
+  auto load_data = [&] {
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      q[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (row[u] < 0) continue;
+      const T* src = dy + row[u] * static_cast<long long>(D) + col0;
+      if constexpr (VEC) {
+        if (unit * (16 / static_cast<int>(sizeof(T))) < cols) q[u] = __ldg(reinterpret_cast<const uint4*>(src) + unit);
+      } else {
+        T* e = reinterpret_cast<T*>(&q[u]);
+#pragma unroll
+        for (int j = 0; j < 16 / static_cast<int>(sizeof(T)); ++j) {
+          const int c = unit * (16 / static_cast<int>(sizeof(T))) + j;
+          if (c < cols) e[j] = src[c];
+        }
       }
     }
+  };
+  load_rows(0);
+  load_data();
+  load_rows(kRunRows);
+  constexpr int kOwn = 4 / static_cast<int>(sizeof(T)) > 0 ? 4 / static_cast<int>(sizeof(T)) : 1;  // columns of an adding lane
+  float acc[kOwn];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u)
-      if (u < got) {
+  for (int j = 0; j < kOwn; ++j) acc[j] = 0.f;
+  int b = 0;
+  for (long long base = 0; base < total; base += kRunRows, b ^= 1) {
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) acc[j] += x[u][j];
+    for (int u = 0; u < kPer; ++u) *reinterpret_cast<uint4*>(&tile[b][first + u * kStep][unit * (16 / sizeof(T))]) = q[u];
+    load_data();  // of the next round
+    load_rows(base + 2 * kRunRows);
+    __syncthreads();  // two buffers: this one is written again after the next barrier, which the adding warp reaches when it is done
+    if (tid < 32) {
+      const int rows = static_cast<int>(total - base < kRunRows ? total - base : kRunRows);
+#pragma unroll 16
+      for (int r = 0; r < rows; ++r) {
+#pragma unroll
+        for (int j = 0; j < kOwn; ++j) acc[j] += ldf(&tile[b][r][tid * kOwn], j);
       }
+    }
   }
-  put_cols<TG, VEC>(dtable + id * ldw + col, acc, accumulate);
+  if (tid < 32) {
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) {
+      const float one[1] = {acc[j]};
+      if (tid * kOwn + j < cols) put_cols<TG, 1>(dtable + id * ldw + col0 + tid * kOwn + j, one, accumulate);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------ fused AdamW
@@ -1003,31 +1054,30 @@ void embedding_forward(const long long* ids, const void* table, long long ldw, i
   });
 }
 
-long long embedding_backward_partial_floats(long long n, int D) { return 2 * ((n + kEmbChunk - 1) / kEmbChunk) * D; }
-
 void embedding_backward(const long long* ids, const long long* order, long long n, const void* dy, int dy_dtype, int D, void* dtable,
-                        bool table_fp32, long long ldw, float* partials, long long table_rows, bool accumulate, cudaStream_t stream) {
+                        bool table_fp32, long long ldw, long long table_rows, bool accumulate, cudaStream_t stream) {
   if (n <= 0 || D <= 0) return;
   const unsigned chunks = static_cast<unsigned>((n + kEmbChunk - 1) / kEmbChunk);
   const bool vec = D % 8 == 0 && ldw % 8 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0 &&
-                   (reinterpret_cast<uintptr_t>(dtable) & 15u) == 0 && (reinterpret_cast<uintptr_t>(partials) & 15u) == 0;
+                   (reinterpret_cast<uintptr_t>(dtable) & 15u) == 0;
   const int per_cta = kEmbThreads * (vec ? 8 : 1);
   const dim3 grid(chunks, (D + per_cta - 1) / per_cta);
 #define RLK_EMB(TG, VEC)                                                                                                          \
   do {                                                                                                                            \
-    embedding_bwd_chunks_kernel<T, TG, VEC><<<grid, kEmbThreads, 0, stream>>>(ids, order, n, static_cast<const T*>(dy), D,         \
-                                                                             static_cast<TG*>(dtable), ldw, partials, table_rows, accumulate); \
+    embedding_bwd_chunks_kernel<T, TG, VEC ? 8 : 1><<<grid, kEmbThreads, 0, stream>>>(ids, order, n, static_cast<const T*>(dy), D, \
+                                                                                     static_cast<TG*>(dtable), ldw, table_rows, accumulate); \
+    const int cols = kRunSlice / static_cast<int>(sizeof(T));                                                                     \
     if (chunks > 1)                                                                                                               \
-      embedding_bwd_runs_kernel<TG, VEC><<<grid, kEmbThreads, 0, stream>>>(ids, n, D, static_cast<TG*>(dtable), ldw, partials,    \
-                                                                          table_rows, accumulate);                                \
+      embedding_bwd_runs_kernel<T, TG, VEC><<<dim3(chunks - 1, (D + cols - 1) / cols), kRunThreads, 0, stream>>>(                  \
+          ids, order, n, static_cast<const T*>(dy), D, static_cast<TG*>(dtable), ldw, table_rows, accumulate);                    \
   } while (0)
   RLK_DISPATCH_T(dy_dtype, {
     if (table_fp32) {
-      if (vec) RLK_EMB(float, 8);
-      else RLK_EMB(float, 1);
+      if (vec) RLK_EMB(float, true);
+      else RLK_EMB(float, false);
     } else {
-      if (vec) RLK_EMB(T, 8);
-      else RLK_EMB(T, 1);
+      if (vec) RLK_EMB(T, true);
+      else RLK_EMB(T, false);
     }
   });
 #undef RLK_EMB

@@ -1259,10 +1259,9 @@ void embedding_bwd(const Tensor& sorted_ids, const Tensor& order, const Tensor& 
   const bool tfp32 = dtable.scalar_type() == torch::kFloat32;
   TORCH_CHECK(tfp32 || dtable.scalar_type() == dy.scalar_type(), "dtable must be float32 or match dy");
   const int D = static_cast<int>(dy.size(1));
-  Tensor partials = torch::empty({rlk::embedding_backward_partial_floats(n, D)}, dy.options().dtype(torch::kFloat32));
   rlk::embedding_backward(reinterpret_cast<const long long*>(sorted_ids.data_ptr<int64_t>()),
                           reinterpret_cast<const long long*>(order.data_ptr<int64_t>()), n, dy.data_ptr(), dtype_code(dy), D,
-                          dtable.data_ptr(), tfp32, dtable.stride(0), partials.data_ptr<float>(), dtable.size(0), accumulate,
+                          dtable.data_ptr(), tfp32, dtable.stride(0), dtable.size(0), accumulate,
                           stream_of(dy));
   after_launch(2);
 }

@@ -226,6 +226,22 @@ def test_embedding_gradient_runs_across_chunks(n, kind, d, dtype):
     assert torch.equal(first, table.grad)
 
 
+@pytest.mark.parametrize("n,kind", [(64, "one"), (65, "one"), (1000, "one"), (20000, "one"), (700, "mixed"), (131, "last")])
+@pytest.mark.parametrize("d,dtype", [(200, torch.bfloat16), (13, torch.float32), (72, torch.float32), (5, torch.float16)])
+def test_embedding_gradient_adds_a_row_in_batch_order(n, kind, d, dtype):
+    """A table row is one 32-bit sum in the order of the batch, however its run lies in the chunks: the same bits."""
+    from rl_engine.kernels.ops.sm100.model_ops import FusedEmbeddingSM100Op
+
+    ids = {"one": torch.full((n,), 3), "mixed": (torch.arange(n) * 7) % 5, "last": (torch.arange(n) > 2) * 6 + 1}[kind].to(DEV)
+    table = _randn(8, d, seed=1, dtype=dtype).requires_grad_(True)
+    dy = _randn(n, d, seed=2, dtype=dtype)
+    FusedEmbeddingSM100Op()(ids, table).backward(dy)
+    want = torch.zeros(8, d)
+    for i, row in zip(ids.tolist(), dy.float().cpu().unbind()):
+        want[i] += row
+    assert torch.equal(table.grad.cpu(), want.to(dtype))
+
+
 def test_embedding_gradient_refuses_ids_outside_the_table():
     from rl_engine.kernels.ops.sm100.model_ops import FusedEmbeddingSM100Op
 
