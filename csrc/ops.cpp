@@ -1488,10 +1488,11 @@ Tensor decode_qkv(const Tensor& x, const Tensor& w, std::optional<Tensor> bias, 
   return q;
 }
 
-// Attention of a decoding step over `parts` disjoint key sets per query (seqs[:, 6] = part * rows) and their merge:
+// Attention of a decoding step over `parts` disjoint key sets per query (seqs[:, 6] = part * rows, with the rows that
+// the table was built for given as part_rows) and their merge:
 // [rows / rep, hkv * rep * 128] in the model's head order.
 Tensor decode_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& seqs, const Tensor& tiles, int64_t parts,
-                        int64_t rep, double softmax_scale) {
+                        int64_t part_rows, int64_t rep, double softmax_scale) {
   auto check3 = [](const Tensor& t, const char* n) {
     TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.dim() == 3 && t.size(2) == 128 && t.is_contiguous() &&
                     reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0,
@@ -1509,6 +1510,7 @@ Tensor decode_attention(const Tensor& q, const Tensor& k, const Tensor& v, const
               "rl_engine.decode_attention: tables must be 16-byte aligned");
   const int64_t rows = q.size(0), hkv = q.size(1);
   TORCH_CHECK(parts >= 1 && rep >= 1 && rows % rep == 0, "rl_engine.decode_attention: rows must be a multiple of rep");
+  TORCH_CHECK(rows == part_rows, "rl_engine.decode_attention: the tables were built for ", part_rows, " query rows, q has ", rows);
   const c10::cuda::CUDAGuard guard(q.device());
   Tensor o = torch::empty({parts * rows, hkv, 128}, q.options());
   Tensor lse = torch::empty({hkv, parts * rows}, q.options().dtype(torch::kFloat32));

@@ -50,6 +50,7 @@ class DecodeStepTables:
     seqs: torch.Tensor          # int32 [parts - 1 + n, 8]; column 6: first output row of the sequence's part
     tiles: torch.Tensor         # int32 [n_tiles, 2] of all sequences
     parts: int
+    rows: int                   # query rows of every part; part i is stored to output rows i * rows ...
     own_begin: int
     prefix: PackedLayout
 
@@ -99,7 +100,8 @@ def decode_step_layouts(prefix: PackedLayout, own: PackedLayout, rows: int, pref
     own_begin = len(seqs)
     tiles += [[own_begin + i, q0] for i, s in enumerate(own.host_seqs) for q0 in range(0, s[1], TILE)]
     table = torch.cat([torch.tensor(seqs, dtype=torch.int32, device=dev).reshape(-1, 8), own.seqs])
-    step = DecodeStepTables(table, torch.tensor(tiles, dtype=torch.int32, device=dev).reshape(-1, 2), own_begin + 1, own_begin, prefix)
+    step = DecodeStepTables(table, torch.tensor(tiles, dtype=torch.int32, device=dev).reshape(-1, 2), own_begin + 1, rows, own_begin,
+                            prefix)
     return replace(own, seqs=table[own_begin:], step=step)
 
 

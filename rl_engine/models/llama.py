@@ -684,6 +684,7 @@ class LlamaModel(nn.Module):
         hq, hkv = cfg.num_heads, cfg.num_kv_heads
         scale = 1.0 / math.sqrt(cfg.head_dim)
         n = token_ids.numel()
+        self._check_step_layouts(n, prefix_layout, self_layout)
         x = self.embed_tokens(token_ids)
         step = self._decode_tables(n, positions, cache, slots, prefix_layout, self_layout)
         if step is not None:
@@ -708,6 +709,15 @@ class LlamaModel(nn.Module):
             gu = self._project(rms_norm(x, p("mlp_norm"), cfg.rms_eps), f"l{i}.w_gate_up")
             x = x + self._project(swiglu_packed(gu), f"l{i}.w_down")
         return rms_norm(x, self.view("final_norm"), cfg.rms_eps)
+
+    def _check_step_layouts(self, n: int, prefix_layout, self_layout) -> None:
+        """Both layouts must hold exactly the ``n * Hq / Hkv`` query rows of this call: the attention kernels store a row of
+        output for every query row of their tables and read back one for every row of the call."""
+        rows = n * (self.cfg.num_heads // self.cfg.num_kv_heads)
+        for what, layout in (("prefix_layout", prefix_layout), ("self_layout", self_layout)):
+            seqs = layout.host_seqs
+            if sum(s[1] for s in seqs) != rows or max((s[0] + s[1] for s in seqs), default=0) != rows:
+                raise ValueError(f"decode_step: {what} was not built for {n} sequences ({rows} query rows)")
 
     def _decode_tables(self, n, positions, cache, slots, prefix_layout, self_layout):
         """The joint tables of ``decode_layouts`` if this call can run on the decode kernels (``_decode_layers``): up to
@@ -753,7 +763,7 @@ class LlamaModel(nn.Module):
             q = ext.decode_qkv(rms_norm(x, p("attn_norm"), cfg.rms_eps), p("wqkv").detach(), p("bqkv").detach() if cfg.qkv_bias else None,
                                self.rope_cos, self.rope_sin, positions, slots, cache[i][0], cache[i][1], cfg.num_heads, partials,
                                counters[i * len(names)])
-            attn = ext.decode_attention(q, cache[i][0], cache[i][1], step.seqs, step.tiles, step.parts, rep, scale)
+            attn = ext.decode_attention(q, cache[i][0], cache[i][1], step.seqs, step.tiles, step.parts, step.rows, rep, scale)
             x = project(attn, i, 1, False, x)
             act = project(rms_norm(x, p("mlp_norm"), cfg.rms_eps), i, 2, True, None)
             x = project(act, i, 3, False, x)
