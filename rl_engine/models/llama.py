@@ -694,6 +694,8 @@ class LlamaModel(nn.Module):
             qkv = self._project(rms_norm(x, p("attn_norm"), cfg.rms_eps), f"l{i}.wqkv")
             if cfg.qkv_bias:
                 qkv = qkv + p("bqkv")
+            if cfg.qk_norm:
+                qkv = ext.qk_norm_fwd(qkv, p("q_norm").detach(), p("k_norm").detach(), hq, hkv, cfg.rms_eps)
             qkv = qkv.view(n, hq + 2 * hkv, cfg.head_dim)
             q, k, v = qkv[:, :hq], qkv[:, hq : hq + hkv], qkv[:, hq + hkv :]
             ext.rope(q, positions, self.rope_cos, self.rope_sin, False, q)
@@ -724,9 +726,10 @@ class LlamaModel(nn.Module):
         128 tokens, layouts that belong together, contiguous caches.  ``None``: the general kernels."""
         cfg, step = self.cfg, getattr(self_layout, "step", None)
         # (fp8 projections keep the general kernels: a code that rounds the other way moves a logit by percents, so their
-        # results are only comparable bit by bit)
+        # results are only comparable bit by bit; so do models with per-head q / k norms, which the projection's epilogue,
+        # straight from the product to the rotation, does not apply)
         if (step is None or not 1 <= n <= 128 or step.prefix is not prefix_layout or cfg.ffn_size % 64 or cfg.hidden_size % 8
-                or self._fp8_linears):
+                or self._fp8_linears or cfg.qk_norm):
             return None
         own = step.seqs[step.own_begin:]
         if self_layout.seqs.data_ptr() != own.data_ptr() or self_layout.seqs.shape != own.shape:

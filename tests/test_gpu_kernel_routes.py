@@ -194,6 +194,40 @@ def test_decode_step_on_the_decode_kernels_matches_the_general_ones(n, p, own, h
     assert torch.equal(layout.step.seqs[layout.step.own_begin :, 5], layout.seqs[:, 5])
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+def test_decode_step_applies_the_head_norms(fp8):
+    """A model with per-head q / k norms: teacher-forced steps against the rows of the packed forward, which normalises the heads.
+    Weights far from one, so that a step without them would miss by the hidden state's own size (measured: 0.5 of its norm).
+    bf16 rounds about ten tensors per layer on either side; e4m3 codes are 2^-4 apart."""
+    from rl_engine.kernels.ops.sm100.attention import grpo_group_layout
+    from rl_engine.models.config import ModelConfig
+    from rl_engine.models.llama import LlamaModel
+
+    cfg = ModelConfig("norms", 512, 256, 2, 4, 2, 128, 448, qk_norm=True)
+    model = LlamaModel(cfg, dtype=torch.bfloat16, device=DEV, seed=5)
+    p, g, l = 70, 3, 5
+    ids = torch.randint(0, 512, (p + g * l,), device=DEV, generator=_gen(6))
+    prompt, comp = ids[:p], ids[p:].view(g, l)
+    with torch.no_grad():
+        for i in range(2):
+            for j, name in enumerate(("q_norm", "k_norm")):
+                model.view(f"l{i}.{name}").copy_(3 * torch.rand(128, device=DEV, generator=_gen(7 + j)))
+        positions = torch.cat([torch.arange(p, device=DEV), (p + torch.arange(l, device=DEV)).repeat(g)])
+        full = model.hidden_states(ids, positions, grpo_group_layout(p, g, l, DEV))[p:].view(g, l, -1)
+        if fp8:
+            model.enable_fp8_inference()
+        cache = model.new_kv_cache(p + g * l)
+        for (ck, cv), (pk, pv) in zip(cache, model.prefix_states(prompt)[1]):
+            ck[:p].copy_(pk)
+            cv[:p].copy_(pv)
+        prefix, own = model.decode_layouts(g, p, l)
+        for t in range(l):
+            pos = torch.full((g,), p + t, dtype=torch.long, device=DEV)
+            got = model.decode_step(comp[:, t].contiguous(), pos, cache, p + torch.arange(g, device=DEV) * l + t, prefix, own)
+            own.seqs[:, 5] += 1
+            assert _rel(got, full[:, t]) < (0.12 if fp8 else 8 * BF16)
+
+
 @pytest.mark.parametrize("m", [1, 32, 100, 128])
 def test_wide_gemm_rows_have_the_same_bits_at_any_number_of_rows(m):
     from rl_engine.kernels.ops.sm100.gemm import gemm
