@@ -658,9 +658,10 @@ class LlamaModel(nn.Module):
     # -- incremental decoding with a key / value cache (rollout side, no autograd) -------------------------
     @torch.no_grad()
     def new_kv_cache(self, rows: int):
-        """Per-layer ``(k, v)`` buffers ``[rows, Hkv, 128]`` for ``decode_step``."""
+        """Per-layer ``(k, v)`` buffers ``[rows, Hkv, 128]`` for ``decode_step``.  Zeroed: attention multiplies the rows of a
+        128-key tile behind a sequence's last key with zero weights, and zero times what memory happens to hold may be NaN."""
         cfg = self.cfg
-        make = lambda: torch.empty(rows, cfg.num_kv_heads, cfg.head_dim, dtype=self.flat.dtype, device=self.flat.device)
+        make = lambda: torch.zeros(rows, cfg.num_kv_heads, cfg.head_dim, dtype=self.flat.dtype, device=self.flat.device)
         return [(make(), make()) for _ in range(cfg.num_layers)]
 
     @torch.no_grad()

@@ -194,11 +194,29 @@ def test_decode_step_on_the_decode_kernels_matches_the_general_ones(n, p, own, h
     assert torch.equal(layout.step.seqs[layout.step.own_begin :, 5], layout.seqs[:, 5])
 
 
+def test_rollout_does_not_read_what_the_cache_memory_held():
+    """Rows of a key tile behind a sequence's last key are multiplied with zero weights; memory that held NaN must not get in."""
+    from rl_engine.executors.native_rollout import NativeRolloutEngine
+    from rl_engine.models.config import ModelConfig
+    from rl_engine.models.llama import LlamaModel
+
+    model = LlamaModel(ModelConfig("cache", 512, 256, 2, 4, 2, 128, 448), dtype=torch.bfloat16, device=DEV, seed=5)
+    prompt = torch.randint(0, 512, (40,), device=DEV, generator=_gen(1))
+    rows = 40 + 3 * 6
+    poison = [torch.full((rows, 2, 128), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(64)]
+    del poison
+    for k, v in model.new_kv_cache(rows):
+        assert bool((k == 0).all()) and bool((v == 0).all())
+    out = NativeRolloutEngine(model, seed=5).generate(prompt, num_generations=3, max_new_tokens=6, top_k=20)
+    assert torch.isfinite(out["rollout_logps"]).all()
+
+
 @pytest.mark.parametrize("fp8", [False, True])
 def test_decode_step_applies_the_head_norms(fp8):
     """A model with per-head q / k norms: teacher-forced steps against the rows of the packed forward, which normalises the heads.
-    Weights far from one, so that a step without them would miss by the hidden state's own size (measured: 0.5 of its norm).
-    bf16 rounds about ten tensors per layer on either side; e4m3 codes are 2^-4 apart."""
+    Weights far from one: a step without the norms misses by 1.03 of the hidden state's norm.  bf16 rounds about ten tensors per
+    layer on either side; e4m3 codes are 2^-3 apart, rounded to within 2^-4, in four products a layer whose errors add up like
+    independent ones: 2^-4 * sqrt(16) at most."""
     from rl_engine.kernels.ops.sm100.attention import grpo_group_layout
     from rl_engine.models.config import ModelConfig
     from rl_engine.models.llama import LlamaModel
@@ -225,7 +243,7 @@ def test_decode_step_applies_the_head_norms(fp8):
             pos = torch.full((g,), p + t, dtype=torch.long, device=DEV)
             got = model.decode_step(comp[:, t].contiguous(), pos, cache, p + torch.arange(g, device=DEV) * l + t, prefix, own)
             own.seqs[:, 5] += 1
-            assert _rel(got, full[:, t]) < (0.12 if fp8 else 8 * BF16)
+            assert _rel(got, full[:, t]) < (0.25 if fp8 else 8 * BF16)
 
 
 @pytest.mark.parametrize("m", [1, 32, 100, 128])
