@@ -404,7 +404,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (j == 0) {
           m_used = cand;  // nothing accumulated yet
         } else if (__any_sync(0xffffffffu, cand - m_used > kLazy)) {  // (-inf) - (-inf) = NaN compares false
-          const float alpha = cand == -INFINITY ? 1.f : fast_exp2(m_used - cand);  // m_used = -inf -> 0
+          // The rescale is a warp's (TMEM is read and written by all lanes), but in a decoding step the rows of a warp are
+          // other sequences' queries: there a row follows its maximum only when its own has grown, so that its bits do
+          // not depend on its neighbours.
+          const bool grown = !STEP || cand - m_used > kLazy;
+          const float alpha = !grown || cand == -INFINITY ? 1.f : fast_exp2(m_used - cand);  // m_used = -inf -> 0
           // O holds the products up to tile j - 1 once P V of that tile has completed; P V of tile j is issued only
           // after every softmax warp has arrived on p_full below, i.e. after this rescale.
           mbar_wait(&o_full[b ^ 1], ((g - 1) >> 1) & 1, abort_flag, err, 200, 7);
@@ -423,7 +427,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           tmem_st_wait();
           tc_fence_before();
           l *= alpha;
-          m_used = cand;
+          if (grown) m_used = cand;
         }
         const float m_safe = m_used == -INFINITY ? 0.f : m_used;
         // P[b] was the A operand of P V two tiles ago: that product must have finished reading it.  (For the first

@@ -2,15 +2,18 @@
 // work that follows a projection done in its epilogue.
 //
 // What bounds it: the weight bytes.  A skinny GEMM that keeps the tokens on the M side pads them to 128 rows, loads 16 KB
-// of mostly empty token tile beside every 8 KB of weight and gets its parallelism from N alone (64 CTAs for a
-// 4096-wide output).  Here the WEIGHT is the 128-row operand and the tokens are the N side (16 .. 128 columns), so a stage
-// is 16 KB of weight and at most as much of tokens, and the (output tile, k-block) units of the whole layer are dealt to the
-// CTAs in equal contiguous ranges: every SM streams the same number of bytes whatever the shape.  A tile that is cut by a range border is
-// summed from fp32 partials in range order by whoever delivers the last one (no spinning, bitwise reproducible, the cut
-// depends on the layer and the machine only, never on the tokens).  The plain GEMMs (bf16 and fp8), whose rows have the
-// same bits at any number of rows, deal whole tiles.
+// of mostly empty token tile beside every 8 KB of weight.  Here the WEIGHT is the row operand and the tokens are the N side
+// (16 .. 128 columns), and a tile holds 64 or 128 rows of the weight (tile_rows_of).  The tensor core always multiplies 128
+// rows: of a tile of 64 it reads whatever lies behind it in shared memory, and those lanes of the accumulator are never looked at.
 //
-// The CTA needs less than half an SM's shared memory on purpose: with programmatic dependent launch the next layer's CTAs
+// K is summed in one piece and every intermediate result is rounded where the separate kernels round it (the product to bf16,
+// then bias, rotation, residual or SwiGLU): a row has the bits of those kernels, with any number of rows, and which kernel a
+// projection runs on is a matter of speed alone.  What that costs: 16 columns or 128, an accumulation into the same columns
+// takes 90 ns a step of 16, so 4096 of K are 22 us and 14336 are 72 us whatever the tile.  Splits of K over CTAs avoid it
+// (50 MB for 32 tokens 19 us), but then a row's bits depend on the route, and the sum of the partials by one CTA made a step of
+// four 1024-wide layers with 128 tokens 845 us instead of 383.
+//
+// A CTA needs less than half an SM's shared memory on purpose: with programmatic dependent launch the next layer's CTAs
 // become resident beside this one's and fetch their first weight stages (weights do not depend on the previous
 // kernel) while this layer's tail drains.
 //
@@ -24,38 +27,43 @@
 namespace rlk {
 namespace {
 
-constexpr int kChunk = 16;  // tokens per epilogue step
 constexpr uint32_t kKernelId = 120u;
 
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-// DEEP: the whole SM for one CTA.
-template <int NT, bool DEEP>
+template <int NT, int WR>
 struct DecSmem {
-  static constexpr int kWBytes = 128 * 128;
+  static constexpr int kChunk = 16;  // tokens per epilogue step
+  static constexpr int kWBytes = WR * 128;
   static constexpr int kXBytes = NT * 128;
   static constexpr int kStageBytes = kWBytes + kXBytes;
-  static constexpr int kStages = DEEP ? 200 * 1024 / kStageBytes : (NT <= 32 ? 5 : (NT == 64 ? 4 : 3));
-  static constexpr int kXch = kStages * kStageBytes;            // float [kChunk][128]
-  static constexpr int kBars = kXch + kChunk * 128 * 4;
-  static constexpr int kBytes = kBars + (2 * kStages + 4) * 8 + 16;
-  static constexpr int kDynamic = kBytes + 1024;
-  static_assert(kDynamic <= (DEEP ? 227 : 113) * 1024, "two CTAs must fit an SM, or one deep one");
+  static constexpr int kXchBytes = kChunk * WR * 4;  // float [kChunk][WR]
+  static constexpr int kLimit = 110 * 1024;          // two CTAs, their static shared memory and the reserved kilobytes fit an SM
+  // the tensor core reads 128 rows from the start of every stage, the last one too
+  static constexpr int kFitRead = (kLimit - 1024 - 128 * 128) / kStageBytes + 1;
+  static constexpr int kFitUsed = (kLimit - 2048 - kXchBytes) / kStageBytes;
+  static constexpr int kFit = kFitRead < kFitUsed ? kFitRead : kFitUsed;
+  static constexpr int kStages = kFit < 16 ? kFit : 16;
+  static constexpr int kXch = kStages * kStageBytes;
+  static constexpr int kBars = kXch + kXchBytes;
+  static constexpr int kUsed = kBars + (2 * kStages + 4) * 8 + 16;
+  static constexpr int kRead = (kStages - 1) * kStageBytes + 128 * 128;
+  static constexpr int kDynamic = (kUsed > kRead ? kUsed : kRead) + 1024;
+  static_assert(kStages >= 2 && kDynamic <= kLimit, "two CTAs must fit an SM");
 };
 
-// The (tile, k-block) units of CTA c: [c T / G, (c + 1) T / G), in units of `step` (one k-block, or a whole tile).
-__device__ __forceinline__ long long range_begin(long long total, int c, int grid, int step = 1) {
-  return total / step * c / grid * step;
-}
-__device__ __forceinline__ int range_owner(long long total, long long unit, int grid) {
-  return static_cast<int>(((unit + 1) * grid - 1) / total);
+// The tiles of CTA c: [c T / G, (c + 1) T / G).
+__device__ __forceinline__ int first_tile(int tiles, int c, int grid) {
+  return static_cast<int>(static_cast<long long>(tiles) * c / grid);
 }
 
-template <int NT, int ELT, int MODE, bool DEEP>
-__global__ void __launch_bounds__(192)
+__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+template <int NT, int WR, int ELT, int MODE>
+__global__ void __launch_bounds__(192, 2)
 decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                      const __grid_constant__ DecodeLinearArgs p, const int tiles, const int k_blocks) {
-  using L = DecSmem<NT, DEEP>;
+  using L = DecSmem<NT, WR>;
+  constexpr int kChunk = L::kChunk;
+  constexpr int kHalf = WR / 2;
   constexpr int kElems = 128 / ELT;  // elements of one 128-byte k-block
   constexpr uint32_t kTmemCols = 2 * NT;
   extern __shared__ uint8_t smem_raw[];
@@ -68,10 +76,8 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* xch = reinterpret_cast<float*>(smem + L::kXch);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long total = static_cast<long long>(tiles) * k_blocks;
   const int grid = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
-  const int step = p.whole_tiles ? k_blocks : 1;
-  const long long u0 = range_begin(total, cta, grid, step), u1 = range_begin(total, cta + 1, grid, step);
+  const int t_begin = first_tile(tiles, cta, grid), t_end = first_tile(tiles, cta + 1, grid);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < L::kStages; ++s) {
@@ -80,7 +86,7 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], 128);
+      mbar_init(&tmem_empty[b], WR);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -98,38 +104,44 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 
   if (warp == 0) {
     if (lane == 0) {
-      auto load_w = [&](long long u, int stage) {
-        const int tile = static_cast<int>(u / k_blocks), k0 = static_cast<int>(u - static_cast<long long>(tile) * k_blocks) * kElems;
+      auto load_w = [&](int tile, int kb, int stage) {
+        const int k0 = kb * kElems;
         uint8_t* sw = smem + stage * L::kStageBytes;
         mbar_arrive_expect_tx(&full_bar[stage], L::kStageBytes);
-        if constexpr (MODE == kDecodeSwiglu) {  // 64 gate rows above the 64 up rows of the same outputs
-          tma_load_2d(sw, &tmap_w, &full_bar[stage], k0, tile * 64);
-          tma_load_2d(sw + L::kWBytes / 2, &tmap_w, &full_bar[stage], k0, p.N / 2 + tile * 64);
+        if constexpr (MODE == kDecodeSwiglu) {  // the gate rows above the up rows of the same outputs
+          tma_load_2d(sw, &tmap_w, &full_bar[stage], k0, tile * kHalf);
+          tma_load_2d(sw + L::kWBytes / 2, &tmap_w, &full_bar[stage], k0, p.N / 2 + tile * kHalf);
+        } else if constexpr (MODE == kDecodeQkv) {  // rows of the first half of a head above their partners in the rotation
+          constexpr int kPerHead = 128 / WR;
+          const int row = tile / kPerHead * 128 + tile % kPerHead * kHalf;
+          tma_load_2d(sw, &tmap_w, &full_bar[stage], k0, row);
+          tma_load_2d(sw + L::kWBytes / 2, &tmap_w, &full_bar[stage], k0, row + 64);
         } else {
-          tma_load_2d(sw, &tmap_w, &full_bar[stage], k0, tile * 128);
+          tma_load_2d(sw, &tmap_w, &full_bar[stage], k0, tile * WR);
         }
       };
-      auto load_x = [&](long long u, int stage) {
-        const int k0 = static_cast<int>(u % k_blocks) * kElems;
-        tma_load_2d(smem + stage * L::kStageBytes + L::kWBytes, &tmap_x, &full_bar[stage], k0, 0);
+      auto load_x = [&](int kb, int stage) {
+        tma_load_2d(smem + stage * L::kStageBytes + L::kWBytes, &tmap_x, &full_bar[stage], kb * kElems, 0);
       };
       // the first stages' weights are requested before the previous kernel has finished, its outputs afterwards
       if (!p.early_weights) grid_dep_wait();
-      const int ahead = static_cast<int>(min(u1 - u0, static_cast<long long>(L::kStages)));
-      for (int s = 0; s < ahead; ++s) load_w(u0 + s, s);
+      const int ahead = t_begin < t_end ? min(k_blocks, L::kStages) : 0;
+      for (int s = 0; s < ahead; ++s) load_w(t_begin, s, s);
       grid_dep_wait();
       grid_dep_launch();
-      for (int s = 0; s < ahead; ++s) load_x(u0 + s, s);
-      int stage = ahead == L::kStages ? 0 : ahead;
+      for (int s = 0; s < ahead; ++s) load_x(s, s);
+      int stage = ahead == L::kStages ? 0 : ahead, kb = ahead;
       uint32_t phase = ahead == L::kStages ? 1 : 0;
-      for (long long u = u0 + ahead; u < u1 && !*abort_flag; ++u) {
-        mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, kKernelId, 1);
-        if (*abort_flag) break;
-        load_w(u, stage);
-        load_x(u, stage);
-        if (++stage == L::kStages) {
-          stage = 0;
-          phase ^= 1;
+      for (int tile = t_begin; tile < t_end && !*abort_flag; ++tile, kb = 0) {
+        for (; kb < k_blocks; ++kb) {
+          mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, kKernelId, 1);
+          if (*abort_flag) break;
+          load_w(tile, kb, stage);
+          load_x(kb, stage);
+          if (++stage == L::kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
     }
@@ -138,15 +150,12 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       constexpr uint32_t idesc = ELT == 1 ? umma_idesc_e4m3(128, NT) : umma_idesc_bf16(128, NT, false, false);
       int stage = 0, buf = 0;
       uint32_t phase = 0, buf_phase = 0;
-      for (long long u = u0; u < u1 && !*abort_flag;) {
-        const int tile = static_cast<int>(u / k_blocks);
-        const long long end = min(u1, static_cast<long long>(tile + 1) * k_blocks);
+      for (int tile = t_begin; tile < t_end && !*abort_flag; ++tile) {
         mbar_wait(&tmem_empty[buf], buf_phase ^ 1, abort_flag, p.err, kKernelId, 2);
         if (*abort_flag) break;
         tc_fence_after();
         const uint32_t d = tmem + buf * NT;
-        bool first = true;
-        for (; u < end; ++u) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
           mbar_wait(&full_bar[stage], phase, abort_flag, p.err, kKernelId, 3);
           if (*abort_flag) break;
           tc_fence_after();
@@ -154,10 +163,9 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const uint64_t da = umma_smem_desc_sw128(sw + k * 32, 16, 1024), db = umma_smem_desc_sw128(sx + k * 32, 16, 1024);
-            if constexpr (ELT == 1) umma_f8(d, da, db, idesc, first && k == 0 ? 0u : 1u);
-            else umma_bf16(d, da, db, idesc, first && k == 0 ? 0u : 1u);
+            if constexpr (ELT == 1) umma_f8(d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+            else umma_bf16(d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
           }
-          first = false;
           umma_commit(&empty_bar[stage]);
           if (++stage == L::kStages) {
             stage = 0;
@@ -171,15 +179,15 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         }
       }
     }
-  } else {
+  } else if ((warp & 3) * 32 < WR) {  // the warps whose lanes of the accumulator hold rows of the tile
     grid_dep_wait();  // everything below reads or overwrites what earlier kernels touch
+    auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(WR) : "memory"); };
     const int quad = warp & 3;
-    const int f = quad * 32 + lane;  // feature within the tile = TMEM lane
+    const int f = quad * 32 + lane;  // row of the tile = TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    __shared__ unsigned int s_last;
     __shared__ long long pos_s[MODE == kDecodeQkv ? NT : 1], slot_s[MODE == kDecodeQkv ? NT : 1];
     if constexpr (MODE == kDecodeQkv) {  // one round trip for all tokens; an index outside its table is reported and skipped
-      for (int t = threadIdx.x - 64; t < p.n; t += 128) {
+      for (int t = f; t < p.n; t += WR) {
         const long long pos = __ldcg(p.positions + t), slot = __ldcg(p.slots + t);
         const bool pos_ok = pos >= 0 && pos < p.table_rows, slot_ok = slot >= 0 && slot < p.cache_rows;
         if (!pos_ok) report_error(p.err, kErrBadIndex, kKernelId, 10);
@@ -187,166 +195,115 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         pos_s[t] = pos_ok ? pos : 0;
         slot_s[t] = slot_ok ? slot : -1;
       }
-      epi_sync();
+      sync();
     }
     int buf = 0;
     uint32_t buf_phase = 0;
-    for (long long u = u0; u < u1;) {
-      const int tile = static_cast<int>(u / k_blocks);
-      const long long t0 = static_cast<long long>(tile) * k_blocks, t1 = t0 + k_blocks;
-      const long long end = min(u1, t1);
-      const bool whole = u == t0 && end == t1;
+    for (int tile = t_begin; tile < t_end; ++tile) {
+      // row of W that this lane holds, its scale and bias
+      constexpr int kPerHead = 128 / WR;
+      int w_row = tile * WR + f;
+      if constexpr (MODE == kDecodeSwiglu) w_row = (f < kHalf ? 0 : p.N / 2) + tile * kHalf + (f & (kHalf - 1));
+      if constexpr (MODE == kDecodeQkv)
+        w_row = tile / kPerHead * 128 + tile % kPerHead * kHalf + (f & (kHalf - 1)) + (f < kHalf ? 0 : 64);
+      const bool live = w_row < p.N;
+      float sw = 1.f, bias = 0.f;
+      if constexpr (ELT == 1) sw = live ? p.scale_w[w_row] : 0.f;
+      if constexpr (MODE == kDecodeQkv) bias = p.bias != nullptr ? __bfloat162float(p.bias[w_row]) : 0.f;
+      // the residual of the first tokens is requested while the products are formed, that of later ones a step ahead
+      __nv_bfloat16 res[MODE == kDecodeStore ? kChunk : 1];
+      auto load_residual = [&](int c0) {
+        if constexpr (MODE == kDecodeStore) {
+          if (p.residual != nullptr && live) {
+#pragma unroll
+            for (int j = 0; j < kChunk; ++j)
+              if (c0 + j < p.n) res[j] = __ldcg(p.residual + static_cast<long long>(c0 + j) * p.ld_residual + w_row);
+          }
+        }
+      };
+      load_residual(0);
       mbar_wait(&tmem_full[buf], buf_phase, abort_flag, p.err, kKernelId, 4);
       tc_fence_after();
       const uint32_t acc = tmem + buf * NT + lane_addr;
-      const int c_first = range_owner(total, t0, grid), c_last = range_owner(total, t1 - 1, grid);
-      // partial slots: 2 c for the tile a range begins in, 2 c + 1 for the one it ends in
-      auto slot_of = [&](int c) {
-        const bool begins = range_begin(total, c, grid) >= t0;
-        return p.partials + static_cast<long long>(2 * c + (begins ? 0 : 1)) * 128 * NT + f * 4;
-      };
-      bool finish = whole;
-      if (!whole) {
-        float* mine = slot_of(cta);
 #pragma unroll 1
-        for (int c0 = 0; c0 < NT; c0 += kChunk) {
-          uint32_t r[kChunk];
-          tmem_ld_32x32b_x16(acc + c0, r);
-          tmem_ld_wait();
+      for (int c0 = 0; c0 < NT; c0 += kChunk) {
+        if (c0 >= p.n) break;
+        float v[kChunk], sx[kChunk];
+        if constexpr (ELT == 1) {
 #pragma unroll
-          for (int j = 0; j < kChunk; j += 4) {
-            *reinterpret_cast<uint4*>(mine + (c0 + j) * 128) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-          }
+          for (int j = 0; j < kChunk; ++j) sx[j] = c0 + j < p.n ? __ldcg(p.scale_x + c0 + j) : 0.f;
         }
-        __threadfence();
-        epi_sync();
-        if (threadIdx.x == 64) {
-          unsigned int old;
-          asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p.counters + tile), "r"(1u) : "memory");
-          s_last = old + 1u == static_cast<unsigned int>(c_last - c_first + 1) ? 1u : 0u;
+        uint32_t r[kChunk];
+        tmem_ld_32x32b_x16(acc + c0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) v[j] = __uint_as_float(r[j]);
+        if constexpr (ELT == 1) {
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j) v[j] = v[j] * sx[j] * sw;  // the order of the 256-wide engines: the same bits
         }
-        epi_sync();
-        finish = s_last != 0u;
-      }
-      if (finish) {
-        // row of W that this lane holds, its scale and bias
-        int w_row = tile * 128 + f;
-        if constexpr (MODE == kDecodeSwiglu) w_row = (f < 64 ? 0 : p.N / 2) + tile * 64 + (f & 63);
-        const bool live = w_row < p.N;
-        float sw = 1.f, bias = 0.f;
-        if constexpr (ELT == 1) sw = live ? p.scale_w[w_row] : 0.f;
-        if constexpr (MODE == kDecodeQkv) bias = p.bias != nullptr ? __bfloat162float(p.bias[w_row]) : 0.f;
-#pragma unroll 1
-        for (int c0 = 0; c0 < NT; c0 += kChunk) {
-          if (c0 >= p.n) break;
-          // everything this step needs from memory is requested together
-          float v[kChunk], sx[kChunk], res[kChunk];
-          if constexpr (ELT == 1) {
+        if constexpr (MODE == kDecodeStore) {
+          if (p.residual != nullptr) {
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) sx[j] = c0 + j < p.n ? __ldcg(p.scale_x + c0 + j) : 0.f;
+            for (int j = 0; j < kChunk; ++j) v[j] = round_bf16(v[j]) + __bfloat162float(res[j]);
+            load_residual(c0 + kChunk);
           }
-          if constexpr (MODE == kDecodeStore) {
-            if (p.residual != nullptr && live) {
+          if (live) {
 #pragma unroll
-              for (int j = 0; j < kChunk; ++j)
-                res[j] = c0 + j < p.n ? __bfloat162float(__ldcg(p.residual + static_cast<long long>(c0 + j) * p.ld_residual + w_row)) : 0.f;
+            for (int j = 0; j < kChunk; ++j) {
+              const int t = c0 + j;
+              if (t < p.n) p.out[static_cast<long long>(t) * p.ldo + w_row] = __float2bfloat16_rn(v[j]);
             }
           }
-          if (whole) {
-            uint32_t r[kChunk];
-            tmem_ld_32x32b_x16(acc + c0, r);
-            tmem_ld_wait();
+        } else {
+          // pairs of rows half a tile apart (gate and up, the two halves of a rotation) meet through shared memory
+          sync();  // the previous step's readers are done
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) v[j] = __uint_as_float(r[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < kChunk; ++j) v[j] = 0.f;
-            // four partials at a time, all their loads in flight together; added in range order
-            constexpr int kAhead = 4;
-#pragma unroll 1
-            for (int c = c_first; c <= c_last; c += kAhead) {
-              float4 q[kAhead][kChunk / 4];
-#pragma unroll
-              for (int a = 0; a < kAhead; ++a) {
-                if (c + a <= c_last) {
-                  const float* part = slot_of(c + a) + c0 * 128;
-#pragma unroll
-                  for (int j = 0; j < kChunk / 4; ++j) q[a][j] = __ldcg(reinterpret_cast<const float4*>(part + j * 512));
-                }
-              }
-#pragma unroll
-              for (int a = 0; a < kAhead; ++a) {
-                if (c + a <= c_last) {
-#pragma unroll
-                  for (int j = 0; j < kChunk / 4; ++j) {
-                    v[4 * j] += q[a][j].x;
-                    v[4 * j + 1] += q[a][j].y;
-                    v[4 * j + 2] += q[a][j].z;
-                    v[4 * j + 3] += q[a][j].w;
-                  }
-                }
-              }
+          for (int j = 0; j < kChunk; ++j) {
+            float x = round_bf16(v[j]);
+            if constexpr (MODE == kDecodeQkv) {
+              if (p.bias != nullptr) x = round_bf16(x + bias);
             }
+            xch[j * WR + f] = x;
           }
-          if constexpr (ELT == 1) {
+          sync();
+          if constexpr (MODE == kDecodeSwiglu) {
+            const int at = f & (kHalf - 1), o = tile * kHalf + at;
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) v[j] = v[j] * sx[j] * sw;  // the order of the 256-wide engines: the same bits
-          }
-          if constexpr (MODE == kDecodeStore) {
-            if (live) {
+            for (int i = 0; i < kChunk / 2; ++i) {  // each half of the lanes takes every other token
+              const int j = 2 * i + (f < kHalf ? 0 : 1), t = c0 + j;
+              const float g = xch[j * WR + at], up = xch[j * WR + kHalf + at];
+              if (t < p.n) p.out[static_cast<long long>(t) * p.ldo + o] = __float2bfloat16_rn(g / (1.f + __expf(-g)) * up);
+            }
+          } else {  // kDecodeQkv
+            const int head = tile / kPerHead, half = tile % kPerHead * kHalf + (f & (kHalf - 1)), kv_heads = p.hkv;
+            const int at = half + (f < kHalf ? 0 : 64);  // feature of the head
+            float cs[kChunk], sn[kChunk];
+            if (head < p.hq + kv_heads) {
 #pragma unroll
               for (int j = 0; j < kChunk; ++j) {
-                const int t = c0 + j;
-                if (t < p.n) {
-                  float x = v[j];
-                  if (p.residual != nullptr) x += res[j];
-                  p.out[static_cast<long long>(t) * p.ldo + w_row] = __float2bfloat16_rn(x);
-                }
+                const long long i = c0 + j < p.n ? pos_s[c0 + j] * 64 + half : half;
+                cs[j] = __ldg(p.cos + i);
+                sn[j] = __ldg(p.sin + i);
               }
             }
-          } else {
-            // pairs of features 64 lanes apart (gate and up, the two halves of a rotation) meet through shared memory
-            epi_sync();  // the previous step's readers are done
+            const int rep = p.hq / kv_heads, kv = head / rep;
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) xch[j * 128 + f] = v[j] + bias;
-            epi_sync();
-            if constexpr (MODE == kDecodeSwiglu) {
-              const int o = tile * 64 + (f & 63);
-#pragma unroll
-              for (int i = 0; i < kChunk / 2; ++i) {  // each half of the lanes takes every other token
-                const int j = 2 * i + (f >> 6), t = c0 + j;
-                const float g = xch[j * 128 + (f & 63)], up = xch[j * 128 + 64 + (f & 63)];
-                if (t < p.n) p.out[static_cast<long long>(t) * p.ldo + o] = __float2bfloat16_rn(g / (1.f + __expf(-g)) * up);
-              }
-            } else {  // kDecodeQkv: one tile is one head
-              const int half = f & 63, kv_heads = p.hkv;
-              float cs[kChunk], sn[kChunk];
-              if (tile < p.hq + kv_heads) {
-#pragma unroll
-                for (int j = 0; j < kChunk; ++j) {
-                  const long long at = c0 + j < p.n ? pos_s[c0 + j] * 64 + half : half;
-                  cs[j] = __ldg(p.cos + at);
-                  sn[j] = __ldg(p.sin + at);
+            for (int j = 0; j < kChunk; ++j) {
+              const int t = c0 + j;
+              if (t < p.n) {
+                float x = xch[j * WR + f];
+                if (head < p.hq + kv_heads) {
+                  const float y = xch[j * WR + (f ^ kHalf)];
+                  x = f < kHalf ? x * cs[j] - y * sn[j] : x * cs[j] + y * sn[j];
                 }
-              }
-              const int rep = p.hq / kv_heads, kv = tile / rep;
-#pragma unroll
-              for (int j = 0; j < kChunk; ++j) {
-                const int t = c0 + j;
-                if (t < p.n) {
-                  float x = xch[j * 128 + f];
-                  if (tile < p.hq + kv_heads) {
-                    const float y = xch[j * 128 + (f ^ 64)];
-                    x = f < 64 ? x * cs[j] - y * sn[j] : x * cs[j] + y * sn[j];
-                  }
-                  const __nv_bfloat16 b = __float2bfloat16_rn(x);
-                  if (tile < p.hq) {
-                    p.q_rows[((static_cast<long long>(t) * rep + tile - kv * rep) * kv_heads + kv) * 128 + f] = b;
-                  } else if (slot_s[t] >= 0) {
-                    const bool is_v = tile >= p.hq + kv_heads;
-                    const int head = tile - p.hq - (is_v ? kv_heads : 0);
-                    (is_v ? p.cache_v : p.cache_k)[(slot_s[t] * kv_heads + head) * 128 + f] = b;
-                  }
+                const __nv_bfloat16 b = __float2bfloat16_rn(x);
+                if (head < p.hq) {
+                  p.q_rows[((static_cast<long long>(t) * rep + head - kv * rep) * kv_heads + kv) * 128 + at] = b;
+                } else if (slot_s[t] >= 0) {
+                  const bool is_v = head >= p.hq + kv_heads;
+                  const int h = head - p.hq - (is_v ? kv_heads : 0);
+                  (is_v ? p.cache_v : p.cache_k)[(slot_s[t] * kv_heads + h) * 128 + at] = b;
                 }
               }
             }
@@ -359,7 +316,6 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         buf = 0;
         buf_phase ^= 1;
       }
-      u = end;
     }
   }
 
@@ -375,68 +331,52 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   }
 }
 
-// CTAs of a launch.  A tile cut between CTAs costs the last of them a round trip through memory (fence, counter, partials:
-// 5 us and more at the end of a 20 us layer), a CTA that holds two cut tiles pays it twice.  So:
-//   - up to two tiles per SM and no fewer than one: a CTA per tile, two to an SM; they share the memory's bandwidth evenly
-//     whether an SM holds one or two (gate / up projection of 32 tokens, 235 MB: 52 -> 45 us).
-//   - fewer: the largest number of equal K splits per tile that the SMs hold, if that uses three quarters of them (each
-//     CTA has one tile: 21 -> 19 and 20 -> 18 us for 50 and 34 MB); ranges that ignore the tile borders otherwise, because
-//     SMs left out cost more than the cut.  A step of four 4096-wide layers and a 128256-row head: 839 -> 792 us.
-int grid_of(int tiles, int k_blocks, bool whole_tiles, int sm_count) {
-  if (whole_tiles) return tiles <= 2 * sm_count ? tiles : sm_count;
-  if (tiles >= sm_count) return tiles <= 2 * sm_count ? tiles : sm_count;
-  const int splits = std::min(sm_count / tiles, k_blocks);
-  if (tiles * splits * 4 >= sm_count * 3 || splits == k_blocks) return tiles * splits;
-  return static_cast<int>(std::min<long long>(static_cast<long long>(tiles) * k_blocks, sm_count));
-}
+// Rows of the weight in a tile.  64 while every tile gets a CTA of its own with two to an SM, 128 beyond, where a CTA walks several:
+// the tiles of 64 end a fifth sooner at 100 tokens (4096 x 4096: 35 against 43 us) and are equal at one, but a CTA's chain of
+// accumulations is as long for 64 rows as for 128 (28672 x 4096: 82 against 37 us).
+int tile_rows_of(int N, int sm_count) { return (N + 63) / 64 <= 2 * sm_count ? 64 : 128; }
 
-template <int NT, int ELT, int MODE, bool DEEP>
-void launch_as(const DecodeLinearArgs& a, int tiles, int k_blocks, int grid, cudaStream_t stream) {
-  using L = DecSmem<NT, DEEP>;
-  const uint32_t w_box = MODE == kDecodeSwiglu ? 64 : 128;
+template <int NT, int WR, int ELT, int MODE>
+void launch(const DecodeLinearArgs& a, cudaStream_t stream) {
+  using L = DecSmem<NT, WR>;
+  const int tiles = (a.N + WR - 1) / WR;
+  const int k_blocks = (a.K * ELT + 127) / 128;
+  // a CTA per tile while two fit every SM (they share the memory's bandwidth evenly whether an SM holds one or two), contiguous
+  // ranges of tiles for one CTA per SM beyond
+  const int grid = tiles <= 2 * a.sm_count ? tiles : a.sm_count;
+  constexpr uint32_t w_box = MODE == kDecodeStore ? WR : WR / 2;
   const CUtensorMap tw = ELT == 1 ? make_tmap_2d_u8(a.w, a.N, a.K, a.ld_w, w_box, 128)
                                   : make_tmap_2d_bf16(a.w, a.N, a.K, a.ld_w, w_box, 64);
   const CUtensorMap tx = ELT == 1 ? make_tmap_2d_u8(a.x, a.n, a.K, a.ld_x, NT, 128) : make_tmap_2d_bf16(a.x, a.n, a.K, a.ld_x, NT, 64);
-  auto kernel = decode_linear_kernel<NT, ELT, MODE, DEEP>;
+  auto kernel = decode_linear_kernel<NT, WR, ELT, MODE>;
   static PerDeviceOnce configured;
   if (configured.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
   launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(192), L::kDynamic, stream, tw, tx, a, tiles, k_blocks);
 }
 
-template <int NT, int ELT, int MODE>
-void launch(const DecodeLinearArgs& a, cudaStream_t stream) {
-  const int tiles = MODE == kDecodeSwiglu ? a.N / 128 : (a.N + 127) / 128;
-  const int k_blocks = (a.K * ELT + 127) / 128;
-  const int grid = grid_of(tiles, k_blocks, a.whole_tiles, a.sm_count);
-  if constexpr (ELT == 1) {
-    // Whole tiles of an 8-bit weight that leave SMs idle: each CTA keeps twice the bytes in flight, with the shared memory of
-    // the second CTA that its SM will not get (with three tokens, 16 projections 425 -> 400 us).
-    if (grid <= a.sm_count / 2) return launch_as<NT, ELT, MODE, true>(a, tiles, k_blocks, grid, stream);
-  }
-  launch_as<NT, ELT, MODE, false>(a, tiles, k_blocks, grid, stream);
+template <int NT, int WR>
+void by_mode(const DecodeLinearArgs& a, cudaStream_t stream) {
+  if (a.fp8) launch<NT, WR, 1, kDecodeStore>(a, stream);
+  else if (a.mode == kDecodeSwiglu) launch<NT, WR, 2, kDecodeSwiglu>(a, stream);
+  else if (a.mode == kDecodeQkv) launch<NT, WR, 2, kDecodeQkv>(a, stream);
+  else launch<NT, WR, 2, kDecodeStore>(a, stream);
 }
 
 template <int NT>
-void by_mode(const DecodeLinearArgs& a, cudaStream_t stream) {
-  if (a.fp8) launch<NT, 1, kDecodeStore>(a, stream);
-  else if (a.mode == kDecodeSwiglu) launch<NT, 2, kDecodeSwiglu>(a, stream);
-  else if (a.mode == kDecodeQkv) launch<NT, 2, kDecodeQkv>(a, stream);
-  else launch<NT, 2, kDecodeStore>(a, stream);
+void by_rows(const DecodeLinearArgs& a, cudaStream_t stream) {
+  const int rows = a.tile_rows > 0 ? a.tile_rows : tile_rows_of(a.N, a.sm_count);
+  if (rows == 64) by_mode<NT, 64>(a, stream);
+  else by_mode<NT, 128>(a, stream);
 }
-
-int padded_tokens(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 : 128)); }
 
 }  // namespace
 
-long long decode_linear_partial_floats(int n, int sm_count) { return 2ll * sm_count * 128 * padded_tokens(n); }
-
 void decode_linear(const DecodeLinearArgs& a, cudaStream_t stream) {
   if (a.n <= 0 || a.N <= 0) return;
-  const int nt = padded_tokens(a.n);
-  if (nt == 16) by_mode<16>(a, stream);
-  else if (nt == 32) by_mode<32>(a, stream);
-  else if (nt == 64) by_mode<64>(a, stream);
-  else by_mode<128>(a, stream);
+  if (a.n <= 16) by_rows<16>(a, stream);
+  else if (a.n <= 32) by_rows<32>(a, stream);
+  else if (a.n <= 64) by_rows<64>(a, stream);
+  else by_rows<128>(a, stream);
 }
 
 }  // namespace rlk

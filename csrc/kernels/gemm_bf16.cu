@@ -160,7 +160,6 @@ void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
         d.N = a.N;
         d.K = a.K;
         d.mode = kDecodeStore;
-        d.whole_tiles = true;
         d.out = static_cast<__nv_bfloat16*>(a.D);
         d.ldo = a.ldd;
         d.sm_count = a.sm_count;

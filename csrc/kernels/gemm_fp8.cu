@@ -172,7 +172,6 @@ void gemm_fp8_rowscaled(const void* a_q, long long lda, const float* scale_a, co
     d.scale_x = scale_a;
     d.scale_w = scale_b;
     d.mode = kDecodeStore;
-    d.whole_tiles = true;
     d.out = static_cast<__nv_bfloat16*>(d_out);
     d.ldo = ldd;
     d.sm_count = sm_count;

@@ -80,7 +80,7 @@ void quantize_rows_e4m3(const void* x, long long ldx, long long rows, int cols, 
 // ------------------------------------------------------- linear layers of a decoding step (decode_linear.cu)
 enum DecodeLinearMode : int {
   kDecodeStore = 0,   // out[t, f] = x W^T (+ residual[t, f])
-  kDecodeSwiglu = 1,  // W = [gate | up]: out[t, f] = silu(gate) * up
+  kDecodeSwiglu = 1,  // W = [gate | up]: out[t, f] = silu(gate) * up; 64 | N / 2
   kDecodeQkv = 2,     // W = [q | k | v] heads of 128: rotary embedding on q and k, q packed for decode attention, k / v to the cache
 };
 struct DecodeLinearArgs {
@@ -92,10 +92,8 @@ struct DecodeLinearArgs {
   const float* scale_x;  // [n] (fp8)
   const float* scale_w;  // [N] (fp8)
   int mode;
-  bool whole_tiles;    // deal whole output tiles: K is summed in one piece, no partials or counters
+  int tile_rows;       // rows of w in a tile: 64 or 128; 0: by size
   bool early_weights;  // no kernel just before this one in the stream writes w
-  float* partials;         // decode_linear_partial_floats floats
-  unsigned int* counters;  // one per 128-row tile of W (64 outputs in the SwiGLU mode), zero before the launch
   __nv_bfloat16* out;
   long long ldo;
   const __nv_bfloat16* residual;  // or null
@@ -114,7 +112,6 @@ struct DecodeLinearArgs {
   int sm_count;
   uint32_t* err;
 };
-long long decode_linear_partial_floats(int n, int sm_count);
 void decode_linear(const DecodeLinearArgs& args, cudaStream_t stream);
 
 // ----------------------------------------------------------------- fused linear -> log-prob

@@ -1386,11 +1386,11 @@ std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor
 namespace {
 
 // Fields shared by the decode projections.
-rlk::DecodeLinearArgs decode_args(const Tensor& x, const Tensor& w, const Tensor& partials, const Tensor& counters, int mode) {
+rlk::DecodeLinearArgs decode_args(const Tensor& x, const Tensor& w, int mode, int64_t tile_rows) {
   check_rowmajor(x, "x");
   check_rowmajor(w, "w");
   TORCH_CHECK(x.scalar_type() == torch::kBFloat16 && w.scalar_type() == torch::kBFloat16, "rl_engine.decode_linear: bf16 operands only");
-  TORCH_CHECK(x.size(1) == w.size(1) && x.size(0) >= 1 && x.size(0) <= 128, "rl_engine.decode_linear: x must be [1..128, K]");
+  TORCH_CHECK(x.size(1) == w.size(1) && x.size(1) >= 1 && x.size(0) >= 1 && x.size(0) <= 128, "rl_engine.decode_linear: x must be [1..128, K]");
   TORCH_CHECK(x.stride(0) % 8 == 0 && w.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 &&
                   reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0,
               "rl_engine.decode_linear: rows must be 16-byte aligned");
@@ -1405,29 +1405,18 @@ rlk::DecodeLinearArgs decode_args(const Tensor& x, const Tensor& w, const Tensor
   a.mode = mode;
   a.early_weights = true;
   a.sm_count = sm_count_of(x.get_device());
-  TORCH_CHECK(partials.is_cuda() && partials.scalar_type() == torch::kFloat32 && partials.is_contiguous() &&
-                  partials.numel() >= rlk::decode_linear_partial_floats(a.n, a.sm_count) && reinterpret_cast<uintptr_t>(partials.data_ptr()) % 16 == 0,
-              "rl_engine.decode_linear: partials too small");
-  TORCH_CHECK(counters.is_cuda() && counters.scalar_type() == torch::kInt32 && counters.is_contiguous() &&
-                  counters.numel() >= (a.N + 127) / 128,
-              "rl_engine.decode_linear: one int32 counter per 128 rows of w");
-  a.partials = partials.data_ptr<float>();
-  a.counters = reinterpret_cast<unsigned int*>(counters.data_ptr<int>());
+  TORCH_CHECK(tile_rows == 0 || tile_rows == 64 || tile_rows == 128, "rl_engine.decode_linear: tiles of 64 or 128 rows");
+  a.tile_rows = static_cast<int>(tile_rows);
   a.err = err_ptr(x);
   return a;
 }
 
 }  // namespace
 
-int64_t decode_linear_partial_floats(int64_t n, int64_t device) {
-  return rlk::decode_linear_partial_floats(static_cast<int>(n), sm_count_of(static_cast<int>(device)));
-}
-
-// x W^T (+ residual), or silu(gate) * up of a packed [gate | up] weight.  counters: zeroed int32, one per 128 rows of w.
-Tensor decode_linear(const Tensor& x, const Tensor& w, bool swiglu, std::optional<Tensor> residual, const Tensor& partials,
-                     const Tensor& counters) {
+// x W^T (+ residual), or silu(gate) * up of a packed [gate | up] weight.  tile_rows: rows of w per tile (0: by size).
+Tensor decode_linear(const Tensor& x, const Tensor& w, bool swiglu, std::optional<Tensor> residual, int64_t tile_rows) {
   const c10::cuda::CUDAGuard guard(x.device());
-  rlk::DecodeLinearArgs a = decode_args(x, w, partials, counters, swiglu ? rlk::kDecodeSwiglu : rlk::kDecodeStore);
+  rlk::DecodeLinearArgs a = decode_args(x, w, swiglu ? rlk::kDecodeSwiglu : rlk::kDecodeStore, tile_rows);
   TORCH_CHECK(!swiglu || (a.N % 128 == 0 && !residual.has_value()), "rl_engine.decode_linear: SwiGLU needs 64 | F and no residual");
   Tensor out = torch::empty({a.n, swiglu ? a.N / 2 : a.N}, x.options().dtype(torch::kBFloat16));
   if (residual.has_value()) {
@@ -1447,10 +1436,9 @@ Tensor decode_linear(const Tensor& x, const Tensor& w, bool swiglu, std::optiona
 // The q / k / v projection of a decoding step: rotary embedding on q and k, k / v written to rows `slots` of the caches,
 // q returned as [n * hq / hkv, hkv, 128] (the query heads of a key / value head are rows).
 Tensor decode_qkv(const Tensor& x, const Tensor& w, std::optional<Tensor> bias, const Tensor& cos_t, const Tensor& sin_t,
-                  const Tensor& positions, const Tensor& slots, Tensor cache_k, Tensor cache_v, int64_t hq, const Tensor& partials,
-                  const Tensor& counters) {
+                  const Tensor& positions, const Tensor& slots, Tensor cache_k, Tensor cache_v, int64_t hq, int64_t tile_rows) {
   const c10::cuda::CUDAGuard guard(x.device());
-  rlk::DecodeLinearArgs a = decode_args(x, w, partials, counters, rlk::kDecodeQkv);
+  rlk::DecodeLinearArgs a = decode_args(x, w, rlk::kDecodeQkv, tile_rows);
   auto cache_ok = [&](const Tensor& c) {
     return c.is_cuda() && c.scalar_type() == torch::kBFloat16 && c.is_contiguous() && c.dim() == 3 && c.size(2) == 128;
   };
@@ -1743,9 +1731,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention_bwd", rlk::traced("rlk::attention_bwd", &attention_bwd), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"),
         py::arg("dout"), py::arg("lse"), py::arg("seqs"), py::arg("q_tiles"), py::arg("kv_items"), py::arg("q_blocks"),
         py::arg("reduce_jobs"), py::arg("num_slots"), py::arg("causal"), py::arg("softmax_scale"), py::arg("packed") = false, py::arg("covered") = false);
-  m.def("decode_linear_partial_floats", rlk::traced("rlk::decode_linear_partial_floats", &decode_linear_partial_floats));
-  m.def("decode_linear", rlk::traced("rlk::decode_linear", &decode_linear));
-  m.def("decode_qkv", rlk::traced("rlk::decode_qkv", &decode_qkv));
+  m.def("decode_linear", rlk::traced("rlk::decode_linear", &decode_linear), py::arg("x"), py::arg("w"), py::arg("swiglu"),
+        py::arg("residual"), py::arg("tile_rows") = 0);
+  m.def("decode_qkv", rlk::traced("rlk::decode_qkv", &decode_qkv), py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("cos"),
+        py::arg("sin"), py::arg("positions"), py::arg("slots"), py::arg("cache_k"), py::arg("cache_v"), py::arg("hq"),
+        py::arg("tile_rows") = 0);
   m.def("decode_attention", rlk::traced("rlk::decode_attention", &decode_attention));
   m.def("error_state", rlk::traced("rlk::error_state", &error_state));
   m.def("reset_error", rlk::traced("rlk::reset_error", &reset_error));

@@ -87,12 +87,14 @@ def make_layout(seqs: Sequence[Sequence[int]], causal: bool, device) -> PackedLa
 def decode_step_layouts(prefix: PackedLayout, own: PackedLayout, rows: int, prefix_len: int, kv_heads: int) -> PackedLayout:
     """``own`` with a private table that is part of a ``DecodeStepTables`` for both layouts.
 
-    The prefix is cut so that its (range, 128-row query tile, head) items are about as many as the machine has SMs: one
-    item walks its key tiles one after the other, and 8 heads alone would keep 8 of 148 SMs busy.  More than 16 ranges
-    cost more in the merge than they save."""
+    The prefix is cut so that the (range, head) items of one 128-row query tile are about as many as the machine has SMs: one
+    item walks its key tiles one after the other, and 8 heads alone would keep 8 of 148 SMs busy.  More than 8 ranges
+    cost more in the merge than they save.  The cut follows from the prefix and the machine alone: a sequence's results keep
+    their bits when others join the step or leave it."""
     dev = own.seqs.device
-    n_tiles, q_tiles = (prefix_len + TILE - 1) // TILE, (rows + TILE - 1) // TILE
-    ranges = max(1, min(n_tiles, 16, 148 // max(1, q_tiles * kv_heads)))
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 148
+    n_tiles = (prefix_len + TILE - 1) // TILE
+    ranges = max(1, min(n_tiles, 8, sms // max(1, kv_heads)))
     per = max(1, -(-n_tiles // ranges)) * TILE
     starts = list(range(0, prefix_len, per))
     seqs = [[0, rows, s, min(per, prefix_len - s), 0, 0, (i + 1) * rows, 0] for i, s in enumerate(starts)]

@@ -688,7 +688,7 @@ class LlamaModel(nn.Module):
         self._check_step_layouts(n, prefix_layout, self_layout)
         x = self.embed_tokens(token_ids)
         step = self._decode_tables(n, positions, cache, slots, prefix_layout, self_layout)
-        if step is not None:
+        if step is not None and n <= 128:
             return self._decode_layers(x.reshape(n, -1), positions, cache, slots, step, scale)
         for i in range(cfg.num_layers):
             p = lambda name: self.view(f"l{i}.{name}")
@@ -705,9 +705,12 @@ class LlamaModel(nn.Module):
             cache[i][1].index_copy_(0, slots, v)
             rep = hq // hkv
             rows = q.reshape(n, hkv, rep, cfg.head_dim).permute(0, 2, 1, 3).reshape(n * rep, hkv, cfg.head_dim)
-            o1, l1 = packed_attention_forward(rows, cache[i][0], cache[i][1], prefix_layout, scale, True)
-            o2, l2 = packed_attention_forward(rows, cache[i][0], cache[i][1], self_layout, scale, True)
-            out = ext.attn_merge2(o1, l1, o2, l2, rep)  # [n, Hq * 128] in the model's head order
+            if step is not None:
+                out = ext.decode_attention(rows.contiguous(), *cache[i], step.seqs, step.tiles, step.parts, step.rows, rep, scale)
+            else:
+                o1, l1 = packed_attention_forward(rows, cache[i][0], cache[i][1], prefix_layout, scale, True)
+                o2, l2 = packed_attention_forward(rows, cache[i][0], cache[i][1], self_layout, scale, True)
+                out = ext.attn_merge2(o1, l1, o2, l2, rep)  # [n, Hq * 128] in the model's head order
             x = x + self._project(out, f"l{i}.wo")
             gu = self._project(rms_norm(x, p("mlp_norm"), cfg.rms_eps), f"l{i}.w_gate_up")
             x = x + self._project(swiglu_packed(gu), f"l{i}.w_down")
@@ -723,13 +726,13 @@ class LlamaModel(nn.Module):
                 raise ValueError(f"decode_step: {what} was not built for {n} sequences ({rows} query rows)")
 
     def _decode_tables(self, n, positions, cache, slots, prefix_layout, self_layout):
-        """The joint tables of ``decode_layouts`` if this call can run on the decode kernels (``_decode_layers``): up to
-        128 tokens, layouts that belong together, contiguous caches.  ``None``: the general kernels."""
+        """The joint tables of ``decode_layouts`` if this call can use them (one attention over all key ranges; up to 128 tokens the
+        projections of ``_decode_layers``): layouts that belong together, contiguous caches.  ``None``: the general kernels."""
         cfg, step = self.cfg, getattr(self_layout, "step", None)
         # (fp8 projections keep the general kernels: a code that rounds the other way moves a logit by percents, so their
         # results are only comparable bit by bit; so do models with per-head q / k norms, which the projection's epilogue,
         # straight from the product to the rotation, does not apply)
-        if (step is None or not 1 <= n <= 128 or step.prefix is not prefix_layout or cfg.ffn_size % 64 or cfg.hidden_size % 8
+        if (step is None or n < 1 or step.prefix is not prefix_layout or cfg.ffn_size % 64 or cfg.hidden_size % 8
                 or self._fp8_linears or cfg.qk_norm):
             return None
         own = step.seqs[step.own_begin:]
@@ -747,30 +750,21 @@ class LlamaModel(nn.Module):
         return step
 
     def _decode_layers(self, x, positions, cache, slots, step, scale):
-        """The layers of ``decode_step`` on the decode kernels: eight launches per layer, each weight streamed once by
-        all SMs; rotary embedding, cache write, residual add and SwiGLU are epilogues of the projections."""
+        """The layers of ``decode_step`` for up to 128 tokens: eight launches per layer, each weight streamed once by all SMs;
+        rotary embedding, cache write, residual add and SwiGLU are epilogues of the projections, with the bits of the
+        separate kernels that more tokens go through."""
         from rl_engine.kernels.ops.base import require_ext
 
         cfg, ext = self.cfg, require_ext()
-        n, rep = x.shape[0], cfg.num_heads // cfg.num_kv_heads
-        names = ("wqkv", "wo", "w_gate_up", "w_down")
-        tiles = [-(-self._shapes[f"l0.{name}"][0] // 128) for name in names]
-        partials = torch.empty(ext.decode_linear_partial_floats(n, x.get_device()), dtype=torch.float32, device=x.device)
-        counters = torch.zeros(cfg.num_layers * sum(tiles), dtype=torch.int32, device=x.device).split(tiles * cfg.num_layers)
-
-        def project(h, i, which, swiglu, residual):
-            return ext.decode_linear(h, self.view(f"l{i}.{names[which]}").detach(), swiglu, residual, partials,
-                                     counters[i * len(names) + which])
-
+        rep = cfg.num_heads // cfg.num_kv_heads
         for i in range(cfg.num_layers):
-            p = lambda name: self.view(f"l{i}.{name}")
-            q = ext.decode_qkv(rms_norm(x, p("attn_norm"), cfg.rms_eps), p("wqkv").detach(), p("bqkv").detach() if cfg.qkv_bias else None,
-                               self.rope_cos, self.rope_sin, positions, slots, cache[i][0], cache[i][1], cfg.num_heads, partials,
-                               counters[i * len(names)])
-            attn = ext.decode_attention(q, cache[i][0], cache[i][1], step.seqs, step.tiles, step.parts, step.rows, rep, scale)
-            x = project(attn, i, 1, False, x)
-            act = project(rms_norm(x, p("mlp_norm"), cfg.rms_eps), i, 2, True, None)
-            x = project(act, i, 3, False, x)
+            p = lambda name: self.view(f"l{i}.{name}").detach()
+            q = ext.decode_qkv(rms_norm(x, p("attn_norm"), cfg.rms_eps), p("wqkv"), p("bqkv") if cfg.qkv_bias else None, self.rope_cos,
+                               self.rope_sin, positions, slots, *cache[i], cfg.num_heads)
+            attn = ext.decode_attention(q, *cache[i], step.seqs, step.tiles, step.parts, step.rows, rep, scale)
+            x = ext.decode_linear(attn, p("wo"), False, x)
+            act = ext.decode_linear(rms_norm(x, p("mlp_norm"), cfg.rms_eps), p("w_gate_up"), True, None)
+            x = ext.decode_linear(act, p("w_down"), False, x)
         return rms_norm(x, self.view("final_norm"), cfg.rms_eps)
 
     def decode_layouts(self, n: int, prefix_len: int, rows_per_sequence: int, own_len: int = 1):

@@ -131,25 +131,52 @@ def test_rmsnorm_weight_gradient_adds_its_chunks_in_order(rows, d):
 # ------------------------------------------------------------------------------------------------ decoding step
 @pytest.mark.parametrize("n", [1, 16, 17, 33, 64, 128])
 @pytest.mark.parametrize("rows,k", [(128, 64), (200, 200), (2560, 1088), (12800, 320), (128 * 149, 136), (128 * 300 - 8, 72)])
-def test_decode_linear(n, rows, k):
-    """Equal K splits, ranges that ignore tile borders, a CTA per tile with two per SM, more tiles than that; ragged last tile,
-    k tail; residual add and SwiGLU epilogues."""
+@pytest.mark.parametrize("tile", [0, 64, 128])
+def test_decode_linear(n, rows, k, tile):
+    """Tiles of 64 and 128 rows: fewer of them than SMs, a CTA per tile with two per SM, more tiles than that; ragged last
+    tile, k tail; residual add and SwiGLU epilogues with the bits of the GEMM and the kernels that follow it."""
     from rl_engine.kernels.ops.base import require_ext
+    from rl_engine.kernels.ops.sm100.gemm import gemm
 
     ext = require_ext()
     x, w = _randn(n, k, seed=n), _randn(rows, k, seed=rows, scale=k ** -0.5)
-    partials = torch.empty(ext.decode_linear_partial_floats(n, 0), device=DEV)
-    counters = lambda: torch.zeros(-(-rows // 128), dtype=torch.int32, device=DEV)
     res = _randn(n, rows, seed=5)
     y = x.double() @ w.double().t()
-    plain = ext.decode_linear(x, w, False, None, partials, counters())
+    product = gemm(torch.cat([x, _randn(200, k, seed=7)]), w)[:n]  # the engine of many rows
+    plain = ext.decode_linear(x, w, False, None, tile)
     assert _rel(plain, y) < BF16 / 2
-    assert torch.equal(plain, ext.decode_linear(x, w, False, None, partials, counters()))
-    assert _rel(ext.decode_linear(x, w, False, res, partials, counters()), y + res.double()) < BF16 / 2
+    assert torch.equal(plain, product)
+    assert torch.equal(ext.decode_linear(x, w, False, res, tile), res + product)
     if rows % 128 == 0:
-        gate, up = y[:, : rows // 2], y[:, rows // 2 :]
-        got = ext.decode_linear(x, w, True, None, partials, counters())
-        assert _rel(got, gate * torch.sigmoid(gate) * up) < BF16 / 2
+        assert torch.equal(ext.decode_linear(x, w, True, None, tile), ext.swiglu_packed_fwd(product.contiguous()))
+
+
+@pytest.mark.parametrize("n", [1, 16, 33, 128])
+@pytest.mark.parametrize("hq,hkv,bias", [(4, 2, False), (8, 1, True), (2, 2, True)])
+@pytest.mark.parametrize("tile", [0, 64, 128])
+def test_decode_qkv(n, hq, hkv, bias, tile):
+    """Projection, bias, rotation, packing of the queries and cache write: the bits of the separate kernels."""
+    from rl_engine.kernels.ops.base import require_ext
+    from rl_engine.kernels.ops.sm100.gemm import gemm
+
+    ext, k, heads = require_ext(), 200, hq + 2 * hkv
+    x, w = _randn(n, k, seed=1), _randn(heads * 128, k, seed=2, scale=0.1)
+    b = _randn(heads * 128, seed=3, scale=0.1) if bias else None
+    angle = torch.rand(50, 64, device=DEV, generator=_gen(4)) * 6
+    cos, sin = angle.cos(), angle.sin()
+    positions = torch.randint(0, 50, (n,), device=DEV, generator=_gen(5))
+    slots = torch.randperm(200, device=DEV, generator=_gen(6))[:n]
+    ck, cv = _randn(200, hkv, 128, seed=7), _randn(200, hkv, 128, seed=8)
+    got_k, got_v = ck.clone(), cv.clone()
+    q = ext.decode_qkv(x, w, b, cos, sin, positions, slots, got_k, got_v, hq, tile)
+    qkv = gemm(torch.cat([x, _randn(200, k, seed=9)]), w)[:n]
+    qkv = (qkv if b is None else qkv + b).view(n, heads, 128)
+    qk = ext.rope(qkv[:, : hq + hkv].contiguous(), positions, cos, sin)
+    ck.index_copy_(0, slots, qk[:, hq:])
+    cv.index_copy_(0, slots, qkv[:, hq + hkv :])
+    rep = hq // hkv
+    assert torch.equal(q, qk[:, :hq].reshape(n, hkv, rep, 128).permute(0, 2, 1, 3).reshape(n * rep, hkv, 128))
+    assert torch.equal(got_k, ck) and torch.equal(got_v, cv)
 
 
 @pytest.mark.parametrize("m", [1, 17, 100, 128])
@@ -192,6 +219,36 @@ def test_decode_step_on_the_decode_kernels_matches_the_general_ones(n, p, own, h
         assert _rel(k, k2) < 4 * BF16 and _rel(v, v2) < 4 * BF16
     layout.seqs[:, 5] += 1  # advanced in place by the caller: both tables follow
     assert torch.equal(layout.step.seqs[layout.step.own_begin :, 5], layout.seqs[:, 5])
+
+
+@pytest.mark.parametrize("p", [1, 200, 3000])
+@pytest.mark.parametrize("heads,kv", [(8, 2), (4, 4)])
+def test_decode_step_rows_have_the_same_bits_at_any_number_of_sequences(p, heads, kv):
+    """Query tiles, prefix ranges, both routes of the projections, row maxima that grow by more than the kernel's lazy step: a
+    sequence's hidden state and cache rows do not depend on who decodes with it."""
+    from rl_engine.models.config import ModelConfig
+    from rl_engine.models.llama import LlamaModel
+
+    cfg, most, own = ModelConfig("rows", 512, 256, 2, heads, kv, 128, 448), 300, 3
+    model = LlamaModel(cfg, dtype=torch.bfloat16, device=DEV, seed=3)
+    start = [(_randn(p + most * own, kv, 128, seed=10 + i, scale=8.0), _randn(p + most * own, kv, 128, seed=20 + i)) for i in range(2)]
+    with torch.no_grad():
+        for i in range(2):
+            model.view(f"l{i}.wqkv")[: heads * 128].mul_(4)
+    tokens = torch.randint(0, 512, (most,), device=DEV, generator=_gen(1))
+    seen = {}
+    for n in (300, 257, 256, 129, 128, 65, 64, 33, 32, 31, 5, 1):
+        cache = [(k[: p + n * own].clone(), v[: p + n * own].clone()) for k, v in start]
+        positions = torch.full((n,), p + own - 1, dtype=torch.long, device=DEV)
+        slots = p + torch.arange(n, device=DEV) * own + own - 1
+        prefix, layout = model.decode_layouts(n, p, own, own)
+        with torch.no_grad():
+            got = model.decode_step(tokens[:n], positions, cache, slots, prefix, layout)
+        rows = [got] + [t[slots] for pair in cache for t in pair]
+        if not seen:
+            seen = rows
+        for a, b in zip(rows, seen):
+            assert torch.equal(a, b[:n]), n
 
 
 def test_rollout_does_not_read_what_the_cache_memory_held():
