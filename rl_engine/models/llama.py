@@ -725,15 +725,18 @@ class LlamaModel(nn.Module):
             if sum(s[1] for s in seqs) != rows or max((s[0] + s[1] for s in seqs), default=0) != rows:
                 raise ValueError(f"decode_step: {what} was not built for {n} sequences ({rows} query rows)")
 
+    def _separate_decode_attention(self) -> bool:
+        """Whether decoding keeps the general kernels throughout.  fp8 projections do: a code that rounds the other way moves a logit
+        by percents, so their results are only comparable bit by bit.  So do models with per-head q / k norms, which the
+        projection's epilogue, straight from the product to the rotation, does not apply."""
+        return bool(self._fp8_linears) or self.cfg.qk_norm
+
     def _decode_tables(self, n, positions, cache, slots, prefix_layout, self_layout):
         """The joint tables of ``decode_layouts`` if this call can use them (one attention over all key ranges; up to 128 tokens the
         projections of ``_decode_layers``): layouts that belong together, contiguous caches.  ``None``: the general kernels."""
         cfg, step = self.cfg, getattr(self_layout, "step", None)
-        # (fp8 projections keep the general kernels: a code that rounds the other way moves a logit by percents, so their
-        # results are only comparable bit by bit; so do models with per-head q / k norms, which the projection's epilogue,
-        # straight from the product to the rotation, does not apply)
         if (step is None or n < 1 or step.prefix is not prefix_layout or cfg.ffn_size % 64 or cfg.hidden_size % 8
-                or self._fp8_linears or cfg.qk_norm):
+                or self._separate_decode_attention()):
             return None
         own = step.seqs[step.own_begin:]
         if self_layout.seqs.data_ptr() != own.data_ptr() or self_layout.seqs.shape != own.shape:
@@ -771,12 +774,16 @@ class LlamaModel(nn.Module):
         """The two layouts of ``decode_step`` for ``n`` sequences whose cache rows are ``[prefix | n x rows_per_sequence]``
         when every sequence holds ``own_len`` tokens including the new one.  Column 5 of ``self_layout.seqs`` is that
         length: a caller that decodes step by step adds one to it in place (the tables are private copies)."""
+        from dataclasses import replace
+
         from rl_engine.kernels.ops.sm100.attention import decode_step_layouts, make_layout
 
         dev = self.flat.device
         rep = self.cfg.num_heads // self.cfg.num_kv_heads
         prefix = make_layout([(0, n * rep, 0, prefix_len, 0, 0)], False, dev)
         own = make_layout([(i * rep, rep, 0, 0, prefix_len + i * rows_per_sequence, own_len) for i in range(n)], False, dev)
+        if self._separate_decode_attention():  # the joint tables would not be read
+            return prefix, replace(own, seqs=own.seqs.clone())
         return prefix, decode_step_layouts(prefix, own, n * rep, prefix_len, self.cfg.num_kv_heads)
 
     def _project(self, x: torch.Tensor, name: str) -> torch.Tensor:

@@ -60,3 +60,14 @@ def test_joint_tables_name_their_query_rows():
         # part i ends inside the output of `parts` times `rows` rows
         ends = own.step.seqs[:, 0] + own.step.seqs[:, 1] + own.step.seqs[:, 6]
         assert int(ends.max()) <= own.step.parts * rows
+
+
+def test_joint_tables_are_built_for_models_whose_step_reads_them():
+    """fp8 projections and per-head norms decode on the general kernels: a private own table, no joint one."""
+    fp8 = _model()
+    fp8._fp8_linears = {"l0.wqkv": object()}
+    for model, joint in ((_model(), True), (fp8, False), (_model(qk_norm=True), False)):
+        prefix, own = model.decode_layouts(3, 300, 16, 2)
+        assert (own.step is not None) == joint
+        own.seqs[:, 5] += 1
+        assert model.decode_layouts(3, 300, 16, 2)[1].seqs[:, 5].eq(2).all()
