@@ -212,6 +212,8 @@ class FusedLinearLogpSM100Op:
     call: ``rl_engine/kernels/ops/cuda/loss/linear_logp.py:353-358``).  ``"sync"``: that host check, raising
     ``ValueError`` at once.  ``"off"``: no check."""
 
+    supports_grad_sink = True  # of ``apply``
+
     def __init__(self, *, check_targets=None, bwd_chunk_tokens: int = DEFAULT_BWD_CHUNK_TOKENS) -> None:
         self._native = NativeLinearLogpOp()
         self.check_targets = target_check_mode(check_targets)

@@ -260,6 +260,8 @@ def _refuse_ids_outside(sorted_ids: torch.Tensor, rows: int) -> None:
 
 
 class FusedEmbeddingSM100Op(torch.nn.Module):
+    supports_grad_sink = True  # of ``forward``
+
     def __init__(self) -> None:
         super().__init__()
         self._native = NativeEmbeddingOp()

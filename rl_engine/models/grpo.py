@@ -252,7 +252,9 @@ def suffix_geometry(p: int, m: int, l: int, device):
 def _head_logps(model, picked: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
     from rl_engine.kernels.registry import kernel_registry
 
-    op, sink = kernel_registry.get_op("linear_logp"), getattr(model, "_grad_sink", lambda name: None)("lm_head")
+    op = kernel_registry.get_op("linear_logp")
+    sinks = getattr(model, "_grad_sink", None) if getattr(op, "supports_grad_sink", False) else None
+    sink = None if sinks is None else sinks("lm_head")
     if sink is None:
         return op(picked, model.lm_head_weight(), ids)
     return op(picked, model.lm_head_weight(), ids, grad_weight_sink=sink)

@@ -419,8 +419,8 @@ class LlamaModel(nn.Module):
     def embed_tokens(self, token_ids: torch.Tensor) -> torch.Tensor:
         from rl_engine.kernels.registry import kernel_registry
 
-        sink = self._grad_sink("embed")
         op = kernel_registry.get_op("embedding")
+        sink = self._grad_sink("embed") if getattr(op, "supports_grad_sink", False) else None
         return op(token_ids, self.view("embed")) if sink is None else op(token_ids, self.view("embed"), grad_sink=sink)
 
     @torch.no_grad()
