@@ -3,6 +3,8 @@
 // Reference counterpart: csrc/ops.cpp:1-99 (pybind of 11-13 functions, launches on the default stream).
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/variable.h>
 #include <torch/extension.h>
 
 #include <cstdlib>
@@ -65,6 +67,15 @@ int sm_count_of(int device) {
 void after_launch(int n = 1) {
   g_launches += n;
   C10_CUDA_KERNEL_LAUNCH_CHECK();
+}
+
+// Whether a hook would see the gradient that autograd adds to the leaf `t`: on the tensor, after its accumulation, or on its
+// AccumulateGrad node (where wrappers that exchange gradients attach; Python cannot list those).
+bool grad_is_watched(const Tensor& t) {
+  namespace impl = torch::autograd::impl;
+  if (!impl::hooks(t).empty() || impl::post_acc_grad_hooks(t) != nullptr) return true;
+  const auto node = impl::try_get_grad_accumulator(t);
+  return node && (!node->pre_hooks().empty() || !node->post_hooks().empty() || !node->tensor_pre_hooks().empty());
 }
 
 // ------------------------------------------------------------------------------------ GEMM
@@ -1668,6 +1679,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
 #endif
   m.def("device_stamp", &device_stamp);
+  m.def("grad_is_watched", &grad_is_watched);
   m.def("trace_enabled", [] { return rlk::trace_enabled(); });
   m.def("gemm", rlk::traced("rlk::gemm", &gemm), py::arg("a"), py::arg("b"), py::arg("a_mn") = false, py::arg("b_mn") = false,
         py::arg("out") = py::none(), py::arg("out_fp32") = false, py::arg("accumulate") = false, py::arg("alpha") = 1.0,

@@ -405,16 +405,18 @@ class LlamaModel(nn.Module):
 
     def _grad_sink(self, name: str) -> Optional[torch.Tensor]:
         """The gradient buffer that a fused backward pass may add to in place of autograd, or ``None``: sinks are off, the
-        parameter is frozen or watched by hooks, or its gradient is not a buffer the kernels can address."""
+        parameter is frozen or watched by hooks (its own, or its ``AccumulateGrad`` node's), or its gradient is not a buffer
+        the kernels can address."""
         if self.sink_weight_grads is None or self.sink_weight_grads != threading.get_ident():
             return None
         p = self.view(name)
         g = p.grad
-        if (g is None or not p.requires_grad or p._backward_hooks or getattr(p, "_post_accumulate_grad_hooks", None)
-                or g.dtype != torch.bfloat16 or g.shape != p.shape or not g.is_contiguous() or g.data_ptr() % 16
-                or g.shape[-1] % 8 or not g.is_cuda):
+        if (g is None or not p.requires_grad or g.dtype != torch.bfloat16 or g.shape != p.shape or not g.is_contiguous()
+                or g.data_ptr() % 16 or g.shape[-1] % 8 or not g.is_cuda):
             return None
-        return g
+        from rl_engine.kernels.ops.base import require_ext
+
+        return None if require_ext().grad_is_watched(p) else g
 
     def embed_tokens(self, token_ids: torch.Tensor) -> torch.Tensor:
         from rl_engine.kernels.registry import kernel_registry

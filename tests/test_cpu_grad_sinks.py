@@ -3,6 +3,7 @@
 import pytest
 import torch
 
+from rl_engine.kernels.ops.base import _C, _EXT_AVAILABLE
 from rl_engine.kernels.registry import kernel_registry
 from rl_engine.models.config import ModelConfig
 from rl_engine.models.grpo import _head_logps
@@ -26,3 +27,19 @@ def test_sinks_go_only_to_operators_that_take_them(monkeypatch):
     grads = torch.autograd.grad(logps.sum(), [model.view("embed"), model.view("lm_head")])
     assert all(float(g.norm()) > 0 for g in grads)
     assert all(float(b.norm()) == 0 for b in buffers.values())
+
+
+@pytest.mark.skipif(not _EXT_AVAILABLE, reason="the native extension is not built")
+def test_every_kind_of_gradient_hook_is_seen():
+    """Hooks on the parameter, after its accumulation and on its AccumulateGrad node (how wrappers attach); a node that exists
+    without hooks is not one."""
+    node_of = lambda p: p.expand_as(p).grad_fn.next_functions[0][0]
+    attach = [lambda p: p.register_hook(lambda g: g), lambda p: p.register_post_accumulate_grad_hook(lambda p: None),
+              lambda p: node_of(p).register_hook(lambda *a: None), lambda p: node_of(p).register_prehook(lambda g: None),
+              lambda p: torch.autograd.graph.register_multi_grad_hook([p], lambda g: None)]
+    for add in attach:
+        p = torch.nn.Parameter(torch.zeros(4, 8))
+        node = node_of(p)  # noqa: F841  (kept alive, as a graph would)
+        assert not _C.grad_is_watched(p)
+        handle = add(p)  # noqa: F841
+        assert _C.grad_is_watched(p)

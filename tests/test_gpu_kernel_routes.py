@@ -533,3 +533,33 @@ def test_gradients_added_by_the_gemms_equal_those_added_by_autograd(micro, chunk
         assert float(g.float().norm()) > 0
     finally:
         op.bwd_chunk_tokens = before
+
+
+@pytest.mark.parametrize("how", ["node", "tensor", "after"])
+def test_hooks_on_a_parameter_see_its_gradient_in_a_trainers_pass(how):
+    """A hook on the AccumulateGrad node, on the parameter or after its accumulation fires as without sinks, and the gradient is
+    the same."""
+    from rl_engine.models.config import ModelConfig
+    from rl_engine.models.grpo import GRPOTrainer, synthetic_batch
+    from rl_engine.models.llama import LlamaModel
+
+    batch = synthetic_batch(640, 70, 6, 90, seed=2).to(DEV)
+    names, grads = ("embed", "l0.wqkv", "l0.mlp_norm", "l1.w_down", "lm_head"), []
+    for watch in (False, True):
+        trainer = GRPOTrainer(LlamaModel(ModelConfig("hooks", 640, 256, 2, 4, 2, 128, 384), dtype=torch.bfloat16, device=DEV, seed=4))
+        trainer.opt.zero_grad()
+        model, seen, nodes = trainer.model, [], []
+        for name in names if watch else ():
+            p = model.view(name)
+            if how == "node":
+                nodes.append(p.expand_as(p).grad_fn.next_functions[0][0])
+                nodes[-1].register_hook(lambda *a, n=name: seen.append(n))
+            elif how == "tensor":
+                p.register_hook(lambda g, n=name: seen.append(n))
+            else:
+                p.register_post_accumulate_grad_hook(lambda p, n=name: seen.append(n))
+        trainer.forward_backward(batch)
+        assert set(seen) == set(names if watch else ())
+        grads.append({n: p.grad.clone() for n, p in model.named_views().items()})
+    for name, want in grads[0].items():
+        assert torch.equal(grads[1][name], want), name
