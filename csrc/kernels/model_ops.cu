@@ -534,6 +534,7 @@ embedding_bwd_chunks_kernel(const long long* __restrict__ ids, const long long* 
                             const T* __restrict__ dy, int D, TG* __restrict__ dtable, long long ldw, long long table_rows,
                             bool accumulate) {
   __shared__ long long id_s[kEmbChunk], row_s[kEmbChunk];
+  if (ids[0] < 0 || ids[n - 1] >= table_rows) return;  // refused by the host: the gradient stays as it was
   const long long r0 = static_cast<long long>(blockIdx.x) * kEmbChunk;
   const int count = static_cast<int>(n - r0 < kEmbChunk ? n - r0 : kEmbChunk);
   for (int i = threadIdx.x; i < count; i += kEmbThreads) {
@@ -565,7 +566,7 @@ embedding_bwd_chunks_kernel(const long long* __restrict__ ids, const long long* 
 #pragma unroll
       for (int j = 0; j < VEC; ++j) acc[j] += x[u][j];
       if (i + 1 < hi && id_s[i + 1] == id_s[i]) continue;
-      if (id_s[i] >= 0 && id_s[i] < table_rows) put_cols<TG, VEC>(dtable + id_s[i] * ldw + col, acc, accumulate);
+      put_cols<TG, VEC>(dtable + id_s[i] * ldw + col, acc, accumulate);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
     }
@@ -584,9 +585,9 @@ embedding_bwd_runs_kernel(const long long* __restrict__ ids, const long long* __
                           const T* __restrict__ dy, int D, TG* __restrict__ dtable, long long ldw, long long table_rows,
                           bool accumulate) {
   const long long r1 = (static_cast<long long>(blockIdx.x) + 1) * kEmbChunk, r0 = r1 - kEmbChunk;
-  if (r1 >= n) return;
+  if (r1 >= n || ids[0] < 0 || ids[n - 1] >= table_rows) return;
   const long long id = ids[r1 - 1];
-  if (ids[r1] != id || id < 0 || id >= table_rows) return;   // no run leaves this chunk to the right
+  if (ids[r1] != id) return;                                 // no run leaves this chunk to the right
   if (r0 > 0 && ids[r0] == id && ids[r0 - 1] == id) return;  // it began further left
   // [begin, end): the ids are sorted, so it is enough to count those that are equal
   const int tid = threadIdx.x;

@@ -1256,7 +1256,7 @@ Tensor embedding_fwd(const Tensor& ids, const Tensor& table) {
 }
 
 // sorted_ids [tokens] (stable sort), order [tokens]: the row of dy each of them belongs to.  Rows of dtable whose id does not
-// occur are left as they are; accumulate adds to the others instead of writing them.
+// occur are left as they are; accumulate adds to the others instead of writing them.  An id outside the table: no row is touched.
 void embedding_bwd(const Tensor& sorted_ids, const Tensor& order, const Tensor& dy, Tensor dtable, bool accumulate) {
   check_rowmajor(dy, "dy");
   check_rowmajor(dtable, "dtable");

@@ -243,8 +243,8 @@ class _Embedding(torch.autograd.Function):
 
 def _refuse_ids_outside(sorted_ids: torch.Tensor, rows: int) -> None:
     """Raises ``ValueError`` from the backward pass that is running if an id lies outside ``[0, rows)``.  The smallest and the
-    largest id are copied out now and looked at when that pass has queued all its kernels (which skip such ids): the
-    host does not stop in the middle of it."""
+    largest id are copied out now and looked at when that pass has queued all its kernels (which then leave the
+    gradient as it was): the host does not stop in the middle of it."""
     n = sorted_ids.numel()
     ends = torch.empty(2, dtype=torch.long, pin_memory=True)
     ends.copy_(sorted_ids[:: n - 1] if n > 1 else sorted_ids.expand(2), non_blocking=True)

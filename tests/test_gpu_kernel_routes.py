@@ -361,6 +361,24 @@ def test_embedding_gradient_refuses_ids_outside_the_table():
             out.sum().backward()
 
 
+@pytest.mark.parametrize("n", [3, 200])
+@pytest.mark.parametrize("bad", [-1, 10])
+def test_refused_ids_leave_the_gradient_buffer_as_it_was(n, bad):
+    """A run inside a chunk and one across a border beside the id outside the table, into a sink that holds a gradient."""
+    from rl_engine.kernels.ops.sm100.model_ops import FusedEmbeddingSM100Op
+
+    table = _randn(10, 64, seed=1).requires_grad_(True)
+    sink = _randn(10, 64, seed=2)
+    before = sink.clone()
+    ids = torch.full((n,), 3, device=DEV)
+    ids[n // 2] = bad
+    out = FusedEmbeddingSM100Op()(ids, table, grad_sink=sink)
+    with pytest.raises(ValueError):
+        out.sum().backward()
+    torch.cuda.synchronize()
+    assert torch.equal(sink, before)
+
+
 # ------------------------------------------------------------------------------------------------ sampler
 def _draws(z, k, p, seed, offset):
     """The kernel's rule in fp64 on the host; a draw within 1e-5 of the border between two tokens allows both."""
