@@ -89,16 +89,10 @@ def _forward_local(hidden2d, weight, target, bias, want_lse: bool, want_entropy:
     )
 
 
-_DZ_CACHE: Dict[Tuple[int, int, int], torch.Tensor] = {}
-
-
-def _dz_workspace(device: torch.device, chunk: int, v_local: int) -> torch.Tensor:
-    v_pad = (v_local + 7) // 8 * 8
-    key = (device.index or 0, chunk, v_pad)
-    buf = _DZ_CACHE.get(key)
-    if buf is None:
-        buf = _DZ_CACHE[key] = torch.empty(chunk, v_pad, dtype=torch.bfloat16, device=device)
-    return buf
+def dz_buffer(device: torch.device, chunk: int, v_local: int) -> torch.Tensor:
+    """``[chunk, V]`` bf16 with 16-byte aligned rows for one backward pass.  From the caching allocator and not kept: two passes on
+    two streams of a device (autograd runs each on its forward's stream) must not share one."""
+    return torch.empty(chunk, (v_local + 7) // 8 * 8, dtype=torch.bfloat16, device=device)
 
 
 def accumulate_grad_weight(ext, dz, h2, grad_w, first: bool, last: bool, dtype, sink=None):
@@ -131,7 +125,7 @@ def linear_logp_backward_local(
     v = weight.shape[0]
     g = grad_logp.reshape(-1).float().contiguous()
     chunk = max(128, min(chunk_tokens, (n + 127) // 128 * 128))
-    dz_buf = _dz_workspace(hidden2d.device, chunk, v)
+    dz_buf = dz_buffer(hidden2d.device, chunk, v)
     grad_h = torch.empty(n, d, dtype=grad_hidden_dtype, device=hidden2d.device) if need_hidden else None
     grad_w = None
     if need_weight and n == 0:

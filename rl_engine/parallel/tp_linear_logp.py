@@ -122,7 +122,7 @@ class _TPLinearLogp(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_logp, _grad_ent):
-        from rl_engine.kernels.ops.sm100.linear_logp import _dz_workspace, accumulate_grad_weight
+        from rl_engine.kernels.ops.sm100.linear_logp import accumulate_grad_weight, dz_buffer
 
         ext = require_ext()
         has_bias, hidden_shape, v_start, tp_group, chunk = ctx.meta
@@ -132,7 +132,7 @@ class _TPLinearLogp(torch.autograd.Function):
         v = w.shape[0]
         ws = _WORKSPACES[(id(tp_group), h2.device.index or 0)]
         g = grad_logp.reshape(-1).float().contiguous()
-        dz_buf = _dz_workspace(h2.device, chunk, v)
+        dz_buf = dz_buffer(h2.device, chunk, v)
         grad_h = torch.empty(n, d, dtype=h2.dtype, device=h2.device)
         grad_w = torch.zeros_like(w) if ctx.needs_input_grad[1] and n == 0 else None
         grad_b = torch.zeros(v, dtype=torch.float32, device=w.device) if has_bias else None

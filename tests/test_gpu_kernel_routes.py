@@ -111,6 +111,31 @@ def test_linear_logp_weight_gradient_adds_its_chunks_in_order(n, chunk):
     assert torch.equal(w.grad, want.to(torch.bfloat16))
 
 
+def test_linear_logp_backward_passes_on_two_streams():
+    """Each stream's gradients are those of the pass on its own."""
+    from rl_engine.kernels.ops.sm100.linear_logp import FusedLinearLogpSM100Op
+
+    n, d, v = 1500, 256, 20000
+    op, streams = FusedLinearLogpSM100Op(bwd_chunk_tokens=512), [torch.cuda.Stream() for _ in range(2)]
+    w = _randn(v, d, seed=1, scale=0.1).requires_grad_(True)
+    hs = [_randn(n, d, seed=2 + i).requires_grad_(True) for i in range(2)]
+    t = torch.randint(0, v, (n,), device=DEV, generator=_gen(4))
+    g = torch.randn(n, device=DEV, generator=_gen(5))
+    want = [torch.autograd.grad(op(h, w, t), [h, w], g) for h in hs]
+    torch.cuda.synchronize()
+    for _ in range(4):
+        logps, got = [], []
+        for s, h in zip(streams, hs):
+            with torch.cuda.stream(s):
+                logps.append(op(h, w, t))
+        for s, lp, h in zip(streams, logps, hs):
+            with torch.cuda.stream(s):
+                got.append(torch.autograd.grad(lp, [h, w], g))
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
 @pytest.mark.parametrize("rows", [8, 24, 1024, 1032, 4000])
 @pytest.mark.parametrize("d", [40, 264])
 def test_rmsnorm_weight_gradient_adds_its_chunks_in_order(rows, d):
