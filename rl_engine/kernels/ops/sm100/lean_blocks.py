@@ -61,11 +61,17 @@ class _NormLinear(torch.autograd.Function):
         return dx.reshape(ctx.x_shape), (dnw if norm_sink is None else None), dw, None, None
 
 
-def _residual(residual, rows: int, cols: int):
-    """``residual`` as the addend of the GEMM's epilogue, or ``None`` if its layout is not fit."""
-    if residual is None or residual.dtype != torch.bfloat16 or cols % 8 or residual.numel() != rows * cols:
+def _residual(residual, shape):
+    """``residual`` as the addend of the GEMM's epilogue, or ``None`` where it is not fit: another shape than the product's (left
+    to the addition to broadcast or refuse), another type, rows that do not start on 16 bytes."""
+    if residual is None or residual.dtype != torch.bfloat16 or shape[-1] % 8 or residual.shape != shape or not residual.is_cuda:
         return None
-    return _as_2d(residual)
+    rows = _as_2d(residual)
+    return None if rows.data_ptr() % 16 or rows.stride(0) % 8 else rows
+
+
+def _product_shape(x: torch.Tensor, w: torch.Tensor) -> torch.Size:
+    return x.shape[:-1] + w.shape[:1]
 
 
 class _SwiGLULinear(torch.autograd.Function):
@@ -75,7 +81,7 @@ class _SwiGLULinear(torch.autograd.Function):
         w2 = _as_2d(w)
         ctx.save_for_backward(gu2, w2)
         ctx.gu_shape, ctx.sink = gate_up.shape, sink
-        y = _gemm_onto(require_ext().swiglu_packed_fwd(gu2), w2, residual)
+        y = _gemm_onto(require_ext().swiglu_packed_fwd(gu2), w2, _residual(residual, _product_shape(gate_up, w)))
         return y.reshape(*gate_up.shape[:-1], w.shape[0])
 
     @staticmethod
@@ -100,7 +106,7 @@ class _ResidualLinear(torch.autograd.Function):
         x2, w2 = _as_2d(x), _as_2d(w)
         ctx.save_for_backward(x2, w2)
         ctx.x_shape, ctx.sink = x.shape, sink
-        return _gemm_onto(x2, w2, residual).reshape(residual.shape)
+        return _gemm_onto(x2, w2, _residual(residual, residual.shape)).reshape(residual.shape)
 
     @staticmethod
     def backward(ctx, dy):
@@ -114,12 +120,12 @@ class _ResidualLinear(torch.autograd.Function):
 def _gemm_onto(x2, w2, residual):
     if residual is None:
         return gemm(x2, w2)
-    return require_ext().gemm(x2, w2, False, False, None, False, False, 1.0, -1, _residual(residual, x2.shape[0], w2.shape[0]))
+    return require_ext().gemm(x2, w2, False, False, None, False, False, 1.0, -1, residual)
 
 
 def residual_linear(residual: torch.Tensor, x: torch.Tensor, w: torch.Tensor, sink=None) -> torch.Tensor:
     """``residual + x @ w.T``: the sum is taken in the GEMM's epilogue."""
-    if _supported(x, w) and _residual(residual, x.numel() // x.shape[-1], w.shape[0]) is not None:
+    if _supported(x, w) and _residual(residual, _product_shape(x, w)) is not None:
         return _ResidualLinear.apply(residual, x, w, sink)
     from rl_engine.kernels.ops.sm100.gemm import matmul_nt
 
@@ -140,7 +146,7 @@ def swiglu_linear(gate_up: torch.Tensor, w: torch.Tensor, residual=None, sink=No
     backward."""
     f = gate_up.shape[-1] // 2
     if _supported(gate_up, w) and f % 8 == 0:
-        if residual is None or _residual(residual, gate_up.numel() // gate_up.shape[-1], w.shape[0]) is not None:
+        if residual is None or _residual(residual, _product_shape(gate_up, w)) is not None:
             return _SwiGLULinear.apply(gate_up, w, residual, sink)
         return residual + _SwiGLULinear.apply(gate_up, w, None, sink)
     from rl_engine.kernels.registry import kernel_registry

@@ -545,6 +545,33 @@ def test_nucleus_sampler_integer_masses(rows, vocab, p, shape):
         assert lo - 2e-5 * float(kept[-1]) <= t <= hi + 2e-5 * float(kept[-1])
 
 
+@pytest.mark.parametrize("form", ["dense", "odd offset", "odd pitch", "transposed", "row", "3-d", "float32"])
+def test_residuals_of_any_layout_are_added(form):
+    """Residuals that the epilogue can address and those that it cannot: the sum (each rounded once, as is the
+    product) and its gradient; a residual that does not broadcast with the product is refused, as by the addition."""
+    from rl_engine.kernels.ops.sm100.lean_blocks import residual_linear, swiglu_linear
+
+    n, k, m = 24, 64, 40
+    x, w = _randn(n, k, seed=1).requires_grad_(True), _randn(m, k, seed=2, scale=0.2).requires_grad_(True)
+    gu, wd = _randn(n, 2 * k, seed=3).requires_grad_(True), _randn(m, k, seed=4, scale=0.2)
+    make = {"dense": lambda: _randn(n, m, seed=5), "odd offset": lambda: _randn(n * m + 1, seed=5)[1:].view(n, m),
+            "odd pitch": lambda: _randn(n, m + 3, seed=5)[:, 1 : m + 1], "transposed": lambda: _randn(m, n, seed=5).t(),
+            "row": lambda: _randn(1, m, seed=5), "3-d": lambda: _randn(2, n // 2, m, seed=5),
+            "float32": lambda: _randn(n, m, seed=5, dtype=torch.float32)}[form]
+    res = make().requires_grad_(True)
+    for fused, product in ((lambda: residual_linear(res, x, w), lambda: x @ w.t()),
+                           (lambda: swiglu_linear(gu, wd, residual=res), lambda: swiglu_linear(gu, wd))):
+        if form == "3-d":
+            with pytest.raises(RuntimeError):
+                fused()
+            continue
+        got, plain = fused(), product()
+        assert got.shape == (res + plain).shape and got.dtype == (res + plain).dtype
+        assert _rel(got.detach(), res.detach().double() + plain.detach().double()) < BF16
+        (a,), (b,) = (torch.autograd.grad(out.sum(), [res]) for out in (got, res + plain))
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("micro", [None, 2])
 @pytest.mark.parametrize("chunk", [4096, 128])
 def test_gradients_added_by_the_gemms_equal_those_added_by_autograd(micro, chunk):
