@@ -336,7 +336,14 @@ namespace rlk {
 // top_k in [1, sample_topk_limit()], top_p in (0, 1] (1 disables the nucleus cut).
 void sample_topk_topp(const void* logits, long long ld, int dtype, int rows, int V, int top_k, float top_p,
                       float temperature, unsigned long long seed, unsigned long long offset, long long* out_ids,
-                      float* out_logprob, cudaStream_t stream);
+                      float* out_logprob, int sm_count, int route, cudaStream_t stream);
+enum SampleRoute : int {
+  kSampleAuto = -1,   // by size
+  kSampleRows = 0,    // one CTA per row
+  kSampleFew = 1,     // slices, bound from an eighth of each (k <= sample_few_limit())
+  kSampleFull = 2,    // slices, bound from all of each
+};
+int sample_few_limit();
 int sample_topk_limit();
 // Full-vocabulary nucleus (top-p only) / plain temperature sampling (top_p = 1).
 void sample_nucleus(const void* logits, long long ld, int dtype, int rows, int V, float top_p, float temperature,

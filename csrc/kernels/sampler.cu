@@ -1,13 +1,13 @@
-// Temperature / top-k / top-p sampling, one CTA (many rows) or one cluster of CTAs (few rows) per row of logits.
+// Temperature / top-k / top-p sampling.
 //
-//   1. a lower bound of the row's k-th largest value: the k-th largest of the maxima of 512 interleaved subsets of the first
-//      eighth of a slice (k <= 256), or of 2048 subsets of all of it (larger k) -- a bound for the row whichever part of it
-//      it comes from.  The slice is then streamed against the bound (what the first sweep read comes from L2) and what reaches it goes to
-//      a candidate buffer in shared memory: about 8 k elements, or 1.4 k, for ordinary logits.  If they do
-//      not fit (masses of ties, a row whose head is unlike its tail), the exact radix select on order-preserving 32-bit keys
-//      (integer histograms in shared memory, 12-bit first digit) takes over;
-//   2. the candidates are cut to at most 2048 by an exact radix select in shared memory where they are more, and bitonic-sorted by (logit descending, index
-//      ascending) -- a total order, so neither the gather order nor the split over CTAs matters -- and cut to the first k plus ties;
+//   1. candidates: a lower bound of the row's k-th largest value from maxima of interleaved subsets, then one streaming pass against
+//      it.  One CTA per row takes 1024 maxima of the whole row (k <= 1024); slices of a row, one CTA or a cluster, take 512 of the
+//      first eighth of each slice, or 2048 of all of it.  The m-th part of n elements has -512 ln(1 - k / 512) m elements or fewer above the
+//      bound from 512 maxima of it: 8.4 k of a row at k = 50, so the bound from an eighth is for small k.  Candidates that do not
+//      fit (masses of ties, a row whose head is unlike its tail) are found by an exact radix select on order-preserving 32-bit
+//      keys (integer histograms in shared memory, 12-bit first digit);
+//   2. slices cut what they have to their exact k-th key first where it is much more; the candidates are bitonic-sorted by (logit descending,
+//      index ascending) -- a total order, so neither the gather order nor the split over CTAs matters -- and cut to the first k plus ties;
 //   3. softmax with temperature over the candidates, inclusive scan in a fixed tree, top-p cut
 //      "keep token i iff the mass strictly before it is <= p" (first token always kept);
 //   4. inverse-CDF draw with a Philox4x32-10 uniform keyed by (seed, row, offset).
@@ -26,11 +26,11 @@ namespace rlk {
 
 namespace {
 
-constexpr int kThreads = 512;
+constexpr int kRowThreads = 1024;  // of the kernel that gives a row one CTA
+constexpr int kThreads = 512;      // of the one that gives it slices
 constexpr int kCap = 2048;       // candidates that are sorted (k <= 1024 plus ties)
 constexpr int kGather = 10240;   // candidates that are gathered: 80 KB, two CTAs per SM
-// Up to this k the bound comes from one maximum per thread over an eighth of the slice; above it from four per thread over all
-// of it (a bound from an eighth would let 8192 candidates through at k = 1024).
+// Up to this k one maximum per thread of an eighth of a slice can give the bound (at 512 there would be none left above it).
 constexpr int kFewLimit = 256;
 constexpr int kSampleShare = 8;
 constexpr int kMinSample = kThreads * 16;  // elements
@@ -144,43 +144,348 @@ __device__ __forceinline__ unsigned long long pack_candidate(uint32_t key, int i
   return (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(i));
 }
 
+// What both kernels keep in shared memory.
+struct SampleState {
+  unsigned long long cand[kCap];
+  float prob[kCap];
+  float warp_tot[32];
+  unsigned int warp_cnt[32];
+  SelectScratch select;
+  unsigned int prefix, remaining, above, pop, count, nkeep, total, bound, overflow;
+  float mass;
+};
+
+// f(vector, index of the vector) for the 16-byte vectors [v0, v1) of `p`, dealt to the block's threads, the next four in flight while
+// four are looked at; f's third argument is the vector's place among the four.
+// AHEAD false: one load at a time, for twice the blocks per SM.
+template <int THREADS, bool AHEAD = true, typename F>
+__device__ __forceinline__ void sweep_vectors(const uint4* __restrict__ p, int v0, int v1, F&& f) {
+  if constexpr (!AHEAD) {
+#pragma unroll 4
+    for (int v = v0 + static_cast<int>(threadIdx.x); v < v1; v += THREADS) f(__ldg(p + v), v, 0);
+    return;
+  }
+  constexpr int kUnroll = 4;
+  uint4 q[kUnroll];
+  int v = v0 + static_cast<int>(threadIdx.x);
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u)
+    if (v + u * THREADS < v1) q[u] = __ldg(p + v + u * THREADS);
+  while (v < v1) {
+    uint4 now[kUnroll];
+    const int at = v;
+    v += kUnroll * THREADS;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      now[u] = q[u];
+      if (v + u * THREADS < v1) q[u] = __ldg(p + v + u * THREADS);
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (at + u * THREADS < v1) f(now[u], at + u * THREADS, u);
+  }
+}
+
+// The candidates of a row by an exact radix select, digits of 12, 8, 8 and 4 bits from the top; after each the threshold bin is
+// located by a parallel suffix scan, until what lies above the bin and the bin itself fit the buffer.  hist: [4096].
+template <int THREADS, typename T>
+__device__ __forceinline__ void radix_candidates(SampleState& s, unsigned int* hist, const T* __restrict__ z, int V, int k) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    s.prefix = 0;
+    s.remaining = static_cast<unsigned int>(k);
+    s.above = 0;
+    s.pop = static_cast<unsigned int>(V);
+  }
+  __syncthreads();
+  int shift = 32;
+#pragma unroll 1
+  for (int pass = 0; pass < 4; ++pass) {
+    const int bits = pass == 0 ? 12 : (pass == 3 ? 4 : 8);
+    if (s.above + s.pop <= static_cast<unsigned int>(kCap)) break;  // uniform: shared values behind a barrier
+    const uint32_t himask = pass == 0 ? 0u : (0xffffffffu << shift);
+    shift -= bits;
+    const int nb = 1 << bits;
+    for (int i = tid; i < nb; i += THREADS) hist[i] = 0;
+    __syncthreads();
+    const uint32_t prefix = s.prefix;
+    for (int i = tid; i < V; i += THREADS) {
+      const uint32_t key = f2key(ldv(z, i));
+      if ((key & himask) == prefix) atomicAdd(&hist[(key >> shift) & static_cast<uint32_t>(nb - 1)], 1u);
+    }
+    __syncthreads();
+    // thread t owns `per` consecutive bins, highest bins first; block-wide exclusive scan of the per-thread sums
+    const int per = (nb + THREADS - 1) / THREADS;
+    const int top = nb - 1 - tid * per;  // highest bin of this thread
+    unsigned int mine = 0;
+    for (int j = 0; j < per; ++j)
+      if (top - j >= 0) mine += hist[top - j];
+    unsigned int incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned int o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+    if (lane == 31) s.warp_cnt[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      unsigned int w = lane < THREADS / 32 ? s.warp_cnt[lane] : 0u;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned int o = __shfl_up_sync(0xffffffffu, w, off);
+        if (lane >= off) w += o;
+      }
+      if (lane < THREADS / 32) s.warp_cnt[lane] = w;
+    }
+    __syncthreads();
+    const unsigned int before = (warp == 0 ? 0u : s.warp_cnt[warp - 1]) + (incl - mine);  // count in higher bins
+    const unsigned int need = s.remaining;
+    __syncthreads();
+    if (before < need && need <= before + mine) {  // exactly one thread: the threshold bin is one of its bins
+      unsigned int acc = before;
+      int bsel = top;
+      for (int j = 0; j < per; ++j) {
+        bsel = top - j;
+        if (acc + hist[bsel] >= need) break;
+        acc += hist[bsel];
+      }
+      s.prefix = prefix | (static_cast<uint32_t>(bsel) << shift);
+      s.remaining = need - acc;
+      s.above += acc;
+      s.pop = hist[bsel];
+    }
+    __syncthreads();
+  }
+  const uint32_t from = s.prefix;  // everything above the threshold bin plus the bin itself
+  if (tid == 0) s.count = 0;
+  __syncthreads();
+  for (int i = tid; i < V; i += THREADS) {
+    const uint32_t key = f2key(ldv(z, i));
+    if (key >= from) {
+      const unsigned int slot = atomicAdd(&s.count, 1u);
+      if (slot < kCap) s.cand[slot] = pack_candidate(key, i);
+    }
+  }
+  __syncthreads();
+}
+
+// Sorts the s.count candidates, cuts them to the first k plus ties, and draws.  The sums are a fixed tree whatever the number of
+// threads (pairs of candidates, groups of 32 pairs, the groups): the draw does not depend on which kernel found the candidates.
+template <int THREADS>
+__device__ __forceinline__ void sort_and_draw(SampleState& s, int k, float top_p, float inv_temp, unsigned long long seed,
+                                              unsigned long long offset, int row, long long* __restrict__ out_ids,
+                                              float* __restrict__ out_logprob) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int n = static_cast<int>(s.count < static_cast<unsigned int>(kCap) ? s.count : kCap);
+  // sort only as many slots as the candidates need (a power of two >= n, at least 64): the usual few dozen
+  // candidates take 21 compare-exchange rounds instead of the 66 of the full buffer
+  int sort_n = 64;
+  while (sort_n < n) sort_n <<= 1;
+  for (int i = n + tid; i < sort_n; i += THREADS) s.cand[i] = 0ull;
+  __syncthreads();
+  // bitonic sort, descending, sort_n elements.  Pairs t = 32 w .. 32 w + 31 at strides up to 32 stay inside the 64 elements
+  // [64 w, 64 w + 64), which one warp owns, so those rounds need no block barrier.
+  for (int size = 2; size <= sort_n; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int t = tid; t < sort_n / 2; t += THREADS) {
+        const int lo = 2 * t - (t & (stride - 1));
+        const int hi = lo + stride;
+        const bool desc = ((lo & size) == 0);
+        const unsigned long long a = s.cand[lo], b = s.cand[hi];
+        if ((a < b) == desc) {
+          s.cand[lo] = b;
+          s.cand[hi] = a;
+        }
+      }
+      if (stride > 32 || (stride == 1 && size >= 64)) __syncthreads();  // the next round crosses the warps' blocks
+      else __syncwarp();
+    }
+  }
+
+  // the candidates may extend below the k-th largest value: keep the first k and everything tied with the k-th
+  {
+    const uint32_t kth_key = static_cast<uint32_t>(s.cand[(k < n ? k : n) - 1] >> 32);
+    if (tid == 0) s.count = 0;
+    __syncthreads();
+    unsigned int local = 0;
+    for (int i = tid; i < n; i += THREADS)
+      if (static_cast<uint32_t>(s.cand[i] >> 32) >= kth_key) ++local;
+    if (local) atomicAdd(&s.count, local);
+    __syncthreads();
+    n = static_cast<int>(s.count);
+  }
+
+  // softmax over the candidates + inclusive scan (fixed tree) + top-p cut
+  const float zmax = key2f(static_cast<uint32_t>(s.cand[0] >> 32));
+  constexpr int kPairs = kCap / 2 / THREADS;  // consecutive pairs of candidates per thread
+  static_assert(kPairs == 1 || kPairs == 2, "512 or 1024 threads");
+  float e[2 * kPairs], pair[kPairs], incl[kPairs];
+#pragma unroll
+  for (int j = 0; j < 2 * kPairs; ++j) {
+    const int i = 2 * kPairs * tid + j;
+    e[j] = i < n ? expf((key2f(static_cast<uint32_t>(s.cand[i] >> 32)) - zmax) * inv_temp) : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < kPairs; ++j) incl[j] = pair[j] = e[2 * j] + e[2 * j + 1];
+  // inclusive scan of 32 pairs: a warp's, or half a warp's where a thread holds two of them
+  const int group = tid * kPairs / 32;
+  if constexpr (kPairs == 1) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const float o = __shfl_up_sync(0xffffffffu, incl[0], off);
+      if (lane >= off) incl[0] += o;
+    }
+  } else {
+    const int l = lane & 15;
+    const float left = __shfl_up_sync(0xffffffffu, incl[1], 1, 16);
+    incl[1] += incl[0];
+    if (l >= 1) incl[0] += left;
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+      const float o0 = __shfl_up_sync(0xffffffffu, incl[0], off, 16), o1 = __shfl_up_sync(0xffffffffu, incl[1], off, 16);
+      if (l >= off) {
+        incl[0] += o0;
+        incl[1] += o1;
+      }
+    }
+  }
+  if ((tid * kPairs + kPairs) % 32 == 0) s.warp_tot[group] = incl[kPairs - 1];
+  __syncthreads();
+  if (warp == 0) {
+    float w = s.warp_tot[lane];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const float o = __shfl_up_sync(0xffffffffu, w, off);
+      if (lane >= off) w += o;
+    }
+    s.warp_tot[lane] = w;  // inclusive over groups
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kPairs; ++j) {
+    const float base = (group == 0 ? 0.f : s.warp_tot[group - 1]) + (incl[j] - pair[j]);  // mass before the pair
+    const int i = 2 * (kPairs * tid + j);
+    s.prob[i] = base + e[2 * j];
+    s.prob[i + 1] = base + e[2 * j] + e[2 * j + 1];
+  }
+  __syncthreads();
+  const float total = s.warp_tot[31];
+  if (tid == 0) s.nkeep = 0;
+  __syncthreads();
+  // keep i iff mass strictly before i <= p * total ; kept set is a prefix, so count it
+  {
+    const float lim = top_p * total;
+    unsigned int local = 0;
+#pragma unroll
+    for (int j = 0; j < 2 * kPairs; ++j) {
+      const int i = 2 * kPairs * tid + j;
+      if (i < n && (i == 0 || s.prob[i - 1] <= lim)) ++local;
+    }
+    if (local) atomicAdd(&s.nkeep, local);
+  }
+  __syncthreads();
+  if (tid != 0) return;
+  // inverse-CDF draw
+  const int nkeep = s.nkeep < 1u ? 1 : static_cast<int>(s.nkeep);
+  const float mass = s.prob[nkeep - 1];
+  const uint4 rnd = philox4x32_10(
+      make_uint4(static_cast<uint32_t>(offset), static_cast<uint32_t>(offset >> 32), static_cast<uint32_t>(row), 0u),
+      make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32)));
+  const float u = (static_cast<float>(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
+  const float target = u * mass;
+  int lo = 0, hi = nkeep - 1;  // first i with prob[i] > target
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (s.prob[mid] > target) hi = mid;
+    else lo = mid + 1;
+  }
+  out_ids[row] = static_cast<long long>(0xffffffffu - static_cast<uint32_t>(s.cand[lo] & 0xffffffffu));
+  if (out_logprob) out_logprob[row] = logf((s.prob[lo] - (lo ? s.prob[lo - 1] : 0.f)) / mass);
+}
+
+// One CTA per row, TWO of them to an SM or one that keeps more loads in flight.  The bound is the k-th largest of 1024 interleaved
+// maxima of the whole row.
+template <typename T, bool TWO>
+__global__ void __launch_bounds__(kRowThreads, TWO ? 2 : 1)
+sample_rows_kernel(const T* __restrict__ logits, long long ld, int V, int top_k, float top_p, float inv_temp, unsigned long long seed,
+                   unsigned long long offset, long long* __restrict__ out_ids, float* __restrict__ out_logprob) {
+  __shared__ unsigned int hist[4096];
+  __shared__ SampleState s;
+  const int row = static_cast<int>(blockIdx.x), tid = threadIdx.x;
+  const T* z = logits + static_cast<long long>(row) * ld;
+  const int k = top_k < 1 ? 1 : (top_k > V ? V : top_k);
+  constexpr int kVec = 16 / sizeof(T);
+  int head = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(z) & 15u)) & 15u) / sizeof(T));
+  if (head > V) head = V;
+  const int nvec = (V - head) / kVec, tail = head + nvec * kVec, rest = head + (V - tail);
+  const uint4* p = reinterpret_cast<const uint4*>(z + head);
+  auto rest_at = [&](int i) { return i < head ? i : tail + (i - head); };
+  if (tid == 0) s.count = 0;
+  uint32_t best = 0u;  // smaller than the key of any number
+  sweep_vectors<kRowThreads, !TWO>(p, 0, nvec, [&](const uint4& q, int, int) {
+    const T* e = reinterpret_cast<const T*>(&q);
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) best = max(best, f2key(ldv(e, j)));
+  });
+  for (int i = tid; i < rest; i += kRowThreads) best = max(best, f2key(ldv(z, rest_at(i))));
+  // two digits (sign, exponent, seven mantissa bits) are enough: a bound a little lower costs a few more candidates
+  const uint32_t from = block_kth_key<2>(s.select, static_cast<unsigned int>(k), [&](auto&& f) { f(best, true); });
+  auto keep = [&](uint32_t key, int i) {
+    const unsigned int slot = atomicAdd(&s.count, 1u);
+    if (slot < kCap) s.cand[slot] = pack_candidate(key, i);
+  };
+  sweep_vectors<kRowThreads, !TWO>(p, 0, nvec, [&](const uint4& q, int v, int) {
+    const T* e = reinterpret_cast<const T*>(&q);
+    uint32_t kk[kVec], top = 0u;
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) {
+      kk[j] = f2key(ldv(e, j));
+      top = max(top, kk[j]);
+    }
+    if (top >= from) {
+#pragma unroll
+      for (int j = 0; j < kVec; ++j)
+        if (kk[j] >= from) keep(kk[j], head + v * kVec + j);
+    }
+  });
+  for (int i = tid; i < rest; i += kRowThreads) {
+    const uint32_t key = f2key(ldv(z, rest_at(i)));
+    if (key >= from) keep(key, rest_at(i));
+  }
+  __syncthreads();
+  const bool fits = s.count <= static_cast<unsigned int>(kCap);  // uniform
+  __syncthreads();
+  if (!fits) radix_candidates<kRowThreads>(s, hist, z, V, k);
+  sort_and_draw<kRowThreads>(s, k, top_p, inv_temp, seed, offset, row, out_ids, out_logprob);
+}
+
+// One CTA or a cluster of CTAs per row, each with a contiguous slice of its 16-byte vectors (the unaligned head and the tail of the row go
+// to the first).  The bound is the k-th largest of 512 interleaved maxima of the first eighth of a slice (`few`), or of 2048 of
+// all of it -- a bound for the row whichever part of it it comes from; the slice is then streamed against it (what the first
+// sweep read comes from L2).
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2)
-sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int top_k, float top_p, float inv_temp,
-                        unsigned long long seed, unsigned long long offset, long long* __restrict__ out_ids,
-                        float* __restrict__ out_logprob) {
+sample_slices_kernel(const T* __restrict__ logits, long long ld, int V, int top_k, float top_p, float inv_temp,
+                     unsigned long long seed, unsigned long long offset, long long* __restrict__ out_ids,
+                     float* __restrict__ out_logprob, bool few) {
   extern __shared__ unsigned long long gather_buf[];  // [kGather]
   unsigned int* hist = reinterpret_cast<unsigned int*>(gather_buf);  // [4096], the radix select over the row only
-  __shared__ unsigned long long cand[kCap];
-  __shared__ float prob[kCap];
-  __shared__ float warp_tot[kThreads / 32];
-  __shared__ unsigned int warp_cnt[kThreads / 32];
-  __shared__ SelectScratch select;
-  __shared__ unsigned int s_prefix, s_remaining, s_above, s_pop, s_count, s_nkeep, s_total, s_bound, s_overflow;
-  __shared__ float s_mass;
+  __shared__ SampleState s;
 
   const int parts = static_cast<int>(cluster_size_x()), part = static_cast<int>(cluster_ctarank());
   const int row = static_cast<int>(blockIdx.x) / parts;
   const T* z = logits + static_cast<long long>(row) * ld;
   const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
   const int k = top_k < 1 ? 1 : (top_k > V ? V : top_k);
 
   if (tid == 0) {
-    s_prefix = 0;
-    s_remaining = static_cast<unsigned int>(k);
-    s_above = 0;
-    s_pop = static_cast<unsigned int>(V);
-    s_count = 0;
-    s_total = 0;
-    s_bound = 0;
-    s_overflow = 0;
+    s.count = 0;
+    s.total = 0;
+    s.bound = 0;
+    s.overflow = 0;
   }
   __syncthreads();
   if (parts > 1) cluster_sync();  // the first CTA's counters are set before anyone adds to them
-
-  // ---- 1. bound from the maxima of a first sweep, then one streaming pass.  The 16-byte vectors of the row
-  //         are dealt to the CTAs in contiguous slices; the unaligned head and the tail of the row go to the first.
   {
     constexpr int kVec = 16 / sizeof(T);
     int head = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(z) & 15u)) & 15u) / sizeof(T));
@@ -190,55 +495,29 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
     const int v0 = min(nvec, part * per), v1 = min(nvec, v0 + per);
     const uint4* p = reinterpret_cast<const uint4*>(z + head);
     constexpr int kUnroll = 4;
-    // f(vector, index) for the vectors [v0, end) dealt to this thread, the next four in flight while four are looked at
-    auto sweep = [&](int end, auto&& f) {
-      uint4 q[kUnroll];
-      int v = v0 + tid;
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
-        if (v + u * kThreads < end) q[u] = __ldg(p + v + u * kThreads);
-      while (v < end) {
-        uint4 now[kUnroll];
-        const int at = v;
-        v += kUnroll * kThreads;
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-          now[u] = q[u];
-          if (v + u * kThreads < end) q[u] = __ldg(p + v + u * kThreads);
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
-          if (at + u * kThreads < end) f(now[u], at + u * kThreads, u);
-      }
-    };
     uint32_t best[kUnroll] = {0u, 0u, 0u, 0u};  // smaller than the key of any number
-    // In a cluster every CTA lets about k x (slice / sample) candidates through, and what all of them send has to fit the
-    // first one's sort buffer: 200 of 77420 in four slices overflowed it (43 us instead of 22 through the exact radix select).
-    const int part_sample = min(v1 - v0, max((v1 - v0) / kSampleShare, kMinSample / kVec));
-    const bool few = k <= kFewLimit &&
-                     (parts == 1 || static_cast<long long>(k) * parts * (v1 - v0) <= static_cast<long long>(kCap) * 3 / 4 * part_sample);
-    const int sample = few ? part_sample : v1 - v0;
-    sweep(v0 + sample, [&](const uint4& q, int, int u) {
+    const int sample = few ? min(v1 - v0, max((v1 - v0) / kSampleShare, kMinSample / kVec)) : v1 - v0;
+    sweep_vectors<kThreads>(p, v0, v0 + sample, [&](const uint4& q, int, int u) {
       const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
       for (int j = 0; j < kVec; ++j) best[u] = max(best[u], f2key(ldv(e, j)));
     });
-    // two digits (sign, exponent, seven mantissa bits) are enough: a bound a little lower costs a few more candidates
+    // two digits, as above
     uint32_t from;
     if (few) {
       const uint32_t top = max(max(best[0], best[1]), max(best[2], best[3]));
-      from = block_kth_key<2>(select, static_cast<unsigned int>(k), [&](auto&& f) { f(top, true); });
+      from = block_kth_key<2>(s.select, static_cast<unsigned int>(k), [&](auto&& f) { f(top, true); });
     } else {
-      from = block_kth_key<2>(select, static_cast<unsigned int>(k), [&](auto&& f) {
+      from = block_kth_key<2>(s.select, static_cast<unsigned int>(k), [&](auto&& f) {
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) f(best[u], true);
       });
     }
     auto keep = [&](uint32_t kk, int i) {
-      const unsigned int slot = atomicAdd(&s_count, 1u);
+      const unsigned int slot = atomicAdd(&s.count, 1u);
       if (slot < kGather) gather_buf[slot] = pack_candidate(kk, i);
     };
-    sweep(v1, [&](const uint4& q, int v, int) {
+    sweep_vectors<kThreads>(p, v0, v1, [&](const uint4& q, int v, int) {
       const T* e = reinterpret_cast<const T*>(&q);
       uint32_t kk[kVec], top = 0u;
 #pragma unroll
@@ -261,246 +540,61 @@ sample_topk_topp_kernel(const T* __restrict__ logits, long long ld, int V, int t
       }
     }
     __syncthreads();
+    // the exact k-th key of the candidates of a slice: fewer of them leave it, or are sorted
+    const unsigned int have = s.count;
+    uint32_t bound = from;
+    if (have > static_cast<unsigned int>(kGather)) {
+      if (tid == 0) {
+        if (parts > 1) cluster_max_u32(mapa_u32(smem_u32(&s.overflow), 0), 1u);
+        else s.overflow = 1u;
+      }
+    } else if (have > static_cast<unsigned int>(parts > 1 ? 2 * k : kCap)) {
+      const int rounds = static_cast<int>((have + kThreads - 1) / kThreads);
+      bound = block_kth_key<4>(s.select, static_cast<unsigned int>(k), [&](auto&& f) {
+        for (int r = 0; r < rounds; ++r) {
+          const unsigned int i = r * kThreads + tid;
+          const bool in = i < have;
+          f(in ? static_cast<uint32_t>(gather_buf[i] >> 32) : 0u, in);
+        }
+      });
+    }
+    const unsigned int mine = min(have, static_cast<unsigned int>(kGather));
     if (parts > 1) {
       // the highest bound of the cluster holds for the row; what reaches it goes to the first CTA's sort buffer
-      const uint32_t bound0 = mapa_u32(smem_u32(&s_bound), 0), total0 = mapa_u32(smem_u32(&s_total), 0);
-      const uint32_t over0 = mapa_u32(smem_u32(&s_overflow), 0), cand0 = mapa_u32(smem_u32(cand), 0);
-      if (tid == 0) {
-        cluster_max_u32(bound0, from);
-        if (s_count > static_cast<unsigned int>(kGather)) cluster_max_u32(over0, 1u);
-      }
+      const uint32_t bound0 = mapa_u32(smem_u32(&s.bound), 0), total0 = mapa_u32(smem_u32(&s.total), 0);
+      const uint32_t cand0 = mapa_u32(smem_u32(s.cand), 0);
+      if (tid == 0) cluster_max_u32(bound0, bound);
       cluster_sync();
-      uint32_t bound;
       asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(bound) : "r"(bound0) : "memory");
-      const int mine = static_cast<int>(min(s_count, static_cast<unsigned int>(kGather)));
-      for (int i = tid; i < mine; i += kThreads) {
-        const unsigned long long c = gather_buf[i];
-        if (static_cast<uint32_t>(c >> 32) >= bound) {
-          const unsigned int slot = cluster_add_u32(total0, 1u);
-          if (slot < kCap) cluster_store_u64(cand0 + slot * 8u, c);
-        }
+      for (unsigned int i0 = 0; i0 < mine; i0 += kThreads) {  // slots are reserved once per warp
+        const unsigned int i = i0 + tid;
+        const unsigned long long c = i < mine ? gather_buf[i] : 0ull;
+        const bool send = i < mine && static_cast<uint32_t>(c >> 32) >= bound;
+        const unsigned int who = __ballot_sync(0xffffffffu, send);
+        unsigned int slot = 0u;
+        if ((tid & 31) == 0 && who != 0u) slot = cluster_add_u32(total0, static_cast<unsigned int>(__popc(who)));
+        slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(who & ((1u << (tid & 31)) - 1u));
+        if (send && slot < kCap) cluster_store_u64(cand0 + slot * 8u, c);
       }
       cluster_sync();
       if (part != 0) return;  // nothing of this CTA is read any more
     } else {
-      const unsigned int have = s_count;
-      if (have > static_cast<unsigned int>(kGather)) {
-        if (tid == 0) s_overflow = 1u;
-      } else {
-        uint32_t bound = 0u;
-        if (have > static_cast<unsigned int>(kCap)) {  // exact k-th key of the candidates
-          const int rounds = static_cast<int>((have + kThreads - 1) / kThreads);
-          bound = block_kth_key<4>(select, static_cast<unsigned int>(k), [&](auto&& f) {
-            for (int r = 0; r < rounds; ++r) {
-              const unsigned int i = r * kThreads + tid;
-              const bool in = i < have;
-              f(in ? static_cast<uint32_t>(gather_buf[i] >> 32) : 0u, in);
-            }
-          });
-        }
-        for (unsigned int i = tid; i < have; i += kThreads) {
-          const unsigned long long c = gather_buf[i];
-          if (static_cast<uint32_t>(c >> 32) >= bound) {
-            const unsigned int slot = atomicAdd(&s_total, 1u);
-            if (slot < kCap) cand[slot] = c;
-          }
+      for (unsigned int i = tid; i < mine; i += kThreads) {
+        const unsigned long long c = gather_buf[i];
+        if (static_cast<uint32_t>(c >> 32) >= bound) {
+          const unsigned int slot = atomicAdd(&s.total, 1u);
+          if (slot < kCap) s.cand[slot] = c;
         }
       }
     }
     __syncthreads();
-    if (tid == 0) s_count = s_total;
+    if (tid == 0) s.count = s.total;
     __syncthreads();
   }
-  // uniform over the block.  Otherwise: radix select over the row, digits of 12, 8, 8 and 4 bits from the top; after each the
-  // threshold bin is located by a parallel suffix scan, until what lies above the bin and the bin itself fit the buffer.
-  const bool gathered = s_overflow == 0u && s_count <= static_cast<unsigned int>(kCap);
+  const bool fits = s.overflow == 0u && s.count <= static_cast<unsigned int>(kCap);  // uniform
   __syncthreads();
-  int shift = 32;
-#pragma unroll 1
-  for (int pass = 0; pass < 4 && !gathered; ++pass) {
-    const int bits = pass == 0 ? 12 : (pass == 3 ? 4 : 8);
-    if (s_above + s_pop <= static_cast<unsigned int>(kCap)) break;  // uniform: shared values behind a barrier
-    const uint32_t himask = pass == 0 ? 0u : (0xffffffffu << shift);
-    shift -= bits;
-    const int nb = 1 << bits;
-    for (int i = tid; i < nb; i += kThreads) hist[i] = 0;
-    __syncthreads();
-    const uint32_t prefix = s_prefix;
-    for (int i = tid; i < V; i += kThreads) {
-      const uint32_t key = f2key(ldv(z, i));
-      if ((key & himask) == prefix) atomicAdd(&hist[(key >> shift) & static_cast<uint32_t>(nb - 1)], 1u);
-    }
-    __syncthreads();
-    // thread t owns `per` consecutive bins, highest bins first; block-wide exclusive scan of the per-thread sums
-    const int per = (nb + kThreads - 1) / kThreads;
-    const int top = nb - 1 - tid * per;  // highest bin of this thread
-    unsigned int mine = 0;
-    for (int j = 0; j < per; ++j)
-      if (top - j >= 0) mine += hist[top - j];
-    unsigned int incl = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const unsigned int o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    if (lane == 31) warp_cnt[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      unsigned int w = lane < kThreads / 32 ? warp_cnt[lane] : 0u;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const unsigned int o = __shfl_up_sync(0xffffffffu, w, off);
-        if (lane >= off) w += o;
-      }
-      if (lane < kThreads / 32) warp_cnt[lane] = w;
-    }
-    __syncthreads();
-    const unsigned int before = (warp == 0 ? 0u : warp_cnt[warp - 1]) + (incl - mine);  // count in higher bins
-    const unsigned int need = s_remaining;
-    __syncthreads();
-    if (before < need && need <= before + mine) {  // exactly one thread: the threshold bin is one of its bins
-      unsigned int acc = before;
-      int bsel = top;
-      for (int j = 0; j < per; ++j) {
-        bsel = top - j;
-        if (acc + hist[bsel] >= need) break;
-        acc += hist[bsel];
-      }
-      s_prefix = prefix | (static_cast<uint32_t>(bsel) << shift);
-      s_remaining = need - acc;
-      s_above += acc;
-      s_pop = hist[bsel];
-    }
-    __syncthreads();
-  }
-  // keys >= gather_from are candidates: everything above the threshold bin plus the bin itself
-  const uint32_t gather_from = s_prefix;
-
-  // ---- 2. gather the candidates (unless 1a already did), then sort (key desc, index asc)
-  if (!gathered) {
-    if (tid == 0) s_count = 0;
-    __syncthreads();
-    for (int i = tid; i < V; i += kThreads) {
-      const uint32_t key = f2key(ldv(z, i));
-      if (key >= gather_from) {
-        const unsigned int slot = atomicAdd(&s_count, 1u);
-        if (slot < kCap) cand[slot] = (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(i));
-      }
-    }
-    __syncthreads();
-  }
-  int n = static_cast<int>(s_count < static_cast<unsigned int>(kCap) ? s_count : kCap);
-  // sort only as many slots as the candidates need (a power of two >= n, at least 64): the usual few dozen
-  // candidates take 21 compare-exchange rounds instead of the 66 of the full buffer
-  int sort_n = 64;
-  while (sort_n < n) sort_n <<= 1;
-  for (int i = n + tid; i < sort_n; i += kThreads) cand[i] = 0ull;
-  __syncthreads();
-  // bitonic sort, descending, sort_n elements.  Pairs t = 32 w .. 32 w + 31 at strides up to 32 stay inside the 64 elements
-  // [64 w, 64 w + 64), which one warp owns, so those rounds need no block barrier.
-  for (int size = 2; size <= sort_n; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = tid; t < sort_n / 2; t += kThreads) {
-        const int lo = 2 * t - (t & (stride - 1));
-        const int hi = lo + stride;
-        const bool desc = ((lo & size) == 0);
-        const unsigned long long a = cand[lo], b = cand[hi];
-        if ((a < b) == desc) {
-          cand[lo] = b;
-          cand[hi] = a;
-        }
-      }
-      if (stride > 32 || (stride == 1 && size >= 64)) __syncthreads();  // the next round crosses the warps' blocks
-      else __syncwarp();
-    }
-  }
-
-  // the gathered set may extend below the k-th largest value: keep the first k and everything tied with the k-th
-  {
-    const uint32_t kth_key = static_cast<uint32_t>(cand[(k < n ? k : n) - 1] >> 32);
-    if (tid == 0) s_count = 0;
-    __syncthreads();
-    unsigned int local = 0;
-    for (int i = tid; i < n; i += kThreads)
-      if (static_cast<uint32_t>(cand[i] >> 32) >= kth_key) ++local;
-    if (local) atomicAdd(&s_count, local);
-    __syncthreads();
-    n = static_cast<int>(s_count);
-  }
-
-  // ---- 3. softmax over candidates + inclusive scan (fixed tree) + top-p cut
-  const float zmax = key2f(static_cast<uint32_t>(cand[0] >> 32));
-  constexpr int kEach = kCap / kThreads;  // consecutive candidates per thread
-  float e[kEach], own = 0.f;
-#pragma unroll
-  for (int j = 0; j < kEach; ++j) {
-    const int i = kEach * tid + j;
-    e[j] = i < n ? expf((key2f(static_cast<uint32_t>(cand[i] >> 32)) - zmax) * inv_temp) : 0.f;
-    own += e[j];
-  }
-  float incl = own;  // thread total, then warp inclusive scan
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const float o = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += o;
-  }
-  if (lane == 31) warp_tot[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    float w = lane < kThreads / 32 ? warp_tot[lane] : 0.f;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const float o = __shfl_up_sync(0xffffffffu, w, off);
-      if (lane >= off) w += o;
-    }
-    if (lane < kThreads / 32) warp_tot[lane] = w;  // inclusive over warps
-  }
-  __syncthreads();
-  {
-    float run = (warp == 0 ? 0.f : warp_tot[warp - 1]) + (incl - own);  // mass before this thread's candidates
-#pragma unroll
-    for (int j = 0; j < kEach; ++j) prob[kEach * tid + j] = run += e[j];
-  }
-  __syncthreads();
-  const float total = warp_tot[kThreads / 32 - 1];
-  if (tid == 0) s_nkeep = 0;
-  __syncthreads();
-  // keep i iff mass strictly before i <= p * total ; kept set is a prefix, so count it
-  {
-    const float lim = top_p * total;
-    unsigned int local = 0;
-#pragma unroll
-    for (int j = 0; j < kEach; ++j) {
-      const int i = kEach * tid + j;
-      if (i < n && (i == 0 || prob[i - 1] <= lim)) ++local;
-    }
-    if (local) atomicAdd(&s_nkeep, local);
-  }
-  __syncthreads();
-  const int nkeep = s_nkeep < 1u ? 1 : static_cast<int>(s_nkeep);
-  if (tid == 0) s_mass = prob[nkeep - 1];
-  __syncthreads();
-
-  // ---- 4. inverse-CDF draw
-  if (tid == 0) {
-    const uint4 rnd = philox4x32_10(
-        make_uint4(static_cast<uint32_t>(offset), static_cast<uint32_t>(offset >> 32), static_cast<uint32_t>(row), 0u),
-        make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32)));
-    const float u = (static_cast<float>(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    const float target = u * s_mass;
-    int lo = 0, hi = nkeep - 1;  // first i with prob[i] > target
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (prob[mid] > target) hi = mid;
-      else lo = mid + 1;
-    }
-    const unsigned long long c = cand[lo];
-    out_ids[row] = static_cast<long long>(0xffffffffu - static_cast<uint32_t>(c & 0xffffffffu));
-    if (out_logprob) {
-      const float e = prob[lo] - (lo ? prob[lo - 1] : 0.f);
-      out_logprob[row] = logf(e / s_mass);
-    }
-  }
+  if (!fits) radix_candidates<kThreads>(s, hist, z, V, k);
+  sort_and_draw<kThreads>(s, k, top_p, inv_temp, seed, offset, row, out_ids, out_logprob);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -856,23 +950,48 @@ void sample_nucleus(const void* logits, long long ld, int dtype, int rows, int V
 namespace {
 
 // CTAs per row: enough for two on every SM, at most eight (the portable cluster size), and slices of at least twice the
-// smallest sample: below that the merge is not repaid.  No more than leave room for k x 3 / 2 candidates of each in the first
+// smallest sample: below that the merge is not repaid.  No more than leave room for 3 / 2 k candidates of each in the first
 // one's sort buffer.
-int sample_parts(int rows, int V, int k) {
+int sample_parts(int rows, int V, int k, int sm_count) {
   int parts = 1;
-  while (parts < 8 && static_cast<long long>(rows) * parts * 2 <= 296 && V / (parts * 2) >= 2 * kMinSample) parts *= 2;
+  while (parts < 8 && static_cast<long long>(rows) * parts <= sm_count && V / (parts * 2) >= 2 * kMinSample) parts *= 2;
   while (parts > 1 && static_cast<long long>(parts) * k * 3 > 2 * kCap) parts /= 2;
   return parts;
 }
 
+// Which kernel, measured over k = 1 .. 1000, 1 .. 256 rows, 5000 .. 151936 columns, fp32 and bf16 (us on one GPU; the draws are the
+// same bits).  Rows that leave SMs idle get a CTA each, with deep loads (37 x 128256 fp32, k = 50: 19 against 23 with one load at a
+// time); slices only where few long rows and a small k repay the cluster (1 x 151936, k = 20: 13 against 19; k = 100: no gain; 37
+// rows: 27 against 21), or where k is so large that the bound from 1024 maxima lets through more than can be sorted (1 x 151936, k =
+// 1000: 48 against 77).  More rows than SMs: two CTAs per SM (256 x 61000 bf16, k = 100: 23, slices 37).  Slices for the smallest k,
+// for long rows with a small one, which they read once and an eighth (256 x 151936 fp32, k = 50: 48 against 59; k = 100: 61 against 60),
+// for short rows, which suit their 512 threads (256 x 16000, k = 20: 12 against 14), and for the largest (256 x 128256, k = 1000: 88
+// against 145).
+int sample_route(int rows, int V, int k, int elem, int sm_count) {
+  if (rows <= sm_count) {
+    if (k > 800 && V > kMinSample) return kSampleFull;
+    return rows * 7 <= sm_count && V >= 9 * kMinSample && k * 3000 <= V ? kSampleFew : kSampleRows;
+  }
+  const bool long_rows = static_cast<long long>(V) * elem >= 384 << 10;
+  if (k <= 10 || (k <= 64 && (long_rows || V <= 2 * kMinSample)) || (k <= kFewLimit && V <= kMinSample)) return kSampleFew;
+  return k > (V > kMinSample ? 640 : 800) ? kSampleFull : kSampleRows;
+}
+
 template <typename T>
 void launch_sample(const void* logits, long long ld, int rows, int V, int top_k, float top_p, float inv_temp,
-                   unsigned long long seed, unsigned long long offset, long long* out_ids, float* out_logprob, cudaStream_t stream) {
-  auto kernel = sample_topk_topp_kernel<T>;
+                   unsigned long long seed, unsigned long long offset, long long* out_ids, float* out_logprob, int sm_count, int route,
+                   cudaStream_t stream) {
+  const int parts = sample_parts(rows, V, top_k, sm_count);
+  if (route == kSampleAuto) route = sample_route(rows, V, top_k, sizeof(T), sm_count);
+  if (route == kSampleRows) {
+    auto kernel = rows > sm_count ? sample_rows_kernel<T, true> : sample_rows_kernel<T, false>;
+    kernel<<<rows, kRowThreads, 0, stream>>>(static_cast<const T*>(logits), ld, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob);
+    return;
+  }
+  auto kernel = sample_slices_kernel<T>;
   constexpr int kBytes = kGather * 8;
   static PerDeviceOnce configured;
   if (configured.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-  const int parts = sample_parts(rows, V, top_k);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * parts);
   cfg.blockDim = dim3(kThreads);
@@ -885,21 +1004,27 @@ void launch_sample(const void* logits, long long ld, int rows, int V, int top_k,
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<const T*>(logits), ld, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob);
+  const bool few = route == kSampleFew;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<const T*>(logits), ld, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, few);
 }
 
 }  // namespace
 
 void sample_topk_topp(const void* logits, long long ld, int dtype, int rows, int V, int top_k, float top_p,
                       float temperature, unsigned long long seed, unsigned long long offset, long long* out_ids,
-                      float* out_logprob, cudaStream_t stream) {
+                      float* out_logprob, int sm_count, int route, cudaStream_t stream) {
   if (rows <= 0) return;
   const float inv_temp = 1.f / temperature;
-  if (dtype == 0) launch_sample<float>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, stream);
-  else if (dtype == 1)
-    launch_sample<__nv_bfloat16>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, stream);
-  else launch_sample<__half>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob, stream);
+  auto launch = [&](auto* typed) {
+    launch_sample<std::remove_pointer_t<decltype(typed)>>(logits, ld, rows, V, top_k, top_p, inv_temp, seed, offset, out_ids, out_logprob,
+                                                          sm_count, route, stream);
+  };
+  if (dtype == 0) launch(static_cast<float*>(nullptr));
+  else if (dtype == 1) launch(static_cast<__nv_bfloat16*>(nullptr));
+  else launch(static_cast<__half*>(nullptr));
 }
+
+int sample_few_limit() { return kFewLimit; }
 
 int sample_topk_limit() { return 1024; }
 

@@ -1309,8 +1309,10 @@ void adamw(Tensor p, std::optional<Tensor> master, const Tensor& g, Tensor m, Te
 
 // ---------------------------------------------------------------------------------- sampler
 std::vector<Tensor> sample(const Tensor& logits, int64_t top_k, double top_p, double temperature, int64_t seed,
-                           int64_t offset, bool want_logprob) {
+                           int64_t offset, bool want_logprob, int64_t route) {
   check_rowmajor(logits, "logits");
+  TORCH_CHECK(route >= rlk::kSampleAuto && route <= rlk::kSampleFull && (route != rlk::kSampleFew || top_k <= rlk::sample_few_limit()),
+              "rl_engine.sample: route is -1 (by size), 0 (a CTA per row), 1 or 2 (slices; 1: k <= ", rlk::sample_few_limit(), ")");
   // top_k == 0 selects the full-vocabulary nucleus kernel (top-p only / plain temperature sampling)
   TORCH_CHECK(top_k >= 0 && top_k <= rlk::sample_topk_limit(), "rl_engine.sample: top_k must be in [0, ",
               rlk::sample_topk_limit(), "] (0 = no top-k)");
@@ -1331,7 +1333,8 @@ std::vector<Tensor> sample(const Tensor& logits, int64_t top_k, double top_p, do
                           static_cast<int>(logits.size(1)), static_cast<int>(top_k), static_cast<float>(top_p),
                           static_cast<float>(temperature), static_cast<unsigned long long>(seed),
                           static_cast<unsigned long long>(offset), reinterpret_cast<long long*>(ids.data_ptr<int64_t>()),
-                          want_logprob ? lp.data_ptr<float>() : nullptr, stream_of(logits));
+                          want_logprob ? lp.data_ptr<float>() : nullptr, sm_count_of(logits.get_device()), static_cast<int>(route),
+                          stream_of(logits));
     after_launch();
   }
   return {ids, lp};
@@ -1738,7 +1741,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding_bwd", rlk::traced("rlk::embedding_bwd", &embedding_bwd), py::arg("sorted_ids"), py::arg("order"), py::arg("dy"),
         py::arg("dtable"), py::arg("accumulate") = false);
   m.def("adamw", rlk::traced("rlk::adamw", &adamw));
-  m.def("sample", rlk::traced("rlk::sample", &sample));
+  m.def("sample", rlk::traced("rlk::sample", &sample), py::arg("logits"), py::arg("top_k"), py::arg("top_p"), py::arg("temperature"),
+        py::arg("seed"), py::arg("offset"), py::arg("want_logprob"), py::arg("route") = -1);
   m.def("attention_fwd", rlk::traced("rlk::attention_fwd", &attention_fwd));
   m.def("attention_bwd", rlk::traced("rlk::attention_bwd", &attention_bwd), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"),
         py::arg("dout"), py::arg("lse"), py::arg("seqs"), py::arg("q_tiles"), py::arg("kv_items"), py::arg("q_blocks"),

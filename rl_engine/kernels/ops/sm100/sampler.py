@@ -1,4 +1,4 @@
-"""Temperature / top-k / top-p sampling on the sm_100a kernel (one CTA per row).
+"""Temperature / top-k / top-p sampling on the sm_100a kernels (a CTA, or slices of a row over a cluster of CTAs).
 
 The draw is a pure function of ``(logits row, top_k, top_p, temperature, seed, offset, row)``;
 ``philox_uniform`` below restates the kernel's random stream on the host so tests can predict it.

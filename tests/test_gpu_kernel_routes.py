@@ -449,6 +449,32 @@ def test_top_k_sampler_over_splits_and_fallbacks(rows, vocab, k, shape):
     assert all(int(i) in a for i, a in zip(ids.cpu(), allowed))
 
 
+@pytest.mark.parametrize("rows,vocab", [(1, 140001), (3, 66000), (20, 50257), (75, 33001), (149, 9000), (160, 101000), (5, 300), (200, 64)])
+@pytest.mark.parametrize("k", [1, 20, 63, 200, 256, 257, 700, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_top_k_draws_do_not_depend_on_the_kernel(rows, vocab, k, dtype):
+    """A CTA per row (both instances), slices with either bound, one to eight of them: the same ids and log-probs, with ties, rows whose
+    head is far below their tail (candidates overflow) and masked stretches; and what the sizes select is one of them."""
+    from rl_engine.kernels.ops.base import require_ext
+
+    ext = require_ext()
+    z = (2 * torch.randn(rows, vocab, device=DEV, generator=_gen(rows + k)))
+    z[rows // 2] += torch.linspace(0, 40, vocab, device=DEV)
+    z[0, : vocab // 2] = float("-inf")
+    z = z.to(dtype)
+    if min(k, vocab) > int((z[0] > float("-inf")).sum()):
+        pytest.skip("ties at -inf fill the buffer")
+    want = ext.sample(z, k, 0.95, 0.8, 7, 11, True, 0)
+    for route in (-1, 1, 2):
+        if route == 1 and k > 256:
+            continue
+        ids, logprob = ext.sample(z, k, 0.95, 0.8, 7, 11, True, route)
+        assert torch.equal(ids, want[0]) and torch.equal(logprob, want[1]), route
+    # the same rows in a batch of another size
+    part = ext.sample(z[:1].contiguous(), k, 0.95, 0.8, 7, 11, True)
+    assert torch.equal(part[0], want[0][:1]) and torch.equal(part[1], want[1][:1])
+
+
 # ------------------------------------------------------------------------------------------------ log-prob gradient
 @pytest.mark.parametrize("v", [5, 1024, 4099, 8192])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
