@@ -148,8 +148,8 @@ void dispatch_out(const GemmArgs& a, cudaStream_t stream) {
     if (a.group_mode == 0 && a.M <= kBM && !a.out_fp32 && !a.accumulate && a.N >= 4 * kSkinnyBN) {
       // With at least one 128-row tile of B per SM (an LM head) the weight-streaming kernel of the decoding step takes it:
       // B is its 128-row operand, so a stage is nearly all weight instead of two thirds padded tokens: 3 tokens on a
-      // 128256 x 4096 head 402 -> 174 us (2.6 -> 6.0 TB/s).  With fewer tiles than SMs, whole tiles leave SMs idle that the
-      // 64-column tiles below reach.
+      // 128256 x 4096 head 402 -> 174 us (2.6 -> 6.0 TB/s).  Narrower products are bound by the chain of accumulations over K, which
+      // is as long on either kernel (4096 x 4096, 32 tokens: 23 and 24 us), and stay on the 64-column tiles below.
       if (a.N >= kBM * a.sm_count && a.alpha == 1.f) {
         DecodeLinearArgs d{};
         d.x = a.A;

@@ -157,8 +157,8 @@ void gemm_fp8_rowscaled(const void* a_q, long long lda, const float* scale_a, co
                         const float* scale_b, void* d_out, long long ldd, int M, int N, int K, bool cta_pair, int sm_count,
                         uint32_t* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return;
-  // A stream over the weight: whole 128-row tiles of it, twice the CTAs of the 128 x 256 tiles below and no loads of padded
-  // tokens.  The 16 projections of a four-layer step with three tokens (4096 / 14336 wide): 582 -> 425 us.
+  // A stream over the weight: tiles of 64 or 128 of its rows, two to four times the CTAs of the 128 x 256 tiles below and no loads
+  // of padded tokens.  A step of four layers with three tokens (4096 / 14336 wide, LM head included): 1368 -> 868 us.
   if (M <= kBM) {
     DecodeLinearArgs d{};
     d.x = a_q;

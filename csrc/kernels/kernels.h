@@ -307,10 +307,11 @@ void swiglu_packed_forward(const __nv_bfloat16* gu, long long ldgu, __nv_bfloat1
                            cudaStream_t stream);
 void swiglu_packed_backward(const __nv_bfloat16* gu, long long ldgu, const __nv_bfloat16* dy, long long lddy,
                             __nv_bfloat16* dgu, long long lddgu, long long rows, int F, cudaStream_t stream);
-// out[n, Hkv * rep * 128] = merge by log-sum-exp of two partial attention results o1 / o2 [n * rep, Hkv, 128] (bf16)
-// with l1 / l2 [Hkv, n * rep]; rows = n * rep.
+// out[n, Hkv * rep * 128] = merge by log-sum-exp of `parts` partial attention results of the same rows = n * rep queries, one behind
+// the other: o [parts * rows, Hkv, 128] (bf16) with lse [Hkv, parts * rows].
 void attn_merge_parts(const __nv_bfloat16* o, const float* lse, __nv_bfloat16* out, int parts, long long rows, int hkv, int rep,
                       cudaStream_t stream);
+// The same of two partial results in buffers of their own: o1 / o2 [n * rep, Hkv, 128] (bf16) with l1 / l2 [Hkv, n * rep].
 void attn_merge2(const void* o1, const float* l1, const void* o2, const float* l2, void* out, long long rows, int hkv,
                  int rep, cudaStream_t stream);
 // table_rows: rows of the cos / sin tables (positions are checked against it in debug-bounds builds)

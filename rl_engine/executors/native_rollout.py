@@ -67,8 +67,8 @@ class NativeRolloutEngine:
         del prompt_kv
         completions = torch.empty(g, max_new_tokens, dtype=torch.long, device=dev)
         tokens = draw(last_state.expand(g, -1).contiguous()).reshape(g)
-        # Step state lives in fixed device tensors that are advanced in place, so that one decoding step (some 14
-        # launches per layer, launch-bound at G tokens) can be captured once as a CUDA graph and replayed per token:
+        # Step state lives in fixed device tensors that are advanced in place, so that one decoding step (eight
+        # launches per layer, more with fp8 projections: bound by their latency at G tokens) can be captured once as a CUDA graph and replayed per token:
         # the token drawn at `step` sits at position p + step and in cache row base + step; its one-token query sees
         # the prompt rows and its own rows so far (sk_len = step + 1, column 5 of the layout table).
         step_tokens = tokens.clone()
